@@ -892,7 +892,7 @@ constexpr size_t kNoAllocBytes =
     + round256(8 * kNoAllocCells)                           // diagonal (f64)
     + 3 * round256(4 * kNoAllocCells)                       // couplings (f32)
     + round256(8 * kNoAllocCells)                           // right-hand side (f64)
-    + 5 * round256(8 * kNoAllocCells)                       // x, r, p, p', Ap (f64)
+    + 7 * round256(8 * kNoAllocCells)                       // x, r, p, p', Ap, z, 1/diagonal (f64)
     + round256(16 * kNoAllocCells)                          // segment descriptors (<= one per cell)
     + round256(kNoAllocCells)                               // segment flags
     + round256(4 * (kNoAllocCells / 1024 + 2))              // scan chunks and the segment count
@@ -972,7 +972,8 @@ EL_API int el_solve_pressure_noalloc(const el_grid* g, const float* phi, float* 
     ctx.p64 = (double*)carve(8 * kNoAllocCells);
     ctx.p64b = (double*)carve(8 * kNoAllocCells);
     ctx.ap64 = (double*)carve(8 * kNoAllocCells);
-    ctx.z64 = ctx.p64b;  // not read by the Jacobi solve
+    ctx.z64 = (double*)carve(8 * kNoAllocCells);
+    ctx.inv64 = (double*)carve(8 * kNoAllocCells);
     SegList& seg = ctx.seg0;
     seg.nsr = (g->ni + 31) / 32;
     seg.total = (long long)seg.nsr * g->nj * g->nk;  // <= n

@@ -40,6 +40,7 @@ struct Scalars {
     double dt;       // step size the step kernels read
     double bb;       // |b|^2 of the current system
     double rz;       // r . z
+    double rz2[2];   // plain FP64 PCG: r . z of the even and the odd iterations
     double alpha, beta;
     double rr;       // |r|^2 (recursively updated residual)
     double thresh;   // stop when rr < thresh (= tol^2 * bb)
@@ -236,6 +237,7 @@ struct el_ctx {
     double* rhs64 = nullptr;
     // FP64 Krylov vectors
     double *x64 = nullptr, *r64 = nullptr, *z64 = nullptr, *p64 = nullptr, *ap64 = nullptr;
+    double* inv64 = nullptr;  // plain FP64 PCG: the reciprocal of the diagonal (0 on empty rows)
     double* p64b = nullptr;  // second direction buffer (the fused K1 writes p out of place)
     // FP32 inner system (mixed solver): the PCG operator as float4 records and the level-0
     // multigrid operator as half4 records
@@ -466,38 +468,75 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// Sums over the first SUMMED threads of a block (at most 1024), thread 0 gets the
+// totals.  What bounds a reduction here is the FP64 pipe: each of the SM's four partitions issues
+// half a lane a clock, so an FP64 addition occupies it for 64 cycles whether one lane of the warp
+// needs it or 32.  A shuffle tree in every warp took 45 of them for 256 threads, the totals all on
+// the partition of warp 0; here the values go through shared memory, a warp sums 256 of them
+// (eight a lane, then one tree: 12 additions), and the summing warps of a block lie on different
+// partitions (consecutive warps; a block starts at a warp of its own number).
+// An FP64 PCG update of 1024 blocks of 256 threads (64^3) ended 6.7 us earlier: 16.8 -> 10.1 us.
 template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double (*sh)[32]) {
+constexpr int kSumChunk = NV < 4 ? NV : 4;
+
+// shared memory of block_sum: a chunk of values of each thread
+template <int NV, int THREADS>
+struct SumScratch {
+    double v[kSumChunk<NV>][THREADS];
+};
+
+template <int NV, int THREADS, int SUMMED>
+__device__ __forceinline__ void block_sum(double (&v)[NV], SumScratch<NV, THREADS>& sh, unsigned first_warp) {
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-    const int nthreads = blockDim.x * blockDim.y * blockDim.z;
-    const int lane = tid & 31, warp = tid >> 5, nwarps = (nthreads + 31) >> 5;
+    constexpr int kWarps = THREADS / 32, kPer = (SUMMED + 255) / 256;  // summing warps a value
+    constexpr int CH = kSumChunk<NV>;
+    const int lane = tid & 31;
+    const int w = ((tid >> 5) + kWarps - (int)(first_warp % kWarps)) % kWarps;  // this warp's place
 #pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        double s = warp_sum(v[q]);
-        if (lane == 0) sh[q][warp] = s;
-    }
-    __syncthreads();
-    if (warp == 0) {
+    for (int q0 = 0; q0 < NV; q0 += CH) {
+        if (q0) __syncthreads();
 #pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double s = lane < nwarps ? sh[q][lane] : 0.0;
-            v[q] = warp_sum(s);
+        for (int c = 0; c < CH; ++c)
+            if (q0 + c < NV) sh.v[c][tid] = v[q0 + c];
+        __syncthreads();
+        for (int u = w; u < CH * kPer; u += kWarps) {
+            const int c = u / kPer, base = (u - c * kPer) * 256;
+            if (q0 + c >= NV) break;
+            double t[8];
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                const int e = base + lane + 32 * m;
+                t[m] = e < SUMMED ? sh.v[c][e] : 0.0;
+            }
+            double s = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+            s = warp_sum(s);
+            if (lane == 0) sh.v[c][base] = s;  // read by this lane only, above
+        }
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                if (q0 + c >= NV) break;
+                double s = sh.v[c][0];
+#pragma unroll
+                for (int p = 1; p < kPer; ++p) s += sh.v[c][256 * p];
+                v[q0 + c] = s;
+            }
         }
     }
-    __syncthreads();
 }
 
 // Returns true in thread 0 of the last block, with out[] holding the grid totals.
 // `partials` must hold (number of blocks) * NV doubles.
-template <int NV>
+// THREADS: the block's threads, SUMMED: those of them (the first ones) that bring values.
+template <int NV, int THREADS = 256, int SUMMED = THREADS>
 __device__ bool grid_sum(double (&v)[NV], double* partials, unsigned* counter, double (&out)[NV]) {
-    __shared__ double sh[NV][32];
+    __shared__ SumScratch<NV, THREADS> sh;
     __shared__ bool last;
     const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-    const int nthreads = blockDim.x * blockDim.y * blockDim.z;
     const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     const unsigned nblocks = gridDim.x * gridDim.y * gridDim.z;
-    block_sum<NV>(v, sh);
+    block_sum<NV, THREADS, SUMMED>(v, sh, bid);
     if (tid == 0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) partials[(size_t)bid * NV + q] = v[q];
@@ -511,11 +550,25 @@ __device__ bool grid_sum(double (&v)[NV], double* partials, unsigned* counter, d
     double acc[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) acc[q] = 0.0;
-    for (unsigned b = tid; b < nblocks; b += nthreads) {
+    // four blocks' partials in flight a thread
+    constexpr int U = NV <= 2 ? 4 : 1;
+    for (unsigned b0 = tid; b0 < nblocks; b0 += U * THREADS) {
+        double t[U][NV];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) acc[q] += __ldcg(&partials[(size_t)b * NV + q]);
+        for (int u = 0; u < U; ++u) {
+            const unsigned b = b0 + u * THREADS;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) t[u][q] = b < nblocks ? __ldcg(&partials[(size_t)b * NV + q]) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (b0 + u * THREADS < nblocks) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) acc[q] += t[u][q];
+            }
     }
-    block_sum<NV>(acc, sh);
+    __syncthreads();
+    block_sum<NV, THREADS, THREADS>(acc, sh, 0);
     if (tid == 0) {
 #pragma unroll
         for (int q = 0; q < NV; ++q) out[q] = acc[q];

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kThreads, Layout<M>::min_blocks) march_kernel(
     if (M == DIRSPMV || M == UPDZ || M == LAST) {
         double acc[1] = {(double)part};
         double tot[1];
-        if (grid_sum<1>(acc, a.partials, a.counter, tot)) {
+        if (grid_sum<1, kThreads, 32 * kComputeWarps>(acc, a.partials, a.counter, tot)) {
             if (M == DIRSPMV) {
                 const double al = s->rz / tot[0];
                 s->alpha = al;

@@ -4,7 +4,8 @@
 // src/project/3d/eulerian_liquid/simulator.cpp:102-109 (x0 = 0, stop on |r|^2 < tol^2 |b|^2 of
 // the recursively updated residual, iteration cap) with three GPU solvers:
 //
-//   EL_SOLVER_JACOBI_FP64  plain FP64 PCG, Jacobi preconditioner (the correctness baseline)
+//   EL_SOLVER_JACOBI_FP64  plain FP64 PCG, Jacobi preconditioner (the correctness baseline;
+//                          jacobi_dir_kernel / jacobi_update_kernel)
 //   EL_SOLVER_MG_FP64      FP64 PCG with a multigrid V-cycle preconditioner
 //   EL_SOLVER_MIXED        FP64 iterative refinement: r = b - A x in FP64, the correction
 //                          solved by FP32 multigrid PCG on the FP32 operator, x += |r| e in FP64
@@ -30,7 +31,7 @@
 // make the V-cycle symmetric, as PCG needs.
 //
 // Per PCG iteration:  K1  p = z + beta p ; Ap = A p ; alpha = rz / p.Ap
-//                     K2  x += alpha p ; r -= alpha Ap ; rr = r.r (; rz = r.D^-1 r for Jacobi)
+//                     K2  x += alpha p ; r -= alpha Ap ; rr = r.r (; z = D^-1 r, rz = r.z for Jacobi)
 //                     V   z = M^-1 r ; rz = r.z ; beta            (multigrid solvers)
 // Scalars live in device memory; once converged the remaining launched kernels return at
 // entry, so the host polls only every `check_every` iterations.
@@ -51,6 +52,10 @@ constexpr int kCoarsestSweeps = 30;
 constexpr int kCoarsestMaxDim = 8;
 constexpr int kCoarsestMaxCells = 512;
 constexpr int kSegThreads = 256;
+// Block size of the PCG kernels that end in a dot product: few, large blocks, because each block's
+// reduction occupies the FP64 pipe (block_sum) -- one block an SM in FP64.
+template <typename V>
+constexpr int kDotThreads = sizeof(V) == 8 ? 1024 : 512;
 
 __device__ __forceinline__ bool finite_d(double v) { return isfinite(v); }
 
@@ -371,50 +376,96 @@ struct St7 {
     V d, cxm, cxp, cym, cyp, czm, czp;   // diagonal and couplings
 };
 
+// which of the stencil's cells exist, and the cell just outside the segment (of lane 0 or of lane
+// 31: one load and one value serve both)
+struct Near7 {
+    bool iym, iyp, izm, izp, ixm, ixp, xp_in;
+    int ce, ie;
+};
+
+__device__ __forceinline__ Near7 near7(const LGeom& g, int c, int i, int j, int k, bool live, int lane) {
+    Near7 n;
+    n.iym = live && j > 0;
+    n.iyp = live && j < g.n1 - 1;
+    n.izm = live && k > 0;
+    n.izp = live && k < g.n2 - 1;
+    n.ixm = lane == 0 && live && i > 0;
+    n.xp_in = live && i + 1 < g.n0;
+    n.ixp = lane == 31 && n.xp_in;
+    n.ce = n.ixm ? c - 1 : c + 1;
+    n.ie = n.ixm ? i - 1 : i + 1;
+    return n;
+}
+
+template <typename V>
+struct Rec7 {
+    Co<V> r0, ym, yp, zm, zp, xe;
+};
+
+template <typename V, bool ALL, typename RF>
+__device__ __forceinline__ Rec7<V> load_rec7(const LGeom& g, const Near7& n, int c, bool live, RF&& recf) {
+    const Co<V> z4{V(0), V(0), V(0), V(0)};
+    Rec7<V> r;
+    r.r0 = live ? recf(c) : z4;
+    r.ym = n.iym ? recf(c - g.s1) : z4;
+    r.yp = (ALL && n.iyp) ? recf(c + g.s1) : z4;
+    r.zm = n.izm ? recf(c - g.s2) : z4;
+    r.zp = (ALL && n.izp) ? recf(c + g.s2) : z4;
+    r.xe = (n.ixm || (ALL && n.ixp)) ? recf(n.ce) : z4;
+    return r;
+}
+
+template <typename Raw>
+struct Raw7 {
+    Raw a0, ym, yp, zm, zp, xe;
+};
+
+template <typename LF>
+__device__ __forceinline__ auto load_raw7(const LGeom& g, const Near7& n, int c, int i, int j, int k, bool live,
+                                          LF&& rawf) {
+    using Raw = decltype(rawf(0, 0, 0, 0));
+    Raw7<Raw> a;
+    a.a0 = live ? rawf(c, i, j, k) : Raw{};
+    a.ym = n.iym ? rawf(c - g.s1, i, j - 1, k) : Raw{};
+    a.yp = n.iyp ? rawf(c + g.s1, i, j + 1, k) : Raw{};
+    a.zm = n.izm ? rawf(c - g.s2, i, j, k - 1) : Raw{};
+    a.zp = n.izp ? rawf(c + g.s2, i, j, k + 1) : Raw{};
+    a.xe = (n.ixm || n.ixp) ? rawf(n.ce, n.ie, j, k) : Raw{};
+    return a;
+}
+
+template <typename V, typename Raw, typename VF>
+__device__ __forceinline__ St7<V> value7(const Near7& n, const Rec7<V>& r, const Raw7<Raw>& a, bool live, int lane,
+                                         VF&& valf) {
+    St7<V> st;
+    st.d = r.r0.d;
+    st.cxp = r.r0.x;
+    st.cyp = r.r0.y;
+    st.czp = r.r0.z;
+    st.cym = r.ym.y;
+    st.czm = r.zm.z;
+    st.v0 = live ? valf(a.a0, r.r0) : V(0);
+    st.vym = n.iym ? valf(a.ym, r.ym) : V(0);
+    st.vyp = n.iyp ? valf(a.yp, r.yp) : V(0);
+    st.vzm = n.izm ? valf(a.zm, r.zm) : V(0);
+    st.vzp = n.izp ? valf(a.zp, r.zp) : V(0);
+    const V sxm = __shfl_up_sync(kFull, st.v0, 1);
+    const V sxp = __shfl_down_sync(kFull, st.v0, 1);
+    const V scm = __shfl_up_sync(kFull, r.r0.x, 1);
+    const V vxe = (n.ixm || n.ixp) ? valf(a.xe, r.xe) : V(0);
+    st.vxm = lane == 0 ? vxe : sxm;
+    st.cxm = lane == 0 ? r.xe.x : scm;
+    st.vxp = n.xp_in ? (lane == 31 ? vxe : sxp) : V(0);
+    return st;
+}
+
 template <typename V, bool ALL, typename RF, typename LF, typename VF>
 __device__ __forceinline__ St7<V> gather7(const LGeom& g, int c, int i, int j, int k, bool live, int lane, RF&& recf,
                                           LF&& rawf, VF&& valf) {
-    const Co<V> z4{V(0), V(0), V(0), V(0)};
-    const bool iym = live && j > 0, iyp = live && j < g.n1 - 1;
-    const bool izm = live && k > 0, izp = live && k < g.n2 - 1;
-    const bool ixm = lane == 0 && live && i > 0;
-    const bool ixp = lane == 31 && live && i + 1 < g.n0;
-    // loads
-    const Co<V> r0 = live ? recf(c) : z4;
-    const Co<V> rym = iym ? recf(c - g.s1) : z4;
-    const Co<V> ryp = (ALL && iyp) ? recf(c + g.s1) : z4;
-    const Co<V> rzm = izm ? recf(c - g.s2) : z4;
-    const Co<V> rzp = (ALL && izp) ? recf(c + g.s2) : z4;
-    const Co<V> rxm = ixm ? recf(c - 1) : z4;
-    const Co<V> rxp = (ALL && ixp) ? recf(c + 1) : z4;
-    using Raw = decltype(rawf(0, 0, 0, 0));
-    const Raw a0 = live ? rawf(c, i, j, k) : Raw{};
-    const Raw aym = iym ? rawf(c - g.s1, i, j - 1, k) : Raw{};
-    const Raw ayp = iyp ? rawf(c + g.s1, i, j + 1, k) : Raw{};
-    const Raw azm = izm ? rawf(c - g.s2, i, j, k - 1) : Raw{};
-    const Raw azp = izp ? rawf(c + g.s2, i, j, k + 1) : Raw{};
-    const Raw axm = ixm ? rawf(c - 1, i - 1, j, k) : Raw{};
-    const Raw axp = ixp ? rawf(c + 1, i + 1, j, k) : Raw{};
-    // values and couplings
-    St7<V> st;
-    st.d = r0.d;
-    st.cxp = r0.x;
-    st.cyp = r0.y;
-    st.czp = r0.z;
-    st.cym = rym.y;
-    st.czm = rzm.z;
-    st.v0 = live ? valf(a0, r0) : V(0);
-    st.vym = iym ? valf(aym, rym) : V(0);
-    st.vyp = iyp ? valf(ayp, ryp) : V(0);
-    st.vzm = izm ? valf(azm, rzm) : V(0);
-    st.vzp = izp ? valf(azp, rzp) : V(0);
-    const V sxm = __shfl_up_sync(kFull, st.v0, 1);
-    const V sxp = __shfl_down_sync(kFull, st.v0, 1);
-    const V scm = __shfl_up_sync(kFull, r0.x, 1);
-    st.vxm = lane == 0 ? (ixm ? valf(axm, rxm) : V(0)) : sxm;
-    st.cxm = lane == 0 ? rxm.x : scm;
-    st.vxp = (live && i + 1 < g.n0) ? (lane == 31 ? valf(axp, rxp) : sxp) : V(0);
-    return st;
+    const Near7 n = near7(g, c, i, j, k, live, lane);
+    const Rec7<V> r = load_rec7<V, ALL>(g, n, c, live, recf);
+    const auto a = load_raw7(g, n, c, i, j, k, live, rawf);
+    return value7<V>(n, r, a, live, lane, valf);
 }
 
 template <typename V>
@@ -440,14 +491,20 @@ struct SplitLoad {
     }
 };
 
-// K1: new direction fused with A p and p.Ap over the active segments.
-// Record operator (FP32 inner / FP64 multigrid).
+__device__ __forceinline__ bool positive(float v) { return v > 0.f; }
+__device__ __forceinline__ bool positive(double v) { return d_positive(v); }  // on the integer pipe
+
+// K1: new direction fused with A p and p.Ap over the active segments (record operator: FP32 inner
+// system, FP64 multigrid).
 template <typename V, typename R>
-__global__ void __launch_bounds__(kSegThreads) dir_spmv_rec_kernel(LGeom g, SegArg seg, const R* __restrict__ A,
-                                                                   const V* __restrict__ z, const V* __restrict__ p_in,
-                                                                   V* __restrict__ p_out, V* __restrict__ ap,
-                                                                   Scalars* s, int first, double* partials,
-                                                                   unsigned* counter) {
+__global__ void __launch_bounds__(kDotThreads<V>) dir_spmv_rec_kernel(LGeom g, SegArg seg, const R* __restrict__ A,
+                                                                      const V* __restrict__ z,
+                                                                      const V* __restrict__ p_in,
+                                                                      V* __restrict__ p_out, V* __restrict__ ap,
+                                                                      Scalars* s, int first, double* partials,
+                                                                      unsigned* counter) {
+    pdl_wait();
+    pdl_trigger();
     if (s->done) return;
     const V beta = first ? V(0) : (V)s->beta;
     DotAcc<V> part = 0;
@@ -458,7 +515,7 @@ __global__ void __launch_bounds__(kSegThreads) dir_spmv_rec_kernel(LGeom g, SegA
     const St7<V> st = gather7<V, false>(g, c, i, j, k, live, lane, recf, rawf, valf);
     if (live) {
         V pc = V(0), apc = V(0);
-        if (st.d > V(0)) {
+        if (positive(st.d)) {
             pc = st.v0;
             apc = apply7(st);
         }
@@ -469,7 +526,7 @@ __global__ void __launch_bounds__(kSegThreads) dir_spmv_rec_kernel(LGeom g, SegA
     SEG_LOOP_END
     double acc[1] = {(double)part};
     double tot[1];
-    if (grid_sum<1>(acc, partials, counter, tot)) {
+    if (grid_sum<1, kDotThreads<V>>(acc, partials, counter, tot)) {
         const double alpha = s->rz / tot[0];
         s->alpha = alpha;
         if (!finite_d(alpha)) {
@@ -479,52 +536,16 @@ __global__ void __launch_bounds__(kSegThreads) dir_spmv_rec_kernel(LGeom g, SegA
     }
 }
 
-// Split FP64 operator with the Jacobi preconditioner applied on the fly (plain FP64 PCG).
-template <typename OT>
-__global__ void __launch_bounds__(kSegThreads) dir_spmv_jacobi_kernel(LGeom g, SegArg seg, SplitOp<OT> A,
-                                                                      const double* __restrict__ r,
-                                                                      const double* __restrict__ p_in,
-                                                                      double* __restrict__ p_out,
-                                                                      double* __restrict__ ap, Scalars* s, int first,
-                                                                      double* partials, unsigned* counter) {
-    if (s->done) return;
-    const double beta = first ? 0.0 : s->beta;
-    double acc[1] = {0.0};
-    const SplitLoad<OT> recf{A};
-    // raw = (r, p) packed as a pair of doubles
-    auto rawf = [&](int q, int, int, int) -> double2 { return make_double2(r[q], first ? 0.0 : p_in[q]); };
-    auto valf = [&](double2 raw, const Co<double>& rec) -> double {
-        return rec.d > 0.0 ? raw.x / rec.d + beta * raw.y : 0.0;
-    };
-    SEG_LOOP_ALL_BEGIN(seg, g)
-    const St7<double> st = gather7<double, true>(g, c, i, j, k, live, lane, recf, rawf, valf);
-    if (live) {
-        const double apc = st.d > 0.0 ? apply7(st) : 0.0;
-        p_out[c] = st.v0;
-        ap[c] = apc;
-        acc[0] += st.v0 * apc;
-    }
-    SEG_LOOP_END
-    double tot[1];
-    if (grid_sum<1>(acc, partials, counter, tot)) {
-        const double alpha = s->rz / tot[0];
-        s->alpha = alpha;
-        if (!finite_d(alpha)) {
-            s->bad = 1;
-            s->done = 1;
-        }
-    }
-}
-
-// K2: x += alpha p ; r -= alpha Ap ; |r|^2 (and r.D^-1 r for Jacobi, giving beta).
-template <typename V, bool JAC>
-__global__ void __launch_bounds__(kSegThreads) update_kernel(LGeom g, SegArg seg, const double* __restrict__ diag,
-                                                             V* __restrict__ x, V* __restrict__ r,
-                                                             const V* __restrict__ p, const V* __restrict__ ap,
-                                                             Scalars* s, double* partials, unsigned* counter) {
+// K2: x += alpha p ; r -= alpha Ap ; |r|^2.
+template <typename V>
+__global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg seg, V* __restrict__ x,
+                                                                V* __restrict__ r, const V* __restrict__ p,
+                                                                const V* __restrict__ ap, Scalars* s,
+                                                                double* partials, unsigned* counter) {
+    pdl_wait();
+    pdl_trigger();
     if (s->done) return;
     const V alpha = (V)s->alpha;
-    double acc[2] = {0.0, 0.0};
     DotAcc<V> part = 0;
     // two segments per warp and iteration, all eight loads issued before any use: the kernel is
     // pure streaming and bound by the loads in flight
@@ -537,10 +558,6 @@ __global__ void __launch_bounds__(kSegThreads) update_kernel(LGeom g, SegArg seg
         x[c] = xc + alpha * pc;
         r[c] = rc;
         part += (DotAcc<V>)rc * (DotAcc<V>)rc;
-        if (JAC) {
-            const double d = diag[c];
-            if (d > 0.0) acc[1] += (double)rc * ((double)rc / d);
-        }
     };
     for (int qs = warp_global; qs < nseg; qs += 2 * nwarps) {
         const int q2 = qs + nwarps;
@@ -564,9 +581,9 @@ __global__ void __launch_bounds__(kSegThreads) update_kernel(LGeom g, SegArg seg
         if (la) finish(ca, pa, apa, xa, ra);
         if (lb) finish(cb, pb, apb, xb, rb);
     }
-    acc[0] = (double)part;
-    double tot[2];
-    if (grid_sum<2>(acc, partials, counter, tot)) {
+    double acc[1] = {(double)part};
+    double tot[1];
+    if (grid_sum<1, kDotThreads<V>>(acc, partials, counter, tot)) {
         s->rr = tot[0];
         s->iter += 1;
         if (!finite_d(tot[0])) {
@@ -575,23 +592,253 @@ __global__ void __launch_bounds__(kSegThreads) update_kernel(LGeom g, SegArg seg
         } else if (tot[0] < s->thresh) {
             s->done = 1;
         }
-        if (JAC) {
-            s->beta = tot[1] / s->rz;
-            s->rz = tot[1];
-        }
     }
 }
 
-// Jacobi start: rz = r . D^-1 r
-__global__ void jacobi_rz_kernel(LGeom g, SegArg seg, const double* __restrict__ diag, const double* __restrict__ r,
-                                 Scalars* s, double* partials, unsigned* counter) {
+// ---------------------------------------------------------------------------------------
+// Plain FP64 PCG with the Jacobi preconditioner: two kernels an iteration.
+//
+// Bound by the FP64 pipe (2 lanes a clock per SM; a division costs nine of its operations) on a
+// large scene, by the chain of latencies on a small one.  So
+//   - the update stores z = D^-1 r, formed with reciprocals of the diagonal taken once a solve, and
+//     the direction reads z: 14 FP64 operations a cell in K1 where r / d at every point of the
+//     stencil took about 80, 5 in K2;
+//   - a kernel leaves its dot products as one partial sum a block, and the next kernel's blocks
+//     each sum those (at most one block an SM) while their own loads are in flight: no fence, ticket
+//     and last block at the end of a launch;
+//   - what no kernel of the iteration writes (segments, coefficients) is loaded before the wait for
+//     the kernel before.
+// Dam break, FP64, both kernels of an iteration: 128^3 115.6 -> 32.1 us, 64^3 38.6 -> 13.9 us.
+//
+// rz of iteration t (0, 1, ...) lives in rz2[t & 1]: K1's blocks read the old one while block 0
+// stores the new one.
+constexpr int kJacThreads = 512;
+constexpr int kJacMaxBlocks = 256;  // at most one block an SM
+
+struct JacPart {
+    double* pap;  // [blocks]      p.Ap   (K1)
+    double* rr;   // [blocks][2]   r.r, r.z   (K2)
+    int blocks;
+};
+
+// The totals of NV values over the blocks' partials, in every thread (a barrier): warp q sums
+// value q, in the same order in every block.
+template <int NV>
+__device__ __forceinline__ void sum_partials(const double* __restrict__ part, int blocks, double (&out)[NV]) {
+    __shared__ double tot[NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < NV) {
+        double t[kJacMaxBlocks / 32];
+#pragma unroll
+        for (int m = 0; m < kJacMaxBlocks / 32; ++m) {
+            const int b = lane + 32 * m;
+            t[m] = b < blocks ? __ldcg(part + (size_t)b * NV + warp) : 0.0;
+        }
+        double v = t[0];
+#pragma unroll
+        for (int m = 1; m < kJacMaxBlocks / 32; ++m)
+            if (32 * m < blocks) v += t[m];
+        v = warp_sum(v);
+        if (lane == 0) tot[warp] = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) out[q] = tot[q];
+}
+
+// |r|^2 and r.z after an update: the stopping test, and beta for the next direction
+struct JacNext {
+    double rr, rz, beta;
+    bool bad, done;
+};
+__device__ __forceinline__ JacNext jacobi_next(const double (&t)[2], double rz_old, double thresh) {
+    JacNext n;
+    n.rr = t[0];
+    n.rz = t[1];
+    n.beta = t[1] / rz_old;
+    n.bad = !finite_d(t[0]);
+    n.done = n.bad || t[0] < thresh;
+    return n;
+}
+__device__ __forceinline__ void jacobi_store(Scalars* s, const JacNext& n, int slot_new) {
+    s->rr = n.rr;
+    s->iter += 1;
+    s->beta = n.beta;
+    s->rz2[slot_new] = n.rz;
+    if (n.bad) s->bad = 1;
+    if (n.done) s->done = 1;
+}
+
+// K1 of iteration t (slot = t & 1).  pending: the update before left its dot products as partials
+// (else s->beta holds the result).
+template <typename OT>
+__global__ void __launch_bounds__(kJacThreads, 1) jacobi_dir_kernel(LGeom g, SegArg seg, SplitOp<OT> A,
+                                                                    const double* __restrict__ z,
+                                                                    const double* __restrict__ p_in,
+                                                                    double* __restrict__ p_out,
+                                                                    double* __restrict__ ap, Scalars* s, int first,
+                                                                    int pending, int slot, JacPart part) {
+    __shared__ SumScratch<1, kJacThreads> sh;
+    const SplitLoad<OT> recf{A};
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    int qs = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nseg = *seg.count;
+    int4 sd = qs < nseg ? seg.desc[qs] : make_int4(0, g.n0, 0, 0);
+    Near7 nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+    Rec7<double> rec = load_rec7<double, false>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+    pdl_wait();
+    pdl_trigger();
+    auto rawf = [&](int q, int, int, int) -> double2 { return make_double2(z[q], first ? 0.0 : p_in[q]); };
+    auto raw = load_raw7(g, nb, sd.x + lane, 0, 0, 0, sd.y + lane < g.n0, rawf);
+    const int done = s->done;
+    double beta = first ? 0.0 : s->beta;
+    if (pending) {
+        const double rz_old = s->rz2[slot ^ 1], thresh = s->thresh;
+        double t[2];
+        sum_partials(part.rr, part.blocks, t);
+        if (done) return;
+        const JacNext n = jacobi_next(t, rz_old, thresh);
+        if (blockIdx.x == 0 && threadIdx.x == 0) jacobi_store(s, n, slot);
+        if (n.done) return;
+        beta = n.beta;
+    } else if (done) {
+        return;
+    }
+    auto valf = [&](double2 v, const Co<double>&) -> double { return first ? v.x : v.x + beta * v.y; };
+    double acc[1] = {0.0};
+    while (true) {
+        const bool live = sd.y + lane < g.n0;
+        const int c = sd.x + lane;
+        const St7<double> st = value7<double>(nb, rec, raw, live, lane, valf);
+        if (live) {
+            double pc = 0.0, apc = 0.0;
+            if (positive(st.d)) {
+                pc = st.v0;
+                apc = apply7(st);
+            }
+            p_out[c] = pc;
+            ap[c] = apc;
+            acc[0] += pc * apc;
+        }
+        qs += nwarps;
+        if (qs >= nseg) break;
+        sd = seg.desc[qs];
+        nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+        rec = load_rec7<double, false>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+        raw = load_raw7(g, nb, sd.x + lane, 0, 0, 0, sd.y + lane < g.n0, rawf);
+    }
+    block_sum<1, kJacThreads, kJacThreads>(acc, sh, 0);
+    if (threadIdx.x == 0) part.pap[blockIdx.x] = acc[0];
+}
+
+// K2 of iteration t: alpha = rz / p.Ap; x += alpha p; r -= alpha Ap; z = D^-1 r; r.r and r.z
+__global__ void __launch_bounds__(kJacThreads, 1) jacobi_update_kernel(LGeom g, SegArg seg,
+                                                                       const double* __restrict__ inv_diag,
+                                                                       double* __restrict__ x, double* __restrict__ r,
+                                                                       double* __restrict__ z,
+                                                                       const double* __restrict__ p,
+                                                                       const double* __restrict__ ap, Scalars* s,
+                                                                       int slot, JacPart part) {
+    __shared__ SumScratch<2, kJacThreads> sh;
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int nseg = *seg.count;
+    constexpr int U = 2;  // segments in flight a warp
+    int qs = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int c[U];
+    bool live[U];
+    double ic[U], pc[U], apc[U], xc[U], rc[U];
+    auto cells = [&]() {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int q = qs + u * nwarps;
+            const int4 sd = q < nseg ? seg.desc[q] : make_int4(0, g.n0, 0, 0);
+            live[u] = sd.y + lane < g.n0;
+            c[u] = sd.x + lane;
+            ic[u] = live[u] ? inv_diag[c[u]] : 0.0;
+        }
+    };
+    auto load = [&]() {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            pc[u] = live[u] ? p[c[u]] : 0.0;
+            apc[u] = live[u] ? ap[c[u]] : 0.0;
+            xc[u] = live[u] ? x[c[u]] : 0.0;
+            rc[u] = live[u] ? r[c[u]] : 0.0;
+        }
+    };
+    cells();
+    pdl_wait();
+    pdl_trigger();
+    load();
+    const int done = s->done;
+    const double rz = s->rz2[slot];
+    double t[1];
+    sum_partials(part.pap, part.blocks, t);
+    if (done) return;
+    const double alpha = rz / t[0];
+    if (!finite_d(alpha)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            s->bad = 1;
+            s->done = 1;
+        }
+        return;
+    }
+    double acc[2] = {0.0, 0.0};
+    while (true) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (live[u]) {
+                const double rn = rc[u] - alpha * apc[u];
+                const double zn = rn * ic[u];
+                x[c[u]] = xc[u] + alpha * pc[u];
+                r[c[u]] = rn;
+                z[c[u]] = zn;
+                acc[0] += rn * rn;
+                acc[1] += rn * zn;
+            }
+        qs += U * nwarps;
+        if (qs >= nseg) break;
+        cells();
+        load();
+    }
+    block_sum<2, kJacThreads, kJacThreads>(acc, sh, 0);
+    if (threadIdx.x == 0) {
+        part.rr[2 * blockIdx.x] = acc[0];
+        part.rr[2 * blockIdx.x + 1] = acc[1];
+    }
+}
+
+// After the last iteration of a batch: its dot products into the scalars (the host polls them)
+__global__ void jacobi_check_kernel(Scalars* s, int slot, JacPart part) {
+    pdl_wait();
+    pdl_trigger();
+    const int done = s->done;
+    const double rz_old = s->rz2[slot], thresh = s->thresh;
+    double t[2];
+    sum_partials(part.rr, part.blocks, t);
+    if (done || threadIdx.x != 0) return;
+    jacobi_store(s, jacobi_next(t, rz_old, thresh), slot ^ 1);
+}
+
+// Jacobi start: the reciprocal diagonal (0 on empty rows), z = D^-1 r and rz = r . z
+__global__ void jacobi_start_kernel(LGeom g, SegArg seg, const double* __restrict__ diag, const double* __restrict__ r,
+                                    double* __restrict__ inv_diag, double* __restrict__ z, Scalars* s,
+                                    double* partials, unsigned* counter) {
     double acc[1] = {0.0};
     SEG_LOOP_BEGIN(seg, g)
     const double d = diag[c];
-    if (d > 0.0) acc[0] += r[c] * (r[c] / d);
+    // (a diagonal below 2^-1000 takes that scale instead: its reciprocal could overflow)
+    const double ic = d_positive(d) ? 1.0 / fmax(d, 0x1p-1000) : 0.0;
+    const double rc = r[c];
+    const double zc = rc * ic;
+    inv_diag[c] = ic;
+    z[c] = zc;
+    acc[0] += rc * zc;
     SEG_LOOP_END
     double tot[1];
-    if (grid_sum<1>(acc, partials, counter, tot)) s->rz = tot[0];
+    if (grid_sum<1>(acc, partials, counter, tot)) s->rz2[0] = tot[0];
 }
 
 // The iterate as a float pair for the double-float residual (el_df.cuh), written with x by the
@@ -1500,6 +1747,14 @@ static int seg_blocks(el_ctx* ctx, long long total_segments) {
     return (int)((need * 32 + kSegThreads - 1) / kSegThreads);
 }
 
+// Blocks of a PCG kernel of kDotThreads<V>: one wave at most, and the tuned warps per SM.
+template <typename V, typename... KArgs>
+static int dot_blocks(el_ctx* ctx, void (*kernel)(KArgs...), long long total_segments) {
+    const long long warps = (long long)ctx->num_sms * ctx->seg_per_sm * (kSegThreads / 32);
+    const long long need = std::max<long long>(1, std::min<long long>(total_segments, warps));
+    return one_wave(ctx, kernel, kDotThreads<V>, (int)((need * 32 + kDotThreads<V> - 1) / kDotThreads<V>));
+}
+
 static SegArg seg_arg(const SegList& l) { return SegArg{l.desc, l.count}; }
 
 // The finest level's restriction is bound by the latency of its gathers: as many warps as can
@@ -1876,39 +2131,56 @@ static int enqueue_mg_iteration(el_ctx* ctx, const RA* A, V* x, V* r, V* z, V*& 
     {
         // reads z, p (not on the first iteration), records; writes p, Ap
         ProfScope prof(ctx, EL_KC_DIR_SPMV, N * (vs * (first ? 3 : 4) + sizeof(RA)));
-        dir_spmv_rec_kernel<V, RA><<<seg_blocks(ctx, seg.total), kSegThreads, 0, ctx->stream>>>(
-            g, seg_arg(seg), A, z, p, p_alt, ap, s, first, ctx->partials, ctx->counter);
+        auto kernel = dir_spmv_rec_kernel<V, RA>;
+        launch_dependent(ctx, kernel, dim3(dot_blocks<V>(ctx, kernel, seg.total)), dim3(kDotThreads<V>), 0, g,
+                         seg_arg(seg), A, (const V*)z, (const V*)p, p_alt, ap, s, first, ctx->partials,
+                         ctx->counter);
     }
     std::swap(p, p_alt);
     {
         // reads x, r, p, Ap; writes x, r
         ProfScope prof(ctx, EL_KC_UPDATE, N * vs * 6);
-        update_kernel<V, false><<<seg_blocks(ctx, seg.total), kSegThreads, 0, ctx->stream>>>(
-            g, seg_arg(seg), nullptr, x, r, p, ap, s, ctx->partials, ctx->counter);
+        auto kernel = update_kernel<V>;
+        launch_dependent(ctx, kernel, dim3(dot_blocks<V>(ctx, kernel, seg.total)), dim3(kDotThreads<V>), 0, g,
+                         seg_arg(seg), x, r, (const V*)p, (const V*)ap, s, ctx->partials, ctx->counter);
     }
     return 2 + enqueue_vcycle<V, R0, RC>(ctx, mg, seg, s, DOT_BETA);
 }
 
+// One iteration of the plain FP64 PCG.  pending: the update before it left its dot products as
+// partials; last: they are summed after this one (the end of a batch).  The slot of rz follows the
+// direction buffers, which alternate every iteration.
 template <typename OT>
 static int enqueue_jacobi_iteration(el_ctx* ctx, const SplitOp<OT>& A, double*& p, double*& p_alt, Scalars* s,
-                                    int first) {
+                                    int first, bool pending, bool last) {
     const LGeom g = make_geom(ctx->ni, ctx->nj, ctx->nk);
     const SegList& seg = ctx->seg0;
     const double N = active_cells(ctx, 0, (double)ctx->ni * ctx->nj * ctx->nk);
+    const int slot = p == ctx->p64 ? 0 : 1;
+    JacPart part;
+    const long long want = (seg.total * 32 + kJacThreads - 1) / kJacThreads;  // a warp a segment
+    part.blocks = (int)std::max<long long>(1, std::min<long long>(want, std::min(ctx->num_sms, kJacMaxBlocks)));
+    part.pap = ctx->partials;
+    part.rr = ctx->partials + kJacMaxBlocks;
     {
-        // reads r, p (not on the first iteration), diag, 3 couplings; writes p, Ap
+        // reads z, p (not on the first iteration), diag, 3 couplings; writes p, Ap
         ProfScope prof(ctx, EL_KC_DIR_SPMV, N * (8.0 * (first ? 4 : 5) + 3 * sizeof(OT)));
-        dir_spmv_jacobi_kernel<OT><<<seg_blocks(ctx, seg.total), kSegThreads, 0, ctx->stream>>>(
-            g, seg_arg(seg), A, ctx->r64, p, p_alt, ctx->ap64, s, first, ctx->partials, ctx->counter);
+        launch_dependent(ctx, jacobi_dir_kernel<OT>, dim3(part.blocks), dim3(kJacThreads), 0, g, seg_arg(seg), A,
+                         (const double*)ctx->z64, (const double*)p, p_alt, ctx->ap64, s, first, (int)pending, slot,
+                         part);
     }
     std::swap(p, p_alt);
     {
-        // reads x, r, p, Ap, diag; writes x, r
-        ProfScope prof(ctx, EL_KC_UPDATE, N * 8.0 * 7);
-        update_kernel<double, true><<<seg_blocks(ctx, seg.total), kSegThreads, 0, ctx->stream>>>(
-            g, seg_arg(seg), A.d, ctx->x64, ctx->r64, p, ctx->ap64, s, ctx->partials, ctx->counter);
+        // reads x, r, p, Ap, the reciprocal diagonal; writes x, r, z
+        ProfScope prof(ctx, EL_KC_UPDATE, N * 8.0 * 8);
+        launch_dependent(ctx, jacobi_update_kernel, dim3(part.blocks), dim3(kJacThreads), 0, g, seg_arg(seg),
+                         (const double*)ctx->inv64, ctx->x64, ctx->r64, ctx->z64, (const double*)p,
+                         (const double*)ctx->ap64, s, slot, part);
     }
-    return 2;
+    if (!last) return 2;
+    ProfScope prof(ctx, EL_KC_OTHER, 0);
+    launch_dependent(ctx, jacobi_check_kernel, dim3(1), dim3(64), 0, s, slot, part);
+    return 3;
 }
 
 // Launch PCG iterations (check_every per poll) until converged or `budget` are launched.
@@ -1926,7 +2198,8 @@ static int run_iterations(el_ctx* ctx, int solver, int which, int budget, int ch
     int st = poll(ctx, out, which);
     if (st != EL_OK) return st;
     if (out->done || budget <= 0) return EL_OK;
-    ctx->launches += enqueue(1);
+    // enqueue(first, position in the batch, last of the batch)
+    ctx->launches += enqueue(1, 0, true);
     launched_iters = 1;
     const int batch = std::max(2, (check_every + 1) / 2 * 2);
     const bool graphs = ctx->use_graphs && ctx->prof_mask == 0;
@@ -1944,7 +2217,7 @@ static int run_iterations(el_ctx* ctx, int solver, int which, int budget, int ch
                 cudaGraph_t graph = nullptr;
                 EL_CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
                 int n = 0;
-                for (int q = 0; q < batch; ++q) n += enqueue(0);
+                for (int q = 0; q < batch; ++q) n += enqueue(0, q, q + 1 == batch);
                 EL_CUDA_TRY(ctx, cudaStreamEndCapture(ctx->stream, &graph));
                 const cudaError_t e = cudaGraphInstantiate(&ctx->iter_graph[solver], graph, 0);
                 cudaGraphDestroy(graph);
@@ -1957,7 +2230,7 @@ static int run_iterations(el_ctx* ctx, int solver, int which, int budget, int ch
             launched_iters += batch;
         } else {
             const int b = std::min(batch, budget - launched_iters);
-            for (int q = 0; q < b; ++q) ctx->launches += enqueue(0);
+            for (int q = 0; q < b; ++q) ctx->launches += enqueue(0, q, q + 1 == b);
             launched_iters += b;
         }
         st = check_launch(ctx, "pcg iteration");
@@ -2060,13 +2333,15 @@ static int solve_t(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st) 
     }
     st->outer_iterations = 1;
     if (prm.solver == EL_SOLVER_JACOBI_FP64) {
-        jacobi_rz_kernel<<<seg_blocks(ctx, ctx->seg0.total), kSegThreads, 0, ctx->stream>>>(
-            g, seg_arg(ctx->seg0), ctx->diag64, ctx->r64, s0, ctx->partials, ctx->counter);
+        jacobi_start_kernel<<<seg_blocks(ctx, ctx->seg0.total), kSegThreads, 0, ctx->stream>>>(
+            g, seg_arg(ctx->seg0), ctx->diag64, ctx->r64, ctx->inv64, ctx->z64, s0, ctx->partials, ctx->counter);
         ctx->launches += 1;
         double* p = ctx->p64;
         double* p_alt = ctx->p64b;
         rc = run_iterations(ctx, EL_SOLVER_JACOBI_FP64, 0, prm.max_iter, check, h,
-                            [&](int first) { return enqueue_jacobi_iteration<T>(ctx, A64, p, p_alt, s0, first); });
+                            [&](int first, int pos, bool last) {
+                                return enqueue_jacobi_iteration<T>(ctx, A64, p, p_alt, s0, first, pos > 0, last);
+                            });
         st->iterations = h->iter;
         st->relres = h->bb > 0 ? sqrt(h->rr / h->bb) : 0.0;
     } else if (prm.solver == EL_SOLVER_MG_FP64) {
@@ -2081,7 +2356,7 @@ static int solve_t(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st) 
         ctx->launches += enqueue_vcycle<double, Rec64, Rec64>(ctx, mg, ctx->seg0, s0, DOT_INIT);
         double* p = ctx->p64;
         double* p_alt = ctx->p64b;
-        rc = run_iterations(ctx, EL_SOLVER_MG_FP64, 0, prm.max_iter, check, h, [&](int first) {
+        rc = run_iterations(ctx, EL_SOLVER_MG_FP64, 0, prm.max_iter, check, h, [&](int first, int, bool) {
             return enqueue_mg_iteration<double, Rec64, Rec64, Rec64>(ctx, ctx->A64rec, ctx->x64, ctx->r64, ctx->z64, p,
                                                                     p_alt, ctx->ap64, s0, first, mg);
         });
@@ -2133,7 +2408,7 @@ static int solve_t(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st) 
                 ctx->launches += enqueue_march_vcycle(ctx, mg, s1, DOT_INIT);
             else
                 ctx->launches += enqueue_vcycle<float, ushort4, float4>(ctx, mg, ctx->seg0, s1, DOT_INIT);
-            rc = run_iterations(ctx, EL_SOLVER_MIXED, 1, prm.max_iter - inner_total, check, &hi, [&](int first) {
+            rc = run_iterations(ctx, EL_SOLVER_MIXED, 1, prm.max_iter - inner_total, check, &hi, [&](int first, int, bool) {
                 if (march) return enqueue_march_iteration(ctx, p, p_alt, r, r_alt, s1, first, mg);
                 return enqueue_mg_iteration<float, float4, ushort4, float4>(ctx, ctx->A32, ctx->x32, ctx->r32, ctx->z32,
                                                                             p, p_alt, ctx->ap32, s1, first, mg);
@@ -2358,6 +2633,10 @@ int setup_solver_storage(el_ctx* ctx, int solver) {
             return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "solver vectors");
         int rc = alloc_seglist(ctx, ctx->seg0, ctx->ni, ctx->nj, ctx->nk);
         if (rc != EL_OK) return rc;
+    }
+    if (solver == EL_SOLVER_JACOBI_FP64 && !ctx->inv64) {
+        ctx->inv64 = (double*)ctx_alloc(ctx, n * 8);
+        if (!ctx->inv64) return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "reciprocal diagonal");
     }
     if (solver == EL_SOLVER_MG_FP64 && ctx->mg64.empty()) {
         ctx->A64rec = (Rec64*)ctx_alloc(ctx, n * sizeof(Rec64));

@@ -449,7 +449,7 @@ int el_nn_adam(int64_t n, float* w, float* g, float* m, float* v, float lr, floa
  * device.  el_solve_pressure_noalloc does what el_solve_pressure does with
  * EL_SOLVER_JACOBI_FP64 (plain FP64 PCG, Jacobi preconditioner), on caller-owned device arrays,
  * and allocates nothing: its scratch (cell flags, the grid-shaped matrix, the PCG vectors,
- * segment lists, reduction partials and scalars) is one fixed array of about 23 MB in the
+ * segment lists, reduction partials and scalars) is one fixed array of about 27 MB in the
  * library's device memory, which every GPU that loads the library holds until the process exits.
  *   - at most EL_NOALLOC_MAX_CELLS cells (64^3); larger grids return EL_ERR_TOO_LARGE before any
  *     device work;
