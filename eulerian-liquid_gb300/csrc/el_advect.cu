@@ -4,14 +4,14 @@
 // (StaggeredGridField, trace_rk2), include/nama/math/interpolation.h (lerp, weno6_interp).
 // Per output sample: sample position -> backtrace through the old velocity (trilinear MAC
 // interpolation at every RK stage) -> trilinear or WENO6 sample of the old field at the foot
-// point.  Two forms: advect_kernel, one thread per sample reading global memory (the stateless
-// operators; any dt), and the tiled kernels below, which stage what a tile of samples reads
-// (the velocity boxes; for WENO6 the level-set box and its x-pass smoothness terms) in shared
-// memory once -- under the CFL limit the foot point moves at most about one cell -- and fall
-// back to the global reads for a sample whose stencil leaves the box.  The boxes arrive by TMA
-// box copies (cp.async.bulk.tensor) wherever the array's row pitch is a multiple of 16 bytes;
-// the parts of a box outside the grid are then filled in from the clamped entries in shared
-// memory, so that a box holds the clamped grid either way.
+// point.  Two forms: advect_kernel, one thread per sample reading global memory (a field other than
+// the advecting velocity on a face grid; WENO6 face samples), and the tiled kernels below, which
+// stage what a tile of samples reads (the velocity boxes; for WENO6 the level-set box and its x-pass
+// smoothness terms) in shared memory once -- under the CFL limit the foot point moves at most about
+// one cell -- and fall back to the global reads for a sample whose stencil leaves the box.  The
+// boxes arrive by TMA box copies (cp.async.bulk.tensor) wherever the array's row pitch is a multiple
+// of 16 bytes; the parts of a box outside the grid are then filled in from the clamped entries in
+// shared memory, so that a box holds the clamped grid either way.
 #include <cstring>
 #include <limits>
 
@@ -45,57 +45,112 @@ struct MacMaps {
     BoxMap c[3];
 };
 
-// floor(t) and t - floor(t), the same values as index_fraction.  FP32: t + 1.5 * 2^23 rounded
-// toward -inf holds floor(t) in its low mantissa bits (exact for |t| < 2^22); outside that range
-// (and for NaN) the index lands millions of cells away, i.e. outside every staged box, and the
-// sample takes the exact global path.
+// Positions.  A face sample's backtrace (and an FP64 cell's) is kept as its displacement in cells,
+// relative to the sample itself: the RK stages are d = -(dt / dx) (weights . velocities), and a read at a displaced
+// position takes the floor and the fraction of the displacement per axis (plus the half cell
+// between cell and face samples).  Against absolute positions this leaves out, per coordinate, two
+// subtractions and a product (FP32) or a division (FP64: fifteen divisions a velocity sample,
+// nine FP64 operations each), and the fraction carries the rounding of a number near 1, not of a
+// coordinate of hundreds of cells.
+//
+// h: -1/2 along the sample's own face axis, 0 along the others and for cell samples; a position
+// d cells away has the coordinate d + h among cell-type samples and d + h + 1/2 among face-type
+// ones, relative to the sample's index.
+//
+// The FP32 level set keeps absolute positions, (x - origin - dx / 2) / dx, as the reference's loops:
+// the ghost-fluid fractions of the projection divide by distances to the surface down to a
+// hundredth of a cell, so that another rounding of the positions, a more exact one too, shows in
+// the projected velocity a thousand times larger.
+
+// floor(e) and e - floor(e).  FP64: within two cells, where every stage of a step under the CFL limit
+// lies, from the high word by integer comparisons (a floor and its conversion are FP64-pipe
+// operations; -1 counts as below -1, with fraction 1: the same point).  FP32: e + 1.5 * 2^23 rounded toward -inf holds floor(e) in its low
+// mantissa bits (exact for |e| < 2^22); outside that range (and for NaN) the index lands millions
+// of cells away, i.e. outside every staged box and grid, and the sample takes the general path.
 template <typename T>
-__device__ __forceinline__ void floor_index(T t, int& idx, T& frac) {
+__device__ __forceinline__ void floor_index(T e, int& idx, T& frac) {
     if constexpr (sizeof(T) == 4) {
         const float big = 12582912.0f;  // 1.5 * 2^23, bit pattern 0x4B400000
-        const float r = __fadd_rd(t, big);
+        const float r = __fadd_rd(e, big);
         idx = (int)((unsigned)__float_as_int(r) - 0x4B400000u);
-        frac = t - (r - big);
+        frac = e - (r - big);
     } else {
-        const T fl = floor(t);
-        idx = (int)fl;
-        frac = t - fl;
+        const int hi = __double2hiint(e);
+        if ((hi & 0x7fffffff) < 0x40000000) {
+            const bool neg = hi < 0, far = (unsigned)(hi & 0x7fffffff) >= 0x3ff00000u;
+            idx = neg ? (far ? -2 : -1) : (far ? 1 : 0);
+            frac = e - __hiloint2double(neg ? (far ? (int)0xc0000000 : (int)0xbff00000) : (far ? 0x3ff00000 : 0), 0);
+        } else {
+            const T fl = floor(e);
+            idx = (int)fl;
+            frac = e - fl;
+        }
     }
 }
 
-// one axis of a trilinear read: index_fraction's floor index and fraction (floor_index: the
-// same values)
+// One axis of a position: floor indices and fractions among cell-type and face-type samples.
 template <typename T>
-__device__ __forceinline__ void axis_index(T pos, T origin, T dx, T inv_dx, int& idx, T& frac) {
-    T t;
-    if constexpr (sizeof(T) == 8)
-        t = (pos - origin - T(0.5) * dx) / dx;
-    else
-        t = (pos - origin - T(0.5) * dx) * inv_dx;
-    floor_index(t, idx, frac);
+struct AxisCF {
+    int c, f;
+    T wc, wf;
+};
+
+// FP32: both floors in packed arithmetic (lane .x cell, .y face), as floor_index, plus base
+__device__ __forceinline__ AxisCF<float> axis_floor(float2 e, int base) {
+    const float big = 12582912.0f;
+    const float2 r = __fadd2_rd(e, make_float2(big, big));
+    const float2 fl = __fadd2_rn(r, make_float2(-big, -big));
+    const float2 w = __ffma2_rn(fl, make_float2(-1.f, -1.f), e);  // e - fl
+    const unsigned b = (unsigned)base - 0x4B400000u;
+    return AxisCF<float>{(int)((unsigned)__float_as_int(r.x) + b), (int)((unsigned)__float_as_int(r.y) + b), w.x, w.y};
 }
 
-// axis_index of one coordinate against two origins; FP32 in packed float2 arithmetic, the same
-// operations as axis_index and floor_index lane by lane
+// d cells away from sample index i
 template <typename T>
-__device__ __forceinline__ void axis_index_pair(T pos, T o1, T o2, T dx, T inv_dx, int& i1, T& f1, int& i2, T& f2) {
+__device__ __forceinline__ AxisCF<T> axis_rel(int i, T d, T h) {
     if constexpr (sizeof(T) == 4) {
-        const float h = 0.5f * dx;
-        const float2 t = __fmul2_rn(__fadd2_rn(__fadd2_rn(make_float2(pos, pos), make_float2(-o1, -o2)),
-                                               make_float2(-h, -h)),
-                                    make_float2(inv_dx, inv_dx));
-        const float big = 12582912.0f;  // 1.5 * 2^23, as floor_index
-        const float2 r = __fadd2_rd(t, make_float2(big, big));
-        const float2 fl = __fadd2_rn(r, make_float2(-big, -big));
-        const float2 f = __fadd2_rn(t, make_float2(-fl.x, -fl.y));
-        i1 = (int)((unsigned)__float_as_int(r.x) - 0x4B400000u);
-        i2 = (int)((unsigned)__float_as_int(r.y) - 0x4B400000u);
-        f1 = f.x;
-        f2 = f.y;
+        return axis_floor(__fadd2_rn(make_float2(d, d), make_float2(h, h + 0.5f)), i);
     } else {
-        axis_index(pos, o1, dx, inv_dx, i1, f1);
-        axis_index(pos, o2, dx, inv_dx, i2, f2);
+        AxisCF<T> a;
+        floor_index(h == T(0) ? d : d + h, a.c, a.wc);
+        floor_index(h == T(0) ? d + T(0.5) : d, a.f, a.wf);
+        a.c = (int)((unsigned)a.c + (unsigned)i);
+        a.f = (int)((unsigned)a.f + (unsigned)i);
+        return a;
     }
+}
+
+// the cell and face coordinates of an absolute FP32 position: (x - origin - dx / 2) / dx with the
+// origins 0 (cells) and -dx / 2 (faces)
+__device__ __forceinline__ float2 coord_abs(float x, float dx, float inv_dx) {
+    const float q = 0.5f * dx;
+    return __fmul2_rn(__fadd2_rn(__fadd2_rn(make_float2(x, x), make_float2(-0.f, q)), make_float2(-q, -q)),
+                      make_float2(inv_dx, inv_dx));
+}
+
+template <typename T>
+struct Vec3T {
+    T x, y, z;
+};
+
+template <typename T>
+struct Axes {
+    AxisCF<T> x, y, z;
+};
+template <typename T>
+__device__ __forceinline__ Axes<T> axes_rel(int i, int j, int k, const Vec3T<T>& h, const Vec3T<T>& d) {
+    return Axes<T>{axis_rel(i, d.x, h.x), axis_rel(j, d.y, h.y), axis_rel(k, d.z, h.z)};
+}
+__device__ __forceinline__ Axes<float> axes_abs(const Vec3T<float>& p, float dx, float inv_dx) {
+    return Axes<float>{axis_floor(coord_abs(p.x, dx, inv_dx), 0), axis_floor(coord_abs(p.y, dx, inv_dx), 0),
+                       axis_floor(coord_abs(p.z, dx, inv_dx), 0)};
+}
+
+// flat index of a sample; 32 bits hold it (every grid has fewer than 2^31 samples), and 64-bit
+// products cost several integer instructions each
+template <typename T>
+__device__ __forceinline__ int cell_index(const GridView<T>& g, int i, int j, int k) {
+    return i + g.n0 * (j + g.n1 * k);
 }
 
 // the 8 points of a trilinear read at floor indices (i, j, k) are inside the grid (then clamping
@@ -105,6 +160,25 @@ __device__ __forceinline__ bool tri_inside(const GridView<T>& g, int i, int j, i
     return (unsigned)i < (unsigned)(g.n0 - 1) && (unsigned)j < (unsigned)(g.n1 - 1) && (unsigned)k < (unsigned)(g.n2 - 1);
 }
 
+// the trilinear combination of 8 loaded points: x, then y, then z lerps; FP32 with the z = 0 and
+// z = 1 halves side by side in packed float2 arithmetic (each lane rounded as its scalar lerp)
+template <typename T>
+__device__ __forceinline__ T tri_mix(T fx, T fy, T fz, T c000, T c100, T c010, T c110, T c001, T c101, T c011,
+                                     T c111) {
+    if constexpr (sizeof(T) == 4) {
+        auto lerp2 = [](float2 a, float2 b, float f) {
+            const float g = 1.f - f;
+            return __ffma2_rn(make_float2(f, f), b, __fmul2_rn(make_float2(g, g), a));
+        };
+        const float2 x0 = lerp2(make_float2(c000, c001), make_float2(c100, c101), fx);
+        const float2 x1 = lerp2(make_float2(c010, c011), make_float2(c110, c111), fx);
+        const float2 y = lerp2(x0, x1, fy);
+        return lerp1(y.x, y.y, fz);
+    } else {
+        return tri_combine(fx, fy, fz, c000, c100, c010, c110, c001, c101, c011, c111);
+    }
+}
+
 // the 8 values of an inside read: one base address and fixed strides
 template <typename T>
 struct Tri8 {
@@ -112,121 +186,164 @@ struct Tri8 {
 };
 template <typename T>
 __device__ __forceinline__ Tri8<T> tri_load(const GridView<T>& g, int i, int j, int k) {
-    const long long sy = g.n0, sz = (long long)g.n0 * g.n1;
-    const T* p = g.d + (i + sy * j + sz * k);
-    return Tri8<T>{{__ldg(p), __ldg(p + 1), __ldg(p + sy), __ldg(p + sy + 1), __ldg(p + sz), __ldg(p + sz + 1),
-                    __ldg(p + sz + sy), __ldg(p + sz + sy + 1)}};
+    const T* p = g.d + cell_index(g, i, j, k);
+    const T *q = p + g.n0, *r = p + g.n0 * g.n1, *t = r + g.n0;
+    return Tri8<T>{{__ldg(p), __ldg(p + 1), __ldg(q), __ldg(q + 1), __ldg(r), __ldg(r + 1), __ldg(t), __ldg(t + 1)}};
 }
-// the trilinear combination of 8 loaded points: x, then y, then z lerps; FP32 with the z = 0 and
-// z = 1 halves side by side in packed float2 arithmetic (each lane rounded as its scalar lerp)
 template <typename T>
 __device__ __forceinline__ T tri_mix(const Tri8<T>& v, T fx, T fy, T fz) {
-    if constexpr (sizeof(T) == 4) {
-        auto lerp2 = [](float2 a, float2 b, float f) {
-            const float g = 1.f - f;
-            return __ffma2_rn(make_float2(f, f), b, __fmul2_rn(make_float2(g, g), a));
-        };
-        const float2 x0 = lerp2(make_float2(v.c[0], v.c[4]), make_float2(v.c[1], v.c[5]), fx);
-        const float2 x1 = lerp2(make_float2(v.c[2], v.c[6]), make_float2(v.c[3], v.c[7]), fx);
-        const float2 y = lerp2(x0, x1, fy);
-        return lerp1(y.x, y.y, fz);
-    } else {
-        TriIdx<T> t;
-        t.fx = fx;
-        t.fy = fy;
-        t.fz = fz;
-        return tri_combine(t, v.c[0], v.c[1], v.c[2], v.c[3], v.c[4], v.c[5], v.c[6], v.c[7]);
-    }
+    return tri_mix(fx, fy, fz, v.c[0], v.c[1], v.c[2], v.c[3], v.c[4], v.c[5], v.c[6], v.c[7]);
 }
 
-// u, v, w at one position from global memory: the three components share six axis coordinates
-// (u at a face in x, cells in y and z; v and w likewise).  When all three reads are inside the
-// grid (the common case) their 24 loads go out together from fixed offsets; otherwise each
-// takes the clamped gather -- the values of three sample_trilinear calls either way
+// trilinear read of the sample's own grid, d cells away from sample (i, j, k)
 template <typename T>
-__device__ __forceinline__ void velocity_at(const Mac<T>& m, T x, T y, T z, T dx, T inv, T& vx, T& vy,
-                                            T& vz) {
-    int ixf, ixc, jyf, jyc, kzf, kzc;
-    T fxf, fxc, fyf, fyc, fzf, fzc;
-    axis_index_pair(x, m.u.ox, m.v.ox, dx, inv, ixf, fxf, ixc, fxc);
-    axis_index_pair(y, m.v.oy, m.u.oy, dx, inv, jyf, fyf, jyc, fyc);
-    axis_index_pair(z, m.w.oz, m.u.oz, dx, inv, kzf, fzf, kzc, fzc);
-    if (tri_inside(m.u, ixf, jyc, kzc) && tri_inside(m.v, ixc, jyf, kzc) && tri_inside(m.w, ixc, jyc, kzf)) {
-        const Tri8<T> a = tri_load(m.u, ixf, jyc, kzc), b = tri_load(m.v, ixc, jyf, kzc),
-                      c = tri_load(m.w, ixc, jyc, kzf);
-        vx = tri_mix(a, fxf, fyc, fzc);
-        vy = tri_mix(b, fxc, fyf, fzc);
-        vz = tri_mix(c, fxc, fyc, fzf);
-    } else {
-        vx = sample_trilinear(m.u, x, y, z, dx, inv);
-        vy = sample_trilinear(m.v, x, y, z, dx, inv);
-        vz = sample_trilinear(m.w, x, y, z, dx, inv);
-    }
+__device__ __forceinline__ T own_at(const GridView<T>& g, int i, int j, int k, const Vec3T<T>& d) {
+    int bi, bj, bk;
+    T fx, fy, fz;
+    floor_index(d.x, bi, fx);
+    floor_index(d.y, bj, fy);
+    floor_index(d.z, bk, fz);
+    bi = (int)((unsigned)bi + (unsigned)i);
+    bj = (int)((unsigned)bj + (unsigned)j);
+    bk = (int)((unsigned)bk + (unsigned)k);
+    if (tri_inside(g, bi, bj, bk)) return tri_mix(tri_load(g, bi, bj, bk), fx, fy, fz);
+    return tri_clamped(g, i, j, k, d.x, d.y, d.z);
 }
 
-// trace_rk2 (ode.h:30-35) or Ralston RK3 (c = 0, 1/2, 3/4; b = 2/9, 1/3, 4/9); h is the
-// signed step (-dt for a backtrace).
-template <typename T, int TRACE>
-__device__ __forceinline__ void backtrace_from(const Mac<T>& m, T ax, T ay, T az, T& x, T& y, T& z, T h, T dx, T inv) {
-    const T h2 = T(0.5) * h;
-    T bx, by, bz;
-    velocity_at(m, x + h2 * ax, y + h2 * ay, z + h2 * az, dx, inv, bx, by, bz);
+// The clamped gathers of u, v, w for a position outside the grid (or a box): d cells away from sample
+// (i, j, k), or at an absolute position.
+template <typename T>
+struct FarRel {
+    int i, j, k;
+    Vec3T<T> h, d;
+    template <int C>
+    __device__ __forceinline__ T at(const GridView<T>& g) const {
+        const T q = T(0.5);
+        return tri_clamped(g, i, j, k, d.x + (h.x + (C == 0 ? q : T(0))), d.y + (h.y + (C == 1 ? q : T(0))),
+                           d.z + (h.z + (C == 2 ? q : T(0))));
+    }
+};
+struct FarAbs {
+    Vec3T<float> p;
+    float dx, inv_dx;
+    template <int C>
+    __device__ __forceinline__ float at(const GridView<float>& g) const {
+        const float2 x = coord_abs(p.x, dx, inv_dx), y = coord_abs(p.y, dx, inv_dx), z = coord_abs(p.z, dx, inv_dx);
+        return tri_clamped(g, 0, 0, 0, C == 0 ? x.y : x.x, C == 1 ? y.y : y.x, C == 2 ? z.y : z.x);
+    }
+};
+
+// u, v, w at one position from global memory: the three components share six axis coordinates (u at
+// a face in x, cells in y and z; v and w likewise).  When all three reads are inside the grid (the
+// common case) their 24 loads go out together from fixed offsets; otherwise each takes the
+// clamped gather -- the same values either way
+template <typename T, typename FAR>
+__device__ __forceinline__ Vec3T<T> velocity_global(const Mac<T>& m, const Axes<T>& a, const FAR& far) {
+    const AxisCF<T>&x = a.x, &y = a.y, &z = a.z;
+    if (tri_inside(m.u, x.f, y.c, z.c) && tri_inside(m.v, x.c, y.f, z.c) && tri_inside(m.w, x.c, y.c, z.f)) {
+        const Tri8<T> u = tri_load(m.u, x.f, y.c, z.c), v = tri_load(m.v, x.c, y.f, z.c), w = tri_load(m.w, x.c, y.c, z.f);
+        return Vec3T<T>{tri_mix(u, x.wf, y.wc, z.wc), tri_mix(v, x.wc, y.wf, z.wc), tri_mix(w, x.wc, y.wc, z.wf)};
+    }
+    return Vec3T<T>{far.template at<0>(m.u), far.template at<1>(m.v), far.template at<2>(m.w)};
+}
+
+// The displacement of trace_rk2 (ode.h:30-35) or Ralston RK3 (c = 0, 1/2, 3/4; b = 2/9, 1/3, 4/9)
+// from the first stage's velocity a; s is the signed step in cells per unit velocity (-dt / dx for
+// a backtrace), at(d) the velocity d cells away.
+template <typename T, int TRACE, typename F>
+__device__ __forceinline__ Vec3T<T> backtrace_from(const Vec3T<T>& a, T s, F&& at) {
+    const T s2 = T(0.5) * s;
+    const Vec3T<T> b = at(Vec3T<T>{s2 * a.x, s2 * a.y, s2 * a.z});
     if constexpr (TRACE == EL_TRACE_RK2) {
-        x = x + h * bx;
-        y = y + h * by;
-        z = z + h * bz;
+        return Vec3T<T>{s * b.x, s * b.y, s * b.z};
     } else {
-        const T h3 = T(0.75) * h;
-        T cx, cy, cz;
-        velocity_at(m, x + h3 * bx, y + h3 * by, z + h3 * bz, dx, inv, cx, cy, cz);
-        const T w1 = h * (T(2) / T(9)), w2 = h * (T(1) / T(3)), w3 = h * (T(4) / T(9));
-        x = x + w1 * ax + w2 * bx + w3 * cx;
-        y = y + w1 * ay + w2 * by + w3 * cy;
-        z = z + w1 * az + w2 * bz + w3 * cz;
+        const T s3 = T(0.75) * s;
+        const Vec3T<T> c = at(Vec3T<T>{s3 * b.x, s3 * b.y, s3 * b.z});
+        const T w1 = s * (T(2) / T(9)), w2 = s * (T(1) / T(3)), w3 = s * (T(4) / T(9));
+        return Vec3T<T>{w1 * a.x + w2 * b.x + w3 * c.x, w1 * a.y + w2 * b.y + w3 * c.y,
+                        w1 * a.z + w2 * b.z + w3 * c.z};
     }
-}
-
-template <typename T, int TRACE>
-__device__ __forceinline__ void backtrace(const Mac<T>& m, T& x, T& y, T& z, T h, T dx, T inv) {
-    T ax, ay, az;
-    velocity_at(m, x, y, z, dx, inv, ax, ay, az);
-    backtrace_from<T, TRACE>(m, ax, ay, az, x, y, z, h, dx, inv);
 }
 
 // The velocity at the centre of cell (i, j, k), the first stage of a level-set backtrace: the
 // trilinear read there has fractions 1/2 along a component's own axis and 0 along the others,
 // so each component is the mean of its two faces (a zero fraction leaves its first value).
-// Exact fractions where index_fraction of the rounded cell position may carry a rounding error
-// of an ulp or so.  The faces of a cell are inside every grid (no clamping).
+// The faces of a cell are inside every grid (no clamping).
 template <typename T>
-__device__ __forceinline__ void cell_velocity(const Mac<T>& m, int i, int j, int k, T& vx, T& vy, T& vz) {
-    const long long cu = lin3(i, j, k, m.u.n0, m.u.n1), cv = lin3(i, j, k, m.v.n0, m.v.n1);
-    const long long cw = lin3(i, j, k, m.w.n0, m.w.n1);
-    vx = lerp1(__ldg(m.u.d + cu), __ldg(m.u.d + cu + 1), T(0.5));
-    vy = lerp1(__ldg(m.v.d + cv), __ldg(m.v.d + cv + m.v.n0), T(0.5));
-    vz = lerp1(__ldg(m.w.d + cw), __ldg(m.w.d + cw + (long long)m.w.n0 * m.w.n1), T(0.5));
+__device__ __forceinline__ Vec3T<T> cell_velocity(const Mac<T>& m, int i, int j, int k) {
+    const T* u = m.u.d + cell_index(m.u, i, j, k);
+    const T* v = m.v.d + cell_index(m.v, i, j, k);
+    const T* w = m.w.d + cell_index(m.w, i, j, k);
+    return Vec3T<T>{lerp1(__ldg(u), __ldg(u + 1), T(0.5)), lerp1(__ldg(v), __ldg(v + m.v.n0), T(0.5)),
+                    lerp1(__ldg(w), __ldg(w + m.w.n0 * m.w.n1), T(0.5))};
 }
 
-// out(x) = src(trace(x, -dt)) for every sample of src's grid (cell centres or one face
-// component); positions are GridBase::pos = (idx + 0.5) * dx + origin (grid.h:355-367).
+// The foot point of cell (i, j, k), as the coordinate among the cells that own_at and sample_weno6
+// take: FP64 the displacement, relative to the cell; FP32 the absolute coordinate (relative to
+// index 0).  vel(axes, far) reads the velocity.
+template <typename T>
+__device__ __forceinline__ int foot_base(int i) {
+    return sizeof(T) == 4 ? 0 : i;
+}
+template <typename T, int TRACE, typename F>
+__device__ __forceinline__ Vec3T<T> level_set_foot(const Vec3T<T>& a, int i, int j, int k, T dt, T dx, T inv_dx, F&& vel) {
+    if constexpr (sizeof(T) == 8) {
+        const Vec3T<T> h{T(0), T(0), T(0)};
+        return backtrace_from<T, TRACE>(a, -dt * inv_dx, [&](const Vec3T<T>& d) {
+            return vel(axes_rel(i, j, k, h, d), FarRel<T>{i, j, k, h, d});
+        });
+    } else {
+        const float h = -dt;
+        const Vec3T<float> p{rn_mul(i + 0.5f, dx), rn_mul(j + 0.5f, dx), rn_mul(k + 0.5f, dx)};
+        auto step = [](const Vec3T<float>& q, float s, const Vec3T<float>& v) {
+            return Vec3T<float>{rn_fma(s, v.x, q.x), rn_fma(s, v.y, q.y), rn_fma(s, v.z, q.z)};
+        };
+        auto at = [&](const Vec3T<float>& q) { return vel(axes_abs(q, dx, inv_dx), FarAbs{q, dx, inv_dx}); };
+        const Vec3T<float> b = at(step(p, 0.5f * h, a));
+        Vec3T<float> q;
+        if constexpr (TRACE == EL_TRACE_RK2) {
+            q = step(p, h, b);
+        } else {
+            const Vec3T<float> c = at(step(p, 0.75f * h, b));
+            q = step(step(step(p, h * (2.f / 9.f), a), h * (1.f / 3.f), b), h * (4.f / 9.f), c);
+        }
+        return Vec3T<float>{coord_abs(q.x, dx, inv_dx).x, coord_abs(q.y, dx, inv_dx).x, coord_abs(q.z, dx, inv_dx).x};
+    }
+}
+
+// out(x) = src(trace(x, -dt)) for every sample of src's grid (comp 0: cell centres, 1..3: a face
+// component).
 template <typename T, int TRACE, int SAMPLE>
-__global__ void __launch_bounds__(256) advect_kernel(GridView<T> src, T* __restrict__ out, Mac<T> mac,
+__global__ void __launch_bounds__(256) advect_kernel(GridView<T> src, int comp, T* __restrict__ out, Mac<T> mac,
                                                      DtArg dt, T dx, T inv_dx) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int k = blockIdx.z;
     if (i >= src.n0 || j >= src.n1) return;
-    const T h = -(T)dt_value(dt);
-    T x = (i + T(0.5)) * dx + src.ox;
-    T y = (j + T(0.5)) * dx + src.oy;
-    T z = (k + T(0.5)) * dx + src.oz;
-    backtrace<T, TRACE>(mac, x, y, z, h, dx, inv_dx);
+    const T dtv = (T)dt_value(dt);
+    const Vec3T<T> zero{T(0), T(0), T(0)};
+    int bi = i, bj = j, bk = k;
+    Vec3T<T> e;
+    if (comp == 0) {
+        auto vel = [&](const Axes<T>& a, const auto& far) { return velocity_global(mac, a, far); };
+        const Vec3T<T> a = vel(axes_rel(i, j, k, zero, zero), FarRel<T>{i, j, k, zero, zero});
+        e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, vel);
+        bi = foot_base<T>(i);
+        bj = foot_base<T>(j);
+        bk = foot_base<T>(k);
+    } else {
+        const Vec3T<T> h{comp == 1 ? T(-0.5) : T(0), comp == 2 ? T(-0.5) : T(0), comp == 3 ? T(-0.5) : T(0)};
+        auto at = [&](const Vec3T<T>& d) {
+            return velocity_global(mac, axes_rel(i, j, k, h, d), FarRel<T>{i, j, k, h, d});
+        };
+        e = backtrace_from<T, TRACE>(at(zero), -dtv * inv_dx, at);
+    }
     T r;
     if constexpr (SAMPLE == EL_SAMPLE_WENO6)
-        r = sample_weno6(src, x, y, z, dx, inv_dx);
+        r = sample_weno6(src, bi, bj, bk, e.x, e.y, e.z);
     else
-        r = sample_trilinear(src, x, y, z, dx, inv_dx);
-    const long long oc = lin3(i, j, k, src.n0, src.n1);
+        r = own_at(src, bi, bj, bk, e);
+    const int oc = cell_index(src, i, j, k);
     if (EL_IN(oc, (long long)src.n0 * src.n1 * src.n2, 1)) out[oc] = r;
 }
 
@@ -244,213 +361,136 @@ __global__ void __launch_bounds__(256) advect_kernel(GridView<T> src, T* __restr
 // The box holds the clamped grid (entry p = value at clamp(box origin + p)), so a sample reads
 // its 8 points at the unclamped indices i, i+1 (j, k likewise) with no clamping and gets exactly
 // the values of the clamped gather lerp() makes; the 8 reads sit at fixed offsets from one
-// address.  The floor of the cell coordinate is taken without conversions (floor_index), and
-// the three components at one position share their cell-centred and face coordinates.  Along
-// x a box starts four entries left of the tile (a box copy starts on a 16-byte boundary) and
-// holds 40 entries; along y and z the halo is two.
+// address.  Along x a box starts four entries left of the tile (a box copy starts on a 16-byte
+// boundary) and holds 40 entries; along y and z the halo is two.
 constexpr int kTileX = 32, kTileY = 8, kTileZ = 8, kHalo = 2, kHaloX = 4;
 constexpr int kBoxX = kTileX + 2 * kHaloX, kBoxY = kTileY + 2 * kHalo, kBoxZ = kTileZ + 2 * kHalo;
+// (Rows 64 words apart in FP32, which leaves no bank conflicts where a floor changes within a warp,
+// measured the same in the velocity kernel: 594 against 579 us at 256^3; two CTAs an SM, not three.)
 constexpr int kBoxN = kBoxX * kBoxY * kBoxZ;
 
-// the cell coordinate of index_fraction: (pos - origin - dx / 2) / dx
-template <typename T>
-__device__ __forceinline__ T cell_coord(T pos, T origin, T dx, T inv_dx) {
-    if constexpr (sizeof(T) == 8)
-        return (pos - origin - T(0.5) * dx) / dx;
-    else
-        return (pos - origin - T(0.5) * dx) * inv_dx;
-}
-
-// one axis of a position: box-relative floor index and fraction
-template <typename T>
-struct AxisPos {
-    int a;
-    T f;
-};
-
-template <typename T>
-__device__ __forceinline__ AxisPos<T> axis_pos(T pos, T origin, int box0, T dx, T inv_dx) {
-    AxisPos<T> p;
-    int idx;
-    floor_index(cell_coord(pos, origin, dx, inv_dx), idx, p.f);
-    p.a = (int)((unsigned)idx - (unsigned)box0);
-    return p;
-}
-
-template <typename T>
-__device__ __forceinline__ T lerp_combine(T fx, T fy, T fz, T c000, T c100, T c010, T c110, T c001, T c101, T c011,
-                                          T c111) {
-    if constexpr (sizeof(T) == 4) {
-        // FP32: the z = 0 and z = 1 halves side by side in packed float2 arithmetic (the same
-        // lerps, x then y, each lane rounded as its scalar operations), then the z lerp
-        auto lerp2 = [](float2 a, float2 b, float f) {
-            const float g = 1.f - f;
-            return __ffma2_rn(make_float2(f, f), b, __fmul2_rn(make_float2(g, g), a));
-        };
-        const float2 x0 = lerp2(make_float2(c000, c001), make_float2(c100, c101), fx);
-        const float2 x1 = lerp2(make_float2(c010, c011), make_float2(c110, c111), fx);
-        const float2 y = lerp2(x0, x1, fy);
-        return lerp1(y.x, y.y, fz);
-    } else {
-        const T lo = lerp1(lerp1(c000, c100, fx), lerp1(c010, c110, fx), fy);
-        const T hi = lerp1(lerp1(c001, c101, fx), lerp1(c011, c111, fx), fy);
-        return lerp1(lo, hi, fz);
-    }
-}
-
-// axis_pos of one coordinate against two origins (FP32: in packed float2 arithmetic, the same
-// operations as cell_coord and floor_index lane by lane)
-template <typename T>
-__device__ __forceinline__ void axis_pos_pair(T pos, T o1, T o2, int box0, T dx, T inv_dx, AxisPos<T>& p1,
-                                              AxisPos<T>& p2) {
-    int i1, i2;
-    axis_index_pair(pos, o1, o2, dx, inv_dx, i1, p1.f, i2, p2.f);
-    p1.a = (int)((unsigned)i1 - (unsigned)box0);
-    p2.a = (int)((unsigned)i2 - (unsigned)box0);
-}
-
-// trilinear sample from a staged box at box-relative (x, y, z); false when the 8 points are not
-// all inside the box.  CHECK = false: the caller knows they are (see advect_velocity_tiled_kernel)
+// trilinear sample from a staged box at box-relative floor indices (x, y, z); false when the 8
+// points are not all inside the box.  CHECK = false: the caller knows they are (see
+// advect_velocity_tiled_kernel)
 template <typename T, bool CHECK = true>
-__device__ __forceinline__ bool staged_lerp(const T* box, const AxisPos<T>& x, const AxisPos<T>& y,
-                                            const AxisPos<T>& z, T& out) {
-    if (CHECK && ((unsigned)x.a >= (unsigned)(kBoxX - 1) || (unsigned)y.a >= (unsigned)(kBoxY - 1) ||
-                  (unsigned)z.a >= (unsigned)(kBoxZ - 1)))
+__device__ __forceinline__ bool staged_lerp(const T* box, int x, int y, int z, T fx, T fy, T fz, T& out) {
+    if (CHECK && ((unsigned)x >= (unsigned)(kBoxX - 1) || (unsigned)y >= (unsigned)(kBoxY - 1) ||
+                  (unsigned)z >= (unsigned)(kBoxZ - 1)))
         return false;
-    const T* p = box + (z.a * kBoxY + y.a) * kBoxX + x.a;
+    const T* p = box + (z * kBoxY + y) * kBoxX + x;
     constexpr int SY = kBoxX, SZ = kBoxX * kBoxY;
-    out = lerp_combine(x.f, y.f, z.f, p[0], p[1], p[SY], p[SY + 1], p[SZ], p[SZ + 1], p[SZ + SY], p[SZ + SY + 1]);
+    out = tri_mix(fx, fy, fz, p[0], p[1], p[SY], p[SY + 1], p[SZ], p[SZ + 1], p[SZ + SY], p[SZ + SY + 1]);
     return true;
 }
 
 template <typename T>
-struct Staged {
-    const T* box;         // shared memory, [z][y][x] over the box
-    int bx0, by0, bz0;    // grid index of the box's first entry
-};
-
-template <typename T, bool CHECK = true>
-__device__ __forceinline__ T sample_staged(const GridView<T>& g, const Staged<T>& b, T x, T y, T z, T dx, T inv) {
-    T r;
-    if (staged_lerp<T, CHECK>(b.box, axis_pos(x, g.ox, b.bx0, dx, inv), axis_pos(y, g.oy, b.by0, dx, inv),
-                              axis_pos(z, g.oz, b.bz0, dx, inv), r) ||
-        !CHECK)
-        return r;
-    return sample_trilinear(g, x, y, z, dx, inv);
-}
-
-template <typename T>
 struct StagedMac {
-    Staged<T> u, v, w;
+    const T* box;         // shared memory: the boxes of u, v, w, each [z][y][x]
+    int bx0, by0, bz0;    // grid index of the boxes' first entry
 };
 
-// u at (face x, cell y, cell z), v at (cell, face, cell), w at (cell, cell, face): six axis
-// positions serve all three (the cell origins are those of the other components' grids)
-template <typename T, bool CHECK = true>
-__device__ __forceinline__ void velocity_at_staged(const Mac<T>& m, const StagedMac<T>& s, T x, T y, T z, T dx, T inv,
-                                                   T& vx, T& vy, T& vz) {
-    AxisPos<T> xf, xc, yf, yc, zf, zc;
-    axis_pos_pair(x, m.u.ox, m.v.ox, s.u.bx0, dx, inv, xf, xc);
-    axis_pos_pair(y, m.v.oy, m.u.oy, s.u.by0, dx, inv, yf, yc);
-    axis_pos_pair(z, m.w.oz, m.u.oz, s.u.bz0, dx, inv, zf, zc);
-    if (!staged_lerp<T, CHECK>(s.u.box, xf, yc, zc, vx) && CHECK) vx = sample_trilinear(m.u, x, y, z, dx, inv);
-    if (!staged_lerp<T, CHECK>(s.v.box, xc, yf, zc, vy) && CHECK) vy = sample_trilinear(m.v, x, y, z, dx, inv);
-    if (!staged_lerp<T, CHECK>(s.w.box, xc, yc, zf, vz) && CHECK) vz = sample_trilinear(m.w, x, y, z, dx, inv);
+// u, v, w at one position through the staged boxes
+template <typename T, bool CHECK, typename FAR>
+__device__ __forceinline__ Vec3T<T> velocity_staged(const Mac<T>& m, const StagedMac<T>& b, const Axes<T>& a,
+                                                    const FAR& far) {
+    auto rel = [](int g, int b0) { return (int)((unsigned)g - (unsigned)b0); };
+    const AxisCF<T>&x = a.x, &y = a.y, &z = a.z;
+    const int xc = rel(x.c, b.bx0), xf = rel(x.f, b.bx0), yc = rel(y.c, b.by0), yf = rel(y.f, b.by0);
+    const int zc = rel(z.c, b.bz0), zf = rel(z.f, b.bz0);
+    Vec3T<T> v;
+    if (!staged_lerp<T, CHECK>(b.box, xf, yc, zc, x.wf, y.wc, z.wc, v.x) && CHECK) v.x = far.template at<0>(m.u);
+    if (!staged_lerp<T, CHECK>(b.box + kBoxN, xc, yf, zc, x.wc, y.wf, z.wc, v.y) && CHECK) v.y = far.template at<1>(m.v);
+    if (!staged_lerp<T, CHECK>(b.box + 2 * kBoxN, xc, yc, zf, x.wc, y.wc, z.wf, v.z) && CHECK)
+        v.z = far.template at<2>(m.w);
+    return v;
 }
 
-// backtrace with the staged velocity: the same stages and arithmetic as backtrace(), from the
-// first stage's velocity (ax, ay, az) at (x, y, z)
-template <typename T, int TRACE, bool CHECK = true>
-__device__ __forceinline__ void backtrace_staged_from(const Mac<T>& m, const StagedMac<T>& sm, T ax, T ay, T az, T& x,
-                                                      T& y, T& z, T h, T dx, T inv) {
-    const T h2 = T(0.5) * h;
-    T bx, by, bz;
-    velocity_at_staged<T, CHECK>(m, sm, x + h2 * ax, y + h2 * ay, z + h2 * az, dx, inv, bx, by, bz);
-    if constexpr (TRACE == EL_TRACE_RK2) {
-        x = x + h * bx;
-        y = y + h * by;
-        z = z + h * bz;
-    } else {
-        const T h3 = T(0.75) * h;
-        T cx, cy, cz;
-        velocity_at_staged<T, CHECK>(m, sm, x + h3 * bx, y + h3 * by, z + h3 * bz, dx, inv, cx, cy, cz);
-        const T w1 = h * (T(2) / T(9)), w2 = h * (T(1) / T(3)), w3 = h * (T(4) / T(9));
-        x = x + w1 * ax + w2 * bx + w3 * cx;
-        y = y + w1 * ay + w2 * by + w3 * cy;
-        z = z + w1 * az + w2 * bz + w3 * cz;
-    }
-}
-
-template <typename T, int TRACE, bool CHECK = true>
-__device__ __forceinline__ void backtrace_staged(const Mac<T>& m, const StagedMac<T>& sm, T& x, T& y, T& z, T h, T dx,
-                                                 T inv) {
-    T ax, ay, az;
-    velocity_at_staged<T, CHECK>(m, sm, x, y, z, dx, inv, ax, ay, az);
-    backtrace_staged_from<T, TRACE, CHECK>(m, sm, ax, ay, az, x, y, z, h, dx, inv);
-}
-
-// The velocity at the centre of a face of component c, the first stage of its backtrace: the
+// The velocity at the centre of a face of component C, the first stage of its backtrace: the
 // trilinear read there has fractions 0 and 1/2 only, so it is the face's own value and the
 // four-point means of the two other components, in the trilinear read's order (x, then y, then
-// z; a zero fraction leaves its first value).  Exact fractions where index_fraction of the
-// rounded face position may carry a rounding error of an ulp or so.  Every point lies in the
-// staged boxes (their halos are at least one entry), which hold the clamped grid.
-template <typename T>
-__device__ __forceinline__ T box_at(const Staged<T>& b, int I, int J, int K) {
-    return b.box[(K * kBoxY + J) * kBoxX + I];
-}
-
+// z; a zero fraction leaves its first value).  (I, J, K): the face, relative to the boxes.  Every
+// point lies in the staged boxes (their halos are at least one entry), which hold the clamped grid.
 template <typename T>
 __device__ __forceinline__ T mid4(T a, T b, T c, T d) {
     return lerp1(lerp1(a, b, T(0.5)), lerp1(c, d, T(0.5)), T(0.5));
 }
 
+// pairs of two samples' values: each lane rounded as the scalar operation
+__device__ __forceinline__ float2 operator*(float s, float2 v) { return __fmul2_rn(make_float2(s, s), v); }
+__device__ __forceinline__ float2 lerp1(float2 a, float2 b, float2 f) {
+    const float2 g = __ffma2_rn(f, make_float2(-1.f, -1.f), make_float2(1.f, 1.f));  // 1 - f, one rounding
+    return __ffma2_rn(f, b, __fmul2_rn(g, a));
+}
+__device__ __forceinline__ float2 lerp1(float2 a, float2 b, float f) { return lerp1(a, b, make_float2(f, f)); }
+__device__ __forceinline__ float2 mid4(float2 a, float2 b, float2 c, float2 d) {
+    return lerp1(lerp1(a, b, 0.5f), lerp1(c, d, 0.5f), 0.5f);
+}
+
+// box entries around the face: M(component, di, dj, dk)
+template <typename V, int C, typename F>
+__device__ __forceinline__ Vec3T<V> face_velocity(F&& M) {
+    if constexpr (C == 0)
+        return Vec3T<V>{M(0, 0, 0, 0), mid4(M(1, -1, 0, 0), M(1, 0, 0, 0), M(1, -1, 1, 0), M(1, 0, 1, 0)),
+                        mid4(M(2, -1, 0, 0), M(2, 0, 0, 0), M(2, -1, 0, 1), M(2, 0, 0, 1))};
+    else if constexpr (C == 1)
+        return Vec3T<V>{mid4(M(0, 0, -1, 0), M(0, 1, -1, 0), M(0, 0, 0, 0), M(0, 1, 0, 0)), M(1, 0, 0, 0),
+                        mid4(M(2, 0, -1, 0), M(2, 0, 0, 0), M(2, 0, -1, 1), M(2, 0, 0, 1))};
+    else
+        return Vec3T<V>{mid4(M(0, 0, 0, -1), M(0, 1, 0, -1), M(0, 0, 0, 0), M(0, 1, 0, 0)),
+                        mid4(M(1, 0, 0, -1), M(1, 0, 1, -1), M(1, 0, 0, 0), M(1, 0, 1, 0)), M(2, 0, 0, 0)};
+}
+
+// The largest |value| met, NaN once one was met.  FP32: a three-input maximum of magnitudes that
+// keeps NaN; FP64: the high word of the magnitude on the integer pipe (NaN's is above every
+// number's), read back as a bound from above.
 template <typename T>
-__device__ __forceinline__ void face_velocity(const StagedMac<T>& s, int c, int i, int j, int k, T& vx, T& vy, T& vz) {
-    const int I = i - s.u.bx0, J = j - s.u.by0, K = k - s.u.bz0;
-    if (c == 0) {
-        vx = box_at(s.u, I, J, K);
-        vy = mid4(box_at(s.v, I - 1, J, K), box_at(s.v, I, J, K), box_at(s.v, I - 1, J + 1, K), box_at(s.v, I, J + 1, K));
-        vz = mid4(box_at(s.w, I - 1, J, K), box_at(s.w, I, J, K), box_at(s.w, I - 1, J, K + 1), box_at(s.w, I, J, K + 1));
-    } else if (c == 1) {
-        vx = mid4(box_at(s.u, I, J - 1, K), box_at(s.u, I + 1, J - 1, K), box_at(s.u, I, J, K), box_at(s.u, I + 1, J, K));
-        vy = box_at(s.v, I, J, K);
-        vz = mid4(box_at(s.w, I, J - 1, K), box_at(s.w, I, J, K), box_at(s.w, I, J - 1, K + 1), box_at(s.w, I, J, K + 1));
-    } else {
-        vx = mid4(box_at(s.u, I, J, K - 1), box_at(s.u, I + 1, J, K - 1), box_at(s.u, I, J, K), box_at(s.u, I + 1, J, K));
-        vy = mid4(box_at(s.v, I, J, K - 1), box_at(s.v, I, J + 1, K - 1), box_at(s.v, I, J, K), box_at(s.v, I, J + 1, K));
-        vz = box_at(s.w, I, J, K);
+struct AbsMax;
+template <>
+struct AbsMax<float> {
+    float m = 0.f;
+    __device__ __forceinline__ void add(float a, float b) {
+        asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(m), "f"(a), "f"(b));
     }
-}
+    __device__ __forceinline__ void add16(const float* p) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        add(q.x, q.y);
+        add(q.z, q.w);
+    }
+    __device__ __forceinline__ void add(float a) { add(a, a); }
+    __device__ __forceinline__ AbsMax shuffled(int o) const { return AbsMax{__shfl_xor_sync(0xffffffffu, m, o)}; }
+    __device__ __forceinline__ void join(const AbsMax& o) { add(o.m, o.m); }
+    __device__ __forceinline__ float value() const { return m; }
+};
+template <>
+struct AbsMax<double> {
+    unsigned m = 0;
+    __device__ __forceinline__ void add(double a) { m = max(m, (unsigned)__double2hiint(a) & 0x7fffffffu); }
+    __device__ __forceinline__ void add16(const double* p) {
+        const double2 q = *reinterpret_cast<const double2*>(p);
+        add(q.x);
+        add(q.y);
+    }
+    __device__ __forceinline__ AbsMax shuffled(int o) const { return AbsMax{__shfl_xor_sync(0xffffffffu, m, o)}; }
+    __device__ __forceinline__ void join(const AbsMax& o) { m = max(m, o.m); }
+    __device__ __forceinline__ double value() const { return __hiloint2double((int)m, -1); }
+};
 
-// max(|a|, |b|) that is NaN when either is (fmax would drop a NaN)
-template <typename T>
-__device__ __forceinline__ T fmax_nan(T m, T v) {
-    const T a = v < T(0) ? -v : v;
-    return (a > m || a != a) ? a : m;
-}
-
-// A box that arrived by a box copy, made the clamped box: an entry outside the grid takes the
-// value of its clamped entry (inside the grid, so the copy filled it), one warp per row; with
-// MAX, vmax gathers the largest |value| of the entries inside the grid (the values the clamped
-// box holds).  A box that lies inside the grid is only scanned for vmax, in 16-byte reads.
-template <typename T, int BX, int BY, int BZ, bool MAX>
-__device__ __forceinline__ void finish_box(T* box, const GridView<T>& g, int bx0, int by0, int bz0, T& vmax) {
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y, nthr = blockDim.x * blockDim.y;
+// A box that arrived by a box copy (rows of PITCH entries, of which the first BX are used), made
+// the clamped box: an entry outside the grid takes the value of its clamped entry (inside the
+// grid, so the copy filled it), one warp per row; with MAX, vmax gathers the largest |value| of the
+// entries inside the grid (the values the clamped box holds).  A box that lies inside the grid is
+// only scanned for vmax, in 16-byte reads.
+template <typename T, int BX, int BY, int BZ, bool MAX, int PITCH = BX>
+__device__ __forceinline__ void finish_box(T* box, const GridView<T>& g, int bx0, int by0, int bz0, AbsMax<T>& vmax) {
+    const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+    const int nthr = blockDim.x * blockDim.y * blockDim.z;
     const bool edge = bx0 < 0 || by0 < 0 || bz0 < 0 || bx0 + BX > g.n0 || by0 + BY > g.n1 || bz0 + BZ > g.n2;
     if (!edge) {
         if constexpr (MAX) {
-            static_assert((BX * BY * BZ * sizeof(T)) % 16 == 0, "whole 16-byte reads");
-            constexpr int nv = BX * BY * BZ * (int)sizeof(T) / 16;
-            for (int e = tid; e < nv; e += nthr) {
-                if constexpr (sizeof(T) == 4) {
-                    const float4 q = reinterpret_cast<const float4*>(box)[e];
-                    vmax = fmax_nan(fmax_nan(fmax_nan(fmax_nan(vmax, q.x), q.y), q.z), q.w);
-                } else {
-                    const double2 q = reinterpret_cast<const double2*>(box)[e];
-                    vmax = fmax_nan(fmax_nan(vmax, q.x), q.y);
-                }
-            }
+            constexpr int per = 16 / (int)sizeof(T), row = BX / per;
+            static_assert(BX % per == 0 && PITCH % per == 0, "whole 16-byte reads");
+#pragma unroll 4
+            for (int e = tid; e < row * BY * BZ; e += nthr) vmax.add16(box + (e / row) * PITCH + (e % row) * per);
         }
         return;
     }
@@ -459,12 +499,12 @@ __device__ __forceinline__ void finish_box(T* box, const GridView<T>& g, int bx0
         const int bz = row / BY, by = row - bz * BY;
         const int cy = clampi(by0 + by, 0, g.n1 - 1) - by0, cz = clampi(bz0 + bz, 0, g.n2 - 1) - bz0;
         const bool row_in = cy == by && cz == bz;
-        const T* src = box + (cz * BY + cy) * BX;
-        T* dst = box + row * BX;
+        const T* src = box + (cz * BY + cy) * PITCH;
+        T* dst = box + row * PITCH;
         for (int x = lane; x < BX; x += 32) {
             const int cx = clampi(bx0 + x, 0, g.n0 - 1) - bx0;
             if (row_in && cx == x) {
-                if (MAX) vmax = fmax_nan(vmax, dst[x]);
+                if (MAX) vmax.add(dst[x]);
             } else {
                 dst[x] = src[cx];
             }
@@ -486,7 +526,7 @@ __device__ __forceinline__ void copy_boxes_begin(uint64_t* bar, unsigned bytes) 
 __device__ __forceinline__ bool copy_boxes_failed(uint64_t* bar) {
     const bool ok = mbar_wait(bar, 0);
     if (!__syncthreads_or(!ok)) return false;
-    if (threadIdx.x == 0 && threadIdx.y == 0) {
+    if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
         atomicOr(&advect_wait_fault, 1u);
         mbar_wait(bar, 0);
     }
@@ -499,21 +539,47 @@ template <typename T>
 __device__ __forceinline__ void nan_column(const GridView<T>& g, T* __restrict__ o, int i, int j, int z0, int nz) {
     if (i >= g.n0 || j >= g.n1) return;
     for (int kk = 0; kk < nz && z0 + kk < g.n2; ++kk) {
-        const long long oc = lin3(i, j, z0 + kk, g.n0, g.n1);
+        const int oc = cell_index(g, i, j, z0 + kk);
         if (EL_IN(oc, (long long)g.n0 * g.n1 * g.n2, 4)) o[oc] = std::numeric_limits<T>::quiet_NaN();
     }
 }
 
 // Stages the clamped boxes of u, v, w around tile (x0, y0, z0): a component with a box map by a
-// box copy (then finish_box), the others by plain loads, rows of kBoxX along x, one warp per row.
-// vmax gathers the largest |value| this thread staged or scanned (NaN if it met one).  `failed`:
-// the box copies did not arrive (the same in every thread).
+// box copy (then finish_box), the others by plain loads (the first 32 entries of a row one warp a
+// row, the last 8 of all rows by all threads).  vmax gathers the largest |value| this thread staged
+// or scanned (NaN if it met one).  `failed`: the box copies did not arrive (the same in every
+// thread).
+template <typename T>
+__device__ __forceinline__ void stage_plain(const GridView<T>& g, T* box, int bx0, int by0, int bz0, int tid, int nthr,
+                                            AbsMax<T>& vmax) {
+    const int lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
+    auto row_of = [&](int row) {
+        const int bz = row / kBoxY, by = row - bz * kBoxY;
+        const int gy = clampi(by0 + by, 0, g.n1 - 1), gz = clampi(bz0 + bz, 0, g.n2 - 1);
+        return g.d + (long long)g.n0 * (gy + (long long)g.n1 * gz);
+    };
+    const int gx = clampi(bx0 + lane, 0, g.n0 - 1);
+#pragma unroll 6
+    for (int row = warp; row < kBoxY * kBoxZ; row += nwarps) {
+        const T v = __ldg(row_of(row) + gx);
+        box[row * kBoxX + lane] = v;
+        vmax.add(v);
+    }
+    constexpr int kTail = kBoxX - 32;
+    const int tx = clampi(bx0 + 32 + tid % kTail, 0, g.n0 - 1);
+#pragma unroll 2
+    for (int e = tid; e < kTail * kBoxY * kBoxZ; e += nthr) {
+        const T v = __ldg(row_of(e / kTail) + tx);
+        box[(e / kTail) * kBoxX + 32 + tid % kTail] = v;
+        vmax.add(v);
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ StagedMac<T> stage_mac(const Mac<T>& m, const MacMaps& maps, T* smem, uint64_t* bar,
-                                                  int x0, int y0, int z0, T& vmax, bool& failed) {
+                                                  int x0, int y0, int z0, AbsMax<T>& vmax, bool& failed) {
     const int bx0 = x0 - kHaloX, by0 = y0 - kHalo, bz0 = z0 - kHalo;
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    const int lane = tid & 31, warp = tid >> 5, nwarps = (blockDim.x * blockDim.y) >> 5;
+    const int tid = threadIdx.x + blockDim.x * threadIdx.y, nthr = blockDim.x * blockDim.y;
     // the flags in registers (a parameter indexed at run time would be copied to local memory)
     const bool on0 = maps.c[0].on != 0, on1 = maps.c[1].on != 0, on2 = maps.c[2].on != 0;
     const int ncopy = (int)on0 + (int)on1 + (int)on2;
@@ -523,23 +589,9 @@ __device__ __forceinline__ StagedMac<T> stage_mac(const Mac<T>& m, const MacMaps
         if (on1) tma_load_3d(smem + kBoxN, &maps.c[1].m, bar, bx0, by0, bz0);
         if (on2) tma_load_3d(smem + 2 * kBoxN, &maps.c[2].m, bar, bx0, by0, bz0);
     }
-    for (int row = warp; row < 3 * kBoxY * kBoxZ; row += nwarps) {
-        const int comp = row / (kBoxY * kBoxZ), r = row - comp * (kBoxY * kBoxZ);
-        if (comp == 0 ? on0 : (comp == 1 ? on1 : on2)) continue;
-        const int bz = r / kBoxY, by = r - bz * kBoxY;
-        const GridView<T>& g = comp == 0 ? m.u : (comp == 1 ? m.v : m.w);
-        T* dst = smem + comp * kBoxN + (bz * kBoxY + by) * kBoxX;
-        const int gy = clampi(by0 + by, 0, g.n1 - 1), gz = clampi(bz0 + bz, 0, g.n2 - 1);
-        const T* src = g.d + (long long)g.n0 * (gy + (long long)g.n1 * gz);
-        const T va = __ldg(src + clampi(bx0 + lane, 0, g.n0 - 1));
-        dst[lane] = va;
-        vmax = fmax_nan(vmax, va);
-        if (lane < kBoxX - 32) {
-            const T vb = __ldg(src + clampi(bx0 + 32 + lane, 0, g.n0 - 1));
-            dst[32 + lane] = vb;
-            vmax = fmax_nan(vmax, vb);
-        }
-    }
+    if (!on0) stage_plain(m.u, smem, bx0, by0, bz0, tid, nthr, vmax);
+    if (!on1) stage_plain(m.v, smem + kBoxN, bx0, by0, bz0, tid, nthr, vmax);
+    if (!on2) stage_plain(m.w, smem + 2 * kBoxN, bx0, by0, bz0, tid, nthr, vmax);
     failed = false;
     if (ncopy) {
         __syncthreads();  // the mbarrier's initialisation is seen by every thread
@@ -550,102 +602,225 @@ __device__ __forceinline__ StagedMac<T> stage_mac(const Mac<T>& m, const MacMaps
             if (on2) finish_box<T, kBoxX, kBoxY, kBoxZ, true>(smem + 2 * kBoxN, m.w, bx0, by0, bz0, vmax);
         }
     }
-    return StagedMac<T>{{smem, bx0, by0, bz0}, {smem + kBoxN, bx0, by0, bz0}, {smem + 2 * kBoxN, bx0, by0, bz0}};
+    return StagedMac<T>{smem, bx0, by0, bz0};
 }
 
-// The largest |velocity| the CTA staged (NaN if it staged a NaN), as the same value in every
-// thread.  Call after the staging, in place of the __syncthreads that ends it.
+// The largest |velocity| the CTA staged (NaN if it staged a NaN; FP64: a bound from above), as the
+// same value in every thread.  Call after the staging, in place of the __syncthreads that ends it.
 template <typename T>
-__device__ __forceinline__ T box_max(T vmax) {
-    __shared__ T wmax[kTileX * kTileY / 32];
-    for (int o = 16; o > 0; o >>= 1) vmax = fmax_nan(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+__device__ __forceinline__ T box_max(AbsMax<T> vmax) {
+    __shared__ decltype(vmax.m) wmax[kTileX * kTileY / 32];
+    for (int o = 16; o > 0; o >>= 1) vmax.join(vmax.shuffled(o));
     const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-    if ((tid & 31) == 0) wmax[tid >> 5] = vmax;
+    if ((tid & 31) == 0) wmax[tid >> 5] = vmax.m;
     __syncthreads();
-    T m = T(0);
+    AbsMax<T> m;
 #pragma unroll
-    for (int q = 0; q < kTileX * kTileY / 32; ++q) m = fmax_nan(m, wmax[q]);
-    return m;
+    for (int q = 0; q < kTileX * kTileY / 32; ++q) m.join(AbsMax<T>{wmax[q]});
+    return m.value();
 }
 
 // A step moves no sample more than one cell when |v| |dt| / dx < 1 over the staged boxes (every
 // RK stage and the foot point are convex combinations of velocities read inside the boxes, by
 // induction): then all of a tile's staged reads fall inside its boxes (the halo is two cells)
 // and the reads need no check.  False for a NaN or infinite velocity or dt.
+// s: the step in cells per unit velocity
 template <typename T>
-__device__ __forceinline__ bool within_one_cell(T vmax, T h, T inv_dx) {
-    const T reach = vmax * (h < T(0) ? -h : h) * inv_dx;
+__device__ __forceinline__ bool within_one_cell(T vmax, T s) {
+    const T reach = vmax * (s < T(0) ? -s : s);
     return reach <= T(0.999);
 }
 
-// the u, v, w samples of a tile (CHECK: each staged read is checked and falls back to the
-// global read outside the box)
-template <typename T, int TRACE, bool CHECK>
-__device__ __forceinline__ void velocity_tile(const Mac<T>& mac, const StagedMac<T>& sm, T* __restrict__ ou,
-                                              T* __restrict__ ov, T* __restrict__ ow, T h, T dx, T inv_dx, int x0,
-                                              int y0, int z0) {
-    const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
-#pragma unroll 1
-    for (int kk = 0; kk < kTileZ; ++kk) {
-        const int k = z0 + kk;
-#pragma unroll 1
-        for (int c = 0; c < 3; ++c) {
-            // the component's grid, box and output, picked by value (no local arrays)
-            GridView<T> g = mac.u;
-            Staged<T> b = sm.u;
-            T* o = ou;
-            if (c == 1) {
-                g = mac.v;
-                b = sm.v;
-                o = ov;
-            } else if (c == 2) {
-                g = mac.w;
-                b = sm.w;
-                o = ow;
-            }
-            if (i >= g.n0 || j >= g.n1 || k >= g.n2) continue;
-            T x = (i + T(0.5)) * dx + g.ox;
-            T y = (j + T(0.5)) * dx + g.oy;
-            T z = (k + T(0.5)) * dx + g.oz;
-            T ax, ay, az;
-            face_velocity(sm, c, i, j, k, ax, ay, az);
-            backtrace_staged_from<T, TRACE, CHECK>(mac, sm, ax, ay, az, x, y, z, h, dx, inv_dx);
-            const long long oc = lin3(i, j, k, g.n0, g.n1);
-            const T r = sample_staged<T, CHECK>(g, b, x, y, z, dx, inv_dx);
-            if (EL_IN(oc, (long long)g.n0 * g.n1 * g.n2, 2)) o[oc] = r;
-        }
-    }
+// one sample of component C (CHECK: each staged read is checked and falls back to the global read
+// outside the box)
+template <typename T, int TRACE, bool CHECK, int C>
+__device__ __forceinline__ void velocity_sample(const Mac<T>& mac, const GridView<T>& g, const StagedMac<T>& sm,
+                                                T* __restrict__ o, T s, int i, int j, int k) {
+    if (i >= g.n0 || j >= g.n1 || k >= g.n2) return;
+    const T* own = sm.box + C * kBoxN;
+    const int I = i - sm.bx0, J = j - sm.by0, K = k - sm.bz0;
+    const Vec3T<T> h{C == 0 ? T(-0.5) : T(0), C == 1 ? T(-0.5) : T(0), C == 2 ? T(-0.5) : T(0)};
+    const Vec3T<T> a = face_velocity<T, C>([&](int c, int di, int dj, int dk) {
+        return sm.box[c * kBoxN + ((K + dk) * kBoxY + J + dj) * kBoxX + I + di];
+    });
+    const Vec3T<T> d = backtrace_from<T, TRACE>(a, s, [&](const Vec3T<T>& e) {
+        return velocity_staged<T, CHECK>(mac, sm, axes_rel(i, j, k, h, e), FarRel<T>{i, j, k, h, e});
+    });
+    int x, y, z;
+    T fx, fy, fz, r;
+    floor_index(d.x, x, fx);
+    floor_index(d.y, y, fy);
+    floor_index(d.z, z, fz);
+    if (!staged_lerp<T, CHECK>(own, (int)((unsigned)I + (unsigned)x), (int)((unsigned)J + (unsigned)y),
+                               (int)((unsigned)K + (unsigned)z), fx, fy, fz, r) &&
+        CHECK)
+        r = tri_clamped(g, i, j, k, d.x, d.y, d.z);
+    const int oc = cell_index(g, i, j, k);
+    if (EL_IN(oc, (long long)g.n0 * g.n1 * g.n2, 2)) o[oc] = r;
 }
 
-// u, v, w of a tile, each advected through the (old) velocity itself
+// Two samples of component C, (i, j, k) and (i, j, k + 1), in packed float2 arithmetic from the
+// boxes to the result: every quantity is a pair of the two samples' values, so no lanes are moved
+// between pairs (with the halves of one trilinear read as the pair, a third of the instructions
+// moved registers).  Each lane is rounded as velocity_sample's scalars.  Only for tiles in which
+// every read lies in the boxes.
+// a pair of floors as byte offsets (times `stride`, plus `base`), and the fractions
+struct AxisPair {
+    unsigned a, b;
+    float2 w;
+};
+__device__ __forceinline__ AxisPair axis_pair(float2 e, unsigned base, unsigned stride) {
+    const float big = 12582912.0f;  // as floor_index
+    const float2 r = __fadd2_rd(e, make_float2(big, big));
+    const float2 fl = __fadd2_rn(r, make_float2(-big, -big));
+    AxisPair p;
+    p.w = __ffma2_rn(fl, make_float2(-1.f, -1.f), e);  // e - fl (packed additions take no negated operand)
+    // the magic number's bits fold into the base (unsigned arithmetic wraps)
+    const unsigned c = base - 0x4B400000u * stride;
+    // (as instructions: the compiler's own folding of this product was seen to lose the stride)
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(p.a) : "r"(__float_as_int(r.x)), "r"(stride), "r"(c));
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(p.b) : "r"(__float_as_int(r.y)), "r"(stride), "r"(c));
+    return p;
+}
+
+// byte strides of a box
+constexpr unsigned kSX = 4, kSY = 4 * kBoxX, kSZ = kSY * kBoxY;
+
+// the entry at shared-memory byte address `at` + OFF
+template <int OFF>
+__device__ __forceinline__ float lds(unsigned at) {
+    float v;
+    asm("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(at), "n"(OFF));
+    return v;
+}
+
+// trilinear reads of a pair of samples, the second one plane above, from the box at byte offset BOX
+// (box0: the boxes' shared-memory address)
+template <int BOX>
+__device__ __forceinline__ float2 tri_pair(unsigned box0, const AxisPair& x, const AxisPair& y, const AxisPair& z) {
+    unsigned p = x.a + y.a + z.a, q = x.b + y.b + z.b;
+    constexpr int SX = kSX, SY = kSY, SZ = kSZ, UP = BOX + SZ;
+    if (!EL_IN(p - box0, 4 * kBoxN - SX - SY - SZ, 5) || !EL_IN(q - box0, 4 * kBoxN - SX - SY - 2 * SZ, 6)) p = q = box0;
+    // (every read is in the box, see the callers; a wrong address would be a fault, not a wrong value)
+    p = box0 + min(p - box0, (unsigned)(4 * kBoxN - SX - SY - SZ - 4));
+    q = box0 + min(q - box0, (unsigned)(4 * kBoxN - SX - SY - 2 * SZ - 4));
+    const float2 x00 = lerp1(make_float2(lds<BOX>(p), lds<UP>(q)), make_float2(lds<BOX + SX>(p), lds<UP + SX>(q)), x.w);
+    const float2 x10 = lerp1(make_float2(lds<BOX + SY>(p), lds<UP + SY>(q)),
+                             make_float2(lds<BOX + SY + SX>(p), lds<UP + SY + SX>(q)), x.w);
+    const float2 x01 = lerp1(make_float2(lds<BOX + SZ>(p), lds<UP + SZ>(q)),
+                             make_float2(lds<BOX + SZ + SX>(p), lds<UP + SZ + SX>(q)), x.w);
+    const float2 x11 = lerp1(make_float2(lds<BOX + SZ + SY>(p), lds<UP + SZ + SY>(q)),
+                             make_float2(lds<BOX + SZ + SY + SX>(p), lds<UP + SZ + SY + SX>(q)), x.w);
+    return lerp1(lerp1(x00, x10, y.w), lerp1(x01, x11, y.w), z.w);
+}
+
+template <int TRACE, int C>
+__device__ __forceinline__ void velocity_pair(const GridView<float>& g, const StagedMac<float>& sm,
+                                              float* __restrict__ o, float s, int i, int j, int k) {
+    if (i >= g.n0 || j >= g.n1 || k >= g.n2) return;
+    const unsigned box0 = (unsigned)__cvta_generic_to_shared(sm.box);
+    const unsigned I = kSX * (i - sm.bx0) + box0;
+    const unsigned J = kSY * (j - sm.by0), K = kSZ * (k - sm.bz0);
+    constexpr int B = 4 * kBoxN;  // bytes of a box
+    constexpr int P = kBoxX;
+    const float* centre = sm.box + ((k - sm.bz0) * kBoxY + j - sm.by0) * P + i - sm.bx0;
+    const Vec3T<float2> a = face_velocity<float2, C>([&](int c, int di, int dj, int dk) {
+        const float* p = centre + (c * kBoxN + (dk * kBoxY + dj) * P + di);
+        return make_float2(p[0], p[P * kBoxY]);
+    });
+    auto cell = [](float2 d, bool face_axis) { return face_axis ? __fadd2_rn(d, make_float2(-0.5f, -0.5f)) : d; };
+    auto face = [](float2 d, bool face_axis) { return face_axis ? d : __fadd2_rn(d, make_float2(0.5f, 0.5f)); };
+    auto at = [&](float2 dx, float2 dy, float2 dz) {
+        const AxisPair xc = axis_pair(cell(dx, C == 0), I, kSX), xf = axis_pair(face(dx, C == 0), I, kSX);
+        const AxisPair yc = axis_pair(cell(dy, C == 1), J, kSY), yf = axis_pair(face(dy, C == 1), J, kSY);
+        const AxisPair zc = axis_pair(cell(dz, C == 2), K, kSZ), zf = axis_pair(face(dz, C == 2), K, kSZ);
+        return Vec3T<float2>{tri_pair<0>(box0, xf, yc, zc), tri_pair<B>(box0, xc, yf, zc), tri_pair<2 * B>(box0, xc, yc, zf)};
+    };
+    const float s2 = 0.5f * s;
+    const Vec3T<float2> b = at(s2 * a.x, s2 * a.y, s2 * a.z);
+    Vec3T<float2> d;
+    if constexpr (TRACE == EL_TRACE_RK2) {
+        d = Vec3T<float2>{s * b.x, s * b.y, s * b.z};
+    } else {
+        const float s3 = 0.75f * s;
+        const Vec3T<float2> c = at(s3 * b.x, s3 * b.y, s3 * b.z);
+        const float w1 = s * (2.f / 9.f), w2 = s * (1.f / 3.f), w3 = s * (4.f / 9.f);
+        auto sum = [&](float2 p, float2 q, float2 r) {
+            return __ffma2_rn(make_float2(w3, w3), r, __ffma2_rn(make_float2(w2, w2), q, w1 * p));
+        };
+        d = Vec3T<float2>{sum(a.x, b.x, c.x), sum(a.y, b.y, c.y), sum(a.z, b.z, c.z)};
+    }
+    const float2 r = tri_pair<C * B>(box0, axis_pair(d.x, I, kSX), axis_pair(d.y, J, kSY), axis_pair(d.z, K, kSZ));
+    const int oc = cell_index(g, i, j, k), plane = g.n0 * g.n1;
+    if (EL_IN(oc, (long long)plane * g.n2, 2)) o[oc] = r.x;
+    if (k + 1 < g.n2 && EL_IN(oc + plane, (long long)plane * g.n2, 2)) o[oc + plane] = r.y;
+}
+
+// The u, v, w samples of a tile of cells.  A component has one more sample than cells along its own
+// axis: where the last tile is full, it also takes that column, row or plane of faces (one entry
+// beyond the tile, which the boxes' halos serve along that axis) rather than a further tile
+// staging three boxes for them.
+template <typename T, int TRACE, bool CHECK>
+__device__ __forceinline__ void velocity_tile(const Mac<T>& mac, const StagedMac<T>& sm, T* __restrict__ ou,
+                                              T* __restrict__ ov, T* __restrict__ ow, T s, int x0, int y0, int z0) {
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int i = x0 + tx, j = y0 + ty;
+    const bool more_u = x0 + kTileX == mac.u.n0 - 1, more_v = y0 + kTileY == mac.v.n1 - 1;
+    const bool more_w = z0 + kTileZ == mac.w.n2 - 1;
+    if constexpr (sizeof(T) == 4 && !CHECK) {
+#pragma unroll 1
+        for (int kk = 0; kk < kTileZ; kk += 2) {
+            velocity_pair<TRACE, 0>(mac.u, sm, ou, s, i, j, z0 + kk);
+            velocity_pair<TRACE, 1>(mac.v, sm, ov, s, i, j, z0 + kk);
+            velocity_pair<TRACE, 2>(mac.w, sm, ow, s, i, j, z0 + kk);
+        }
+    } else {
+#pragma unroll 1
+        for (int kk = 0; kk < kTileZ; ++kk) {
+            velocity_sample<T, TRACE, CHECK, 0>(mac, mac.u, sm, ou, s, i, j, z0 + kk);
+            velocity_sample<T, TRACE, CHECK, 1>(mac, mac.v, sm, ov, s, i, j, z0 + kk);
+            velocity_sample<T, TRACE, CHECK, 2>(mac, mac.w, sm, ow, s, i, j, z0 + kk);
+        }
+    }
+    // 8 x 8 faces by two warps, 32 x 8 by all
+    if (more_u && ty < 2) velocity_sample<T, TRACE, CHECK, 0>(mac, mac.u, sm, ou, s, x0 + kTileX, y0 + (tx & 7), z0 + 4 * ty + (tx >> 3));
+    if (more_v) velocity_sample<T, TRACE, CHECK, 1>(mac, mac.v, sm, ov, s, i, y0 + kTileY, z0 + ty);
+    if (more_w) velocity_sample<T, TRACE, CHECK, 2>(mac, mac.w, sm, ow, s, i, j, z0 + kTileZ);
+}
+
+// u, v, w of a tile, each advected through the (old) velocity itself.  FP32: bound by shared-memory
+// loads (66 a sample, seven trilinear reads) and issue (285 instructions a sample, from 617):
+// 256^3 RK3 0.96 -> 0.58 ms, three per-sample launches of 256 x 128 x 192 took 0.62 ms for what
+// now takes 0.24.  FP64: bound by its FP64 operations (155 a sample, from 350): 128^3 RK3 5.04 ->
+// 1.81 ms.
 template <typename T, int TRACE>
-__global__ void __launch_bounds__(kTileX * kTileY, 3) advect_velocity_tiled_kernel(
-    Mac<T> mac, T* __restrict__ ou, T* __restrict__ ov, T* __restrict__ ow, DtArg dt, T dx, T inv_dx,
+__global__ void __launch_bounds__(kTileX * kTileY, sizeof(T) == 4 ? 3 : 1) advect_velocity_tiled_kernel(
+    Mac<T> mac, T* __restrict__ ou, T* __restrict__ ov, T* __restrict__ ow, DtArg dt, T inv_dx,
     const __grid_constant__ MacMaps maps) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* smem = reinterpret_cast<T*>(align128(smem_raw));
     __shared__ uint64_t bar;
     const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY, z0 = blockIdx.z * kTileZ;
-    T vmax = T(0);
+    AbsMax<T> vmax;
     bool failed;
     const StagedMac<T> sm = stage_mac(mac, maps, smem, &bar, x0, y0, z0, vmax, failed);
     if (failed) {
         const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
-        nan_column(mac.u, ou, i, j, z0, kTileZ);
-        nan_column(mac.v, ov, i, j, z0, kTileZ);
-        nan_column(mac.w, ow, i, j, z0, kTileZ);
+        nan_column(mac.u, ou, i, j, z0, kTileZ + 1);
+        nan_column(mac.v, ov, i, j, z0, kTileZ + 1);
+        nan_column(mac.w, ow, i, j, z0, kTileZ + 1);
         return;
     }
     const T bm = box_max(vmax);  // ends the staging (a barrier)
-    const T h = -(T)dt_value(dt);
-    if (within_one_cell(bm, h, inv_dx))
-        velocity_tile<T, TRACE, false>(mac, sm, ou, ov, ow, h, dx, inv_dx, x0, y0, z0);
+    const T s = -(T)dt_value(dt) * inv_dx;
+    if (within_one_cell(bm, s))
+        velocity_tile<T, TRACE, false>(mac, sm, ou, ov, ow, s, x0, y0, z0);
     else
-        velocity_tile<T, TRACE, true>(mac, sm, ou, ov, ow, h, dx, inv_dx, x0, y0, z0);
+        velocity_tile<T, TRACE, true>(mac, sm, ou, ov, ow, s, x0, y0, z0);
 }
 
-// the level set (cells) through the staged velocity; phi itself from global memory
-template <typename T, int TRACE, int SAMPLE>
+// the level set (cells) through the staged velocity; phi itself from global memory (trilinear)
+template <typename T, int TRACE>
 __global__ void __launch_bounds__(kTileX * kTileY) advect_phi_tiled_kernel(GridView<T> src, T* __restrict__ out,
                                                                            Mac<T> mac, DtArg dt, T dx, T inv_dx,
                                                                            const __grid_constant__ MacMaps maps) {
@@ -653,249 +828,445 @@ __global__ void __launch_bounds__(kTileX * kTileY) advect_phi_tiled_kernel(GridV
     T* smem = reinterpret_cast<T*>(align128(smem_raw));
     __shared__ uint64_t bar;
     const int x0 = blockIdx.x * kTileX, y0 = blockIdx.y * kTileY, z0 = blockIdx.z * kTileZ;
-    T vmax = T(0);
+    AbsMax<T> vmax;
     bool failed;
     const StagedMac<T> sm = stage_mac(mac, maps, smem, &bar, x0, y0, z0, vmax, failed);
     if (failed) {
         nan_column(src, out, x0 + threadIdx.x, y0 + threadIdx.y, z0, kTileZ);
         return;
     }
-    const bool inside = within_one_cell(box_max(vmax), -(T)dt_value(dt), inv_dx);  // ends the staging
-    const T h = -(T)dt_value(dt);
+    const T dtv = (T)dt_value(dt);
+    const bool inside = within_one_cell(box_max(vmax), dtv * inv_dx);  // ends the staging
     const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
     if (i >= src.n0 || j >= src.n1) return;
 #pragma unroll 1
     for (int kk = 0; kk < kTileZ; ++kk) {
         const int k = z0 + kk;
         if (k >= src.n2) break;
-        T x = (i + T(0.5)) * dx + src.ox;
-        T y = (j + T(0.5)) * dx + src.oy;
-        T z = (k + T(0.5)) * dx + src.oz;
-        T ax, ay, az;
-        cell_velocity(mac, i, j, k, ax, ay, az);
+        const Vec3T<T> a = cell_velocity(mac, i, j, k);
+        Vec3T<T> e;
         if (inside)
-            backtrace_staged_from<T, TRACE, false>(mac, sm, ax, ay, az, x, y, z, h, dx, inv_dx);
+            e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, [&](const Axes<T>& q, const auto& far) {
+                return velocity_staged<T, false>(mac, sm, q, far);
+            });
         else
-            backtrace_staged_from<T, TRACE, true>(mac, sm, ax, ay, az, x, y, z, h, dx, inv_dx);
-        T r;
-        if constexpr (SAMPLE == EL_SAMPLE_WENO6)
-            r = sample_weno6(src, x, y, z, dx, inv_dx);
-        else
-            r = sample_trilinear(src, x, y, z, dx, inv_dx);
-        const long long oc = lin3(i, j, k, src.n0, src.n1);
+            e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, [&](const Axes<T>& q, const auto& far) {
+                return velocity_staged<T, true>(mac, sm, q, far);
+            });
+        const int oc = cell_index(src, i, j, k);
+        const T r = own_at(src, foot_base<T>(i), foot_base<T>(j), foot_base<T>(k), e);
         if (EL_IN(oc, (long long)src.n0 * src.n1 * src.n2, 3)) out[oc] = r;
     }
 }
 
 // ---------------------------------------------------------------------------------------
 // WENO6 level set, tiled.  Under the CFL limit the foot point of a cell lies within one cell
-// of it, so the 6^3 stencils of a 32 x 8 x 4 tile of cells read phi within [tile - 3, tile + 4]:
-// the CTA stages that clamped box (39 x 15 x 11 nodes) once.  The smoothness indicators of an x-pass
-// depend only on the six values it reads, not on the sample's fraction, so they are formed once
-// per (row, floor index) of the box -- (eps + IS_s)^2, in FP32 its reciprocal, for the 34 floor
-// indices of each of the 165 rows -- and shared by every sample whose stencil uses that row
-// segment, instead of being recomputed by all 36 x-passes of every sample.  The y- and z-passes
-// combine per-sample values and are evaluated in full.  The backtrace reads the velocity from
-// global memory (L1-served).  A foot point outside the box (a larger dt) takes the global
-// sample_weno6 path, with the same arithmetic.  The box arrives by one box copy where the cell
-// grid's row pitch allows it; along x it then starts four cells left of the tile (a 16-byte
-// boundary) and holds 40 entries, of which the first is never read.
-constexpr int kWX = 32, kWY = 8, kWZ = 4;
-constexpr int kWBX = kWX + 8, kWBY = kWY + 7, kWBZ = kWZ + 7;  // nodes [tile - 4, tile + 4] x [tile - 3, tile + 4]^2
-constexpr int kWRows = kWBY * kWBZ;
-constexpr int kWBases = kWX + 2;                 // floor indices [tile - 1, tile + 32]
-constexpr int kWBoxN = kWBX * kWRows;            // phi box (a multiple of 16 bytes)
-constexpr int kWQ = kWRows * kWBases;            // one indicator plane
+// of it, so the 6^3 stencils of a 32 x 8 x WZ tile of cells read phi within [tile - 3, tile + 4]:
+// the CTA stages that clamped box (39 x 15 x (WZ + 7) nodes) once, by one box copy where the cell
+// grid's row pitch allows it (along x it then starts four cells left of the tile, a 16-byte
+// boundary, and holds 40 entries, of which the first is never read).
+//
+// The six-point combination, relative to its middle candidate.  Neighbouring candidates are cubics
+// through three common nodes, so they differ by a fourth difference times a fixed polynomial:
+//   p_a - p_b = -D0 (x+1) x (x-1) / 6,   p_c - p_b = D1 x (x-1) (x-2) / 6,
+//   D0 = v4 - 4 v3 + 6 v2 - 4 v1 + v0,   D1 = v5 - 4 v4 + 6 v3 - 4 v2 + v1,
+// and with the nonlinear weights alpha_s = C_s / q_s, q_s = (eps + IS_s)^2, taken relative to the
+// middle one (ra = qb / qa, rc = qb / qc),
+//   sum(alpha p) / sum(alpha) = p_b + (Ka ra D0 + Kc rc D1) / (Cb + Ca ra + Cc rc),
+// Ka = -Ca (x+1) x (x-1) / 6, Kc = Cc x (x-1) (x-2) / 6: one candidate instead of three, and in FP64
+// one division instead of four.  ra, rc, ra D0 and rc D1 of an x-pass depend only on the six
+// values it reads, not on the sample's fraction: they are formed once per (row, floor index) of the
+// box (34 floor indices of each row) and shared by every sample whose stencil uses that row
+// segment, instead of being formed by each of the 36 x-passes of every sample.  In FP32 they are
+// one 16-byte entry {ra, ra D0, rc, rc D1}, so that the numerator and denominator of a pass are two
+// packed multiply-adds; in FP64 {ra, rc} and the plane of D0 (D1 is the next floor index's D0), three
+// doubles an entry.  The y- and z-passes combine per-sample values and are evaluated in full.
+//
+// FP32 is bound by instruction issue and the shared-memory loads (1380 instructions a sample, from
+// 2450; 256^3: 1.48 -> 1.07 ms, the per-sample kernel took 1.03 ms for 203 x 149 x 181 cells that
+// now take 0.45).  FP64 by its FP64 operations (1400 a sample; 128^3: 11.2 -> 5.6 ms, the pipe 88 %
+// busy).
+//
+// A foot point outside the box (a larger dt), and a result that is not finite, takes the global
+// sample_weno6 path: its weights alpha_s stay finite where ratios of the q_s overflow (level-set
+// jumps of 1e6 and more; an FP32 entry whose ratios could lose a weight to flushing is made NaN).
+constexpr int kWX = 32, kWY = 8;
+constexpr int kWNodes = kWX + 8, kWBY = kWY + 7;  // nodes [tile - 4, tile + 4] x [tile - 3, tile + 4]
+constexpr int kWBases = kWX + 2;               // floor indices [tile - 1, tile + 32]
 
-template <typename T, int TRACE>
-__global__ void __launch_bounds__(kWX * kWY, sizeof(T) == 4 ? 2 : 1)
+template <typename T, int WZ, int NZ>
+struct WenoTile {
+    static constexpr int kBZ = WZ + 7;             // nodes [tile - 3, tile + 4] along z
+    static constexpr int kRows = kWBY * kBZ;
+    // FP32: rows of the box and of the entries a multiple of 32 banks apart, so that lanes whose
+    // foot points lie in neighbouring rows do not meet on a bank (203 x 149 x 181: 563 -> 488 us)
+    static constexpr int kBX = sizeof(T) == 4 ? 64 : kWNodes;
+    static constexpr int kEP = sizeof(T) == 4 ? 40 : kWBases;
+    static constexpr int kBoxN = kBX * kRows;      // phi box (a multiple of 16 bytes)
+    static constexpr int kEntries = kRows * kWBases;
+    static constexpr int kDiffs = kWBases + 1;     // FP64: D0 of the floor indices and of one more
+    static constexpr int kFoot = kWX * kWY * WZ;   // FP32: the samples' displacements, x, y, z planes
+    static constexpr int kBytes =
+        kBoxN * (int)sizeof(T) + kRows * kEP * 16 + (sizeof(T) == 4 ? kFoot * 12 : kRows * kDiffs * 8);
+    static constexpr int kNZ = NZ;                 // planes at a time
+    static constexpr int kThreads = kWX * kWY * kNZ;
+};
+
+// the part of the combination that depends on x only
+template <typename T>
+struct WenoX {
+    T L[4];          // p_b = sum_m L[m] v[m + 1]
+    T Ca, Cb, Cc, Ka, Kc;
+};
+
+template <typename T>
+__device__ __forceinline__ WenoX<T> weno_x(T x) {
+    WenoX<T> w;
+    const T xp = x + T(1), xm = x - T(1), x2 = x - T(2);
+    // p_b in Newton form on nodes -1, 0, 1, 2
+    const T n2 = xp * x * T(0.5), n3 = xp * x * xm * T(1.0 / 6.0);
+    w.L[0] = T(1) - xp + n2 - n3;
+    w.L[1] = xp - T(2) * n2 + T(3) * n3;
+    w.L[2] = n2 - T(3) * n3;
+    w.L[3] = n3;
+    w.Ca = (T(2) - x) * (T(3) - x) * T(1.0 / 20.0);
+    w.Cb = (T(3) - x) * (x + T(2)) * T(1.0 / 10.0);
+    w.Cc = (x + T(2)) * xp * T(1.0 / 20.0);
+    w.Ka = -w.Ca * n3;
+    w.Kc = w.Cc * (x * xm * x2 * T(1.0 / 6.0));
+    return w;
+}
+
+__device__ __forceinline__ float rcp_approx(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// q_s = (eps + IS_s)^2 of the three candidates, times a common factor, and the fourth differences
+// D0, D1.  Each 180 IS_s is 244 times a sum of squares of combinations of the first differences
+// (the quadratic form factored from its leading term; IS_2's is IS_0's read from the right):
+//   form(a, b, c) = (a + B b + G c)^2 + D (b + E c)^2 + Z c^2,
+// nine operations with the square, and in float the squares do not cancel where the quadratic
+// form's terms do.  The common factor (244 / 180)^2 drops out of the weights' ratios and, with eps
+// scaled alike, out of their normalisation.
+template <typename V, typename O>
+__device__ __forceinline__ void weno_q(const V (&v)[6], V& qa, V& qb, V& qc, V& D0, V& D1, O) {
+    V d[6];
+#pragma unroll
+    for (int m = 1; m < 6; ++m) d[m] = O::sub(v[m], v[m - 1]);
+    auto form = [&](V a, V b, V c, double B, double G, double D, double E, double Z) {
+        const V y1 = O::fma(O::k(G), c, O::fma(O::k(B), b, a)), y2 = O::fma(O::k(E), c, b);
+        V t = O::fma(O::mul(O::k(Z), c), c, O::k(1e-6 * 180.0 / 244.0));
+        t = O::fma(y1, y1, O::fma(O::mul(O::k(D), y2), y2, t));
+        return O::mul(t, t);
+    };
+    constexpr double kB = -1171.0 / 488, kG = 683.0 / 488, kD = 152295.0 / 238144, kE = -1.0 / 1, kZ = 45.0 / 61;
+    constexpr double kB1 = -781.0 / 488, kG1 = 293.0 / 488, kD1 = 327975.0 / 238144, kE1 = -10153.0 / 21865, kZ1 = 91377.0 / 266753;
+    qa = form(d[1], d[2], d[3], kB, kG, kD, kE, kZ);
+    qb = form(d[2], d[3], d[4], kB1, kG1, kD1, kE1, kZ1);
+    qc = form(d[5], d[4], d[3], kB, kG, kD, kE, kZ);
+    D0 = O::fma(O::k(3.0), O::sub(d[2], d[3]), O::sub(d[4], d[1]));
+    D1 = O::fma(O::k(3.0), O::sub(d[3], d[4]), O::sub(d[5], d[2]));
+}
+
+template <typename T>
+struct ScalarOps {
+    static __device__ __forceinline__ T k(double c) { return T(c); }
+    static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
+    static __device__ __forceinline__ T sub(T a, T b) { return a - b; }
+    static __device__ __forceinline__ T fma(T a, T b, T c) { return rn_fma(a, b, c); }
+};
+struct PairOps {
+    static __device__ __forceinline__ float2 k(double c) { return make_float2((float)c, (float)c); }
+    static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+    static __device__ __forceinline__ float2 sub(float2 a, float2 b) {
+        return __ffma2_rn(b, make_float2(-1.f, -1.f), a);  // one rounding, no negations in registers
+    }
+    static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+};
+
+// num / den (den a positive normal double) in five FP64 operations instead of the nine of a
+// division: a float reciprocal of the leading bits, one Newton step, and one correction by the
+// residual (P. Markstein, IBM J. Res. Dev. 34, 1990); within an ulp.  Outside the floats' range the
+// division itself.
+__device__ __forceinline__ bool in_float_range(double v) {  // 2^-120 <= v < 2^120
+    return (unsigned)(__double2hiint(v) - 0x38700000) < 0x0f000000u;
+}
+__device__ __forceinline__ double rcp_newton(double v) {
+    const float f = __int_as_float(__funnelshift_l(__double2loint(v), __double2hiint(v) - 0x38000000, 3));
+    const unsigned b = (unsigned)__float_as_int(rcp_approx(f));
+    const double r = __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    return fma(r, fma(-v, r, 1.0), r);  // 44 bits
+}
+__device__ __forceinline__ double div_newton(double num, double den) {
+    if (!in_float_range(den)) return num / den;
+    const double r = rcp_newton(den), q = num * r;
+    return fma(fma(-den, q, num), r, q);
+}
+// 1 / v to within an ulp (one more Newton step)
+__device__ __forceinline__ double inverse(double v) {
+    if (!in_float_range(v)) return 1.0 / v;
+    const double r = rcp_newton(v);
+    return fma(r, fma(-v, r, 1.0), r);
+}
+
+// a y- or z-pass.  FP32: the weights alpha_s by reciprocals (as the general path's, finite for any
+// q_s); FP64: the ratios of the q_s by one division.
+__device__ __forceinline__ float weno_pass(const WenoX<float>& w, const float (&v)[6]) {
+    float qa, qb, qc, D0, D1;
+    weno_q(v, qa, qb, qc, D0, D1, ScalarOps<float>());
+    const float ia = rcp_approx(qa), ib = rcp_approx(qb), ic = rcp_approx(qc);
+    const float pb = fmaf(w.L[3], v[4], fmaf(w.L[2], v[3], fmaf(w.L[1], v[2], w.L[0] * v[1])));
+    const float den = fmaf(w.Cc, ic, fmaf(w.Ca, ia, w.Cb * ib));
+    const float num = fmaf(w.Kc * ic, D1, w.Ka * ia * D0);
+    return fmaf(num, rcp_approx(den), pb);
+}
+__device__ __forceinline__ float2 weno_pass(const WenoX<float>& w, const float2 (&v)[6]) {
+    using O = PairOps;
+    auto b2 = [](float x) { return make_float2(x, x); };
+    auto rcp2 = [](float2 q) { return make_float2(rcp_approx(q.x), rcp_approx(q.y)); };
+    float2 qa, qb, qc, D0, D1;
+    weno_q(v, qa, qb, qc, D0, D1, O());
+    const float2 ia = rcp2(qa), ib = rcp2(qb), ic = rcp2(qc);
+    const float2 pb = O::fma(b2(w.L[3]), v[4],
+                             O::fma(b2(w.L[2]), v[3], O::fma(b2(w.L[1]), v[2], O::mul(b2(w.L[0]), v[1]))));
+    const float2 den = O::fma(b2(w.Cc), ic, O::fma(b2(w.Ca), ia, O::mul(b2(w.Cb), ib)));
+    const float2 num = O::fma(O::mul(b2(w.Kc), ic), D1, O::mul(O::mul(b2(w.Ka), ia), D0));
+    return O::fma(num, rcp2(den), pb);
+}
+__device__ __forceinline__ double weno_pass(const WenoX<double>& w, const double (&v)[6]) {
+    double qa, qb, qc, D0, D1;
+    weno_q(v, qa, qb, qc, D0, D1, ScalarOps<double>());
+    const double inv = inverse(qa * qc);
+    const double ra = qb * qc * inv, rc = qb * qa * inv;
+    const double pb = fma(w.L[3], v[4], fma(w.L[2], v[3], fma(w.L[1], v[2], w.L[0] * v[1])));
+    const double den = fma(w.Cc, rc, fma(w.Ca, ra, w.Cb));
+    return pb + div_newton(fma(w.Kc * rc, D1, w.Ka * ra * D0), den);
+}
+
+template <typename T, int TRACE, int WZ, int NZ>
+__global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
     advect_phi_weno_tiled_kernel(GridView<T> src, T* __restrict__ out, Mac<T> mac, DtArg dt, T dx, T inv_dx,
                                  const __grid_constant__ BoxMap pmap) {
+    using W = WenoTile<T, WZ, NZ>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* pbox = reinterpret_cast<T*>(align128(smem_raw));  // [z][y][x]
-    // [s][row][floor index]; in FP32 s = 0, 1 interleaved ({qa, qb} pairs), then the s = 2 plane
-    T* qbox = pbox + kWBoxN;
-    const T* pb = pbox + 1;  // the box from node tile - 3 along x
+    const T* pb = pbox + 1;                              // the box from node tile - 3 along x
+    // FP32: float4 entries [row][floor index]; FP64: double2 entries, then D0 [row][kDiffs]
+    void* const entries = pbox + W::kBoxN;
     __shared__ uint64_t bar;
-    const int x0 = blockIdx.x * kWX, y0 = blockIdx.y * kWY, z0 = blockIdx.z * kWZ;
+    const int x0 = blockIdx.x * kWX, y0 = blockIdx.y * kWY, z0 = blockIdx.z * WZ;
     const int bx0 = x0 - 4, by0 = y0 - 3, bz0 = z0 - 3;
-    const int tid = threadIdx.x + kWX * threadIdx.y;
+    const int tid = threadIdx.x + kWX * (threadIdx.y + kWY * threadIdx.z);
     const int lane = tid & 31, warp = tid >> 5;
     if (pmap.on) {
         if (tid == 0) {
-            copy_boxes_begin(&bar, (unsigned)(kWBoxN * sizeof(T)));
+            copy_boxes_begin(&bar, (unsigned)(W::kBoxN * sizeof(T)));
             tma_load_3d(pbox, &pmap.m, &bar, bx0, by0, bz0);
         }
+    }
+    // the thread's foot points while the box is on its way: their global reads are in flight together
+    const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
+    const bool column = i < src.n0 && j < src.n1;
+    const T dtv = (T)dt_value(dt);
+    // (FP32 keeps them in shared memory until their turn, for the registers of more warps)
+    [[maybe_unused]] Vec3T<T> foot[sizeof(T) == 4 ? 1 : WZ / W::kNZ];
+    [[maybe_unused]] float* const sfoot = reinterpret_cast<float*>(pbox + W::kBoxN) + W::kRows * W::kEP * 4 + tid;
+#pragma unroll
+    for (int q = 0; q < WZ / W::kNZ; ++q) {
+        const int k = z0 + (int)threadIdx.z + q * W::kNZ;
+        Vec3T<T> d{T(0), T(0), T(0)};
+        if (column && k < src.n2)
+            d = level_set_foot<T, TRACE>(cell_velocity(mac, i, j, k), i, j, k, dtv, dx, inv_dx,
+                                         [&](const Axes<T>& a, const auto& far) { return velocity_global(mac, a, far); });
+        if constexpr (sizeof(T) == 4) {
+            sfoot[q * W::kThreads] = d.x;
+            sfoot[q * W::kThreads + W::kFoot] = d.y;
+            sfoot[q * W::kThreads + 2 * W::kFoot] = d.z;
+        } else {
+            foot[q] = d;
+        }
+    }
+    if (pmap.on) {
         __syncthreads();  // the mbarrier's initialisation is seen by every thread
         if (copy_boxes_failed(&bar)) {
-            nan_column(src, out, x0 + threadIdx.x, y0 + threadIdx.y, z0, kWZ);
+            nan_column(src, out, x0 + threadIdx.x, y0 + threadIdx.y, z0, WZ);
             return;
         }
-        T unused = T(0);
-        finish_box<T, kWBX, kWBY, kWBZ, false>(pbox, src, bx0, by0, bz0, unused);
+        AbsMax<T> unused;
+        finish_box<T, kWNodes, kWBY, W::kBZ, false, W::kBX>(pbox, src, bx0, by0, bz0, unused);
     } else {
-        for (int row = warp; row < kWRows; row += (kWX * kWY) / 32) {
+        for (int row = warp; row < W::kRows; row += W::kThreads / 32) {
             const int bz = row / kWBY, by = row - bz * kWBY;
             const int gy = clampi(by0 + by, 0, src.n1 - 1), gz = clampi(bz0 + bz, 0, src.n2 - 1);
-            const T* s = src.d + (long long)src.n0 * (gy + (long long)src.n1 * gz);
-            T* d = pbox + row * kWBX;
-            d[lane] = __ldg(s + clampi(bx0 + lane, 0, src.n0 - 1));
-            if (lane < kWBX - 32) d[32 + lane] = __ldg(s + clampi(bx0 + 32 + lane, 0, src.n0 - 1));
+            const T* p = src.d + (long long)src.n0 * (gy + (long long)src.n1 * gz);
+            T* d = pbox + row * W::kBX;
+            d[lane] = __ldg(p + clampi(bx0 + lane, 0, src.n0 - 1));
+            if (lane < kWNodes - 32) d[32 + lane] = __ldg(p + clampi(bx0 + 32 + lane, 0, src.n0 - 1));
         }
     }
     __syncthreads();
     if constexpr (sizeof(T) == 4) {
         // two (row, floor index) entries a thread per pass in packed float2 arithmetic
-        constexpr int kStep = kWX * kWY;
-        for (int e0 = tid; e0 < kWQ; e0 += 2 * kStep) {
-            const int e1 = e0 + kStep < kWQ ? e0 + kStep : e0;  // the tail repeats its first entry
+        float4* q = static_cast<float4*>(entries);
+        for (int e0 = tid; e0 < W::kEntries; e0 += 2 * W::kThreads) {
+            const int e1 = e0 + W::kThreads < W::kEntries ? e0 + W::kThreads : e0;  // the tail repeats its entry
             const int r0 = e0 / kWBases, r1 = e1 / kWBases;
-            const float* va = pb + r0 * kWBX + (e0 - r0 * kWBases);
-            const float* vb = pb + r1 * kWBX + (e1 - r1 * kWBases);
+            const int b0 = e0 - r0 * kWBases, b1 = e1 - r1 * kWBases;
+            const float* va = pb + r0 * W::kBX + b0;
+            const float* vb = pb + r1 * W::kBX + b1;
             float2 v[6];
 #pragma unroll
             for (int m = 0; m < 6; ++m) v[m] = make_float2(va[m], vb[m]);
-            float2 qa, qb, qc;
-            weno6_sq2(v, qa, qb, qc);
-            reinterpret_cast<float2*>(qbox)[e0] = make_float2(qa.x, qb.x);  // one 8-byte load for both
-            qbox[2 * kWQ + e0] = qc.x;
-            if (e1 != e0) {
-                reinterpret_cast<float2*>(qbox)[e1] = make_float2(qa.y, qb.y);
-                qbox[2 * kWQ + e1] = qc.y;
-            }
+            float2 qa, qb, qc, D0, D1;
+            weno_q(v, qa, qb, qc, D0, D1, PairOps());
+            auto entry = [](float a, float b, float c, float d0, float d1) {
+                // q_s below 1e25: with q_s >= 1e-12 the ratios stay below 1e37, and so does the
+                // denominator (a reciprocal of 2^126 or more would be flushed to zero)
+                const float ra = fmaxf(fmaxf(a, b), c) < 1e25f ? b * rcp_approx(a) : __int_as_float(0x7fc00000);
+                const float rc = b * rcp_approx(c);
+                return make_float4(ra, ra * d0, rc, rc * d1);
+            };
+            q[r0 * W::kEP + b0] = entry(qa.x, qb.x, qc.x, D0.x, D1.x);
+            if (e1 != e0) q[r1 * W::kEP + b1] = entry(qa.y, qb.y, qc.y, D0.y, D1.y);
         }
     } else {
-        for (int e = tid; e < kWQ; e += kWX * kWY) {
+        double2* q = static_cast<double2*>(entries);
+        double* D = reinterpret_cast<double*>(q + W::kRows * W::kEP);
+        for (int e = tid; e < W::kEntries; e += W::kThreads) {
             const int row = e / kWBases, b = e - row * kWBases;
-            const T* v = pb + row * kWBX + b;
-            T qa, qb, qc;
-            weno6_sq(v[0], v[1], v[2], v[3], v[4], v[5], qa, qb, qc);
-            qbox[e] = qa;
-            qbox[kWQ + e] = qb;
-            qbox[2 * kWQ + e] = qc;
+            const T* p = pb + row * W::kBX + b;
+            const double v[6] = {p[0], p[1], p[2], p[3], p[4], p[5]};
+            double qa, qb, qc, D0, D1;
+            weno_q(v, qa, qb, qc, D0, D1, ScalarOps<double>());
+            const double inv = inverse(qa * qc);
+            q[e] = make_double2(qb * qc * inv, qb * qa * inv);
+            D[row * W::kDiffs + b] = D0;
+            if (b == kWBases - 1) D[row * W::kDiffs + b + 1] = D1;
         }
     }
     __syncthreads();
-    const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
-    if (i >= src.n0 || j >= src.n1) return;
-    const T h = -(T)dt_value(dt);
+    if (!column) return;
 #pragma unroll 1
-    for (int kk = 0; kk < kWZ; ++kk) {
-        const int k = z0 + kk;
+    for (int n = 0; n < WZ / W::kNZ; ++n) {
+        const int kk = (int)threadIdx.z + n * W::kNZ, k = z0 + kk;
         if (k >= src.n2) break;
-        T x = (i + T(0.5)) * dx + src.ox;
-        T y = (j + T(0.5)) * dx + src.oy;
-        T z = (k + T(0.5)) * dx + src.oz;
-        T ax, ay, az;
-        cell_velocity(mac, i, j, k, ax, ay, az);
-        backtrace_from<T, TRACE>(mac, ax, ay, az, x, y, z, h, dx, inv_dx);
+        Vec3T<T> d;
+        if constexpr (sizeof(T) == 4) {
+            d = Vec3T<T>{sfoot[n * W::kThreads], sfoot[n * W::kThreads + W::kFoot], sfoot[n * W::kThreads + 2 * W::kFoot]};
+        } else {
+            d = foot[0];  // registers, not a dynamically indexed array
+#pragma unroll
+            for (int q = 1; q < WZ / W::kNZ; ++q) {
+                d.x = n == q ? foot[q].x : d.x;
+                d.y = n == q ? foot[q].y : d.y;
+                d.z = n == q ? foot[q].z : d.z;
+            }
+        }
         // stencil origin (floor - 2) relative to the box, per axis
-        const AxisPos<T> px = axis_pos(x, src.ox, x0 - 1, dx, inv_dx);
-        const AxisPos<T> py = axis_pos(y, src.oy, y0 - 1, dx, inv_dx);
-        const AxisPos<T> pz = axis_pos(z, src.oz, z0 - 1, dx, inv_dx);
-        T r;
-        if ((unsigned)px.a < (unsigned)kWBases && (unsigned)py.a < (unsigned)(kWY + 2) &&
-            (unsigned)pz.a < (unsigned)(kWZ + 2)) {
-            const WenoAxis<T> wx = weno_axis(px.f);
-            const WenoAxis<T> wy = weno_axis(py.f);
+        int px, py, pz;
+        T fx, fy, fz;
+        floor_index(d.x, px, fx);
+        floor_index(d.y, py, fy);
+        floor_index(d.z, pz, fz);
+        px = (int)((unsigned)px + (unsigned)(foot_base<T>(i) - x0 + 1));
+        py = (int)((unsigned)py + (unsigned)(foot_base<T>(j) - y0 + 1));
+        pz = (int)((unsigned)pz + (unsigned)(foot_base<T>(k) - z0 + 1));
+        T r = T(0);
+        bool ok = false;
+        if ((unsigned)px < (unsigned)kWBases && (unsigned)py < (unsigned)(kWY + 2) && (unsigned)pz < (unsigned)(WZ + 2)) {
+            const WenoX<T> wx = weno_x(fx), wy = weno_x(fy);
             T zl[6];
             if constexpr (sizeof(T) == 4) {
-                // FP32: packed float2 arithmetic (two lanes per instruction, each rounded as its
-                // scalar operation): the x-passes of rows dj and dj + 1, and the y-passes of
-                // planes dk and dk + 1, together; the expressions of weno6_combine / weno6_eval
+                const float4* q = static_cast<const float4*>(entries);
+                const float2 Ka{wx.Ca, wx.Ka}, Kc{wx.Cc, wx.Kc}, Kb{wx.Cb, 0.f};
 #pragma unroll
                 for (int dk = 0; dk < 6; dk += 2) {
-                    float2 yl2[6];  // .x: plane dk, .y: plane dk + 1
+                    float2 yl[6];  // .x: plane dk, .y: plane dk + 1, evaluated together
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int row0 = (pz.a + dk + h) * kWBY + py.a;
+                    for (int u = 0; u < 2; ++u) {
+                        const int row0 = (pz + dk + u) * kWBY + py;
 #pragma unroll
-                        for (int dj = 0; dj < 6; dj += 2) {
-                            const int row = row0 + dj;
-                            const float* va = pb + row * kWBX + px.a;
-                            const float* vb = va + kWBX;
-                            const float2 qa2 = reinterpret_cast<const float2*>(qbox)[row * kWBases + px.a];
-                            const float2 qb2 = reinterpret_cast<const float2*>(qbox)[(row + 1) * kWBases + px.a];
-                            const float* qc = qbox + 2 * kWQ + row * kWBases + px.a;
-                            float2 v[6];
-#pragma unroll
-                            for (int m = 0; m < 6; ++m) v[m] = make_float2(va[m], vb[m]);
-                            const float2 rr = weno6_combine2(wx, v, make_float2(qa2.x, qb2.x),
-                                                             make_float2(qa2.y, qb2.y), make_float2(qc[0], qc[kWBases]));
-                            if (h == 0) {
-                                yl2[dj].x = rr.x;
-                                yl2[dj + 1].x = rr.y;
-                            } else {
-                                yl2[dj].y = rr.x;
-                                yl2[dj + 1].y = rr.y;
-                            }
+                        for (int dj = 0; dj < 6; ++dj) {
+                            const float* v = pb + (row0 + dj) * W::kBX + px;
+                            const float4 e = q[(row0 + dj) * W::kEP + px];
+                            const float p = fmaf(wx.L[3], v[4], fmaf(wx.L[2], v[3], fmaf(wx.L[1], v[2], wx.L[0] * v[1])));
+                            // {denominator, numerator}
+                            const float2 t = __ffma2_rn(Kc, make_float2(e.z, e.w), __ffma2_rn(Ka, make_float2(e.x, e.y), Kb));
+                            const float y = fmaf(t.y, rcp_approx(t.x), p);
+                            if (u == 0)
+                                yl[dj].x = y;
+                            else
+                                yl[dj].y = y;
                         }
                     }
-                    const float2 zv = weno6_eval2(wy, yl2);
+                    const float2 zv = weno_pass(wy, yl);
                     zl[dk] = zv.x;
                     zl[dk + 1] = zv.y;
                 }
             } else {
+                const double2* q = static_cast<const double2*>(entries);
+                const double* D = reinterpret_cast<const double*>(q + W::kRows * W::kEP);
 #pragma unroll
-            for (int dk = 0; dk < 6; ++dk) {
-                const int row0 = (pz.a + dk) * kWBY + py.a;
-                T yl[6];
+                for (int dk = 0; dk < 6; ++dk) {
+                    const int row0 = (pz + dk) * kWBY + py;
+                    double yl[6];
 #pragma unroll
-                for (int dj = 0; dj < 6; ++dj) {
-                    const int row = row0 + dj;
-                    const T* v = pb + row * kWBX + px.a;
-                    const T* q = qbox + row * kWBases + px.a;
-                    yl[dj] = weno6_combine(wx, v[0], v[1], v[2], v[3], v[4], v[5], q[0], q[kWQ], q[2 * kWQ]);
+                    for (int dj = 0; dj < 6; ++dj) {
+                        const int row = row0 + dj;
+                        const T* v = pb + row * W::kBX + px;
+                        const double2 e = q[row * kWBases + px];
+                        const double* dd = D + row * W::kDiffs + px;
+                        const double p = fma(wx.L[3], v[4], fma(wx.L[2], v[3], fma(wx.L[1], v[2], wx.L[0] * v[1])));
+                        const double den = fma(wx.Cc, e.y, fma(wx.Ca, e.x, wx.Cb));
+                        yl[dj] = p + div_newton(fma(wx.Kc * e.y, dd[1], wx.Ka * e.x * dd[0]), den);
+                    }
+                    const double zv = weno_pass(wy, yl);
+                    // registers, not a dynamically indexed array
+                    zl[0] = dk == 0 ? zv : zl[0];
+                    zl[1] = dk == 1 ? zv : zl[1];
+                    zl[2] = dk == 2 ? zv : zl[2];
+                    zl[3] = dk == 3 ? zv : zl[3];
+                    zl[4] = dk == 4 ? zv : zl[4];
+                    zl[5] = dk == 5 ? zv : zl[5];
                 }
-                const T zv = weno6_eval(wy, yl[0], yl[1], yl[2], yl[3], yl[4], yl[5]);
-                zl[0] = dk == 0 ? zv : zl[0];
-                zl[1] = dk == 1 ? zv : zl[1];
-                zl[2] = dk == 2 ? zv : zl[2];
-                zl[3] = dk == 3 ? zv : zl[3];
-                zl[4] = dk == 4 ? zv : zl[4];
-                zl[5] = dk == 5 ? zv : zl[5];
             }
-            }
-            r = weno6_eval(weno_axis(pz.f), zl[0], zl[1], zl[2], zl[3], zl[4], zl[5]);
-        } else {
-            r = sample_weno6(src, x, y, z, dx, inv_dx);
+            r = weno_pass(weno_x(fz), zl);
+            ok = isfinite(r);
         }
-        const long long oc = lin3(i, j, k, src.n0, src.n1);
+        if (!ok) r = sample_weno6(src, foot_base<T>(i), foot_base<T>(j), foot_base<T>(k), d.x, d.y, d.z);
+        const int oc = cell_index(src, i, j, k);
         if (EL_IN(oc, (long long)src.n0 * src.n1 * src.n2, 3)) out[oc] = r;
     }
 }
 
 // Grid views of the scene's grids (staggered_grid.h:100-112): comp 0 = cells, 1/2/3 = u/v/w.
 template <typename T>
-GridView<T> make_view(const void* d, int ni, int nj, int nk, T dx, int comp) {
-    GridView<T> g{static_cast<const T*>(d), ni, nj, nk, T(0), T(0), T(0)};
-    const T half = T(0.5) * dx;
-    if (comp == 1) { g.n0 = ni + 1; g.ox = T(0) - half; }
-    if (comp == 2) { g.n1 = nj + 1; g.oy = T(0) - half; }
-    if (comp == 3) { g.n2 = nk + 1; g.oz = T(0) - half; }
-    return g;
+GridView<T> make_view(const void* d, int ni, int nj, int nk, int comp) {
+    return GridView<T>{static_cast<const T*>(d), ni + (comp == 1), nj + (comp == 2), nk + (comp == 3)};
 }
 
 template <typename T, int TRACE, int SAMPLE>
-static void launch_one(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, int rows,
+static void launch_one(const GridView<T>& src, int comp, void* out, const Mac<T>& mac, DtArg dt, T dx, int rows,
                        cudaStream_t s) {
     dim3 block(32, rows, 1);
     dim3 grid((src.n0 + 31) / 32, (src.n1 + rows - 1) / rows, src.n2);
-    advect_kernel<T, TRACE, SAMPLE><<<grid, block, 0, s>>>(src, static_cast<T*>(out), mac, dt, dx,
+    advect_kernel<T, TRACE, SAMPLE><<<grid, block, 0, s>>>(src, comp, static_cast<T*>(out), mac, dt, dx,
                                                            T(1) / dx);
 }
 
 template <typename T>
-static void launch_dispatch(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx,
+static void launch_dispatch(const GridView<T>& src, int comp, void* out, const Mac<T>& mac, DtArg dt, T dx,
                             int trace, int sample, int rows, cudaStream_t s) {
     if (trace == EL_TRACE_RK2 && sample == EL_SAMPLE_TRILINEAR)
-        launch_one<T, EL_TRACE_RK2, EL_SAMPLE_TRILINEAR>(src, out, mac, dt, dx, rows, s);
+        launch_one<T, EL_TRACE_RK2, EL_SAMPLE_TRILINEAR>(src, comp, out, mac, dt, dx, rows, s);
     else if (trace == EL_TRACE_RK2 && sample == EL_SAMPLE_WENO6)
-        launch_one<T, EL_TRACE_RK2, EL_SAMPLE_WENO6>(src, out, mac, dt, dx, rows, s);
+        launch_one<T, EL_TRACE_RK2, EL_SAMPLE_WENO6>(src, comp, out, mac, dt, dx, rows, s);
     else if (trace == EL_TRACE_RK3 && sample == EL_SAMPLE_TRILINEAR)
-        launch_one<T, EL_TRACE_RK3, EL_SAMPLE_TRILINEAR>(src, out, mac, dt, dx, rows, s);
+        launch_one<T, EL_TRACE_RK3, EL_SAMPLE_TRILINEAR>(src, comp, out, mac, dt, dx, rows, s);
     else
-        launch_one<T, EL_TRACE_RK3, EL_SAMPLE_WENO6>(src, out, mac, dt, dx, rows, s);
+        launch_one<T, EL_TRACE_RK3, EL_SAMPLE_WENO6>(src, comp, out, mac, dt, dx, rows, s);
 }
 
 // Launch the advection of `which` (0 = cell-centred grid `in`, 1..3 = face component) into out.
@@ -905,10 +1276,10 @@ static int advect_launch(int ni, int nj, int nk, double dx_d, int comp, void* ou
                          const void* vu, const void* vv, const void* vw, DtArg dt, int trace,
                          int sample, int rows, cudaStream_t s) {
     const T dx = (T)dx_d;
-    Mac<T> mac{make_view<T>(vu, ni, nj, nk, dx, 1), make_view<T>(vv, ni, nj, nk, dx, 2),
-               make_view<T>(vw, ni, nj, nk, dx, 3)};
-    GridView<T> src = make_view<T>(in, ni, nj, nk, dx, comp);
-    launch_dispatch<T>(src, out, mac, dt, dx, trace, sample, rows, s);
+    Mac<T> mac{make_view<T>(vu, ni, nj, nk, 1), make_view<T>(vv, ni, nj, nk, 2),
+               make_view<T>(vw, ni, nj, nk, 3)};
+    GridView<T> src = make_view<T>(in, ni, nj, nk, comp);
+    launch_dispatch<T>(src, comp, out, mac, dt, dx, trace, sample, rows, s);
     return 1;
 }
 
@@ -934,30 +1305,49 @@ static MacMaps mac_maps(const Mac<T>& mac, bool copy) {
 
 // the tiled kernels: the level set (any scheme), and the velocity advecting itself (trilinear);
 // dynamic shared memory holds the boxes plus 128 bytes to align them
-template <typename T, int TRACE, int SAMPLE>
+template <typename T, int TRACE>
 static int launch_phi_tiled(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, bool copy,
                             cudaStream_t s) {
     const int smem = 3 * kBoxN * (int)sizeof(T) + 128;
-    if (cudaFuncSetAttribute(advect_phi_tiled_kernel<T, TRACE, SAMPLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(advect_phi_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem) != cudaSuccess)
         return -1;
     const dim3 grid((src.n0 + kTileX - 1) / kTileX, (src.n1 + kTileY - 1) / kTileY, (src.n2 + kTileZ - 1) / kTileZ);
-    advect_phi_tiled_kernel<T, TRACE, SAMPLE><<<grid, dim3(kTileX, kTileY, 1), smem, s>>>(
+    advect_phi_tiled_kernel<T, TRACE><<<grid, dim3(kTileX, kTileY, 1), smem, s>>>(
         src, static_cast<T*>(out), mac, dt, dx, T(1) / dx, mac_maps(mac, copy));
     return 1;
 }
 
+template <typename T, int TRACE, int WZ, int NZ>
+static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, bool copy,
+                                cudaStream_t s) {
+    using W = WenoTile<T, WZ, NZ>;
+    const int smem = W::kBytes + 128;
+    if (cudaFuncSetAttribute(advect_phi_weno_tiled_kernel<T, TRACE, WZ, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             smem) != cudaSuccess)
+        return -1;
+    const dim3 grid((src.n0 + kWX - 1) / kWX, (src.n1 + kWY - 1) / kWY, (src.n2 + WZ - 1) / WZ);
+    advect_phi_weno_tiled_kernel<T, TRACE, WZ, NZ><<<grid, dim3(kWX, kWY, W::kNZ), smem, s>>>(
+        src, static_cast<T*>(out), mac, dt, dx, T(1) / dx, box_map(src, copy, W::kBX, kWBY, W::kBZ));
+    return 1;
+}
+
+// FP32: a CTA of 1024 threads per tile, four planes at a time.  Tiles of eight planes form 3.7
+// entries a sample against 5.5 of four planes (256^3: 1072 against 1230 us; 151 x 97 x 133: 156
+// against 177); where every tile of four planes has an SM of its own, those finish sooner (48^3:
+// 18.8 against 30.0 us).  512 and 768 threads a tile took 1187 and 1130 us at 256^3.
+constexpr int kSMs = 152;
+
 template <typename T, int TRACE>
 static int launch_phi_weno_tiled(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, bool copy,
                                  cudaStream_t s) {
-    const int smem = (kWBoxN + 3 * kWQ) * (int)sizeof(T) + 128;
-    if (cudaFuncSetAttribute(advect_phi_weno_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
-        return -1;
-    const dim3 grid((src.n0 + kWX - 1) / kWX, (src.n1 + kWY - 1) / kWY, (src.n2 + kWZ - 1) / kWZ);
-    advect_phi_weno_tiled_kernel<T, TRACE><<<grid, dim3(kWX, kWY, 1), smem, s>>>(
-        src, static_cast<T*>(out), mac, dt, dx, T(1) / dx, box_map(src, copy, kWBX, kWBY, kWBZ));
-    return 1;
+    if constexpr (sizeof(T) == 4) {
+        const long long tiles4 = (long long)((src.n0 + kWX - 1) / kWX) * ((src.n1 + kWY - 1) / kWY) * ((src.n2 + 3) / 4);
+        if (tiles4 > kSMs) return launch_phi_weno_tile<T, TRACE, 8, 4>(src, out, mac, dt, dx, copy, s);
+        return launch_phi_weno_tile<T, TRACE, 4, 4>(src, out, mac, dt, dx, copy, s);
+    } else {
+        return launch_phi_weno_tile<T, TRACE, 4, 1>(src, out, mac, dt, dx, copy, s);
+    }
 }
 
 template <typename T, int TRACE>
@@ -967,11 +1357,11 @@ static int launch_velocity_tiled(const Mac<T>& mac, void* ou, void* ov, void* ow
     if (cudaFuncSetAttribute(advect_velocity_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem) != cudaSuccess)
         return -1;
-    // tiles over the largest extent of the three face grids
-    const dim3 grid((mac.u.n0 + kTileX - 1) / kTileX, (mac.v.n1 + kTileY - 1) / kTileY,
-                    (mac.w.n2 + kTileZ - 1) / kTileZ);
+    // tiles of cells
+    const dim3 grid((mac.v.n0 + kTileX - 1) / kTileX, (mac.u.n1 + kTileY - 1) / kTileY,
+                    (mac.u.n2 + kTileZ - 1) / kTileZ);
     advect_velocity_tiled_kernel<T, TRACE><<<grid, dim3(kTileX, kTileY, 1), smem, s>>>(
-        mac, static_cast<T*>(ou), static_cast<T*>(ov), static_cast<T*>(ow), dt, dx, T(1) / dx, mac_maps(mac, copy));
+        mac, static_cast<T*>(ou), static_cast<T*>(ov), static_cast<T*>(ow), dt, T(1) / dx, mac_maps(mac, copy));
     return 1;
 }
 
@@ -980,23 +1370,23 @@ static int advect_phi_tiled_t(int ni, int nj, int nk, double dx_d, void* out, co
                               const void* vv, const void* vw, DtArg dt, int trace, int sample, bool copy,
                               cudaStream_t s) {
     const T dx = (T)dx_d;
-    Mac<T> mac{make_view<T>(vu, ni, nj, nk, dx, 1), make_view<T>(vv, ni, nj, nk, dx, 2),
-               make_view<T>(vw, ni, nj, nk, dx, 3)};
-    GridView<T> src = make_view<T>(in, ni, nj, nk, dx, 0);
+    Mac<T> mac{make_view<T>(vu, ni, nj, nk, 1), make_view<T>(vv, ni, nj, nk, 2),
+               make_view<T>(vw, ni, nj, nk, 3)};
+    GridView<T> src = make_view<T>(in, ni, nj, nk, 0);
     if (sample == EL_SAMPLE_WENO6)
         return trace == EL_TRACE_RK2 ? launch_phi_weno_tiled<T, EL_TRACE_RK2>(src, out, mac, dt, dx, copy, s)
                                      : launch_phi_weno_tiled<T, EL_TRACE_RK3>(src, out, mac, dt, dx, copy, s);
     if (trace == EL_TRACE_RK2)
-        return launch_phi_tiled<T, EL_TRACE_RK2, EL_SAMPLE_TRILINEAR>(src, out, mac, dt, dx, copy, s);
-    return launch_phi_tiled<T, EL_TRACE_RK3, EL_SAMPLE_TRILINEAR>(src, out, mac, dt, dx, copy, s);
+        return launch_phi_tiled<T, EL_TRACE_RK2>(src, out, mac, dt, dx, copy, s);
+    return launch_phi_tiled<T, EL_TRACE_RK3>(src, out, mac, dt, dx, copy, s);
 }
 
 template <typename T>
 static int advect_velocity_tiled_t(int ni, int nj, int nk, double dx_d, void* ou, void* ov, void* ow, const void* vu,
                                    const void* vv, const void* vw, DtArg dt, int trace, bool copy, cudaStream_t s) {
     const T dx = (T)dx_d;
-    Mac<T> mac{make_view<T>(vu, ni, nj, nk, dx, 1), make_view<T>(vv, ni, nj, nk, dx, 2),
-               make_view<T>(vw, ni, nj, nk, dx, 3)};
+    Mac<T> mac{make_view<T>(vu, ni, nj, nk, 1), make_view<T>(vv, ni, nj, nk, 2),
+               make_view<T>(vw, ni, nj, nk, 3)};
     if (trace == EL_TRACE_RK2) return launch_velocity_tiled<T, EL_TRACE_RK2>(mac, ou, ov, ow, dt, dx, copy, s);
     return launch_velocity_tiled<T, EL_TRACE_RK3>(mac, ou, ov, ow, dt, dx, copy, s);
 }
