@@ -843,8 +843,12 @@ EL_API int el_advect_collocated_grid(const el_grid* g, int dtype, void* out, con
                                      void* stream) {
     if (!valid_grid(g, dtype) || !out || !in || !vu || !vv || !vw || out == in || !valid_scheme(trace, sample))
         return EL_ERR_INVALID_ARGUMENT;
-    advect_any(dtype, g->ni, g->nj, g->nk, g->dx, 0, out, in, vu, vv, vw, nullptr, dt, trace, sample,
-               (cudaStream_t)stream);
+    // the tiled kernels, as advect_level_set (they stage nothing outside their launch)
+    const int n = advect_phi_tiled(dtype, g->ni, g->nj, g->nk, g->dx, out, in, vu, vv, vw, nullptr, dt, trace, sample,
+                                   true, (cudaStream_t)stream);
+    if (n < 0)
+        advect_any(dtype, g->ni, g->nj, g->nk, g->dx, 0, out, in, vu, vv, vw, nullptr, dt, trace, sample,
+                   (cudaStream_t)stream);
     return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
 }
 
@@ -861,6 +865,12 @@ EL_API int el_advect_staggered_grid(const el_grid* g, int dtype, void* ou, void*
             if (outs[a] == ins[b] || outs[a] == (a == 0 ? iu : a == 1 ? iv : iw)) return EL_ERR_INVALID_ARGUMENT;
     const void* src[3] = {iu, iv, iw};
     void* dst[3] = {ou, ov, ow};
+    // a velocity advecting itself with trilinear reads: the tiled kernel, the three components in
+    // one launch; any other field, and WENO6 reads, by the per-sample kernel
+    if (sample == EL_SAMPLE_TRILINEAR && iu == vu && iv == vv && iw == vw &&
+        advect_velocity_tiled(dtype, g->ni, g->nj, g->nk, g->dx, ou, ov, ow, vu, vv, vw, nullptr, dt, trace, true,
+                              (cudaStream_t)stream) > 0)
+        return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
     for (int c = 0; c < 3; ++c)
         advect_any(dtype, g->ni, g->nj, g->nk, g->dx, c + 1, dst[c], src[c], vu, vv, vw, nullptr, dt, trace, sample,
                    (cudaStream_t)stream);
