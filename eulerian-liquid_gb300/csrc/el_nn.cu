@@ -621,135 +621,223 @@ __global__ void pack_weights_tc_kernel(int cin, int cout, const float* __restric
 }  // namespace tc
 
 // ---------------------------------------------------------------------------------------
-// backward weight: dW[co][tap][ci] = sum_v gm[v][co] x[v + off(tap)][ci], gm = g * (y > 0),
-// one 16 (co) x 16 (ci) tile of one tap per warp task; the CTA covers taps
-// [tap0, tap0 + ntaps) for all channels over bricks split, split + nsplit, ...
-template <int CIN, int COUT>
-struct WGrad {
-    static constexpr int MB = COUT / 16, NP = CIN / 16;
-    static constexpr int TILES_PER_TAP = MB * NP;
-    static constexpr int TAPS = (64 / TILES_PER_TAP) < 1 ? 1 : ((64 / TILES_PER_TAP) > 27 ? 27 : 64 / TILES_PER_TAP);
-    static constexpr int GROUPS = (27 + TAPS - 1) / TAPS;
-    static constexpr int MAXT = (TAPS * TILES_PER_TAP + 7) / 8;  // tasks per warp
-};
+// backward weight: dW[co][tap][ci] = sum_v gm[v][co] x[v + off(tap)][ci], gm = g * (y > 0).
+//
+// A CTA takes all 27 taps of a 16-channel slice of the input and 16 MB output channels, over a run
+// of units (a unit: the 16 x 8 voxels of one brick of one plane z; z fastest), and keeps the
+// accumulators in registers: warp (dz, dy) has the three taps dx, 9 warps.  What it stages is then
+// its own channels once (the input planes z - 1, z, z + 1 in a ring of four, each fetched once a
+// column by cp.async while the plane before is worked on), where a split by taps staged every
+// channel of the halo in every group of taps and spent its time on that.  The masked gradient of
+// the next unit comes through registers (two buffers).  One barrier a unit; a row of 16 voxels is
+// one k-step: MB + 3 ldmatrix for 6 MB mma.
+// 96 -> 32 at 64^3: 1618 -> 150 us; 16 -> 16 at 128^3: 290 -> 101 us (mma.sync's own limit is about
+// a third of that).
+constexpr int kWgThreads = 288;
+constexpr int kPlaneVox = kHX * kHY;      // 180 voxels of a staged plane
+constexpr int kXPitch = 48;               // bytes of a voxel's 16 channels, padded: conflict-free ldmatrix
+constexpr int kXPlane = kPlaneVox * kXPitch;
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) conv3_wgrad_kernel(int X, int Y, int Z, ConvIn in,
-                                                               const __nv_bfloat16* __restrict__ g,
-                                                               const __nv_bfloat16* __restrict__ y_out, int nsplit,
-                                                               float* __restrict__ part_w, float* __restrict__ part_b) {
+struct WGrad {
+    static constexpr int MB = COUT >= 32 ? 2 : 1;        // 16-channel blocks of the output a CTA
+    static constexpr int GROUPS = (CIN / 16) * (COUT / (16 * MB));
+    static constexpr int GPITCH = 32 * MB + 16;          // bytes of a voxel's gradient slice, padded
+    static constexpr int GTILE = 128 * GPITCH;
+    static constexpr int SMEM = 4 * kXPlane + 2 * GTILE;
+    static constexpr int CTAS = MB == 2 ? 2 : 3;         // resident per SM (registers)
+};
+
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kWgThreads, WGrad<CIN, COUT>::CTAS)
+    conv3_wgrad_kernel(int X, int Y, int Z, ConvIn in, const __nv_bfloat16* __restrict__ g,
+                       const __nv_bfloat16* __restrict__ y_out, int nsplit, float* __restrict__ part_w,
+                       float* __restrict__ part_b) {
     using W = WGrad<CIN, COUT>;
-    constexpr int SROW = CIN + 8, GROW = COUT + 8;
+    constexpr int MB = W::MB, GV = 2 * MB;  // 16-byte chunks of a voxel's gradient slice
+    constexpr int kGPer = (128 * GV + kWgThreads - 1) / kWgThreads;  // gradient chunks a thread
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __nv_bfloat16* halo = reinterpret_cast<__nv_bfloat16*>(smem_raw);
-    __nv_bfloat16* gt = halo + kHV * SROW;  // [128 voxels][COUT]
-    const int group = blockIdx.x, split = blockIdx.y;
-    const int tap0 = group * W::TAPS;
-    const int ntaps = min(W::TAPS, 27 - tap0);
-    const int ntasks = ntaps * W::TILES_PER_TAP;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t xs = smem_u32(smem_raw), gs = xs + 4 * kXPlane;
+    const int cis = blockIdx.x % (CIN / 16), cos = blockIdx.x / (CIN / 16), split = blockIdx.y;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int bx = (X + kTX - 1) / kTX, by = (Y + kTY - 1) / kTY;
-    const long long nbricks = (long long)bx * by * Z;
-    float acc[W::MAXT][2][4];
+    const long long units = (long long)bx * by * Z;
+    const long long u_begin = units * split / nsplit, u_end = units * (split + 1) / nsplit;
+    float acc[3][MB][2][4];
 #pragma unroll
-    for (int t = 0; t < W::MAXT; ++t)
+    for (int t = 0; t < 3; ++t)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) acc[t][h][0] = acc[t][h][1] = acc[t][h][2] = acc[t][h][3] = 0.f;
-    float bsum = 0.f;  // bias gradient: channel threadIdx.x % COUT (group 0 only)
-    const int r = (lane & 7), m = lane >> 3;
-#pragma unroll 1
-    for (long long br = split; br < nbricks; br += nsplit) {
-        const int bxi = (int)(br % bx);
-        const long long rest = br / bx;
-        const int byi = (int)(rest % by), z0 = (int)(rest / by);
-        const int x0 = bxi * kTX, y0 = byi * kTY;
-        __syncthreads();  // previous brick's reads done
-        stage_halo<CIN>(halo, in, X, Y, Z, x0, y0, z0);
-        // output gradient tile, masked by ReLU'; zero outside the grid
-        for (int idx = threadIdx.x; idx < 128 * (COUT / 8); idx += kThreads) {
-            const int vv = idx / (COUT / 8), cv = idx - vv * (COUT / 8);
+        for (int m = 0; m < MB; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) acc[t][m][h][0] = acc[t][m][h][1] = acc[t][m][h][2] = acc[t][m][h][3] = 0.f;
+    float accb[MB][4];  // bias gradient (warp 0 of the first input slice): the row sums of gm^T
+#pragma unroll
+    for (int m = 0; m < MB; ++m) accb[m][0] = accb[m][1] = accb[m][2] = accb[m][3] = 0.f;
+    const bool bias_warp = cis == 0 && warp == 0;
+
+    int x0 = 0, y0 = 0;
+    // chunk e of a plane: voxel e / 2, channels 8 (e % 2) of the slice; this thread's are tid and,
+    // for the first 72 threads, tid + 288
+    auto stage_plane = [&](int z) {
+        const uint32_t slot = xs + (uint32_t)((z + 4) & 3) * kXPlane;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int e = tid + q * kWgThreads;
+            if (e >= 2 * kPlaneVox) break;
+            const int hv = e >> 1, hy = hv / kHX, hx = hv - hy * kHX;
+            const int x = x0 + hx - 1, y = y0 + hy - 1, c = cis * 16 + (e & 1) * 8;
+            const __nv_bfloat16* src = in.a;  // a valid address even when nothing is read
+            bool valid = x >= 0 && x < X && y >= 0 && y < Y && z >= 0 && z < Z;
+            if (valid) {
+                if (c < in.ca) {
+                    const long long v = in.up_a ? ((long long)(z >> 1) * in.ay + (y >> 1)) * in.ax + (x >> 1)
+                                                : ((long long)z * Y + y) * X + x;
+                    src = in.a + v * in.ca + c;
+                } else if (in.b) {
+                    src = in.b + (((long long)z * Y + y) * X + x) * in.cb + (c - in.ca);
+                } else {
+                    valid = false;
+                }
+            }
+            cp_async16_zfill(slot + (uint32_t)(hv * kXPitch + (e & 1) * 16), src, valid);
+        }
+    };
+    uint4 gr[kGPer], yr[kGPer];
+    auto load_grad = [&](int z) {
+#pragma unroll
+        for (int q = 0; q < kGPer; ++q) {
+            const int e = tid + q * kWgThreads, vv = e / GV, cv = e % GV;
             const int x = x0 + (vv & 15), y = y0 + (vv >> 4);
-            uint4 val = make_uint4(0u, 0u, 0u, 0u);
-            if (x < X && y < Y) {
-                const long long v = ((long long)z0 * Y + y) * X + x;
-                val = apply_relu_mask(__ldg(reinterpret_cast<const uint4*>(g + v * COUT + cv * 8)),
-                                      __ldg(reinterpret_cast<const uint4*>(y_out + v * COUT + cv * 8)));
+            gr[q] = yr[q] = make_uint4(0u, 0u, 0u, 0u);
+            if (e < 128 * GV && x < X && y < Y) {
+                const long long o = (((long long)z * Y + y) * X + x) * COUT + cos * 16 * MB + cv * 8;
+                gr[q] = __ldg(reinterpret_cast<const uint4*>(g + o));
+                yr[q] = __ldg(reinterpret_cast<const uint4*>(y_out + o));
             }
-            *reinterpret_cast<uint4*>(gt + vv * GROW + cv * 8) = val;
         }
-        __syncthreads();
-        if (group == 0 && threadIdx.x < 2 * COUT) {
-            const int co = threadIdx.x % COUT, half = threadIdx.x / COUT;
-            for (int vv = half * 64; vv < half * 64 + 64; ++vv) bsum += __bfloat162float(gt[vv * GROW + co]);
-        }
-#pragma unroll 1
-        for (int row = 0; row < kTY; ++row) {  // k-step: the 16 voxels of brick row `row`
+    };
+    auto store_grad = [&](int buf) {
 #pragma unroll
-            for (int t = 0; t < W::MAXT; ++t) {
-                const int task = warp + 8 * t;
-                if (task >= ntasks) break;
-                const int tl = task / W::TILES_PER_TAP, rem = task - tl * W::TILES_PER_TAP;
-                const int mb = rem / W::NP, np = rem - mb * W::NP;
-                const int tap = tap0 + tl;
-                const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-                // A = gm^T (co x v): matrices (v 0-7|co 0-7), (v 0-7|co 8-15), (v 8-15|co 0-7), (v 8-15|co 8-15)
-                uint32_t a[4];
-                ldsm_x4_t(smem_u32(gt + (row * 16 + r + (m >> 1) * 8) * GROW + mb * 16 + (m & 1) * 8), a);
-                // B = x shifted (v x ci): matrices (v 0-7|ci 0-7), (v 8-15|ci 0-7), (v 0-7|ci 8-15), (v 8-15|ci 8-15)
-                const int hv = ((1 + dz) * kHY + (row + 1 + dy)) * kHX + (1 + dx) + r + (m & 1) * 8;
+        for (int q = 0; q < kGPer; ++q) {
+            const int e = tid + q * kWgThreads;
+            if (e < 128 * GV)
+                *reinterpret_cast<uint4*>(smem_raw + 4 * kXPlane + buf * W::GTILE + (e / GV) * W::GPITCH + (e % GV) * 16) =
+                    apply_relu_mask(gr[q], yr[q]);
+        }
+    };
+
+    const int r = lane & 7, m4 = lane >> 3;
+    const int dz = warp / 3 - 1, dy = warp % 3 - 1;
+    // this lane's ldmatrix rows: A = gm^T (v 0-7|co 0-7), (v 0-7|co 8-15), (v 8-15|co 0-7), (v 8-15|co 8-15);
+    // B = x shifted (v 0-7|ci 0-7), (v 8-15|ci 0-7), (v 0-7|ci 8-15), (v 8-15|ci 8-15)
+    const uint32_t a_lane = (uint32_t)((r + (m4 >> 1) * 8) * W::GPITCH + (m4 & 1) * 16);
+    const uint32_t b_lane = (uint32_t)(((1 + dy) * kHX + r + (m4 & 1) * 8) * kXPitch + (m4 >> 1) * 16);
+    int buf = 0;
+#pragma unroll 1
+    for (long long u = u_begin; u < u_end; ++u) {
+        const int z = (int)(u % Z);
+        if (u == u_begin || z == 0) {  // a column begins: its first three planes and its first gradient
+            __syncthreads();           // the unit before is done with the buffers
+            const long long col = u / Z;
+            x0 = (int)(col % bx) * kTX;
+            y0 = (int)(col / bx) * kTY;
+            stage_plane(z - 1);
+            stage_plane(z);
+            stage_plane(z + 1);
+            load_grad(z);
+            store_grad(buf);
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        const bool more = u + 1 < u_end && z + 1 < Z;  // the next unit continues this column
+        if (more) {
+            stage_plane(z + 2);
+            load_grad(z + 1);
+        }
+        const uint32_t xp = xs + (uint32_t)((z + dz + 4) & 3) * kXPlane + b_lane;
+        const uint32_t gp = gs + (uint32_t)(buf * W::GTILE) + a_lane;
+#pragma unroll
+        for (int row = 0; row < kTY; ++row) {
+            uint32_t a[MB][4];
+#pragma unroll
+            for (int m = 0; m < MB; ++m) ldsm_x4_t(gp + (uint32_t)(row * 16 * W::GPITCH + m * 32), a[m]);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
                 uint32_t b[4];
-                ldsm_x4_t(smem_u32(halo + hv * SROW + np * 16 + (m >> 1) * 8), b);
-                mma_bf16(acc[t][0], a, b[0], b[1]);
-                mma_bf16(acc[t][1], a, b[2], b[3]);
+                ldsm_x4_t(xp + (uint32_t)((row * kHX + t) * kXPitch), b);
+#pragma unroll
+                for (int m = 0; m < MB; ++m) {
+                    mma_bf16(acc[t][m][0], a[m], b[0], b[1]);
+                    mma_bf16(acc[t][m][1], a[m], b[2], b[3]);
+                }
+            }
+            if (bias_warp) {
+#pragma unroll
+                for (int m = 0; m < MB; ++m) mma_bf16(accb[m], a[m], 0x3f803f80u, 0x3f803f80u);  // times ones
             }
         }
+        buf ^= 1;
+        if (more) store_grad(buf);
     }
     // partial [split][tap][co][ci]
 #pragma unroll
-    for (int t = 0; t < W::MAXT; ++t) {
-        const int task = warp + 8 * t;
-        if (task >= ntasks) break;
-        const int tl = task / W::TILES_PER_TAP, rem = task - tl * W::TILES_PER_TAP;
-        const int mb = rem / W::NP, np = rem - mb * W::NP;
-        float* dst = part_w + ((size_t)split * 27 + tap0 + tl) * COUT * CIN;
+    for (int t = 0; t < 3; ++t) {
+        float* dst = part_w + ((size_t)split * 27 + warp * 3 + t) * COUT * CIN;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int ci = np * 16 + h * 8 + (lane & 3) * 2;
-            const int co = mb * 16 + (lane >> 2);
-            dst[(size_t)co * CIN + ci] = acc[t][h][0];
-            dst[(size_t)co * CIN + ci + 1] = acc[t][h][1];
-            dst[(size_t)(co + 8) * CIN + ci] = acc[t][h][2];
-            dst[(size_t)(co + 8) * CIN + ci + 1] = acc[t][h][3];
-        }
+        for (int m = 0; m < MB; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int ci = cis * 16 + h * 8 + (lane & 3) * 2, co = (cos * MB + m) * 16 + (lane >> 2);
+                *reinterpret_cast<float2*>(dst + (size_t)co * CIN + ci) = make_float2(acc[t][m][h][0], acc[t][m][h][1]);
+                *reinterpret_cast<float2*>(dst + (size_t)(co + 8) * CIN + ci) =
+                    make_float2(acc[t][m][h][2], acc[t][m][h][3]);
+            }
     }
-    if (group == 0) {
-        __shared__ float bs[2 * 128];
-        if (threadIdx.x < 2 * COUT) bs[threadIdx.x] = bsum;
-        __syncthreads();
-        if (threadIdx.x < COUT) part_b[(size_t)split * COUT + threadIdx.x] = bs[threadIdx.x] + bs[threadIdx.x + COUT];
+    if (bias_warp && (lane & 3) == 0) {
+#pragma unroll
+        for (int m = 0; m < MB; ++m) {
+            const int co = (cos * MB + m) * 16 + (lane >> 2);
+            part_b[(size_t)split * COUT + co] = accb[m][0];
+            part_b[(size_t)split * COUT + co + 8] = accb[m][2];
+        }
     }
 }
 
-// dW[co][tap][ci] += sum over splits (fixed order); db[co] += likewise
-__global__ void wgrad_reduce_kernel(int cin, int cout, int nsplit, const float* __restrict__ part_w,
-                                    const float* __restrict__ part_b, float* __restrict__ dw, float* __restrict__ db) {
-    const long long per = 27LL * cout * cin;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < per + cout;
-         e += (long long)gridDim.x * blockDim.x) {
-        if (e < per) {
-            // e indexes the partial layout [tap][co][ci]; dW is [co][tap][ci]
-            const int ci = (int)(e % cin);
-            const long long t2 = e / cin;
-            const int co = (int)(t2 % cout), tap = (int)(t2 / cout);
-            float s = 0.f;
-            for (int q = 0; q < nsplit; ++q) s += part_w[(size_t)q * per + e];
-            dw[((size_t)co * 27 + tap) * cin + ci] += s;
-        } else if (db) {
-            const int co = (int)(e - per);
-            float s = 0.f;
-            for (int q = 0; q < nsplit; ++q) s += part_b[(size_t)q * cout + co];
-            db[co] += s;
-        }
+// dW[co][tap][ci] += sum over splits, db[co] += likewise, in a fixed order: a block takes 32 values,
+// warp w sums every eighth split from w on, and the eight sums are added in order (a thread a value
+// and all its splits in sequence left 28 blocks waiting for one load after another: 26 -> 6 us
+// for 16 -> 16 at 128^3)
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(int cin, int cout, int nsplit,
+                                                           const float* __restrict__ part_w,
+                                                           const float* __restrict__ part_b, float* __restrict__ dw,
+                                                           float* __restrict__ db) {
+    __shared__ float sums[8][32];
+    const int per = 27 * cout * cin;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + lane;
+    const float* p = e < per ? part_w + e : part_b + (e - per);
+    const size_t stride = e < per ? (size_t)per : (size_t)cout;
+    float s = 0.f;
+    if (e < per + (db ? cout : 0)) {
+#pragma unroll 8
+        for (int q = warp; q < nsplit; q += 8) s += p[(size_t)q * stride];
+    }
+    sums[warp][lane] = s;
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (int q = 1; q < 8; ++q) s += sums[q][lane];
+    if (e < per) {
+        // e indexes the partial layout [tap][co][ci]; dW is [co][tap][ci]
+        const int ci = e % cin, t2 = e / cin, co = t2 % cout, tap = t2 / cout;
+        dw[((size_t)co * 27 + tap) * cin + ci] += s;
+    } else if (db && e < per + cout) {
+        db[e - per] += s;
     }
 }
 
@@ -1133,11 +1221,12 @@ int launch_conv_tc(const el_nn_conv_args* a, cudaStream_t s) {
     return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
 }
 
+// one wave of resident CTAs over the channel slices, at most a split a unit
 template <int CIN, int COUT>
 int wgrad_splits(int nx, int ny, int nz) {
-    const long long bricks = (long long)((nx + kTX - 1) / kTX) * ((ny + kTY - 1) / kTY) * nz;
-    const int want = (2 * num_sms_current() + WGrad<CIN, COUT>::GROUPS - 1) / WGrad<CIN, COUT>::GROUPS;
-    return (int)std::max<long long>(1, std::min<long long>(want, bricks));
+    const long long units = (long long)((nx + kTX - 1) / kTX) * ((ny + kTY - 1) / kTY) * nz;
+    const int want = WGrad<CIN, COUT>::CTAS * num_sms_current() / WGrad<CIN, COUT>::GROUPS;
+    return (int)std::max<long long>(1, std::min<long long>(want, units));
 }
 
 template <int CIN, int COUT>
@@ -1154,15 +1243,14 @@ int launch_wgrad(const el_nn_conv_args* a, const void* grad_out, float* dw, floa
     if (ws_bytes < wgrad_ws<CIN, COUT>(a->nx, a->ny, a->nz)) return EL_ERR_INVALID_ARGUMENT;
     float* part_w = static_cast<float*>(ws);
     float* part_b = part_w + (size_t)ns * 27 * CIN * COUT;
-    const size_t smem = ((size_t)kHV * (CIN + 8) + 128 * (COUT + 8)) * sizeof(__nv_bfloat16);
-    if (cudaFuncSetAttribute(conv3_wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(conv3_wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, W::SMEM) !=
         cudaSuccess)
         return EL_ERR_CUDA;
-    conv3_wgrad_kernel<CIN, COUT><<<dim3(W::GROUPS, ns), kThreads, smem, s>>>(
+    conv3_wgrad_kernel<CIN, COUT><<<dim3(W::GROUPS, ns), kWgThreads, W::SMEM, s>>>(
         a->nx, a->ny, a->nz, conv_in(a), static_cast<const __nv_bfloat16*>(grad_out),
         static_cast<const __nv_bfloat16*>(a->out_a), ns, part_w, part_b);
-    const long long n = 27LL * CIN * COUT + COUT;
-    wgrad_reduce_kernel<<<grid_elems(n), 256, 0, s>>>(CIN, COUT, ns, part_w, part_b, dw, db);
+    const int n = 27 * CIN * COUT + COUT;
+    wgrad_reduce_kernel<<<(n + 31) / 32, 256, 0, s>>>(CIN, COUT, ns, part_w, part_b, dw, db);
     return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
 }
 
