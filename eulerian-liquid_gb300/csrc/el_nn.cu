@@ -47,6 +47,12 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// 16 bytes to shared memory, zeros where !valid (src is then any valid address)
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
+}
+
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -177,34 +183,45 @@ __global__ void __launch_bounds__(kThreads) conv3_kernel(int X, int Y, int Z, Co
 }
 
 // ---------------------------------------------------------------------------------------
-// The same convolution on the 5th-generation tensor cores (tcgen05), for layers whose 27 taps
-// of weights fit in shared memory next to the input brick.  A CTA of 4 warps owns an
-// 8 (x) x 16 (y) x 1 (z) brick: M = 128 voxels, one TMEM lane each; N = output channels in TMEM
-// columns (FP32).  Both operands sit in shared memory in the no-swizzle K-major layout, whose
-// unit is an 8-row x 16-byte core matrix:
-//   A: the input brick with its halo (10 x 18 x 3 voxels), channel-chunk major: chunk c
-//      (channels 8c..8c+7) of voxel v at (c * 540 + v) * 16 bytes.  Eight x-consecutive voxels
-//      are one core matrix, the next 8 rows (the next y) are 10 voxels further (SBO = 160 B),
-//      the next chunk along K is 540 voxels further (LBO = 8640 B); tap (dx, dy, dz) only moves
-//      the start address, so the 27 shifted operands need no copies.
+// The same convolution on the 5th-generation tensor cores (tcgen05).  A unit is the 8 (x) x 16 (y)
+// voxels of one column in one plane z: M = 128 voxels, one TMEM lane each; N = output channels in TMEM
+// columns (FP32).  A CTA owns a range of units (z fastest) and takes it in runs within a column, with
+// one accumulator per unit of a run; the input channels go in slices of SC.  For each slice it fetches
+// the slice's 27 taps of weights (once for all runs, if there is one slice) and marches the run's
+// planes; after the last slice the run is stored.  Both operands sit in shared memory in the no-swizzle
+// K-major layout, whose unit is an 8-row x 16-byte core matrix:
+//   A: a ring of five input planes with their halo (10 x 18 voxels), channel-chunk major: chunk c
+//      (channels 8c..8c+7) of voxel v of ring slot s at ((5 c + s) * 180 + v) * 16 bytes.  Eight
+//      x-consecutive voxels are one core matrix, the next 8 rows (the next y) are 10 voxels further
+//      (SBO = 160 B), the next chunk along K is five planes further (LBO = 14400 B); tap
+//      (dx, dy, dz) only moves the start address, so the 27 shifted operands need no copies.
 //   B: per tap, [channel chunk][output channel] x 16 bytes: SBO = 128 B, LBO = cout * 16 B.
-// One thread issues the 27 * cin / 16 MMAs (K = 16 each) into one accumulator and commits them to
-// an mbarrier; the 4 warps wait (bounded), read their 32 TMEM lanes (tcgen05.ld) and store.
-// The CTA is persistent over bricks: the weights are staged once.
+// One thread issues the 27 * SC / 16 MMAs (K = 16 each) of a unit and commits them to one of two
+// mbarriers; while they run, the plane two units ahead is fetched (cp.async, zero-filled outside the
+// grid; with a ReLU mask, through registers).
+// A plane of a column is staged once a slice (bricks of one plane staged three, and that staging was
+// most of the time), and several CTAs on an SM cover each other's staging: SC and the CTAs an SM are
+// chosen together so that weights and ring fit (EL_NN_TC_PAIRS; all 48 channels of 48 -> 16 at once
+// left one CTA an SM: 589 us against 222).  An MMA reads 4 KB of A whatever N is, about 32 clocks: that
+// and the staging bound the narrow layers (16 -> 16 at 128^3: 48 us of MMA).  Forward / backward data,
+// before (bricks) and now: 16 -> 16 at 128^3 166 / 258 -> 88 / 116 us; 32 -> 96 at 64^3 196 -> 66.
 namespace tc {
 
 __device__ int g_error;  // set when a bounded wait gave up; read and cleared by el_nn_take_error
 
-constexpr int TX = 8, TY = 16, HX = TX + 2, HY = TY + 2, HZ = 3, HV = HX * HY * HZ;  // 540 halo voxels
-constexpr int kThreads = 128;
+constexpr int TX = 8, TY = 16, HX = TX + 2, HY = TY + 2, PV = HX * HY;  // 180 voxels of a staged plane
+constexpr int kThreads = 256;
+constexpr int kRing = 5;     // planes z - 1, z, z + 1 of a unit, z + 2 landing, z + 3 on its way
+
+__device__ __forceinline__ int ring_slot(int z) { return (int)((unsigned)(z + kRing) % (unsigned)kRing); }
 
 template <int CIN, int COUT>
 struct Shape {
     static constexpr int KC = CIN / 8;                 // 16-byte channel chunks
     static constexpr int WB = 27 * KC * COUT * 16;     // weight bytes
-    static constexpr int HB = KC * HV * 16;            // input brick bytes
-    static constexpr int SMEM = WB + HB + 16;          // + mbarrier and TMEM address
-    static constexpr uint32_t NCOL = COUT <= 32 ? 32u : (COUT <= 64 ? 64u : 128u);
+    static constexpr int LBO = kRing * PV * 16;            // bytes from a channel chunk to the next
+    static constexpr int HB = KC * LBO;                // the ring
+    static constexpr int SMEM = WB + HB + COUT * 4 + 32;  // + bias, two mbarriers and the TMEM address
     // BF16 x BF16 -> FP32, both K-major, M = 128, N = COUT
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COUT >> 3) << 17) |
                                       ((uint32_t)(128 >> 4) << 24);
@@ -235,243 +252,108 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t phase) {
     }
 }
 
-template <int CIN>
-__device__ __forceinline__ void stage_brick(unsigned char* hsm, const ConvIn& in, int X, int Y, int Z, int x0, int y0,
-                                            int z0) {
-    constexpr int KC = CIN / 8;
-    for (int idx = threadIdx.x; idx < HV * KC; idx += kThreads) {
-        const int hv = idx / KC, cv = idx - hv * KC;
-        const int hx = hv % HX, t = hv / HX, hy = t % HY, hz = t / HY;
-        const int x = x0 + hx - 1, y = y0 + hy - 1, z = z0 + hz - 1;
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (x >= 0 && x < X && y >= 0 && y < Y && z >= 0 && z < Z) {
-            const int c = cv * 8;
-            const long long fine = ((long long)z * Y + y) * X + x;
-            if (c < in.ca) {
-                const long long va = in.up_a ? ((long long)(z >> 1) * in.ay + (y >> 1)) * in.ax + (x >> 1) : fine;
-                val = __ldg(reinterpret_cast<const uint4*>(in.a + va * in.ca + c));
-            } else if (in.b) {
-                val = __ldg(reinterpret_cast<const uint4*>(in.b + fine * in.cb + (c - in.ca)));
-            }
-            if (in.mask) val = apply_relu_mask(val, __ldg(reinterpret_cast<const uint4*>(in.mask + fine * CIN + c)));
+// The staging of a column's planes, KC channel chunks from chunk c0 of the input on.  Chunk idx of a
+// plane: voxel idx / KC, channel chunk idx % KC (consecutive threads read consecutive bytes of a
+// voxel); a thread's chunks are the same in every plane, so what depends on x and y is formed once a
+// column.
+template <int KC>
+struct ColumnStage {
+    static constexpr int N = PV * KC, PER = (N + kThreads - 1) / kThreads;
+    int va[PER], vf[PER];  // voxel within a plane of `a`, and at full resolution (-1: outside the grid)
+    __device__ __forceinline__ void column(const ConvIn& in, int X, int Y, int x0, int y0) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int hv = ((int)threadIdx.x + q * kThreads) / KC, hy = hv / HX, hx = hv - hy * HX;
+            const int x = x0 + hx - 1, y = y0 + hy - 1;
+            const bool inside = hv < PV && x >= 0 && x < X && y >= 0 && y < Y;
+            vf[q] = inside ? y * X + x : -1;
+            va[q] = in.up_a ? (y >> 1) * in.ax + (x >> 1) : vf[q];
         }
-        *reinterpret_cast<uint4*>(hsm + ((size_t)cv * HV + hv) * 16) = val;
     }
-}
-
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) conv3_tc_kernel(int X, int Y, int Z, ConvIn in,
-                                                            const uint4* __restrict__ wtc,
-                                                            const float* __restrict__ bias, int relu,
-                                                            __nv_bfloat16* __restrict__ out_a, int oca,
-                                                            __nv_bfloat16* __restrict__ out_b) {
-    using S = Shape<CIN, COUT>;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    unsigned char* wsm = smem_raw;
-    unsigned char* hsm = smem_raw + S::WB;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + S::WB + S::HB);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem_raw + S::WB + S::HB + 8);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int q = tid; q < S::WB / 16; q += kThreads) reinterpret_cast<uint4*>(wsm)[q] = __ldg(wtc + q);
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
-                     "r"(S::NCOL)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(mbar)), "r"(1) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *tslot;
-    const uint32_t wbase = smem_u32(wsm), hbase = smem_u32(hsm), mbar_a = smem_u32(mbar);
-    const int bx = (X + TX - 1) / TX, by = (Y + TY - 1) / TY;
-    const long long nbricks = (long long)bx * by * Z;
-    uint32_t phase = 0;
-    for (long long br = blockIdx.x; br < nbricks; br += gridDim.x) {
-        const int x0 = (int)(br % bx) * TX;
-        const long long rest = br / bx;
-        const int y0 = (int)(rest % by) * TY, z0 = (int)(rest / by);
-        stage_brick<CIN>(hsm, in, X, Y, Z, x0, y0, z0);
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // visible to the tensor cores
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll 1
-            for (int tap = 0; tap < 27; ++tap) {
-                const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-                const uint32_t a0 = hbase + (uint32_t)(((dz * HY + dy) * HX + dx) * 16);
-                const uint32_t b0 = wbase + (uint32_t)(tap * S::KC * COUT * 16);
+    // plane z into its ring slot
+    __device__ __forceinline__ void plane(unsigned char* ring, const ConvIn& in, int X, int Y, int Z, int c0, int z) const {
+        constexpr int LBO = kRing * PV * 16;
+        unsigned char* slot = ring + (size_t)ring_slot(z) * PV * 16;
+        const bool z_in = z >= 0 && z < Z;
+        const long long pa = (long long)(in.up_a ? z >> 1 : z) * in.ax * in.ay, pf = (long long)z * X * Y;
+        auto source = [&](int q) -> const __nv_bfloat16* {
+            const int c = (c0 + ((int)threadIdx.x + q * kThreads) % KC) * 8;
+            if (!z_in || vf[q] < 0) return nullptr;
+            if (c < in.ca) return in.a + (pa + va[q]) * in.ca + c;
+            return in.b ? in.b + (pf + vf[q]) * in.cb + (c - in.ca) : nullptr;
+        };
+        if (in.mask) {  // the mask is applied on the way: through registers, a few chunks in flight
+            constexpr int U = PER < 3 ? PER : 3;
 #pragma unroll
-                for (int s = 0; s < S::KC / 2; ++s) {
-                    const uint64_t da = smem_desc(a0 + (uint32_t)(2 * s * HV * 16), HV * 16, HX * 16);
-                    const uint64_t db = smem_desc(b0 + (uint32_t)(2 * s * COUT * 16), COUT * 16, 128);
-                    const uint32_t acc = (tap | s) ? 1u : 0u;
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\t"
-                        "setp.ne.b32 p, %4, 0;\n\t"
-                        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                        "l"(da), "l"(db), "r"(S::IDESC), "r"(acc)
-                        : "memory");
-                }
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             mbar_a)
-                         : "memory");
-        }
-        const bool ok = mbar_wait(mbar_a, phase);
-        phase ^= 1u;
-        if (!__syncthreads_and(ok)) {
-            if (tid == 0) atomicExch(&g_error, 1);
-            break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        // row r = 32 warp + lane of the accumulator is voxel (x0 + r % 8, y0 + r / 8, z0)
-        const int r = warp * 32 + lane;
-        const int x = x0 + (r & 7), y = y0 + (r >> 3);
-        const bool live = x < X && y < Y;
-        const long long v = ((long long)z0 * Y + y) * X + x;
+            for (int q0 = 0; q0 < PER; q0 += U) {
+                uint4 v[U], m[U];
 #pragma unroll
-        for (int c0 = 0; c0 < COUT; c0 += 16) {
-            uint32_t q[16];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];\n"
-                : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]),
-                  "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]),
-                  "=r"(q[15])
-                : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (live) {
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint4 o;
-                    __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int co = c0 + h * 8 + 2 * e;
-                        float f0 = __uint_as_float(q[h * 8 + 2 * e]), f1 = __uint_as_float(q[h * 8 + 2 * e + 1]);
-                        if (bias) {
-                            f0 += bias[co];
-                            f1 += bias[co + 1];
-                        }
-                        if (relu) {
-                            f0 = fmaxf(f0, 0.f);
-                            f1 = fmaxf(f1, 0.f);
-                        }
-                        op[e] = __floats2bfloat162_rn(f0, f1);
+                for (int q = 0; q < U; ++q) {
+                    const __nv_bfloat16* p = q0 + q < PER ? source(q0 + q) : nullptr;
+                    const int c = (c0 + ((int)threadIdx.x + (q0 + q) * kThreads) % KC) * 8;
+                    v[q] = m[q] = make_uint4(0u, 0u, 0u, 0u);
+                    if (p) {
+                        v[q] = __ldg(reinterpret_cast<const uint4*>(p));
+                        m[q] = __ldg(reinterpret_cast<const uint4*>(in.mask + (pf + vf[q0 + q]) * (in.ca + in.cb) + c));
                     }
-                    const int cb = c0 + h * 8;
-                    if (cb < oca)
-                        *reinterpret_cast<uint4*>(out_a + v * oca + cb) = o;
-                    else
-                        *reinterpret_cast<uint4*>(out_b + v * (COUT - oca) + (cb - oca)) = o;
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    const int idx = (int)threadIdx.x + (q0 + q) * kThreads;
+                    if (q0 + q < PER && idx < N)
+                        *reinterpret_cast<uint4*>(slot + (size_t)(idx % KC) * LBO + (idx / KC) * 16) =
+                            apply_relu_mask(v[q], m[q]);
                 }
             }
+            return;
         }
-        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();  // accumulator read and brick consumed before the next brick
+        const uint32_t base = smem_u32(slot);
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int idx = (int)threadIdx.x + q * kThreads;
+            if (idx >= N) break;
+            const __nv_bfloat16* p = source(q);
+            cp_async16_zfill(base + (uint32_t)((idx % KC) * LBO + (idx / KC) * 16), p ? p : in.a, p != nullptr);
+        }
     }
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(S::NCOL) : "memory");
-}
-
-// Pipelined variant, for the layers where two input bricks fit next to the weights: the copy of
-// brick i+1 (cp.async, 16 bytes per thread and chunk, zero-filled outside the grid) and the
-// epilogue of brick i-1 run while the tensor cores work on brick i, with two input buffers and
-// two accumulators (2 * cout TMEM columns) used in turn.  A ReLU mask (backward data) is applied
-// while staging, so that case stages with ordinary loads at the same point.
-template <int CIN, int COUT>
-struct PipeShape {
-    static constexpr int KC = CIN / 8;
-    static constexpr int WB = 27 * KC * COUT * 16;
-    static constexpr int HB = KC * HV * 16;
-    static constexpr int SMEM = WB + 2 * HB + 32;
-    static constexpr uint32_t NCOL = 2 * COUT <= 32 ? 32u : (2 * COUT <= 64 ? 64u : (2 * COUT <= 128 ? 128u : 256u));
-    static constexpr bool FITS = SMEM <= 220 * 1024;
 };
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
-}
-
-template <int CIN>
-__device__ __forceinline__ void stage_brick_async(unsigned char* hsm, const ConvIn& in, int X, int Y, int Z, int x0,
-                                                  int y0, int z0) {
-    if (in.mask) {  // needs the mask applied on the way: ordinary loads
-        stage_brick<CIN>(hsm, in, X, Y, Z, x0, y0, z0);
-        return;
-    }
-    constexpr int KC = CIN / 8;
-    const uint32_t base = smem_u32(hsm);
-    for (int idx = threadIdx.x; idx < HV * KC; idx += kThreads) {
-        const int hv = idx / KC, cv = idx - hv * KC;
-        const int hx = hv % HX, t = hv / HX, hy = t % HY, hz = t / HY;
-        const int x = x0 + hx - 1, y = y0 + hy - 1, z = z0 + hz - 1;
-        const bool inside = x >= 0 && x < X && y >= 0 && y < Y && z >= 0 && z < Z;
-        const int c = cv * 8;
-        const __nv_bfloat16* src = in.a;  // a valid address even when nothing is read
-        bool valid = false;
-        if (inside) {
-            const long long fine = ((long long)z * Y + y) * X + x;
-            if (c < in.ca) {
-                const long long va = in.up_a ? ((long long)(z >> 1) * in.ay + (y >> 1)) * in.ax + (x >> 1) : fine;
-                src = in.a + va * in.ca + c;
-                valid = true;
-            } else if (in.b) {
-                src = in.b + fine * in.cb + (c - in.ca);
-                valid = true;
-            }
-        }
-        cp_async16(base + (uint32_t)(((size_t)cv * HV + hv) * 16), src, valid);
-    }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-
-// accumulator columns [col, col + COUT) of this warp's 32 lanes -> bias, ReLU, bf16, store
+// accumulator columns [col, col + COUT) of this warp's 32 lanes -> bias, ReLU, bf16, store; the two
+// warps of a lane quarter take alternate groups of 16 channels (bias: in shared memory)
 template <int COUT>
 __device__ __forceinline__ void tc_epilogue(uint32_t tmem, uint32_t col, int X, int Y, int x0, int y0, int z0,
-                                            const float* __restrict__ bias, int relu, __nv_bfloat16* out_a, int oca,
+                                            const float* bias, int relu, __nv_bfloat16* out_a, int oca,
                                             __nv_bfloat16* out_b) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = warp * 32 + lane;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quarter = warp & 3;
+    const int r = quarter * 32 + lane;
     const int x = x0 + (r & 7), y = y0 + (r >> 3);
     const bool live = x < X && y < Y;
     const long long v = ((long long)z0 * Y + y) * X + x;
 #pragma unroll
     for (int c0 = 0; c0 < COUT; c0 += 16) {
+        if (((c0 >> 4) & 1) != (warp >> 2)) continue;
         uint32_t q[16];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
             "[%16];\n"
             : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]),
               "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
-            : "r"(tmem + ((uint32_t)(warp * 32) << 16) + col + (uint32_t)c0));
+            : "r"(tmem + ((uint32_t)(quarter * 32) << 16) + col + (uint32_t)c0));
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
         if (!live) continue;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             uint4 o;
             __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+            const float4 b0 = *reinterpret_cast<const float4*>(bias + c0 + h * 8);
+            const float4 b1 = *reinterpret_cast<const float4*>(bias + c0 + h * 8 + 4);
+            const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int co = c0 + h * 8 + 2 * e;
-                float f0 = __uint_as_float(q[h * 8 + 2 * e]), f1 = __uint_as_float(q[h * 8 + 2 * e + 1]);
-                if (bias) {
-                    f0 += bias[co];
-                    f1 += bias[co + 1];
-                }
-                if (relu) {
-                    f0 = fmaxf(f0, 0.f);
-                    f1 = fmaxf(f1, 0.f);
-                }
+                float f0 = __uint_as_float(q[h * 8 + 2 * e]) + bb[2 * e];
+                float f1 = __uint_as_float(q[h * 8 + 2 * e + 1]) + bb[2 * e + 1];
+                f0 = relu ? fmaxf(f0, 0.f) : f0;
+                f1 = relu ? fmaxf(f1, 0.f) : f1;
                 op[e] = __floats2bfloat162_rn(f0, f1);
             }
             const int cb = c0 + h * 8;
@@ -483,49 +365,64 @@ __device__ __forceinline__ void tc_epilogue(uint32_t tmem, uint32_t col, int X, 
     }
 }
 
+// the MMAs of the unit in plane z into the accumulator at tmem_acc (first: which they start), committed
+// to mbar (one thread).  A descriptor's address field counts 16 bytes, so a tap is one addition to it.
 template <int CIN, int COUT>
-__device__ __forceinline__ void tc_issue(uint32_t tmem_acc, uint32_t hbase, uint32_t wbase, uint32_t mbar) {
-    using S = PipeShape<CIN, COUT>;
+__device__ __forceinline__ void tc_issue(uint32_t tmem_acc, uint32_t ring, uint32_t wbase, uint32_t mbar, int z,
+                                         bool first) {
+    using S = Shape<CIN, COUT>;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint64_t d0 = smem_desc(ring, S::LBO, HX * 16);
+    uint64_t db = smem_desc(wbase, COUT * 16, 128);
 #pragma unroll 1
-    for (int tap = 0; tap < 27; ++tap) {
-        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-        const uint32_t a0 = hbase + (uint32_t)(((dz * HY + dy) * HX + dx) * 16);
-        const uint32_t b0 = wbase + (uint32_t)(tap * S::KC * COUT * 16);
+    for (int dz = 0; dz < 3; ++dz) {
+        const uint64_t dplane = d0 + (uint64_t)(ring_slot(z - 1 + dz) * PV);
 #pragma unroll
-        for (int s = 0; s < S::KC / 2; ++s) {
-            const uint64_t da = smem_desc(a0 + (uint32_t)(2 * s * HV * 16), HV * 16, HX * 16);
-            const uint64_t db = smem_desc(b0 + (uint32_t)(2 * s * COUT * 16), COUT * 16, 128);
-            const uint32_t acc = (tap | s) ? 1u : 0u;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "setp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_acc),
-                "l"(da), "l"(db), "r"(Shape<CIN, COUT>::IDESC), "r"(acc)
-                : "memory");
-        }
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+            for (int s = 0; s < S::KC / 2; ++s) {
+                const uint64_t da = dplane + (uint64_t)((t / 3) * HX + t % 3 + 2 * s * (S::LBO / 16));
+                const uint32_t acc = (!first || (dz | t | s)) ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_acc),
+                    "l"(da), "l"(db), "r"(S::IDESC), "r"(acc)
+                    : "memory");
+                db += 2 * COUT;
+            }
     }
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar)
                  : "memory");
 }
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads) conv3_tc_pipe_kernel(int X, int Y, int Z, ConvIn in,
-                                                                 const uint4* __restrict__ wtc,
-                                                                 const float* __restrict__ bias, int relu,
-                                                                 __nv_bfloat16* __restrict__ out_a, int oca,
-                                                                 __nv_bfloat16* __restrict__ out_b) {
-    using S = PipeShape<CIN, COUT>;
+template <int CIN, int COUT, int SC, int CTAS>
+struct RunShape {
+    using S = Shape<SC, COUT>;                                                      // a slice's layout
+    static constexpr int SLICES = CIN / SC;
+    static constexpr uint32_t NCOL = CTAS == 1 ? 512u : (CTAS == 2 ? 256u : 128u);  // of the SM's 512
+    static constexpr int MAX_RUN = (int)NCOL / COUT < 16 ? (int)NCOL / COUT : 16;   // accumulators
+};
+
+template <int CIN, int COUT, int SC, int CTAS>
+__global__ void __launch_bounds__(kThreads, CTAS) conv3_tc_kernel(int X, int Y, int Z, ConvIn in,
+                                                                      const uint4* __restrict__ wtc,
+                                                                      const float* __restrict__ bias, int relu,
+                                                                      __nv_bfloat16* __restrict__ out_a, int oca,
+                                                                      __nv_bfloat16* __restrict__ out_b) {
+    using SS = RunShape<CIN, COUT, SC, CTAS>;
+    using S = typename SS::S;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* wsm = smem_raw;
-    unsigned char* hsm[2] = {smem_raw + S::WB, smem_raw + S::WB + S::HB};
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + S::WB + 2 * S::HB);  // two
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem_raw + S::WB + 2 * S::HB + 16);
+    unsigned char* ring = smem_raw + S::WB;
+    float* sbias = reinterpret_cast<float*>(smem_raw + S::WB + S::HB);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + S::WB + S::HB + COUT * 4);  // two
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(smem_raw + S::WB + S::HB + COUT * 4 + 16);
     const int tid = threadIdx.x, warp = tid >> 5;
-    for (int q = tid; q < S::WB / 16; q += kThreads) reinterpret_cast<uint4*>(wsm)[q] = __ldg(wtc + q);
+    if (tid < COUT) sbias[tid] = bias ? bias[tid] : 0.f;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
-                     "r"(S::NCOL)
+                     "r"(SS::NCOL)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
@@ -538,69 +435,83 @@ __global__ void __launch_bounds__(kThreads) conv3_tc_pipe_kernel(int X, int Y, i
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
-    const uint32_t wbase = smem_u32(wsm), hb[2] = {smem_u32(hsm[0]), smem_u32(hsm[1])};
+    const uint32_t wbase = smem_u32(wsm), rbase = smem_u32(ring);
     const uint32_t mb[2] = {smem_u32(mbar), smem_u32(mbar + 1)};
-    const int bx = (X + TX - 1) / TX, by = (Y + TY - 1) / TY;
-    const long long nbricks = (long long)bx * by * Z;
-    const long long mine = nbricks > blockIdx.x ? (nbricks - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    auto origin = [&](long long i, int& x0, int& y0, int& z0) {
-        const long long br = blockIdx.x + i * gridDim.x;
-        x0 = (int)(br % bx) * TX;
-        const long long rest = br / bx;
-        y0 = (int)(rest % by) * TY;
-        z0 = (int)(rest / by);
-    };
+    const int bx = (X + TX - 1) / TX, by = (Y + TY - 1) / TY, per = SS::MAX_RUN;
+    const long long units = (long long)bx * by * Z;
+    const long long u_end = units * (blockIdx.x + 1) / gridDim.x;
     uint32_t phase[2] = {0u, 0u};
     bool ok = true;
-    int x0, y0, z0;
-    if (mine > 0) {
-        origin(0, x0, y0, z0);
-        stage_brick_async<CIN>(hsm[0], in, X, Y, Z, x0, y0, z0);
-    }
-    for (long long i = 0; i < mine && ok; ++i) {
-        const int b = (int)(i & 1);
-        cp_async_wait_all();
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // brick i visible to the tensor cores
-        __syncthreads();
-        if (tid == 0) tc_issue<CIN, COUT>(tmem + (uint32_t)(b * COUT), hb[b], wbase, mb[b]);
-        if (i > 0) {
-            // brick i-1: its MMAs are done, so its buffer takes brick i+1 while its result is stored
-            const bool mine_ok = mbar_wait(mb[b ^ 1], phase[b ^ 1]);
-            phase[b ^ 1] ^= 1u;
-            ok = __syncthreads_and(mine_ok) != 0;  // uniform across the block
-            if (!ok) break;
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    auto finish_wait = [&](int b) {  // the MMAs committed to mbarrier b; uniform over the block
+        const bool mine_ok = mbar_wait(mb[b], phase[b]);
+        phase[b] ^= 1u;
+        const bool all = __syncthreads_and(mine_ok) != 0;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        return all;
+    };
+    ColumnStage<S::KC> stage;
+    int b = 0;
+    bool fresh = true;  // no weights fetched yet
+    for (long long u = units * blockIdx.x / gridDim.x; u < u_end && ok;) {
+        // what is left of this CTA's units in this column, as runs of about one length
+        const long long colu = u / Z;
+        const int x0 = (int)(colu % bx) * TX, y0 = (int)(colu / bx) * TY;
+        const int z_begin = (int)(u - colu * Z), left = (int)min((long long)(Z - z_begin), u_end - u);
+        const int nruns = (left + per - 1) / per, z_end = z_begin + (left + nruns - 1) / nruns;
+        u += z_end - z_begin;
+        stage.column(in, X, Y, x0, y0);
+#pragma unroll 1
+        for (int sl = 0; sl < SS::SLICES && ok; ++sl) {
+            // every MMA of the slice before has completed: its weights and planes may be overwritten
+            const int c0 = sl * S::KC;
+            for (int q = tid; q < S::WB / 16 && (SS::SLICES > 1 || fresh); q += kThreads) {
+                constexpr int T = S::KC * COUT;  // 16-byte pieces of a tap of the slice
+                const int tap = q / T, o = q - tap * T;
+                cp_async16_zfill(wbase + (uint32_t)q * 16, wtc + (size_t)tap * (CIN / 8) * COUT + (size_t)c0 * COUT + o, true);
+            }
+            stage.plane(ring, in, X, Y, Z, c0, z_begin - 1);
+            stage.plane(ring, in, X, Y, Z, c0, z_begin);
+            stage.plane(ring, in, X, Y, Z, c0, z_begin + 1);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            if (z_begin + 1 < z_end) stage.plane(ring, in, X, Y, Z, c0, z_begin + 2);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+#pragma unroll 1
+            for (int z = z_begin; z < z_end; ++z) {
+                asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // plane z + 1 has landed
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                __syncthreads();
+                if (tid == 0)
+                    tc_issue<SC, COUT>(tmem + (uint32_t)((z - z_begin) * COUT), rbase, wbase, mb[b], z, sl == 0);
+                if (z > z_begin) {
+                    ok = finish_wait(b ^ 1);  // the slot of plane z - 2 is free
+                    if (!ok) break;
+                }
+                if (z + 2 < z_end) stage.plane(ring, in, X, Y, Z, c0, z + 3);
+                asm volatile("cp.async.commit_group;\n" ::: "memory");
+                b ^= 1;
+            }
+            if (ok) ok = finish_wait(b ^ 1);
         }
-        if (i + 1 < mine) {
-            int x1, y1, z1;
-            origin(i + 1, x1, y1, z1);
-            stage_brick_async<CIN>(hsm[b ^ 1], in, X, Y, Z, x1, y1, z1);
-        }
-        if (i > 0) {
-            int xp, yp, zp;
-            origin(i - 1, xp, yp, zp);
-            tc_epilogue<COUT>(tmem, (uint32_t)((b ^ 1) * COUT), X, Y, xp, yp, zp, bias, relu, out_a, oca, out_b);
-        }
+        if (!ok) break;
+        fresh = false;
+        for (int z = z_begin; z < z_end; ++z)
+            tc_epilogue<COUT>(tmem, (uint32_t)((z - z_begin) * COUT), X, Y, x0, y0, z, sbias, relu, out_a, oca, out_b);
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();  // the accumulator just read is free for brick i+1
+        __syncthreads();  // the accumulators are read before the next run writes them
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     }
-    if (ok && mine > 0) {  // ok is uniform here
-        const long long i = mine - 1;
-        const int b = (int)(i & 1);
-        ok = __syncthreads_and(mbar_wait(mb[b], phase[b])) != 0;
-        if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            origin(i, x0, y0, z0);
-            tc_epilogue<COUT>(tmem, (uint32_t)(b * COUT), X, Y, x0, y0, z0, bias, relu, out_a, oca, out_b);
-        }
+    if (!ok && tid == 0) {
+        atomicExch(&g_error, 1);
+        mbar_wait(mb[0], phase[0]);  // once more (bounded), for MMAs still in flight
+        mbar_wait(mb[1], phase[1]);
     }
-    if (!ok && tid == 0) atomicExch(&g_error, 1);
-    cp_async_wait_all();
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(S::NCOL) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(SS::NCOL) : "memory");
 }
 
 // FP32 master [co][27][ci] -> the B layout above: [tap][ci / 8][co][ci % 8]
@@ -647,11 +558,6 @@ struct WGrad {
     static constexpr int SMEM = 4 * kXPlane + 2 * GTILE;
     static constexpr int CTAS = MB == 2 ? 2 : 3;         // resident per SM (registers)
 };
-
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
-}
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kWgThreads, WGrad<CIN, COUT>::CTAS)
@@ -1131,18 +1037,6 @@ int num_sms_current() {
     return sms;
 }
 
-// resident CTAs per SM for a kernel of `threads` threads and `smem` dynamic shared bytes, from the
-// device's shared memory per SM (the occupancy query alone reported one CTA per SM for these)
-int resident_per_sm(int threads, int smem) {
-    int dev = 0, per_sm_smem = 0, reserved = 0, max_threads = 2048;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&per_sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-    cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-    cudaDeviceGetAttribute(&max_threads, cudaDevAttrMaxThreadsPerMultiProcessor, dev);
-    const int by_smem = per_sm_smem / (smem + reserved);
-    return std::max(1, std::min(by_smem, max_threads / threads));
-}
-
 int grid_elems(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 152LL * 16)); }
 
 ConvIn conv_in(const el_nn_conv_args* a) {
@@ -1172,50 +1066,18 @@ int launch_conv(const el_nn_conv_args* a, cudaStream_t s) {
     return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
 }
 
-template <int CIN, int COUT>
-int launch_conv_tc_pipe(const el_nn_conv_args* a, cudaStream_t s) {
-    using S = tc::PipeShape<CIN, COUT>;
-    // the largest shared-memory carve-out, so that the occupancy below (and the launch) get it
-    if (cudaFuncSetAttribute(tc::conv3_tc_pipe_kernel<CIN, COUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-        return EL_ERR_CUDA;
-    if (cudaFuncSetAttribute(tc::conv3_tc_pipe_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             S::SMEM) != cudaSuccess)
-        return EL_ERR_CUDA;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc::conv3_tc_pipe_kernel<CIN, COUT>, tc::kThreads,
-                                                      S::SMEM) != cudaSuccess)
-        return EL_ERR_CUDA;
-    per_sm = std::max(per_sm, resident_per_sm(tc::kThreads, S::SMEM));
-    const long long bricks =
-        (long long)((a->nx + tc::TX - 1) / tc::TX) * ((a->ny + tc::TY - 1) / tc::TY) * a->nz;
-    const int grid = (int)std::max<long long>(1, std::min<long long>(bricks, (long long)num_sms_current() * per_sm));
-    tc::conv3_tc_pipe_kernel<CIN, COUT><<<grid, tc::kThreads, S::SMEM, s>>>(
-        a->nx, a->ny, a->nz, conv_in(a), static_cast<const uint4*>(a->weights_tc), a->bias, a->relu,
-        static_cast<__nv_bfloat16*>(a->out_a), a->out_a_channels, static_cast<__nv_bfloat16*>(a->out_b));
-    return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
-}
-
-template <int CIN, int COUT>
+template <int CIN, int COUT, int SC, int CTAS>
 int launch_conv_tc(const el_nn_conv_args* a, cudaStream_t s) {
-    if constexpr (tc::PipeShape<CIN, COUT>::FITS) return launch_conv_tc_pipe<CIN, COUT>(a, s);
-    using S = tc::Shape<CIN, COUT>;
-    // the largest shared-memory carve-out, so that the occupancy below (and the launch) get it
-    if (cudaFuncSetAttribute(tc::conv3_tc_kernel<CIN, COUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    using SS = tc::RunShape<CIN, COUT, SC, CTAS>;
+    if (cudaFuncSetAttribute(tc::conv3_tc_kernel<CIN, COUT, SC, CTAS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
         return EL_ERR_CUDA;
-    if (cudaFuncSetAttribute(tc::conv3_tc_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(tc::conv3_tc_kernel<CIN, COUT, SC, CTAS>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, SS::S::SMEM) != cudaSuccess)
         return EL_ERR_CUDA;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tc::conv3_tc_kernel<CIN, COUT>, tc::kThreads,
-                                                      S::SMEM) != cudaSuccess)
-        return EL_ERR_CUDA;
-    per_sm = std::max(per_sm, resident_per_sm(tc::kThreads, S::SMEM));
-    const long long bricks =
-        (long long)((a->nx + tc::TX - 1) / tc::TX) * ((a->ny + tc::TY - 1) / tc::TY) * a->nz;
-    const int grid = (int)std::max<long long>(1, std::min<long long>(bricks, (long long)num_sms_current() * per_sm));
-    tc::conv3_tc_kernel<CIN, COUT><<<grid, tc::kThreads, S::SMEM, s>>>(
+    const long long units = (long long)((a->nx + tc::TX - 1) / tc::TX) * ((a->ny + tc::TY - 1) / tc::TY) * a->nz;
+    const int grid = (int)std::min<long long>(units, (long long)num_sms_current() * CTAS);
+    tc::conv3_tc_kernel<CIN, COUT, SC, CTAS><<<grid, tc::kThreads, SS::S::SMEM, s>>>(
         a->nx, a->ny, a->nz, conv_in(a), static_cast<const uint4*>(a->weights_tc), a->bias, a->relu,
         static_cast<__nv_bfloat16*>(a->out_a), a->out_a_channels, static_cast<__nv_bfloat16*>(a->out_b));
     return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
@@ -1258,9 +1120,13 @@ int launch_wgrad(const el_nn_conv_args* a, const void* grad_out, float* dw, floa
 #define EL_NN_CONV_PAIRS(X)                                                                                      \
     X(16, 16) X(16, 32) X(32, 32) X(32, 64) X(64, 64) X(128, 64) X(96, 32) X(48, 16) X(32, 16) X(64, 32) X(64, 128) \
         X(32, 96) X(16, 48)
-// pairs whose 27 taps of weights fit in shared memory with the input brick: the tcgen05 kernel
-#define EL_NN_TC_PAIRS(X) \
-    X(16, 16) X(16, 32) X(32, 32) X(32, 64) X(48, 16) X(32, 16) X(64, 32) X(16, 48) X(32, 96)
+// the same on the tcgen05 kernel: input channels a slice, resident CTAs an SM (the fastest of the
+// combinations that fit, over the layers' grids; e.g. 32 -> 32 at 64^3 in slices of 16, three CTAs: 41 us
+// against 31; 96 -> 32 in slices of 16, three CTAs: 100 against 75; 64 -> 32 at 32^3: 22.7 against 18.6)
+#define EL_NN_TC_PAIRS(X)                                                                                    \
+    X(16, 16, 16, 4) X(16, 32, 16, 4) X(32, 32, 32, 2) X(32, 64, 32, 1) X(64, 64, 32, 1) X(128, 64, 32, 1)   \
+        X(96, 32, 32, 2) X(48, 16, 16, 4) X(32, 16, 32, 2) X(64, 32, 32, 2) X(64, 128, 16, 1) X(32, 96, 32, 1) \
+        X(16, 48, 16, 3)
 // forward pairs (backward weight)
 #define EL_NN_FWD_PAIRS(X) X(16, 16) X(16, 32) X(32, 32) X(32, 64) X(64, 64) X(128, 64) X(96, 32) X(48, 16)
 
@@ -1277,19 +1143,18 @@ bool valid_conv(const el_nn_conv_args* a) {
 #define EL_API extern "C" __attribute__((visibility("default")))
 
 EL_API int el_nn_tc_supported(int cin, int cout) {
-#define EL_NN_CASE(CI, CO) \
+#define EL_NN_CASE(CI, CO, SC, CTAS) \
     if (cin == CI && cout == CO) return 1;
     EL_NN_TC_PAIRS(EL_NN_CASE)
 #undef EL_NN_CASE
     return 0;
 }
 
-// pairs where the tcgen05 kernel measured faster than the mma.sync one on GB300 (128^3 network
-// grids): the small-cin layers; with cin >= 32 and cout <= 64 the persistent tcgen05 CTAs are
-// limited to one or two per SM by the staged weights and lose to the register-tiled kernel
-EL_API int el_nn_tc_preferred(int cin, int cout) {
-    return (cin == 16 && (cout == 16 || cout == 32 || cout == 48)) || (cin == 32 && cout == 96);
-}
+// Every pair: no layer of the network measured slower on the tcgen05 kernel than on the mma.sync one
+// (us, mma.sync / tcgen05: 16 -> 16 at 128^3 230 / 88, 48 -> 16 664 / 222, 16 -> 48 363 / 188; at 64^3
+// 32 -> 32 65 / 31, 96 -> 32 212 / 75; at 32^3 64 -> 64 34 / 21, 128 -> 64 106 / 33, 16 -> 32 10.5 / 8.4;
+// at 8^3 64 -> 64 29 / 13).
+EL_API int el_nn_tc_preferred(int cin, int cout) { return el_nn_tc_supported(cin, cout); }
 
 EL_API int el_nn_take_error(void) {
     int e = 0;
@@ -1304,8 +1169,8 @@ EL_API int el_nn_conv3_forward(const el_nn_conv_args* a, void* stream) {
         a->out_a_channels > 0 && a->out_a_channels <= a->cout && a->out_a_channels % 8 == 0 &&
         (a->out_a_channels == a->cout || a->out_b)) {
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-#define EL_NN_CASE(CI, CO) \
-        if (a->cin == CI && a->cout == CO) return launch_conv_tc<CI, CO>(a, s);
+#define EL_NN_CASE(CI, CO, SC, CTAS) \
+        if (a->cin == CI && a->cout == CO) return launch_conv_tc<CI, CO, SC, CTAS>(a, s);
         EL_NN_TC_PAIRS(EL_NN_CASE)
 #undef EL_NN_CASE
     }

@@ -404,13 +404,13 @@ size_t el_nn_packed_weight_bytes(int cin, int cout);
 int el_nn_pack_weights(int cin, int cout, const float* w, void* packed_fwd, void* packed_bwd, void* stream);
 /* The same weights in the tcgen05 kernel's shared-memory operand layout (27*cin*cout*2 bytes
  * each), forward and (if packed_bwd is not NULL) backward data.  el_nn_tc_supported(cin, cout)
- * says whether a (cin, cout) call can use them: (16,16) (16,32) (32,32) (32,64) (48,16) (32,16)
- * (64,32) (16,48) (32,96), the pairs whose 27 taps fit in shared memory with the input brick.
+ * says whether a (cin, cout) call can use them: every pair of the network, forward and backward
+ * data.
  * el_nn_take_error returns (and clears) 1 if a tcgen05 kernel's bounded wait for its MMAs gave
  * up, 0 otherwise, -1 if it could not be read. */
 int el_nn_pack_weights_tc(int cin, int cout, const float* w, void* packed_fwd, void* packed_bwd, void* stream);
 int el_nn_tc_supported(int cin, int cout);
-/* 1 where the tcgen05 kernel measured faster than the mma.sync one on GB300 (small cin) */
+/* 1 where the tcgen05 kernel measured no slower than the mma.sync one on GB300 (every pair) */
 int el_nn_tc_preferred(int cin, int cout);
 int el_nn_take_error(void);
 /* 2x2x2 average pooling; its backward is el_nn_spread(scale 1/8, accumulate 1) */

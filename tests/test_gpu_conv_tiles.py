@@ -1,7 +1,15 @@
-"""The weight-gradient kernel at the edges of its tiles, all channel pairs: grids smaller than a tile,
-ragged in x and y, of one plane, longer than a run.  References are float64 on bf16-representable
-inputs; products are exact, and the FP32 accumulation of n <= 6120 voxels adds at most (n / 16) * 2^-23:
-5e-5."""
+"""The weight-gradient and tcgen05 convolution kernels at the edges of their tiles, all channel pairs.
+
+Both stage a column of planes and work on a run of units: grids smaller than a tile, ragged in x and y,
+of one plane, longer than a run, and with more columns than blocks.  References are float64 on
+bf16-representable inputs.
+
+  - weight gradients (FP32 out): products are exact, at most (n / 16) * 2^-23 of accumulation for the
+    n <= 6120 voxels here: 5e-5;
+  - bf16 outputs, each element: half an ulp of rounding, 2^-8 |y| (8 significant bits), and the FP32
+    accumulation's 27 * 128 / 16 steps of 2^-23 max |y|, doubled: 5e-5 max |y|;
+  - tcgen05 against mma.sync on a large grid: FP32 sums in another order (< 2e-5 apart) round
+    differently in a share 2e-5 * 2^8 of the outputs, by 2^-8 each: 5e-4."""
 
 import ctypes as C
 
@@ -9,7 +17,7 @@ import numpy as np
 import pytest
 
 from conftest import rel_err
-from test_gpu_nn import _args, _rand, _ws, bf, dev, up2
+from test_gpu_nn import _args, _pack, _rand, _ws, bf, conv_ref, dev, up2
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +63,61 @@ def test_weight_gradient(cin, cout, shape, up):
     rw, rb = wgrad_ref(x, g * (y > 0))
     assert rel_err(dw.cpu().numpy(), rw.reshape(-1).numpy()) < 5e-5
     assert rel_err(db.cpu().numpy(), rb.numpy()) < 5e-5
+
+
+PAIRS = FWD + [(32, 16), (64, 32), (64, 128), (32, 96), (16, 48)]
+
+
+def _run_conv(W, shape, cin, cout, xd, w, bias, mask, split, tc):
+    L = W.lib()
+    nx, ny, nz = shape
+    fwd, _ = _pack(L, w.numpy(), cin, cout)
+    args = _args(W, shape, cin, cout, xd, cin, 0)
+    args.weights, args.relu = fwd.data_ptr(), 1 if bias is not None else 0
+    args.bias = bias.data_ptr() if bias is not None else None
+    args.mask = mask.data_ptr() if mask is not None else None
+    if tc:
+        pt = torch.empty_like(fwd)
+        wd = torch.from_numpy(w.numpy().astype(np.float32)).cuda()
+        assert L.el_nn_pack_weights_tc(cin, cout, wd.data_ptr(), pt.data_ptr(), None, None) == 0
+        args.weights_tc = pt.data_ptr()
+    out_a = torch.empty((nz, ny, nx, split), dtype=torch.bfloat16, device="cuda")
+    out_b = torch.empty((nz, ny, nx, cout - split), dtype=torch.bfloat16, device="cuda")
+    args.out_a, args.out_a_channels, args.out_b = out_a.data_ptr(), split, out_b.data_ptr()
+    assert L.el_nn_conv3_forward(C.byref(args), None) == 0
+    torch.cuda.synchronize()
+    assert L.el_nn_take_error() == 0
+    return torch.cat([out_a, out_b], 3)
+
+
+def _within_rounding(got, ref):
+    return bool(((got.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 5e-5 * ref.abs().max()).all())
+
+
+@pytest.mark.parametrize("cin,cout", PAIRS)
+@pytest.mark.parametrize("shape", SHAPES)
+def test_tcgen05_convolution(cin, cout, shape):
+    W = _ws()
+    assert W.lib().el_nn_tc_supported(cin, cout) == 1
+    nx, ny, nz = shape
+    rng = np.random.default_rng(cin + 3 * cout + nz)
+    x, m = bf(_rand(rng, nz, ny, nx, cin)), bf(_rand(rng, nz, ny, nx, cin))
+    w = bf(_rand(rng, cout, 27, cin, scale=(2.0 / (27 * cin)) ** 0.5))
+    bias = torch.from_numpy(_rand(rng, cout, scale=0.1))
+    xd, md = dev(x), dev(m)
+    got = _run_conv(W, shape, cin, cout, xd, w, bias.cuda(), None, cout - 8, True)
+    assert _within_rounding(got, torch.relu(conv_ref(x, w, bias.double())))
+    got = _run_conv(W, shape, cin, cout, xd, w, None, md, cout, True)
+    assert _within_rounding(got, conv_ref(x * (m > 0), w))
+
+
+@pytest.mark.parametrize("cin,cout", PAIRS)
+def test_tcgen05_convolution_more_units_than_a_wave(cin, cout):
+    W = _ws()
+    shape = (40, 33, 330)  # 4950 units in 15 columns: several runs a block, across columns
+    gen = torch.Generator(device="cuda").manual_seed(cin + cout)
+    xd = torch.randn((330, 33, 40, cin), device="cuda", generator=gen).to(torch.bfloat16)
+    w = bf(_rand(np.random.default_rng(cin), cout, 27, cin, scale=(2.0 / (27 * cin)) ** 0.5))
+    tc = _run_conv(W, shape, cin, cout, xd, w, None, None, cout, True).float()
+    mma = _run_conv(W, shape, cin, cout, xd, w, None, None, cout, False).float()
+    assert float((tc - mma).norm() / mma.norm()) < 5e-4
