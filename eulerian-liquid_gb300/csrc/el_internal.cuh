@@ -91,6 +91,7 @@ struct MGLevel {
     V* b = nullptr;
     V* x = nullptr;
     V* t = nullptr;
+    V* rd = nullptr;  // FP64: the reciprocal of the diagonal, 0 on empty rows
     SegList seg;
 };
 

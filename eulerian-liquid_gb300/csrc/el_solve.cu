@@ -59,6 +59,9 @@ constexpr int kDotThreads = sizeof(V) == 8 ? 1024 : 512;
 
 __device__ __forceinline__ bool finite_d(double v) { return isfinite(v); }
 
+__device__ __forceinline__ bool positive(float v) { return v > 0.f; }
+__device__ __forceinline__ bool positive(double v) { return d_positive(v); }  // on the integer pipe
+
 // ---------------------------------------------------------------------------------------
 // coefficient records
 
@@ -317,9 +320,13 @@ __global__ void pack32_kernel(long long n, const double* __restrict__ d, const O
 
 template <typename OT>
 __global__ void pack64_kernel(long long n, const double* __restrict__ d, const OT* __restrict__ ox,
-                              const OT* __restrict__ oy, const OT* __restrict__ oz, Rec64* __restrict__ a) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x)
-        a[c] = Rec64{d[c], (double)ox[c], (double)oy[c], (double)oz[c]};
+                              const OT* __restrict__ oy, const OT* __restrict__ oz, Rec64* __restrict__ a,
+                              double* __restrict__ rd) {
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
+        const double dc = d[c];
+        a[c] = Rec64{dc, (double)ox[c], (double)oy[c], (double)oz[c]};
+        rd[c] = positive(dc) ? 1.0 / dc : 0.0;
+    }
 }
 
 // Coarse records A_c = 1/2 P^T A P over 2x2x2 blocks.  The FP32 hierarchy (float4 coarse
@@ -327,7 +334,8 @@ __global__ void pack64_kernel(long long n, const double* __restrict__ d, const O
 // carry at most 24 significant bits, and FP64 arithmetic runs at a small fraction of the FP32
 // rate on this GPU -- the FP64 hierarchy in FP64.
 template <typename RF, typename RC>
-__global__ void coarsen_kernel(LGeom F, const RF* __restrict__ fr, LGeom C, RC* __restrict__ cr) {
+__global__ void coarsen_kernel(LGeom F, const RF* __restrict__ fr, LGeom C, RC* __restrict__ cr,
+                               double* __restrict__ rd) {
     using A = typename std::conditional<sizeof(RC) == sizeof(float4), float, double>::type;
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
@@ -352,8 +360,10 @@ __global__ void coarsen_kernel(LGeom F, const RF* __restrict__ fr, LGeom C, RC* 
     const long long q = I + C.s1 * J + C.s2 * K;
     if constexpr (sizeof(RC) == sizeof(float4))
         cr[q] = make_float4(dc, A(0.5) * sx, A(0.5) * sy, A(0.5) * sz);
-    else
+    else {
         cr[q] = Rec64{dc, 0.5 * sx, 0.5 * sy, 0.5 * sz};
+        rd[q] = positive(dc) ? 1.0 / dc : 0.0;
+    }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -491,8 +501,6 @@ struct SplitLoad {
     }
 };
 
-__device__ __forceinline__ bool positive(float v) { return v > 0.f; }
-__device__ __forceinline__ bool positive(double v) { return d_positive(v); }  // on the integer pipe
 
 // K1: new direction fused with A p and p.Ap over the active segments (record operator: FP32 inner
 // system, FP64 multigrid).
@@ -536,11 +544,12 @@ __global__ void __launch_bounds__(kDotThreads<V>) dir_spmv_rec_kernel(LGeom g, S
     }
 }
 
-// K2: x += alpha p ; r -= alpha Ap ; |r|^2.
+// K2: x += alpha p ; r -= alpha Ap ; |r|^2; FP64 also t = the V-cycle's first sweep from zero.
 template <typename V>
 __global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg seg, V* __restrict__ x,
                                                                 V* __restrict__ r, const V* __restrict__ p,
-                                                                const V* __restrict__ ap, Scalars* s,
+                                                                const V* __restrict__ ap, V* __restrict__ t,
+                                                                const V* __restrict__ rd, Scalars* s,
                                                                 double* partials, unsigned* counter) {
     pdl_wait();
     pdl_trigger();
@@ -557,6 +566,7 @@ __global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg 
         const V rc = rc0 - alpha * apc;
         x[c] = xc + alpha * pc;
         r[c] = rc;
+        if (sizeof(V) == 8) t[c] = rn_mul(rn_mul(V(kSweep1), rc), rd[c]);
         part += (DotAcc<V>)rc * (DotAcc<V>)rc;
     };
     for (int qs = warp_global; qs < nseg; qs += 2 * nwarps) {
@@ -881,6 +891,14 @@ __global__ void solve_init_kernel(LGeom g, SegArg seg, const double* __restrict_
     }
 }
 
+// the FP64 V-cycle's first sweep from zero for the first residual (later ones: update_kernel)
+__global__ void first_sweep_kernel(LGeom g, SegArg seg, const double* __restrict__ r, const double* __restrict__ rd,
+                                   double* __restrict__ t) {
+    SEG_LOOP_BEGIN(seg, g)
+    t[c] = rn_mul(rn_mul(kSweep1, r[c]), rd[c]);
+    SEG_LOOP_END
+}
+
 // ---- warm start: x0 = alpha g with g the pressure grid as it stands --------------------
 // x = g on fluid cells (0 elsewhere); the residual kernel then gives r0 = b - A g.
 template <typename T>
@@ -1158,21 +1176,22 @@ __global__ void __launch_bounds__(kSegThreads, 4) residual_df_kernel(LGeom g, Se
 // ---------------------------------------------------------------------------------------
 // multigrid smoothing over the active segments of one level
 //
-// MODE 0: two sweeps from x = 0 (the first, omega b / D, formed on the fly)
+// MODE 0: two sweeps from x = 0 (the first, omega b / D, formed on the fly; FP32)
 // MODE 1: one sweep from x_in + P e (e = coarse correction, formed on the fly)
 // MODE 2: one sweep from x_in.   DOT (finest level, last sweep): rz = b . x_out and beta.
+//
+// In FP64 these kernels are bound by the FP64 pipe (2 lanes a clock per SM; a division costs about nine
+// of its operations, a comparison one), so nothing in a sweep divides or compares there: the
+// reciprocals of the diagonal are taken once a solve (rd), the sign of a diagonal is read as an
+// integer, and the first sweep from zero is stored by the kernel that forms b (update_kernel on the
+// finest level, the restrictions below), not divided out at every point of the second sweep's stencil.
+// 128^3 pool, finest level: second sweep from zero 97 -> 17 us (reads t), prolongation sweep 40 -> 23,
+// last sweep 38 -> 21.
 enum { SM_ZERO2 = 0, SM_PROLONG = 1, SM_PLAIN = 2 };
 
-// a / b inside the multigrid preconditioner: FP32 takes the fast division (within 2 ulp; the
-// preconditioner only has to be a fixed symmetric operator, not correctly rounded), FP64 the
-// exact one
-template <typename V>
-__device__ __forceinline__ V mg_div(V a, V b) {
-    if constexpr (sizeof(V) == 4)
-        return __fdividef(a, b);
-    else
-        return a / b;
-}
+// a / d inside the FP32 multigrid preconditioner: the fast division (within 2 ulp; the preconditioner
+// only has to be a fixed symmetric operator, not correctly rounded)
+__device__ __forceinline__ float mg_div(float a, float d) { return __fdividef(a, d); }
 enum { DOT_NONE = 0, DOT_INIT = 1, DOT_BETA = 2 };
 
 // A value of an iterate or right-hand side.  COH: through L2 only (ld.global.cg), for arrays
@@ -1193,8 +1212,9 @@ template <typename V, typename R, int MODE, int DOT, bool COH = false>
 __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegArg& seg, const R* __restrict__ A,
                                                      const V* __restrict__ b, const V* __restrict__ x_in,
                                                      const LGeom& gc, const V* __restrict__ e, V* __restrict__ x_out,
-                                                     int wg, int nw) {
-    const V w_first = V(kSweep1);
+                                                     const V* __restrict__ rd, int wg, int nw) {
+    static_assert(sizeof(V) == 4 || MODE != SM_ZERO2, "FP64 stores the first sweep");
+    [[maybe_unused]] const V w_first = V(kSweep1);
     const V omega = V(MODE == SM_PROLONG ? kSweep1 : kSweep2);
     DotAcc<V> part = 0;
     const RecLoad<V, R> recf{A};
@@ -1206,15 +1226,22 @@ __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegAr
         return v;
     };
     auto valf = [&](V raw, const Co<V>& rec) -> V {
-        if (!(rec.d > V(0))) return V(0);
-        return MODE == SM_ZERO2 ? mg_div(rn_mul(w_first, raw), rec.d) : raw;
+        if (!positive(rec.d)) return V(0);
+        if constexpr (MODE == SM_ZERO2) return mg_div(rn_mul(w_first, raw), rec.d);
+        return raw;
     };
     SEG_LOOP_ALL_W_BEGIN(seg, g, wg, nw)
     const St7<V> st = gather7<V, true>(g, c, i, j, k, live, lane, recf, rawf, valf);
     if (live) {
-        const V bc = ldv<COH>(b, c);
+        const V bc = ldv<COH>(b, c), rc = sizeof(V) == 8 ? rd[c] : V(0);
         V xo = V(0);
-        if (st.d > V(0)) xo = rn_add(st.v0, mg_div(rn_mul(omega, rn_sub(bc, apply7(st))), st.d));
+        if (positive(st.d)) {
+            const V q = rn_mul(omega, rn_sub(bc, apply7(st)));
+            if constexpr (sizeof(V) == 8)
+                xo = rn_fma(q, rc, st.v0);
+            else
+                xo = rn_add(st.v0, mg_div(q, st.d));
+        }
         if (EL_IN(c, (long long)g.s2 * g.n2, 30)) x_out[c] = xo;
         if (DOT != DOT_NONE) part += (DotAcc<V>)bc * (DotAcc<V>)xo;
     }
@@ -1226,12 +1253,12 @@ template <typename V, typename R, int MODE, int DOT>
 __global__ void __launch_bounds__(kSegThreads) smooth_kernel(LGeom g, SegArg seg, const R* __restrict__ A,
                                                              const V* __restrict__ b, const V* __restrict__ x_in,
                                                              LGeom gc, const V* __restrict__ e,
-                                                             V* __restrict__ x_out, Scalars* s, double* partials,
-                                                             unsigned* counter) {
+                                                             V* __restrict__ x_out, const V* __restrict__ rd,
+                                                             Scalars* s, double* partials, unsigned* counter) {
     pdl_wait();
     pdl_trigger();
     if (s->done) return;
-    const DotAcc<V> part = smooth_segments<V, R, MODE, DOT>(g, seg, A, b, x_in, gc, e, x_out,
+    const DotAcc<V> part = smooth_segments<V, R, MODE, DOT>(g, seg, A, b, x_in, gc, e, x_out, rd,
                                                             (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
                                                             (gridDim.x * blockDim.x) >> 5);
     if (DOT != DOT_NONE) {
@@ -1255,7 +1282,8 @@ __global__ void __launch_bounds__(kSegThreads) smooth_kernel(LGeom g, SegArg seg
 template <typename V, typename R>
 __global__ void __launch_bounds__(kSegThreads, sizeof(V) == 4 ? 5 : 4) restrict_kernel(LGeom g, const R* __restrict__ A, const V* __restrict__ b,
                                                                const V* __restrict__ x, LGeom gc, SegArg cseg,
-                                                               V* __restrict__ bc, const Scalars* s) {
+                                                               V* __restrict__ bc, V* __restrict__ tc,
+                                                               const V* __restrict__ rdc, const Scalars* s) {
     if (s->done) return;
     const RecLoad<V, R> recf{A};
     auto rawf = [&](int q, int, int, int) -> V { return x[q]; };
@@ -1281,15 +1309,18 @@ __global__ void __launch_bounds__(kSegThreads, sizeof(V) == 4 ? 5 : 4) restrict_
                     const bool live = i < g.n0;
                     const int c = i + g.s1 * j + g.s2 * k;
                     const St7<V> st = gather7<V, false>(g, c, i, j, k, live, lane, recf, rawf, valf);
-                    if (live && st.d > V(0)) sum[h] += rn_sub(b[c], apply7(st));
+                    if (live && positive(st.d)) sum[h] += rn_sub(b[c], apply7(st));
                 }
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const V pair = sum[h] + __shfl_down_sync(kFull, sum[h], 1);
             const int I = I0 + 16 * h + (lane >> 1);
-            if ((lane & 1) == 0 && I < gc.n0 && EL_IN(I + gc.s1 * J + gc.s2 * K, (long long)gc.s2 * gc.n2, 31))
-                bc[I + gc.s1 * J + gc.s2 * K] = pair;
+            const int q = I + gc.s1 * J + gc.s2 * K;
+            if ((lane & 1) == 0 && I < gc.n0 && EL_IN(q, (long long)gc.s2 * gc.n2, 31)) {
+                bc[q] = pair;
+                if (sizeof(V) == 8) tc[q] = rn_mul(rn_mul(V(kSweep1), pair), rdc[q]);
+            }
         }
     }
 }
@@ -1308,7 +1339,7 @@ template <typename V, typename R, bool COH = false>
 __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* __restrict__ A,
                                                        const V* __restrict__ b, const V* __restrict__ x,
                                                        const LGeom& gc, const SegArg& cseg, V* __restrict__ bc,
-                                                       V (*part)[4][2][16], int quad, int nquads, int quad_b,
+                                                       V* __restrict__ tc, const V* __restrict__ rdc, V (*part)[4][2][16], int quad, int nquads, int quad_b,
                                                        int sub) {
     const RecLoad<V, R> recf{A};
     auto rawf = [&](int q, int, int, int) -> V { return ldv<COH>(x, q); };
@@ -1329,7 +1360,7 @@ __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* 
                 const bool live = i < g.n0;
                 const int c = i + g.s1 * j + g.s2 * k;
                 const St7<V> st = gather7<V, false>(g, c, i, j, k, live, lane, recf, rawf, valf);
-                if (live && st.d > V(0)) sum[h] = rn_sub(ldv<COH>(b, c), apply7(st));
+                if (live && positive(st.d)) sum[h] = rn_sub(ldv<COH>(b, c), apply7(st));
             }
         }
 #pragma unroll
@@ -1344,8 +1375,11 @@ __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* 
             const V tot = ((part[quad_b][0][h][q] + part[quad_b][1][h][q]) + part[quad_b][2][h][q]) +
                           part[quad_b][3][h][q];
             const int I = I0 + 16 * h + q;
-            if (I < gc.n0 && EL_IN(I + gc.s1 * J + gc.s2 * K, (long long)gc.s2 * gc.n2, 32))
-                bc[I + gc.s1 * J + gc.s2 * K] = tot;
+            const int o = I + gc.s1 * J + gc.s2 * K;
+            if (I < gc.n0 && EL_IN(o, (long long)gc.s2 * gc.n2, 32)) {
+                bc[o] = tot;
+                if (sizeof(V) == 8) tc[o] = rn_mul(rn_mul(V(kSweep1), tot), rdc[o]);
+            }
         }
         asm volatile("bar.sync %0, %1;" ::"r"(1 + quad_b), "r"(128) : "memory");
     }
@@ -1355,6 +1389,7 @@ template <typename V, typename R>
 __global__ void __launch_bounds__(kSegThreads, 4) restrict_quad_kernel(LGeom g, const R* __restrict__ A,
                                                                     const V* __restrict__ b, const V* __restrict__ x,
                                                                     LGeom gc, SegArg cseg, V* __restrict__ bc,
+                                                                    V* __restrict__ tc, const V* __restrict__ rdc,
                                                                     const Scalars* s) {
     pdl_wait();
     pdl_trigger();
@@ -1362,58 +1397,84 @@ __global__ void __launch_bounds__(kSegThreads, 4) restrict_quad_kernel(LGeom g, 
     __shared__ V part[kQuadsPerBlock][4][2][16];
     const int wb = threadIdx.x >> 5;                  // warp in the block
     const int quad_b = wb >> 2, sub = wb & 3;         // quad in the block, row of the quad
-    restrict_quad_segments<V, R>(g, A, b, x, gc, cseg, bc, part, blockIdx.x * kQuadsPerBlock + quad_b,
+    restrict_quad_segments<V, R>(g, A, b, x, gc, cseg, bc, tc, rdc, part, blockIdx.x * kQuadsPerBlock + quad_b,
                                  gridDim.x * kQuadsPerBlock, quad_b, sub);
 }
 
 
-// Coarsest level: omega-Jacobi sweeps from zero in one block's shared memory.
+// Coarsest level: omega-Jacobi sweeps from zero in one block's shared memory, a thread a cell, its
+// row in registers.  In FP64 the row is scaled by omega / D beforehand, which leaves a sweep seven
+// multiply-adds (the FP64 pipe of one SM bounds it): 512 cells 38 -> 21 us
 template <typename V, typename R>
 __global__ void __launch_bounds__(kCoarsestMaxCells) coarsest_kernel(LGeom g, const R* __restrict__ A,
                                                                      const V* __restrict__ b, V* __restrict__ x,
-                                                                     int sweeps, const Scalars* s) {
+                                                                     const V* __restrict__ rd, int sweeps,
+                                                                     const Scalars* s) {
     if (s->done) return;
-    __shared__ V sd[kCoarsestMaxCells], sx[kCoarsestMaxCells], sy[kCoarsestMaxCells], sz[kCoarsestMaxCells];
-    __shared__ V sb[kCoarsestMaxCells], xa[kCoarsestMaxCells], xb[kCoarsestMaxCells];
+    __shared__ V xs[2][kCoarsestMaxCells];
     const int n = g.n0 * g.n1 * g.n2;
     const int c = threadIdx.x;
     const V omega = V(kOmega);
-    if (c < n) {
-        const auto r = ldrec(A, c);
-        sd[c] = (V)r.d;
-        sx[c] = (V)r.x;
-        sy[c] = (V)r.y;
-        sz[c] = (V)r.z;
-        sb[c] = b[c];
-        xa[c] = sd[c] > V(0) ? mg_div(rn_mul(omega, sb[c]), sd[c]) : V(0);
-    }
-    __syncthreads();
     const int i = c % g.n0, j = (c / g.n0) % g.n1, k = c / (g.n0 * g.n1);
     const int s1 = g.n0, s2 = g.n0 * g.n1;
-    V* cur = xa;
-    V* nxt = xb;
-    for (int it = 1; it < sweeps; ++it) {
-        if (c < n) {
-            V xo = V(0);
-            const V d = sd[c];
-            if (d > V(0)) {
-                V a = rn_mul(d, cur[c]);
-                if (i > 0) a = rn_fma(sx[c - 1], cur[c - 1], a);
-                if (i < g.n0 - 1) a = rn_fma(sx[c], cur[c + 1], a);
-                if (j > 0) a = rn_fma(sy[c - s1], cur[c - s1], a);
-                if (j < g.n1 - 1) a = rn_fma(sy[c], cur[c + s1], a);
-                if (k > 0) a = rn_fma(sz[c - s2], cur[c - s2], a);
-                if (k < g.n2 - 1) a = rn_fma(sz[c], cur[c + s2], a);
-                xo = rn_add(cur[c], mg_div(rn_mul(omega, rn_sub(sb[c], a)), d));
-            }
-            nxt[c] = xo;
-        }
-        __syncthreads();
-        V* t = cur;
-        cur = nxt;
-        nxt = t;
+    const Co<V> z4{V(0), V(0), V(0), V(0)};
+    auto rec = [&](bool in, int q) -> Co<V> {
+        if (!in) return z4;
+        const auto r = ldrec(A, q);
+        return Co<V>{(V)r.d, (V)r.x, (V)r.y, (V)r.z};
+    };
+    const bool in = c < n;
+    const Co<V> r0 = rec(in, c);
+    const bool act = positive(r0.d);
+    const bool hxm = act && i > 0, hxp = act && i < g.n0 - 1, hym = act && j > 0, hyp = act && j < g.n1 - 1;
+    const bool hzm = act && k > 0, hzp = act && k < g.n2 - 1;
+    V cxm = rec(hxm, c - 1).x, cym = rec(hym, c - s1).y, czm = rec(hzm, c - s2).z;
+    V cxp = hxp ? r0.x : V(0), cyp = hyp ? r0.y : V(0), czp = hzp ? r0.z : V(0);
+    // an absent neighbour: coefficient 0 at the cell itself
+    const int qxm = hxm ? c - 1 : c, qxp = hxp ? c + 1 : c, qym = hym ? c - s1 : c, qyp = hyp ? c + s1 : c;
+    const int qzm = hzm ? c - s2 : c, qzp = hzp ? c + s2 : c;
+    V bc = in ? b[c] : V(0);
+    V x0 = V(0);
+    if constexpr (sizeof(V) == 8) {
+        const V w = act ? rn_mul(omega, rd[c]) : V(0);
+        cxm = rn_mul(cxm, -w);
+        cxp = rn_mul(cxp, -w);
+        cym = rn_mul(cym, -w);
+        cyp = rn_mul(cyp, -w);
+        czm = rn_mul(czm, -w);
+        czp = rn_mul(czp, -w);
+        x0 = bc = rn_mul(bc, w);
+    } else {
+        if (act) x0 = mg_div(rn_mul(omega, bc), r0.d);
     }
-    if (c < n) x[c] = cur[c];
+    xs[0][c] = x0;
+    __syncthreads();
+    for (int it = 1; it < sweeps; ++it) {
+        const V* cur = xs[(it - 1) & 1];
+        if (act) {
+            if constexpr (sizeof(V) == 8) {
+                V a = rn_fma(V(1.0 - kOmega), x0, bc);
+                a = rn_fma(cxm, cur[qxm], a);
+                a = rn_fma(cxp, cur[qxp], a);
+                a = rn_fma(cym, cur[qym], a);
+                a = rn_fma(cyp, cur[qyp], a);
+                a = rn_fma(czm, cur[qzm], a);
+                x0 = rn_fma(czp, cur[qzp], a);
+            } else {
+                V a = rn_mul(r0.d, x0);
+                if (hxm) a = rn_fma(cxm, cur[qxm], a);
+                if (hxp) a = rn_fma(cxp, cur[qxp], a);
+                if (hym) a = rn_fma(cym, cur[qym], a);
+                if (hyp) a = rn_fma(cyp, cur[qyp], a);
+                if (hzm) a = rn_fma(czm, cur[qzm], a);
+                if (hzp) a = rn_fma(czp, cur[qzp], a);
+                x0 = rn_add(x0, mg_div(rn_mul(omega, rn_sub(bc, a)), r0.d));
+            }
+        }
+        xs[it & 1][c] = x0;
+        __syncthreads();
+    }
+    if (in) x[c] = x0;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1714,10 +1775,10 @@ __global__ void __launch_bounds__(kBottomThreads, 1) mg_coarse_cycle_kernel(cons
     for (int l = a.from; l < a.pre_end; ++l) {
         const CoarseLevel& F = a.lv[l];
         const CoarseLevel& C = a.lv[l + 1];
-        smooth_segments<float, float4, SM_ZERO2, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, nullptr, F.g, nullptr, F.x,
+        smooth_segments<float, float4, SM_ZERO2, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, nullptr, F.g, nullptr, F.x, nullptr,
                                                                  wg, nw);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
-        restrict_quad_segments<float, float4, true>(F.g, F.rec, F.b, F.x, C.g, C.seg, C.b, part, quad, nquads,
+        restrict_quad_segments<float, float4, true>(F.g, F.rec, F.b, F.x, C.g, C.seg, C.b, nullptr, nullptr, part, quad, nquads,
                                                     quad_b, sub);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
     }
@@ -1730,10 +1791,10 @@ __global__ void __launch_bounds__(kBottomThreads, 1) mg_coarse_cycle_kernel(cons
         const CoarseLevel& F = a.lv[l];
         const CoarseLevel& C = a.lv[l + 1];
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
-        smooth_segments<float, float4, SM_PROLONG, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, F.x, C.g, C.x, F.t, wg,
+        smooth_segments<float, float4, SM_PROLONG, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, F.x, C.g, C.x, F.t, nullptr, wg,
                                                                    nw);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
-        smooth_segments<float, float4, SM_PLAIN, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, F.t, F.g, nullptr, F.x, wg,
+        smooth_segments<float, float4, SM_PLAIN, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, F.t, F.g, nullptr, F.x, nullptr, wg,
                                                                  nw);
     }
 }
@@ -1835,7 +1896,8 @@ static int build_hierarchy(el_ctx* ctx, std::vector<MGLevel<V>>& mg, size_t coar
     L0.n2 = ctx->nk;
     const long long n = (long long)ctx->ni * ctx->nj * ctx->nk;
     L0.t = (V*)ctx_alloc(ctx, n * sizeof(V));
-    if (!L0.t) return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "multigrid");
+    if (sizeof(V) == 8) L0.rd = (V*)ctx_alloc(ctx, n * sizeof(V));
+    if (!L0.t || (sizeof(V) == 8 && !L0.rd)) return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "multigrid");
     mg.push_back(L0);
     while (std::max(mg.back().n0, std::max(mg.back().n1, mg.back().n2)) > kCoarsestMaxDim) {
         MGLevel<V> C;
@@ -1847,7 +1909,8 @@ static int build_hierarchy(el_ctx* ctx, std::vector<MGLevel<V>>& mg, size_t coar
         C.b = (V*)ctx_alloc(ctx, m * sizeof(V));
         C.x = (V*)ctx_alloc(ctx, m * sizeof(V));
         C.t = (V*)ctx_alloc(ctx, m * sizeof(V));
-        if (!C.rec || !C.b || !C.x || !C.t) return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "multigrid");
+        if (sizeof(V) == 8) C.rd = (V*)ctx_alloc(ctx, m * sizeof(V));
+        if (!C.rec || !C.b || !C.x || !C.t || (sizeof(V) == 8 && !C.rd)) return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "multigrid");
         int rc = alloc_seglist(ctx, C.seg, C.n0, C.n1, C.n2);
         if (rc != EL_OK) return rc;
         mg.push_back(C);
@@ -1869,9 +1932,9 @@ static int enqueue_coarsen(el_ctx* ctx, std::vector<MGLevel<V>>& mg) {
             ProfScope prof(ctx, EL_KC_MG_COARSE, (double)F.n0 * F.n1 * F.n2 * (l == 0 ? sizeof(R0) : sizeof(RC)) +
                                                      (double)C.n0 * C.n1 * C.n2 * sizeof(RC));
             if (l == 0)
-                coarsen_kernel<R0, RC><<<grid, block, 0, ctx->stream>>>(gf, (const R0*)F.rec, gc, (RC*)C.rec);
+                coarsen_kernel<R0, RC><<<grid, block, 0, ctx->stream>>>(gf, (const R0*)F.rec, gc, (RC*)C.rec, (double*)C.rd);
             else
-                coarsen_kernel<RC, RC><<<grid, block, 0, ctx->stream>>>(gf, (const RC*)F.rec, gc, (RC*)C.rec);
+                coarsen_kernel<RC, RC><<<grid, block, 0, ctx->stream>>>(gf, (const RC*)F.rec, gc, (RC*)C.rec, (double*)C.rd);
         }
         launched += 1 + enqueue_seglist_rec<RC>(ctx, C.seg, gc, (const RC*)C.rec);
     }
@@ -1886,7 +1949,7 @@ static void launch_smooth(el_ctx* ctx, const MGLevel<V>& F, const SegList& seg, 
     const int blocks = one_wave(ctx, smooth_kernel<V, R, MODE, DOT>, kSegThreads, seg_blocks(ctx, seg.total));
     launch_dependent(ctx, smooth_kernel<V, R, MODE, DOT>, dim3(blocks), dim3(kSegThreads), 0, g,
                      seg_arg(seg), (const R*)F.rec, (const V*)F.b, x_in, gc, C ? (const V*)C->x : (const V*)nullptr,
-                     x_out, s, ctx->partials, ctx->counter);
+                     x_out, (const V*)F.rd, s, ctx->partials, ctx->counter);
 }
 
 // The coarse part of an FP32 V-cycle, levels [from, pre_end) and the bottom pair, as one
@@ -1942,7 +2005,7 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
         // too small to coarsen: the coarsest sweeps solve it, one more sweep gives the dot
         MGLevel<V>& C = mg[0];
         coarsest_kernel<V, R0><<<1, kCoarsestMaxCells, 0, ctx->stream>>>(make_geom(C.n0, C.n1, C.n2), (const R0*)C.rec,
-                                                                         C.b, C.t, kCoarsestSweeps, s);
+                                                                         C.b, C.t, C.rd, kCoarsestSweeps, s);
         if (dot == DOT_INIT)
             launch_smooth<V, R0, SM_PLAIN, DOT_INIT>(ctx, C, seg0, C.t, nullptr, C.x, s);
         else
@@ -1970,12 +2033,15 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
         MGLevel<V>& C = mg[l + 1];
         const double rb = l == 0 ? sizeof(R0) : sizeof(RC);
         {
-            // reads b and records; writes x
-            ProfScope prof(ctx, l == 0 ? EL_KC_SMOOTH : EL_KC_MG_COARSE, act(l, F) * (2 * vs + rb));
+            // reads b and records (FP64: t and rd); writes x
+            ProfScope prof(ctx, l == 0 ? EL_KC_SMOOTH : EL_KC_MG_COARSE, act(l, F) * ((vs == 8 ? 4 : 2) * vs + rb));
+            // the two sweeps from zero; FP64: the first is in t already
+            constexpr int mode = sizeof(V) == 8 ? SM_PLAIN : SM_ZERO2;
+            const V* first = sizeof(V) == 8 ? F.t : nullptr;
             if (l == 0)
-                launch_smooth<V, R0, SM_ZERO2, DOT_NONE>(ctx, F, segof(l), nullptr, nullptr, F.x, s);
+                launch_smooth<V, R0, mode, DOT_NONE>(ctx, F, segof(l), first, nullptr, F.x, s);
             else
-                launch_smooth<V, RC, SM_ZERO2, DOT_NONE>(ctx, F, segof(l), nullptr, nullptr, F.x, s);
+                launch_smooth<V, RC, mode, DOT_NONE>(ctx, F, segof(l), first, nullptr, F.x, s);
         }
         {
             // reads b, x and records; writes the coarse b
@@ -1983,13 +2049,13 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
             const LGeom gf = make_geom(F.n0, F.n1, F.n2), gc = make_geom(C.n0, C.n1, C.n2);
             if (l == 0)
                 restrict_kernel<V, R0><<<restrict_blocks(ctx, C.seg.total), kSegThreads, 0, ctx->stream>>>(
-                    gf, (const R0*)F.rec, F.b, F.x, gc, seg_arg(C.seg), C.b, s);
+                    gf, (const R0*)F.rec, F.b, F.x, gc, seg_arg(C.seg), C.b, C.t, C.rd, s);
             else
                 launch_dependent(ctx, restrict_quad_kernel<V, RC>,
                                  dim3(one_wave(ctx, restrict_quad_kernel<V, RC>, kSegThreads,
                                                seg_blocks(ctx, 4 * C.seg.total))),
                                  dim3(kSegThreads), 0, gf, (const RC*)F.rec, (const V*)F.b, (const V*)F.x, gc,
-                                 seg_arg(C.seg), C.b, (const Scalars*)s);
+                                 seg_arg(C.seg), C.b, C.t, (const V*)C.rd, (const Scalars*)s);
         }
         launched += 2;
     }
@@ -2019,7 +2085,7 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
         MGLevel<V>& C = mg[L - 1];
         ProfScope prof(ctx, EL_KC_MG_COARSE, cells(C) * (3 * vs + sizeof(RC)));
         coarsest_kernel<V, RC><<<1, kCoarsestMaxCells, 0, ctx->stream>>>(make_geom(C.n0, C.n1, C.n2), (const RC*)C.rec,
-                                                                         C.b, C.x, kCoarsestSweeps, s);
+                                                                         C.b, C.x, C.rd, kCoarsestSweeps, s);
         ++launched;
     }
     for (int l = down_end - 1; l >= from; --l) {
@@ -2142,7 +2208,8 @@ static int enqueue_mg_iteration(el_ctx* ctx, const RA* A, V* x, V* r, V* z, V*& 
         ProfScope prof(ctx, EL_KC_UPDATE, N * vs * 6);
         auto kernel = update_kernel<V>;
         launch_dependent(ctx, kernel, dim3(dot_blocks<V>(ctx, kernel, seg.total)), dim3(kDotThreads<V>), 0, g,
-                         seg_arg(seg), x, r, (const V*)p, (const V*)ap, s, ctx->partials, ctx->counter);
+                         seg_arg(seg), x, r, (const V*)p, (const V*)ap, mg[0].t, (const V*)mg[0].rd, s, ctx->partials,
+                         ctx->counter);
     }
     return 2 + enqueue_vcycle<V, R0, RC>(ctx, mg, seg, s, DOT_BETA);
 }
@@ -2349,11 +2416,14 @@ static int solve_t(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st) 
         mg[0].rec = ctx->A64rec;
         mg[0].b = ctx->r64;
         mg[0].x = ctx->z64;
-        pack64_kernel<T><<<grid1d(ctx, n), 256, 0, ctx->stream>>>(n, ctx->diag64, A64.x, A64.y, A64.z, ctx->A64rec);
+        pack64_kernel<T><<<grid1d(ctx, n), 256, 0, ctx->stream>>>(n, ctx->diag64, A64.x, A64.y, A64.z, ctx->A64rec,
+                                                                  mg[0].rd);
         ctx->launches += 1 + enqueue_coarsen<double, Rec64, Rec64>(ctx, mg);
         rc = record_active(ctx, ctx->seg0, ctx->ni, &mg);
         if (rc != EL_OK) return rc;
-        ctx->launches += enqueue_vcycle<double, Rec64, Rec64>(ctx, mg, ctx->seg0, s0, DOT_INIT);
+        first_sweep_kernel<<<seg_blocks(ctx, ctx->seg0.total), kSegThreads, 0, ctx->stream>>>(
+            g, seg_arg(ctx->seg0), ctx->r64, mg[0].rd, mg[0].t);
+        ctx->launches += 1 + enqueue_vcycle<double, Rec64, Rec64>(ctx, mg, ctx->seg0, s0, DOT_INIT);
         double* p = ctx->p64;
         double* p_alt = ctx->p64b;
         rc = run_iterations(ctx, EL_SOLVER_MG_FP64, 0, prm.max_iter, check, h, [&](int first, int, bool) {
