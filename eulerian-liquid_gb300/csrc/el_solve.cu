@@ -511,27 +511,42 @@ __global__ void __launch_bounds__(kDotThreads<V>) dir_spmv_rec_kernel(LGeom g, S
                                                                       V* __restrict__ p_out, V* __restrict__ ap,
                                                                       Scalars* s, int first, double* partials,
                                                                       unsigned* counter) {
+    const RecLoad<V, R> recf{A};
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    int qs = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nseg = *seg.count;
+    int4 sd = qs < nseg ? seg.desc[qs] : make_int4(0, g.n0, 0, 0);
+    Near7 nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+    Rec7<V> rec = load_rec7<V, false>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
     pdl_wait();
     pdl_trigger();
     if (s->done) return;
     const V beta = first ? V(0) : (V)s->beta;
     DotAcc<V> part = 0;
-    const RecLoad<V, R> recf{A};
     auto rawf = [&](int q, int, int, int) -> V { return first ? z[q] : z[q] + beta * p_in[q]; };
     auto valf = [](V raw, const Co<V>&) -> V { return raw; };
-    SEG_LOOP_ALL_PF_BEGIN(seg, g)
-    const St7<V> st = gather7<V, false>(g, c, i, j, k, live, lane, recf, rawf, valf);
-    if (live) {
-        V pc = V(0), apc = V(0);
-        if (positive(st.d)) {
-            pc = st.v0;
-            apc = apply7(st);
+    while (qs < nseg) {
+        const bool live = sd.y + lane < g.n0;
+        const int c = sd.x + lane;
+        const auto raw = load_raw7(g, nb, c, 0, 0, 0, live, rawf);
+        const St7<V> st = value7<V>(nb, rec, raw, live, lane, valf);
+        qs += nwarps;
+        if (qs < nseg) sd = seg.desc[qs];
+        if (live) {
+            V pc = V(0), apc = V(0);
+            if (positive(st.d)) {
+                pc = st.v0;
+                apc = apply7(st);
+            }
+            p_out[c] = pc;
+            ap[c] = apc;
+            part += (DotAcc<V>)pc * (DotAcc<V>)apc;
         }
-        p_out[c] = pc;
-        ap[c] = apc;
-        part += (DotAcc<V>)pc * (DotAcc<V>)apc;
+        if (qs >= nseg) break;
+        nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+        rec = load_rec7<V, false>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
     }
-    SEG_LOOP_END
     double acc[1] = {(double)part};
     double tot[1];
     if (grid_sum<1, kDotThreads<V>>(acc, partials, counter, tot)) {
@@ -551,17 +566,20 @@ __global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg 
                                                                 const V* __restrict__ ap, V* __restrict__ t,
                                                                 const V* __restrict__ rd, Scalars* s,
                                                                 double* partials, unsigned* counter) {
-    pdl_wait();
-    pdl_trigger();
-    if (s->done) return;
-    const V alpha = (V)s->alpha;
-    DotAcc<V> part = 0;
     // two segments per warp and iteration, all eight loads issued before any use: the kernel is
     // pure streaming and bound by the loads in flight
     const int lane = threadIdx.x & 31;
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int nseg = *seg.count;
+    const int qe = warp_global + nwarps;
+    int4 sa = warp_global < nseg ? seg.desc[warp_global] : make_int4(0, 0, 0, 0);
+    int4 sb = qe < nseg ? seg.desc[qe] : sa;
+    pdl_wait();
+    pdl_trigger();
+    if (s->done) return;
+    const V alpha = (V)s->alpha;
+    DotAcc<V> part = 0;
     auto finish = [&](int c, V pc, V apc, V xc, V rc0) {
         const V rc = rc0 - alpha * apc;
         x[c] = xc + alpha * pc;
@@ -571,8 +589,10 @@ __global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg 
     };
     for (int qs = warp_global; qs < nseg; qs += 2 * nwarps) {
         const int q2 = qs + nwarps;
-        const int4 sa = seg.desc[qs];
-        const int4 sb = q2 < nseg ? seg.desc[q2] : sa;
+        if (qs != warp_global) {
+            sa = seg.desc[qs];
+            sb = q2 < nseg ? seg.desc[q2] : sa;
+        }
         const bool la = sa.y + lane < g.n0, lb = q2 < nseg && sb.y + lane < g.n0;
         const int ca = sa.x + lane, cb = sb.x + lane;
         V pa = V(0), apa = V(0), xa = V(0), ra = V(0), pb = V(0), apb = V(0), xb = V(0), rb = V(0);
@@ -1207,12 +1227,14 @@ __device__ __forceinline__ V ldv(const V* p, int q) {
 
 // One smoothing sweep over the active segments of a level, warp wg of nw warps taking segments
 // wg, wg + nw, ...; returns the thread's share of b.x when DOT is set.
-// ZERO2: first sweep (formed on the fly) w1, this sweep w2; PROLONG: w1; PLAIN: w2
-template <typename V, typename R, int MODE, int DOT, bool COH = false>
+// ZERO2: first sweep (formed on the fly) w1, this sweep w2; PROLONG: w1; PLAIN: w2.  start() is called
+// once the first segment's list entry and records, which no kernel of an iteration writes, are on
+// their way, and before anything else is read; false ends the call.
+template <typename V, typename R, int MODE, int DOT, bool COH = false, typename Start>
 __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegArg& seg, const R* __restrict__ A,
                                                      const V* __restrict__ b, const V* __restrict__ x_in,
                                                      const LGeom& gc, const V* __restrict__ e, V* __restrict__ x_out,
-                                                     const V* __restrict__ rd, int wg, int nw) {
+                                                     const V* __restrict__ rd, int wg, int nw, Start&& start) {
     static_assert(sizeof(V) == 4 || MODE != SM_ZERO2, "FP64 stores the first sweep");
     [[maybe_unused]] const V w_first = V(kSweep1);
     const V omega = V(MODE == SM_PROLONG ? kSweep1 : kSweep2);
@@ -1230,22 +1252,37 @@ __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegAr
         if constexpr (MODE == SM_ZERO2) return mg_div(rn_mul(w_first, raw), rec.d);
         return raw;
     };
-    SEG_LOOP_ALL_W_BEGIN(seg, g, wg, nw)
-    const St7<V> st = gather7<V, true>(g, c, i, j, k, live, lane, recf, rawf, valf);
-    if (live) {
-        const V bc = ldv<COH>(b, c), rc = sizeof(V) == 8 ? rd[c] : V(0);
-        V xo = V(0);
-        if (positive(st.d)) {
-            const V q = rn_mul(omega, rn_sub(bc, apply7(st)));
-            if constexpr (sizeof(V) == 8)
-                xo = rn_fma(q, rc, st.v0);
-            else
-                xo = rn_add(st.v0, mg_div(q, st.d));
+    const int lane = threadIdx.x & 31;
+    int qs = wg;
+    const int nseg = *seg.count;
+    int4 sd = qs < nseg ? seg.desc[qs] : make_int4(0, g.n0, 0, 0);
+    Near7 nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+    Rec7<V> rec = load_rec7<V, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+    if (!start()) return part;
+    while (qs < nseg) {
+        const bool live = sd.y + lane < g.n0;
+        const int c = sd.x + lane;
+        const auto raw = load_raw7(g, nb, c, sd.y + lane, sd.z, sd.w, live, rawf);
+        const V bc = live ? ldv<COH>(b, c) : V(0), rc = sizeof(V) == 8 && live ? rd[c] : V(0);
+        const St7<V> st = value7<V>(nb, rec, raw, live, lane, valf);
+        if (live) {
+            V xo = V(0);
+            if (positive(st.d)) {
+                const V q = rn_mul(omega, rn_sub(bc, apply7(st)));
+                if constexpr (sizeof(V) == 8)
+                    xo = rn_fma(q, rc, st.v0);
+                else
+                    xo = rn_add(st.v0, mg_div(q, st.d));
+            }
+            if (EL_IN(c, (long long)g.s2 * g.n2, 30)) x_out[c] = xo;
+            if (DOT != DOT_NONE) part += (DotAcc<V>)bc * (DotAcc<V>)xo;
         }
-        if (EL_IN(c, (long long)g.s2 * g.n2, 30)) x_out[c] = xo;
-        if (DOT != DOT_NONE) part += (DotAcc<V>)bc * (DotAcc<V>)xo;
+        qs += nw;
+        if (qs >= nseg) break;
+        sd = seg.desc[qs];
+        nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+        rec = load_rec7<V, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
     }
-    SEG_LOOP_END
     return part;
 }
 
@@ -1255,12 +1292,16 @@ __global__ void __launch_bounds__(kSegThreads) smooth_kernel(LGeom g, SegArg seg
                                                              LGeom gc, const V* __restrict__ e,
                                                              V* __restrict__ x_out, const V* __restrict__ rd,
                                                              Scalars* s, double* partials, unsigned* counter) {
-    pdl_wait();
-    pdl_trigger();
-    if (s->done) return;
+    bool go = false;
+    auto start = [&] {
+        pdl_wait();
+        pdl_trigger();
+        return go = !s->done;
+    };
     const DotAcc<V> part = smooth_segments<V, R, MODE, DOT>(g, seg, A, b, x_in, gc, e, x_out, rd,
                                                             (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-                                                            (gridDim.x * blockDim.x) >> 5);
+                                                            (gridDim.x * blockDim.x) >> 5, start);
+    if (!go) return;
     if (DOT != DOT_NONE) {
         double acc[1] = {(double)part};
         double tot[1];
@@ -1284,6 +1325,9 @@ __global__ void __launch_bounds__(kSegThreads, sizeof(V) == 4 ? 5 : 4) restrict_
                                                                const V* __restrict__ x, LGeom gc, SegArg cseg,
                                                                V* __restrict__ bc, V* __restrict__ tc,
                                                                const V* __restrict__ rdc, const Scalars* s) {
+    const int nseg = *cseg.count;
+    pdl_wait();
+    pdl_trigger();
     if (s->done) return;
     const RecLoad<V, R> recf{A};
     auto rawf = [&](int q, int, int, int) -> V { return x[q]; };
@@ -1291,7 +1335,6 @@ __global__ void __launch_bounds__(kSegThreads, sizeof(V) == 4 ? 5 : 4) restrict_
     const int lane = threadIdx.x & 31;
     const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int nseg = *cseg.count;
     for (int qs = warp_global; qs < nseg; qs += nwarps) {
         const int4 sd = cseg.desc[qs];
         const int I0 = sd.y, J = sd.z, K = sd.w;
@@ -1334,34 +1377,56 @@ __global__ void __launch_bounds__(kSegThreads, sizeof(V) == 4 ? 5 : 4) restrict_
 constexpr int kQuadsPerBlock = kSegThreads / 128;
 
 // The quads' walk: quad `quad` of `nquads`, the block's quad quad_b (named barrier 1 + quad_b),
-// row `sub` of it; part = the block's [quads][4][2][16] sums in shared memory.
-template <typename V, typename R, bool COH = false>
+// row `sub` of it; part = the block's [quads][4][2][16] sums in shared memory; start() as for
+// smooth_segments.
+template <typename V, typename R, bool COH = false, typename Start>
 __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* __restrict__ A,
                                                        const V* __restrict__ b, const V* __restrict__ x,
                                                        const LGeom& gc, const SegArg& cseg, V* __restrict__ bc,
-                                                       V* __restrict__ tc, const V* __restrict__ rdc, V (*part)[4][2][16], int quad, int nquads, int quad_b,
-                                                       int sub) {
+                                                       V* __restrict__ tc, const V* __restrict__ rdc,
+                                                       V (*part)[4][2][16], int quad, int nquads, int quad_b,
+                                                       int sub, Start&& start) {
     const RecLoad<V, R> recf{A};
     auto rawf = [&](int q, int, int, int) -> V { return ldv<COH>(x, q); };
     auto valf = [](V raw, const Co<V>&) -> V { return raw; };
     const int lane = threadIdx.x & 31;
     const int kk = sub >> 1, jj = sub & 1;
+    int qs = quad;
     const int nseg = *cseg.count;
-    for (int qs = quad; qs < nseg; qs += nquads) {
-        const int4 sd = cseg.desc[qs];
-        const int I0 = sd.y, J = sd.z, K = sd.w;
-        const int j = 2 * J + jj, k = 2 * K + kk;
-        V sum[2] = {V(0), V(0)};  // fine i in [2*I0, 2*I0+32) and [2*I0+32, 2*I0+64)
-        // warp-uniform: the row exists for all lanes or for none
-        if (j < g.n1 && k < g.n2) {
+    int4 sd = qs < nseg ? cseg.desc[qs] : make_int4(0, g.n0, 0, 0);
+    // half h of the quad's row under a coarse segment: its fine cell at this lane, and that cell's
+    // records (the row exists for all lanes of the warp or for none)
+    Near7 nb[2];
+    Rec7<V> rec[2];
+    auto cell = [&](int h, int& c, int& i, int& j, int& k) -> bool {
+        i = 2 * sd.y + 32 * h + lane;
+        j = 2 * sd.z + jj;
+        k = 2 * sd.w + kk;
+        c = i + g.s1 * j + g.s2 * k;
+        return i < g.n0 && j < g.n1 && k < g.n2;
+    };
+    auto records = [&] {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = 2 * I0 + 32 * h + lane;
-                const bool live = i < g.n0;
-                const int c = i + g.s1 * j + g.s2 * k;
-                const St7<V> st = gather7<V, false>(g, c, i, j, k, live, lane, recf, rawf, valf);
-                if (live && positive(st.d)) sum[h] = rn_sub(ldv<COH>(b, c), apply7(st));
-            }
+        for (int h = 0; h < 2; ++h) {
+            int c, i, j, k;
+            const bool live = cell(h, c, i, j, k);
+            nb[h] = near7(g, c, i, j, k, live, lane);
+            rec[h] = load_rec7<V, false>(g, nb[h], c, live, recf);
+        }
+    };
+    records();
+    if (!start()) return;
+    while (qs < nseg) {
+        const int I0 = sd.y, J = sd.z, K = sd.w;
+        V sum[2] = {V(0), V(0)};  // fine i in [2*I0, 2*I0+32) and [2*I0+32, 2*I0+64)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            int c, i, j, k;
+            const bool live = cell(h, c, i, j, k);
+            const auto raw = load_raw7(g, nb[h], c, i, j, k, live, rawf);
+            const V bv = live ? ldv<COH>(b, c) : V(0);
+            const St7<V> st = value7<V>(nb[h], rec[h], raw, live, lane, valf);
+            if (live && positive(st.d)) sum[h] = rn_sub(bv, apply7(st));
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -1382,6 +1447,10 @@ __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* 
             }
         }
         asm volatile("bar.sync %0, %1;" ::"r"(1 + quad_b), "r"(128) : "memory");
+        qs += nquads;
+        if (qs >= nseg) break;
+        sd = cseg.desc[qs];
+        records();
     }
 }
 
@@ -1391,14 +1460,15 @@ __global__ void __launch_bounds__(kSegThreads, 4) restrict_quad_kernel(LGeom g, 
                                                                     LGeom gc, SegArg cseg, V* __restrict__ bc,
                                                                     V* __restrict__ tc, const V* __restrict__ rdc,
                                                                     const Scalars* s) {
-    pdl_wait();
-    pdl_trigger();
-    if (s->done) return;
     __shared__ V part[kQuadsPerBlock][4][2][16];
     const int wb = threadIdx.x >> 5;                  // warp in the block
     const int quad_b = wb >> 2, sub = wb & 3;         // quad in the block, row of the quad
     restrict_quad_segments<V, R>(g, A, b, x, gc, cseg, bc, tc, rdc, part, blockIdx.x * kQuadsPerBlock + quad_b,
-                                 gridDim.x * kQuadsPerBlock, quad_b, sub);
+                                 gridDim.x * kQuadsPerBlock, quad_b, sub, [&] {
+                                     pdl_wait();
+                                     pdl_trigger();
+                                     return !s->done;
+                                 });
 }
 
 
@@ -1410,7 +1480,6 @@ __global__ void __launch_bounds__(kCoarsestMaxCells) coarsest_kernel(LGeom g, co
                                                                      const V* __restrict__ b, V* __restrict__ x,
                                                                      const V* __restrict__ rd, int sweeps,
                                                                      const Scalars* s) {
-    if (s->done) return;
     __shared__ V xs[2][kCoarsestMaxCells];
     const int n = g.n0 * g.n1 * g.n2;
     const int c = threadIdx.x;
@@ -1433,10 +1502,13 @@ __global__ void __launch_bounds__(kCoarsestMaxCells) coarsest_kernel(LGeom g, co
     // an absent neighbour: coefficient 0 at the cell itself
     const int qxm = hxm ? c - 1 : c, qxp = hxp ? c + 1 : c, qym = hym ? c - s1 : c, qyp = hyp ? c + s1 : c;
     const int qzm = hzm ? c - s2 : c, qzp = hzp ? c + s2 : c;
+    [[maybe_unused]] const V w = sizeof(V) == 8 && act ? rn_mul(omega, rd[c]) : V(0);
+    pdl_wait();
+    pdl_trigger();
+    if (s->done) return;
     V bc = in ? b[c] : V(0);
     V x0 = V(0);
     if constexpr (sizeof(V) == 8) {
-        const V w = act ? rn_mul(omega, rd[c]) : V(0);
         cxm = rn_mul(cxm, -w);
         cxp = rn_mul(cxp, -w);
         cym = rn_mul(cym, -w);
@@ -1531,10 +1603,11 @@ constexpr int bottom_smem_bytes() {
 }
 
 // the bottom's passes by one CTA of kBottomThreads threads, staged in bottom_smem
+template <typename Start>
 __device__ __forceinline__ void bottom_cycle(const LGeom& gf, const float4* __restrict__ recf,
                                              const float* __restrict__ bf, float* __restrict__ xf, const LGeom& gc,
                                              const float4* __restrict__ recc, int sweeps,
-                                             unsigned char* bottom_smem) {
+                                             unsigned char* bottom_smem, Start&& start) {
     float4* sr = reinterpret_cast<float4*>(bottom_smem);
     float* sb = reinterpret_cast<float*>(sr + kBottomMaxCells);
     float* s1 = sb + kBottomMaxCells;
@@ -1562,11 +1635,10 @@ __device__ __forceinline__ void bottom_cycle(const LGeom& gf, const float4* __re
     const int ci = tid & 7, cj = (tid >> 3) & 7, ck = tid >> 6;
     const bool clive = tid < kCoarsestMaxCells && ci < gc.n0 && cj < gc.n1 && ck < gc.n2;
     const int cq = clive ? ci + gc.s1 * cj + gc.s2 * ck : 0;
-    for (int c = tid; c < nf; c += kBottomThreads) {
-        sr[c] = recf[c];
-        sb[c] = __ldcg(bf + c);  // written by other CTAs of the fused coarse cycle
-    }
+    for (int c = tid; c < nf; c += kBottomThreads) sr[c] = recf[c];
     for (int c = tid; c < nc; c += kBottomThreads) cr[c] = recc[c];
+    if (!start()) return;
+    for (int c = tid; c < nf; c += kBottomThreads) sb[c] = __ldcg(bf + c);  // written by other CTAs of the fused coarse cycle
     __syncthreads();
     // two sweeps from zero: the first is pointwise
 #pragma unroll
@@ -1682,11 +1754,12 @@ __global__ void __launch_bounds__(kBottomThreads) mg_bottom_kernel(LGeom gf, con
                                                                    float* __restrict__ xf, LGeom gc,
                                                                    const float4* __restrict__ recc, int sweeps,
                                                                    const Scalars* s) {
-    pdl_wait();
-    pdl_trigger();
-    if (s->done) return;
     extern __shared__ __align__(16) unsigned char bottom_smem[];
-    bottom_cycle(gf, recf, bf, xf, gc, recc, sweeps, bottom_smem);
+    bottom_cycle(gf, recf, bf, xf, gc, recc, sweeps, bottom_smem, [&] {
+        pdl_wait();
+        pdl_trigger();
+        return !s->done;
+    });
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1765,6 +1838,7 @@ __global__ void __launch_bounds__(kBottomThreads, 1) mg_coarse_cycle_kernel(cons
     const int wg = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     const int wb = threadIdx.x >> 5, quad_b = wb >> 2, sub = wb & 3;
     const int quad = blockIdx.x * kCoopQuads + quad_b, nquads = gridDim.x * kCoopQuads;
+    auto now = [] { return true; };
     auto fail = [&]() {
         if (threadIdx.x == 0) {
             s->fault = 1;
@@ -1776,26 +1850,26 @@ __global__ void __launch_bounds__(kBottomThreads, 1) mg_coarse_cycle_kernel(cons
         const CoarseLevel& F = a.lv[l];
         const CoarseLevel& C = a.lv[l + 1];
         smooth_segments<float, float4, SM_ZERO2, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, nullptr, F.g, nullptr, F.x, nullptr,
-                                                                 wg, nw);
+                                                                 wg, nw, now);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
         restrict_quad_segments<float, float4, true>(F.g, F.rec, F.b, F.x, C.g, C.seg, C.b, nullptr, nullptr, part, quad, nquads,
-                                                    quad_b, sub);
+                                                    quad_b, sub, now);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
     }
     if (blockIdx.x == 0) {
         const CoarseLevel& F = a.lv[a.pre_end];
         const CoarseLevel& C = a.lv[a.pre_end + 1];
-        bottom_cycle(F.g, F.rec, F.b, F.x, C.g, C.rec, a.sweeps, bottom_smem);
+        bottom_cycle(F.g, F.rec, F.b, F.x, C.g, C.rec, a.sweeps, bottom_smem, now);
     }
     for (int l = a.pre_end - 1; l >= a.from; --l) {
         const CoarseLevel& F = a.lv[l];
         const CoarseLevel& C = a.lv[l + 1];
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
         smooth_segments<float, float4, SM_PROLONG, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, F.x, C.g, C.x, F.t, nullptr, wg,
-                                                                   nw);
+                                                                   nw, now);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
         smooth_segments<float, float4, SM_PLAIN, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, F.t, F.g, nullptr, F.x, nullptr, wg,
-                                                                 nw);
+                                                                 nw, now);
     }
 }
 
@@ -2004,8 +2078,8 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
     if (L == 1) {
         // too small to coarsen: the coarsest sweeps solve it, one more sweep gives the dot
         MGLevel<V>& C = mg[0];
-        coarsest_kernel<V, R0><<<1, kCoarsestMaxCells, 0, ctx->stream>>>(make_geom(C.n0, C.n1, C.n2), (const R0*)C.rec,
-                                                                         C.b, C.t, C.rd, kCoarsestSweeps, s);
+        launch_dependent(ctx, coarsest_kernel<V, R0>, dim3(1), dim3(kCoarsestMaxCells), 0, make_geom(C.n0, C.n1, C.n2),
+                         (const R0*)C.rec, (const V*)C.b, C.t, (const V*)C.rd, (int)kCoarsestSweeps, (const Scalars*)s);
         if (dot == DOT_INIT)
             launch_smooth<V, R0, SM_PLAIN, DOT_INIT>(ctx, C, seg0, C.t, nullptr, C.x, s);
         else
@@ -2048,8 +2122,9 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
             ProfScope prof(ctx, l == 0 ? EL_KC_RESTRICT : EL_KC_MG_COARSE, act(l, F) * (2 * vs + rb) + act(l + 1, C) * vs);
             const LGeom gf = make_geom(F.n0, F.n1, F.n2), gc = make_geom(C.n0, C.n1, C.n2);
             if (l == 0)
-                restrict_kernel<V, R0><<<restrict_blocks(ctx, C.seg.total), kSegThreads, 0, ctx->stream>>>(
-                    gf, (const R0*)F.rec, F.b, F.x, gc, seg_arg(C.seg), C.b, C.t, C.rd, s);
+                launch_dependent(ctx, restrict_kernel<V, R0>, dim3(restrict_blocks(ctx, C.seg.total)), dim3(kSegThreads),
+                                 0, gf, (const R0*)F.rec, (const V*)F.b, (const V*)F.x, gc, seg_arg(C.seg), C.b, C.t,
+                                 (const V*)C.rd, (const Scalars*)s);
             else
                 launch_dependent(ctx, restrict_quad_kernel<V, RC>,
                                  dim3(one_wave(ctx, restrict_quad_kernel<V, RC>, kSegThreads,
@@ -2084,8 +2159,8 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
     } else {
         MGLevel<V>& C = mg[L - 1];
         ProfScope prof(ctx, EL_KC_MG_COARSE, cells(C) * (3 * vs + sizeof(RC)));
-        coarsest_kernel<V, RC><<<1, kCoarsestMaxCells, 0, ctx->stream>>>(make_geom(C.n0, C.n1, C.n2), (const RC*)C.rec,
-                                                                         C.b, C.x, C.rd, kCoarsestSweeps, s);
+        launch_dependent(ctx, coarsest_kernel<V, RC>, dim3(1), dim3(kCoarsestMaxCells), 0, make_geom(C.n0, C.n1, C.n2),
+                         (const RC*)C.rec, (const V*)C.b, C.x, (const V*)C.rd, (int)kCoarsestSweeps, (const Scalars*)s);
         ++launched;
     }
     for (int l = down_end - 1; l >= from; --l) {
