@@ -385,27 +385,14 @@ __global__ void scatter_pressure_kernel(long long n, const double* __restrict__ 
 
 // update_velocity_using_pressure (projection.cpp:93-134): faces with index in [1, n) along
 // their normal and [1, n-1) along the two tangential axes, as the reference's loops.
-// one face given the level set and pressure of its two cells (a: below, b: above).  FP64: its pipe (2
-// lanes a clock per SM; a division costs about nine of its operations, a comparison one) bounds the
-// kernel, so signs are read as integers and a face between two fluid cells (theta = 1) skips what theta
-// needs, with the same bits: UVFIG us at 128^3.
-__device__ __forceinline__ bool below_zero(float v) { return v < 0.f; }
-__device__ __forceinline__ bool below_zero(double v) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
-}
+// one face given the level set and pressure of its two cells (a: below, b: above)
 template <typename T>
 __device__ __forceinline__ void update_face(T pa, T pb, T qa, T qb, long long fi, T* __restrict__ f, T dt, T dx) {
-    const bool na = below_zero(pa), nb = below_zero(pb);
-    if (nb || na) {
-        const T num = mul_rn(dt, qb - qa);
-        if (sizeof(T) == 8 && na && nb) {
-            f[fi] = f[fi] - num / dx;
-            return;
-        }
+    if (pb < T(0) || pa < T(0)) {
         T theta = T(1);
         if (pb >= T(0) || pa >= T(0)) theta = fraction_inside(pa, pb);
         theta = theta < T(0.01) ? T(0.01) : theta;
+        const T num = mul_rn(dt, qb - qa);
         const T den = mul_rn(dx, theta);
         f[fi] = f[fi] - num / den;
     }
