@@ -34,6 +34,8 @@ int launch_time_step(el_ctx* ctx, double cfl, unsigned long long* scratch_max);
 int launch_set_dt(el_ctx* ctx, double dt);
 int launch_emit(el_ctx* ctx, int target, int kind, const double* a, int na);
 int solve_system(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st);
+bool solve_graph_ready(el_ctx* ctx, const el_solve_params& prm);
+int solve_system_graph(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st);
 int setup_solver_storage(el_ctx* ctx, int solver);
 int launch_substep(el_ctx* ctx, double cfl, double dt_frame, const BatchRecord* rec, unsigned long long* scratch_max);
 int enqueue_solve_device(el_ctx* ctx, const el_solve_params& prm, int kernels[3]);
@@ -231,6 +233,7 @@ EL_API int el_ctx_destroy(el_ctx* ctx) {
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     for (auto& g : ctx->iter_graph)
         if (g) cudaGraphExecDestroy(g);
+    if (ctx->solve_graph) cudaGraphExecDestroy(ctx->solve_graph);
     for (auto& bs : ctx->body_stream)
         if (bs) cudaStreamDestroy(bs);
     for (auto& ss : ctx->side)
@@ -285,13 +288,18 @@ EL_API int el_ctx_set_tuning(el_ctx* ctx, const el_tuning* t) {
     ctx->solver_tiles = t->solver_tiles;
     ctx->coarse_fused = t->coarse_fused;
     ctx->dependent_launch = t->dependent_launch;
-    // cached PCG iteration graphs hold the old launch shapes
+    // cached graphs of the solve hold the old launch shapes
     cudaStreamSynchronize(ctx->stream);
     for (auto& g : ctx->iter_graph)
         if (g) {
             cudaGraphExecDestroy(g);
             g = nullptr;
         }
+    if (ctx->solve_graph) {
+        cudaGraphExecDestroy(ctx->solve_graph);
+        ctx->solve_graph = nullptr;
+    }
+    ctx->solve_last = el_ctx::SolveKey{};
     return EL_OK;
 }
 
@@ -613,15 +621,26 @@ static int solve_pressure_impl(el_ctx* ctx, const el_solve_params& prm, el_solve
     ctx->launches += build_prof(ctx, inner32);
     rc = check_launch(ctx, "build_matrix");
     if (rc != EL_OK) return rc;
-    EL_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->hscal, ctx->dscal, sizeof(Scalars), cudaMemcpyDeviceToHost, ctx->stream));
-    EL_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    // a solve like the one before runs as one graph, with the fluid cells read back at its end (a
+    // system without any is empty: the graph's loops end at once)
+    const bool graph = solve_graph_ready(ctx, prm);
+    if (graph) {
+        rc = solve_system_graph(ctx, prm, st);
+        if (rc != EL_OK) return rc;
+    } else {
+        EL_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->hscal, ctx->dscal, sizeof(Scalars), cudaMemcpyDeviceToHost, ctx->stream));
+        EL_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    }
     st->fluid_cells = ctx->hscal->count;
     if (ctx->hscal->count == 0) {
+        *st = el_solve_stats{};
         st->status = EL_ERR_NO_FLUID;
         return set_error(ctx, EL_ERR_NO_FLUID, "No fluid");
     }
-    rc = solve_system(ctx, prm, st);
-    if (rc != EL_OK) return rc;
+    if (!graph) {
+        rc = solve_system(ctx, prm, st);
+        if (rc != EL_OK) return rc;
+    }
     ctx->launches += launch_scatter_pressure(ctx);
     ctx->launches += launch_update_velocity(ctx, ctx->dscal, 0.0);
     return check_launch(ctx, "update_velocity_using_pressure");

@@ -54,6 +54,7 @@ struct Scalars {
     int outer;       // mixed solver: refinement sweeps done
     int inner_total; // mixed solver: inner iterations summed over the sweeps
     int inner_passes;// device-driven mixed solver: passes of its PCG loop
+    int iter_limit;  // iterations after which an inner solve stops as if it had converged
     int fault;       // a bounded device wait gave up (the solve reports EL_ERR_TIMEOUT)
     int df_shift;    // mixed solver: the power of two 2^df_shift that brings |b| near 1 in the
                      // double-float residual (scale invariance for its float pairs)
@@ -277,6 +278,20 @@ struct el_ctx {
     int iter_graph_len[3] = {0, 0, 0};
     int iter_graph_kernels[3] = {0, 0, 0};
     bool use_graphs = true;
+    // the mixed solve as one graph (solve_graph): the parameters of the last mixed solve, and the
+    // graph made for them once a second solve in a row had the same
+    struct SolveKey {
+        double tol = 0.0, inner_floor = 0.0;
+        int max_iter = 0, max_outer = 0;
+        bool records = false, valid = false;
+        bool operator==(const SolveKey& o) const {
+            return tol == o.tol && inner_floor == o.inner_floor && max_iter == o.max_iter &&
+                   max_outer == o.max_outer && records == o.records && valid == o.valid;
+        }
+    };
+    SolveKey solve_last, solve_graph_key;
+    cudaGraphExec_t solve_graph = nullptr;
+    int solve_graph_kernels[3] = {0, 0, 0};  // outside the loops, a refinement sweep, a pass of the PCG loop
 
     // per-kernel-class timing (el_ctx_profile_begin / _end)
     uint32_t prof_mask = 0;

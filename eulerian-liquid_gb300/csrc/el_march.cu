@@ -507,11 +507,12 @@ __global__ void __launch_bounds__(kThreads, Layout<M>::min_blocks) march_kernel(
                 }
             } else if (M == UPDZ) {
                 s->rr = tot[0];
-                s->iter += 1;
+                const int iter = s->iter + 1;
+                s->iter = iter;
                 if (!isfinite(tot[0])) {
                     s->bad = 1;
                     s->done = 1;
-                } else if (tot[0] < s->thresh) {
+                } else if (tot[0] < s->thresh || iter >= s->iter_limit) {
                     s->done = 1;
                 }
             } else {
