@@ -1555,211 +1555,196 @@ __global__ void __launch_bounds__(kCoarsestMaxCells) coarsest_kernel(LGeom g, co
 
 // ---------------------------------------------------------------------------------------
 // The bottom of the FP32 V-cycle in one CTA.  Coarsening stops once the largest dimension is
-// at most 8, so the level above the coarsest holds at most 16^3 = 4096 cells: that level and
-// the coarsest fit in one CTA's shared memory (126 KB with float4 records).  One launch of 1024
-// threads does what the segment kernels do in five: the two sweeps from zero, the restriction,
-// the coarsest level's 30 sweeps, the prolongation sweep and the last sweep -- the same
-// expressions in the same order, over the dense level (cells with no diagonal come out 0, as
-// they contribute nothing to their neighbours), with barriers between the passes instead of
-// kernel boundaries.  Only the level's final x goes back to global memory (the finer level's
-// prolongation reads it).
-constexpr int kBottomMaxCells = 4096;
-constexpr int kBottomThreads = 1024;
-// Each thread owns fixed cells: on the level, (i, j) = (t mod 16, t / 16 mod 16) and the planes
-// k = t / 256 + 4 m, m = 0..3 (the level is at most 16 cells a side: its coarse level is at
-// most 8); on the coarsest, thread t < 512 owns (t mod 8, t / 8 mod 8, t / 64).  No index is
-// divided at run time, and the coarsest cell's record stays in registers across its sweeps.
-constexpr int kBottomDim = 16, kBottomPlanes = kBottomThreads / (kBottomDim * kBottomDim);
-constexpr int kBottomCells = kBottomDim / kBottomPlanes;  // cells per thread on the level
+// at most 8, so the level above the coarsest holds at most 16^3 cells: one launch of 1024 threads
+// does what the segment kernels do in five: the two sweeps from zero, the restriction, the coarsest
+// level's solve, the prolongation sweep and the last sweep, over the dense level (cells with no
+// diagonal come out 0, as they contribute nothing to their neighbours), with barriers between the
+// passes instead of kernel boundaries.  Only the level's final x goes back to global memory (the
+// finer level's prolongation reads it).
+//
+// One SM's shared memory bounds the passes: a float4 record a neighbour, read in every pass, was 23
+// wavefronts a warp and cell.  So a thread owns C cells in a row along z, (t mod 16, t / 16 mod 16,
+// C (t / 256) + m), with their couplings, right-hand side and values in registers, and reads only the
+// neighbours' values in x and y and above and below its own; the couplings are loaded before the wait
+// for the kernel before.  512 threads of eight cells: 1024 of four (the fused coarse cycle's) leave
+// a thread 64 registers, which the coarsest level's rows do not fit beside the level's.
+// 16^3 and 8^3: 17.5 -> 13.4 us, of which 1.6 may pass before the kernel before ends; 12^3 and 6^3
+// 14.0 -> 11.7.  The coarsest level's 30 sweeps are bound by the latency of a sweep (a barrier, the
+// neighbours' values, seven dependent multiply-adds): with a cell a thread 0.13 us each, with two 0.16,
+// with four 0.31.
+constexpr int kBottomThreads = 512;   // of mg_bottom_kernel
+constexpr int kCycleThreads = 1024;   // of mg_coarse_cycle_kernel
+constexpr int kBottomDim = 16;        // the level's cells are (i, j, k) at i + 16 j + 256 k in shared memory
+// the coarsest level's cells are at i + 8 j + 64 k; kBottomCoarseThreads threads own them
+constexpr int kBottomCoarseThreads = 512;
 
-// neighbour bits of a cell: 1 -x, 2 +x, 4 -y, 8 +y, 16 -z, 32 +z inside the level
-__device__ __forceinline__ unsigned inside_bits(int i, int j, int k, const LGeom& g) {
-    return (i > 0 ? 1u : 0u) | (i < g.n0 - 1 ? 2u : 0u) | (j > 0 ? 4u : 0u) | (j < g.n1 - 1 ? 8u : 0u) |
-           (k > 0 ? 16u : 0u) | (k < g.n2 - 1 ? 32u : 0u);
+struct BottomSmem {
+    float v[2][kBottomDim * kBottomDim * kBottomDim];
+    float4 rec[kCoarsestMaxCells];  // the coarsest level's
+    float c[2][kCoarsestMaxCells];
+};
+
+// C cells along z, (i, j, k0 + m), of a dense level of at most N cells an axis, stored with pitches N and
+// N * N: couplings (0 towards cells outside), and the places of the neighbours outside the C (the cell
+// itself where there is none)
+template <int C, int N>
+struct Column {
+    static constexpr int PY = N, PZ = N * N;
+    float d[C], cxm[C], cxp[C], cym[C], cyp[C], cz[C + 1];  // cz[m]: between k0 + m - 1 and k0 + m
+    int at, xm, xp, ym, yp, zm, zp;
+    bool live[C];
+    template <typename RF>
+    __device__ __forceinline__ void load(int i, int j, int k0, int n0, int n1, int n2, RF&& recf) {
+        at = i + PY * j + PZ * k0;
+        xm = i > 0 ? -1 : 0;
+        xp = i + 1 < N ? 1 : 0;
+        ym = j > 0 ? -PY : 0;
+        yp = j + 1 < N ? PY : 0;
+        zm = k0 > 0 ? -PZ : 0;
+        zp = k0 + C < N ? C * PZ : (C - 1) * PZ;
+        const bool row = i < n0 && j < n1;
+        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+        cz[0] = row && k0 > 0 && k0 < n2 ? recf(i, j, k0 - 1).w : 0.f;
+#pragma unroll
+        for (int m = 0; m < C; ++m) {
+            live[m] = row && k0 + m < n2;
+            const float4 r = live[m] ? recf(i, j, k0 + m) : z4;
+            d[m] = r.x;
+            cxp[m] = i + 1 < n0 ? r.y : 0.f;
+            cyp[m] = j + 1 < n1 ? r.z : 0.f;
+            cz[m + 1] = k0 + m + 1 < n2 ? r.w : 0.f;
+            cxm[m] = live[m] && i > 0 ? recf(i - 1, j, k0 + m).y : 0.f;
+            cym[m] = live[m] && j > 0 ? recf(i, j - 1, k0 + m).z : 0.f;
+        }
+    }
+    // A x at the four cells, x also in v[] (of every cell of the level)
+    __device__ __forceinline__ void apply(const float* v, const float (&x)[C], float (&ax)[C]) const {
+        const float* q = v + at;
+        const float below = q[zm], above = q[zp];
+#pragma unroll
+        for (int m = 0; m < C; ++m) {
+            const float* c = q + m * PZ;
+            ax[m] = stencil7(d[m], x[m], cxm[m], c[xm], cxp[m], c[xp], cym[m], c[ym], cyp[m], c[yp], cz[m],
+                             m ? x[m - 1] : below, cz[m + 1], m + 1 < C ? x[m + 1] : above);
+        }
+    }
+};
+
+// The coarsest level (right-hand side in sm.c[0], the result too): damped Jacobi from zero as
+// coarsest_kernel, by kBottomCoarseThreads threads on named barrier 15.
+__device__ __forceinline__ void coarsest_solve(BottomSmem& sm, int tid, const LGeom& gc) {
+    constexpr int C = kCoarsestMaxCells / kBottomCoarseThreads;
+    const float omega = (float)kOmega;
+    Column<C, 8> A;
+    A.load(tid & 7, (tid >> 3) & 7, C * (tid >> 6), gc.n0, gc.n1, gc.n2,
+           [&](int i, int j, int k) { return sm.rec[i + 8 * j + 64 * k]; });
+    float b[C], x[C], t[C];
+#pragma unroll
+    for (int m = 0; m < C; ++m) {
+        b[m] = sm.c[0][A.at + 64 * m];
+        x[m] = A.d[m] > 0.f ? mg_div(rn_mul(omega, b[m]), A.d[m]) : 0.f;
+    }
+    auto put = [&](float* v) {
+#pragma unroll
+        for (int m = 0; m < C; ++m) v[A.at + 64 * m] = x[m];
+        asm volatile("bar.sync 15, %0;" ::"r"(kBottomCoarseThreads) : "memory");
+    };
+    static_assert(kCoarsestSweeps % 2 == 0, "the last sweep's values go to sm.c[0]");
+#pragma unroll 2
+    for (int it = 1; it < kCoarsestSweeps; ++it) {
+        float* v = sm.c[it & 1];
+        put(v);
+        A.apply(v, x, t);
+#pragma unroll
+        for (int m = 0; m < C; ++m)
+            x[m] = A.d[m] > 0.f ? rn_add(x[m], mg_div(rn_mul(omega, rn_sub(b[m], t[m])), A.d[m])) : 0.f;
+    }
+    put(sm.c[0]);
 }
 
-// the 7-point stencil of cell c of a dense level held in shared memory (float4 records); a
-// neighbour outside the level gives coupling and value 0
-__device__ __forceinline__ St7<float> dense_st7(const float4* rec, const float* v, int c, unsigned in,
-                                                const LGeom& g) {
-    St7<float> st;
-    const float4 r0 = rec[c];
-    st.d = r0.x;
-    st.cxp = r0.y;
-    st.cyp = r0.z;
-    st.czp = r0.w;
-    st.cxm = (in & 1u) ? rec[c - 1].y : 0.f;
-    st.cym = (in & 4u) ? rec[c - g.s1].z : 0.f;
-    st.czm = (in & 16u) ? rec[c - g.s2].w : 0.f;
-    st.v0 = v[c];
-    st.vxm = (in & 1u) ? v[c - 1] : 0.f;
-    st.vxp = (in & 2u) ? v[c + 1] : 0.f;
-    st.vym = (in & 4u) ? v[c - g.s1] : 0.f;
-    st.vyp = (in & 8u) ? v[c + g.s1] : 0.f;
-    st.vzm = (in & 16u) ? v[c - g.s2] : 0.f;
-    st.vzp = (in & 32u) ? v[c + g.s2] : 0.f;
-    return st;
-}
-
-constexpr int bottom_smem_bytes() {
-    return kBottomMaxCells * (int)(sizeof(float4) + 3 * sizeof(float)) +
-           kCoarsestMaxCells * (int)(sizeof(float4) + 3 * sizeof(float));
-}
-
-// the bottom's passes by one CTA of kBottomThreads threads, staged in bottom_smem
-template <typename Start>
+// the bottom's passes by one CTA of 4096 / C threads
+template <int C, typename Start>
 __device__ __forceinline__ void bottom_cycle(const LGeom& gf, const float4* __restrict__ recf,
                                              const float* __restrict__ bf, float* __restrict__ xf, const LGeom& gc,
-                                             const float4* __restrict__ recc, int sweeps,
-                                             unsigned char* bottom_smem, Start&& start) {
-    float4* sr = reinterpret_cast<float4*>(bottom_smem);
-    float* sb = reinterpret_cast<float*>(sr + kBottomMaxCells);
-    float* s1 = sb + kBottomMaxCells;
-    float* s2 = s1 + kBottomMaxCells;
-    float4* cr = reinterpret_cast<float4*>(s2 + kBottomMaxCells);
-    float* c1 = reinterpret_cast<float*>(cr + kCoarsestMaxCells);
-    float* c2 = c1 + kCoarsestMaxCells;
-    const float omega = (float)kOmega;  // the coarsest level's sweeps
+                                             const float4* __restrict__ recc, unsigned char* bottom_smem,
+                                             Start&& start) {
+    BottomSmem& sm = *reinterpret_cast<BottomSmem*>(bottom_smem);
     const float w1 = (float)kSweep1, w2 = (float)kSweep2;
-    const int nf = gf.n0 * gf.n1 * gf.n2, nc = gc.n0 * gc.n1 * gc.n2;
     const int tid = threadIdx.x;
-    // this thread's cells of the level: index (-1: none) and neighbour bits
-    const int fi = tid & (kBottomDim - 1), fj = (tid / kBottomDim) & (kBottomDim - 1);
-    const int fk0 = tid / (kBottomDim * kBottomDim);
-    int fc[kBottomCells];
-    unsigned fin[kBottomCells];
-#pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int k = fk0 + kBottomPlanes * m;
-        const bool live = fi < gf.n0 && fj < gf.n1 && k < gf.n2;
-        fc[m] = live ? fi + gf.s1 * fj + gf.s2 * k : -1;
-        fin[m] = live ? inside_bits(fi, fj, k, gf) : 0u;
+    const int fi = tid & 15, fj = (tid >> 4) & 15, k0 = C * (tid >> 8);
+    Column<C, 16> A;
+    A.load(fi, fj, k0, gf.n0, gf.n1, gf.n2,
+           [&](int i, int j, int k) { return recf[i + gf.s1 * j + gf.s2 * k]; });
+    if (tid < kCoarsestMaxCells) {
+        const int ci = tid & 7, cj = (tid >> 3) & 7, ck = tid >> 6;
+        sm.rec[tid] = ci < gc.n0 && cj < gc.n1 && ck < gc.n2 ? recc[ci + gc.s1 * cj + gc.s2 * ck]
+                                                             : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    // this thread's cell of the coarsest level
-    const int ci = tid & 7, cj = (tid >> 3) & 7, ck = tid >> 6;
-    const bool clive = tid < kCoarsestMaxCells && ci < gc.n0 && cj < gc.n1 && ck < gc.n2;
-    const int cq = clive ? ci + gc.s1 * cj + gc.s2 * ck : 0;
-    for (int c = tid; c < nf; c += kBottomThreads) sr[c] = recf[c];
-    for (int c = tid; c < nc; c += kBottomThreads) cr[c] = recc[c];
     if (!start()) return;
-    for (int c = tid; c < nf; c += kBottomThreads) sb[c] = __ldcg(bf + c);  // written by other CTAs of the fused coarse cycle
-    __syncthreads();
+    float b[C], x[C], t[C];
+#pragma unroll
+    for (int m = 0; m < C; ++m)  // (b may have been written by other CTAs of the fused coarse cycle)
+        b[m] = A.live[m] ? __ldcg(bf + fi + gf.s1 * fj + gf.s2 * (k0 + m)) : 0.f;
+    auto put = [&](float* v) {
+#pragma unroll
+        for (int m = 0; m < C; ++m) v[A.at + 256 * m] = x[m];
+        __syncthreads();
+    };
+    auto sweep = [&](const float* v, float w) {
+        A.apply(v, x, t);
+#pragma unroll
+        for (int m = 0; m < C; ++m)
+            x[m] = A.d[m] > 0.f ? rn_add(x[m], mg_div(rn_mul(w, rn_sub(b[m], t[m])), A.d[m])) : 0.f;
+    };
     // two sweeps from zero: the first is pointwise
 #pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int c = fc[m];
-        if (c < 0) continue;
-        const float d = sr[c].x;
-        s1[c] = d > 0.f ? mg_div(rn_mul(w1, sb[c]), d) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int c = fc[m];
-        if (c < 0) continue;
-        const St7<float> st = dense_st7(sr, s1, c, fin[m], gf);
-        float xo = 0.f;
-        if (st.d > 0.f) xo = rn_add(st.v0, mg_div(rn_mul(w2, rn_sub(sb[c], apply7(st))), st.d));
-        s2[c] = xo;
-    }
-    __syncthreads();
+    for (int m = 0; m < C; ++m) x[m] = A.d[m] > 0.f ? mg_div(rn_mul(w1, b[m]), A.d[m]) : 0.f;
+    put(sm.v[0]);
+    sweep(sm.v[0], w2);
+    put(sm.v[1]);
     // residual, then its 2 x 2 x 2 sums onto the coarsest level (order of the segment kernels:
-    // i-pairs of the rows (jj, kk) = (0,0), (1,0), (0,1), (1,1), summed in that order)
+    // i-pairs of the rows (jj, kk) = (0,0), (1,0), (0,1), (1,1), summed in that order); a warp holds
+    // 16 cells in x of two rows in y
+    A.apply(sm.v[1], x, t);
+    {
+        float p[C], q[C];
 #pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int c = fc[m];
-        if (c < 0) continue;
-        const St7<float> st = dense_st7(sr, s2, c, fin[m], gf);
-        s1[c] = st.d > 0.f ? rn_sub(sb[c], apply7(st)) : 0.f;
+        for (int m = 0; m < C; ++m) {
+            const float r = A.d[m] > 0.f ? rn_sub(b[m], t[m]) : 0.f;
+            p[m] = r + __shfl_down_sync(kFull, r, 1);
+            q[m] = __shfl_down_sync(kFull, p[m], 16);
+        }
+        if (!(tid & 17)) {
+            float* c = sm.c[0] + (fi >> 1) + 8 * (fj >> 1) + 64 * (k0 >> 1);
+#pragma unroll
+            for (int h = 0; h < C / 2; ++h) c[64 * h] = ((p[2 * h] + q[2 * h]) + p[2 * h + 1]) + q[2 * h + 1];
+        }
     }
     __syncthreads();
-    // the coarsest cell's record, rhs and neighbour bits in registers for all its sweeps
-    float cbq = 0.f, cd = 0.f, cxm = 0.f, cxp = 0.f, cym = 0.f, cyp = 0.f, czm = 0.f, czp = 0.f;
-    unsigned cin = 0u;
-    if (clive) {
-        auto res = [&](int i, int j, int k) -> float {
-            return (i < gf.n0 && j < gf.n1 && k < gf.n2) ? s1[i + gf.s1 * j + gf.s2 * k] : 0.f;
-        };
-        float part[4];
-#pragma unroll
-        for (int sub = 0; sub < 4; ++sub) {
-            const int jj = sub & 1, kk = sub >> 1;
-            part[sub] = res(2 * ci, 2 * cj + jj, 2 * ck + kk) + res(2 * ci + 1, 2 * cj + jj, 2 * ck + kk);
-        }
-        cbq = ((part[0] + part[1]) + part[2]) + part[3];
-        cin = inside_bits(ci, cj, ck, gc);
-        const float4 r = cr[cq];
-        cd = r.x;
-        cxp = r.y;
-        cyp = r.z;
-        czp = r.w;
-        if (cin & 1u) cxm = cr[cq - 1].y;
-        if (cin & 4u) cym = cr[cq - gc.s1].z;
-        if (cin & 16u) czm = cr[cq - gc.s2].w;
-        // the coarsest level: damped Jacobi from zero, as coarsest_kernel
-        c1[cq] = cd > 0.f ? mg_div(rn_mul(omega, cbq), cd) : 0.f;
-    }
+    if (tid < kBottomCoarseThreads) coarsest_solve(sm, tid, gc);
     __syncthreads();
-    float* cur = c1;
-    float* nxt = c2;
-    for (int it = 1; it < sweeps; ++it) {
-        if (clive) {
-            float xo = 0.f;
-            if (cd > 0.f) {
-                const float x0 = cur[cq];
-                float a = rn_mul(cd, x0);
-                if (cin & 1u) a = rn_fma(cxm, cur[cq - 1], a);
-                if (cin & 2u) a = rn_fma(cxp, cur[cq + 1], a);
-                if (cin & 4u) a = rn_fma(cym, cur[cq - gc.s1], a);
-                if (cin & 8u) a = rn_fma(cyp, cur[cq + gc.s1], a);
-                if (cin & 16u) a = rn_fma(czm, cur[cq - gc.s2], a);
-                if (cin & 32u) a = rn_fma(czp, cur[cq + gc.s2], a);
-                xo = rn_add(x0, mg_div(rn_mul(omega, rn_sub(cbq, a)), cd));
-            }
-            nxt[cq] = xo;
-        }
-        __syncthreads();
-        float* t = cur;
-        cur = nxt;
-        nxt = t;
-    }
     // prolongation (x + P e) and a sweep, then the last sweep into global memory
+    {
+        const float* e = sm.c[0] + (fi >> 1) + 8 * (fj >> 1) + 64 * (k0 >> 1);
 #pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int c = fc[m];
-        if (c < 0) continue;
-        const int k = fk0 + kBottomPlanes * m;
-        s1[c] = s2[c] + cur[(fi >> 1) + gc.s1 * (fj >> 1) + gc.s2 * (k >> 1)];
+        for (int m = 0; m < C; ++m) x[m] = A.live[m] ? x[m] + e[64 * (m / 2)] : 0.f;
     }
-    __syncthreads();
+    put(sm.v[0]);
+    sweep(sm.v[0], w1);
+    put(sm.v[1]);
+    sweep(sm.v[1], w2);
 #pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int c = fc[m];
-        if (c < 0) continue;
-        const St7<float> st = dense_st7(sr, s1, c, fin[m], gf);
-        float xo = 0.f;
-        if (st.d > 0.f) xo = rn_add(st.v0, mg_div(rn_mul(w1, rn_sub(sb[c], apply7(st))), st.d));
-        s2[c] = xo;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int m = 0; m < kBottomCells; ++m) {
-        const int c = fc[m];
-        if (c < 0) continue;
-        const St7<float> st = dense_st7(sr, s2, c, fin[m], gf);
-        float xo = 0.f;
-        if (st.d > 0.f) xo = rn_add(st.v0, mg_div(rn_mul(w2, rn_sub(sb[c], apply7(st))), st.d));
-        xf[c] = xo;
-    }
+    for (int m = 0; m < C; ++m)
+        if (A.live[m]) xf[fi + gf.s1 * fj + gf.s2 * (k0 + m)] = x[m];
 }
 
 __global__ void __launch_bounds__(kBottomThreads) mg_bottom_kernel(LGeom gf, const float4* __restrict__ recf,
                                                                    const float* __restrict__ bf,
                                                                    float* __restrict__ xf, LGeom gc,
-                                                                   const float4* __restrict__ recc, int sweeps,
+                                                                   const float4* __restrict__ recc,
                                                                    const Scalars* s) {
     extern __shared__ __align__(16) unsigned char bottom_smem[];
-    bottom_cycle(gf, recf, bf, xf, gc, recc, sweeps, bottom_smem, [&] {
+    bottom_cycle<8>(gf, recf, bf, xf, gc, recc, bottom_smem, [&] {
         pdl_wait();
         pdl_trigger();
         return !s->done;
@@ -1779,7 +1764,7 @@ __global__ void __launch_bounds__(kBottomThreads) mg_bottom_kernel(LGeom gf, con
 // (ld.global.cg).  Every barrier wait is bounded: a CTA that gives up marks the solve as failed
 // (fault, bad, done) and leaves; the other CTAs' waits then run out too.
 constexpr int kCoarseMaxLevels = 16;
-constexpr int kCoopQuads = kBottomThreads / 128;  // restriction quads per CTA
+constexpr int kCoopQuads = kCycleThreads / 128;  // restriction quads per CTA
 constexpr long long kBarrierPolls = 1ll << 21;    // past the first 4096, each poll sleeps ~100 ns: ~0.2 s
 
 struct CoarseLevel {
@@ -1833,7 +1818,7 @@ __device__ __forceinline__ bool coarse_grid_barrier(unsigned* bar, unsigned nblo
     return ok_s != 0;
 }
 
-__global__ void __launch_bounds__(kBottomThreads, 1) mg_coarse_cycle_kernel(const __grid_constant__ CoarseCycle a,
+__global__ void __launch_bounds__(kCycleThreads, 1) mg_coarse_cycle_kernel(const __grid_constant__ CoarseCycle a,
                                                                             Scalars* s) {
     if (s->done) return;  // read by every CTA before any can change it: all leave, or none
     extern __shared__ __align__(16) unsigned char bottom_smem[];
@@ -1863,7 +1848,7 @@ __global__ void __launch_bounds__(kBottomThreads, 1) mg_coarse_cycle_kernel(cons
     if (blockIdx.x == 0) {
         const CoarseLevel& F = a.lv[a.pre_end];
         const CoarseLevel& C = a.lv[a.pre_end + 1];
-        bottom_cycle(F.g, F.rec, F.b, F.x, C.g, C.rec, a.sweeps, bottom_smem, now);
+        bottom_cycle<4>(F.g, F.rec, F.b, F.x, C.g, C.rec, bottom_smem, now);
     }
     for (int l = a.pre_end - 1; l >= a.from; --l) {
         const CoarseLevel& F = a.lv[l];
@@ -2039,7 +2024,7 @@ static bool coarse_fused_usable(const el_ctx* ctx, int L) {
 
 static int coarse_cycle_grid(const el_ctx* ctx, const SegList& seg_from) {
     const long long cap = (long long)ctx->num_sms * ctx->coarse_per_sm;
-    const long long want = (seg_from.total + kBottomThreads / 32 - 1) / (kBottomThreads / 32);
+    const long long want = (seg_from.total + kCycleThreads / 32 - 1) / (kCycleThreads / 32);
     return (int)std::max<long long>(1, std::min(cap, want));
 }
 
@@ -2051,12 +2036,11 @@ static int launch_coarse_cycle(el_ctx* ctx, std::vector<MGLevel<float>>& mg, int
     }
     a.from = from;
     a.pre_end = pre_end;
-    a.sweeps = kCoarsestSweeps;
     a.bar = ctx->coarse_bar;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(coarse_cycle_grid(ctx, mg[from].seg), 1, 1);
-    cfg.blockDim = dim3(kBottomThreads, 1, 1);
-    cfg.dynamicSmemBytes = bottom_smem_bytes();
+    cfg.blockDim = dim3(kCycleThreads, 1, 1);
+    cfg.dynamicSmemBytes = (int)sizeof(BottomSmem);
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -2154,10 +2138,9 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
             MGLevel<V>& C = mg[L - 1];
             // reads the level's records and b and the coarsest records; writes the level's x
             ProfScope prof(ctx, EL_KC_MG_COARSE, cells(F) * (sizeof(RC) + 2 * vs) + cells(C) * sizeof(RC));
-            launch_dependent(ctx, mg_bottom_kernel, dim3(1), dim3(kBottomThreads), bottom_smem_bytes(),
+            launch_dependent(ctx, mg_bottom_kernel, dim3(1), dim3(kBottomThreads), (int)sizeof(BottomSmem),
                              make_geom(F.n0, F.n1, F.n2), (const float4*)F.rec, (const float*)F.b, F.x,
-                             make_geom(C.n0, C.n1, C.n2), (const float4*)C.rec, (int)kCoarsestSweeps,
-                             (const Scalars*)s);
+                             make_geom(C.n0, C.n1, C.n2), (const float4*)C.rec, (const Scalars*)s);
             ++launched;
         }
     } else {
@@ -2851,7 +2834,7 @@ int setup_solver_storage(el_ctx* ctx, int solver) {
     }
     if (solver == EL_SOLVER_MIXED && !ctx->x32) {
         EL_CUDA_TRY(ctx, cudaFuncSetAttribute(mg_bottom_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              bottom_smem_bytes()));
+                                              (int)sizeof(BottomSmem)));
         // the fused coarse cycle: 1024-thread CTAs, all resident, where cooperative launches
         // exist; otherwise the per-level launches stay in use
         int coop = 0;
@@ -2859,10 +2842,10 @@ int setup_solver_storage(el_ctx* ctx, int solver) {
         ctx->coarse_per_sm = 0;
         if (coop) {
             EL_CUDA_TRY(ctx, cudaFuncSetAttribute(mg_coarse_cycle_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  bottom_smem_bytes()));
+                                                  (int)sizeof(BottomSmem)));
             int per_sm = 0;
             EL_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mg_coarse_cycle_kernel,
-                                                                          kBottomThreads, bottom_smem_bytes()));
+                                                                          kCycleThreads, (int)sizeof(BottomSmem)));
             ctx->coarse_bar = (unsigned*)ctx_alloc(ctx, 64);
             if (!ctx->coarse_bar) return set_error(ctx, EL_ERR_OUT_OF_MEMORY, "coarse cycle barrier");
             ctx->coarse_per_sm = per_sm;
