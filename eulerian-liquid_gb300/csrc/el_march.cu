@@ -30,7 +30,7 @@
 //   PROLONG   one sweep from x + P e (e = the coarse correction)
 //   LAST      the last sweep, and r.z for beta
 // The expressions and their order are those of el_solve.cu's dir_spmv_rec_kernel,
-// update_kernel, smooth_kernel and restrict_kernel; only the dot products' summation order
+// update_kernel, smooth_kernel and restrict_quad_kernel; only the dot products' summation order
 // differs (per CTA instead of per segment warp).
 //
 // Conditions (el::march_supported): the finest level's rows are a multiple of 16 bytes (ni a

@@ -1320,75 +1320,26 @@ __global__ void __launch_bounds__(kSegThreads) smooth_kernel(LGeom g, SegArg seg
     }
 }
 
-// Residual of a level summed onto the coarse right-hand side (R = P^T), one warp per active
-// coarse segment: the warp walks the 64 x 2 x 2 fine cells under it one fine row segment at a
-// time (one fine cell per lane, coalesced), the i-pairs are summed by shuffle.  Used from the
-// finest level, where the grid of warps is capped well below the number of coarse segments.
-template <typename V, typename R>
-__global__ void __launch_bounds__(kSegThreads, sizeof(V) == 4 ? 5 : 4) restrict_kernel(LGeom g, const R* __restrict__ A, const V* __restrict__ b,
-                                                               const V* __restrict__ x, LGeom gc, SegArg cseg,
-                                                               V* __restrict__ bc, V* __restrict__ tc,
-                                                               const V* __restrict__ rdc, const Scalars* s) {
-    const int nseg = *cseg.count;
-    pdl_wait();
-    pdl_trigger();
-    if (s->done) return;
-    const RecLoad<V, R> recf{A};
-    auto rawf = [&](int q, int, int, int) -> V { return x[q]; };
-    auto valf = [](V raw, const Co<V>&) -> V { return raw; };
-    const int lane = threadIdx.x & 31;
-    const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int qs = warp_global; qs < nseg; qs += nwarps) {
-        const int4 sd = cseg.desc[qs];
-        const int I0 = sd.y, J = sd.z, K = sd.w;
-        V sum[2] = {V(0), V(0)};  // fine i in [2*I0, 2*I0+32) and [2*I0+32, 2*I0+64)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = 2 * I0 + 32 * h + lane;
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk)
-#pragma unroll
-                for (int jj = 0; jj < 2; ++jj) {
-                    const int j = 2 * J + jj, k = 2 * K + kk;
-                    // warp-uniform: the row exists for all lanes or for none
-                    if (j >= g.n1 || k >= g.n2) continue;
-                    const bool live = i < g.n0;
-                    const int c = i + g.s1 * j + g.s2 * k;
-                    const St7<V> st = gather7<V, false>(g, c, i, j, k, live, lane, recf, rawf, valf);
-                    if (live && positive(st.d)) sum[h] += rn_sub(b[c], apply7(st));
-                }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const V pair = sum[h] + __shfl_down_sync(kFull, sum[h], 1);
-            const int I = I0 + 16 * h + (lane >> 1);
-            const int q = I + gc.s1 * J + gc.s2 * K;
-            if ((lane & 1) == 0 && I < gc.n0 && EL_IN(q, (long long)gc.s2 * gc.n2, 31)) {
-                bc[q] = pair;
-                if (sizeof(V) == 8) tc[q] = rn_mul(rn_mul(V(kSweep1), pair), rdc[q]);
-            }
-        }
-    }
-}
-
-// The same below the finest level, where the coarse segments are few: a quad of four
+// Residual of a level summed onto the coarse right-hand side (R = P^T): a quad of four
 // warps takes one active coarse segment: warp (kk, jj) of the quad walks the fine row
 // (2J + jj, 2K + kk) under it, 64 fine cells as two 32-cell halves (one fine cell per lane,
-// coalesced), and sums the i-pairs by shuffle; the quad then adds its four rows in a fixed order
-// through shared memory (deterministic).  Four rows in flight per coarse segment instead of
-// eight gathers in sequence: the kernel is bound by the latency of the gathers.
+// coalesced); the quad then adds its four rows in a fixed order through shared memory
+// (deterministic).  Four rows in flight per coarse segment: the kernel is bound by the latency of
+// the gathers.  The finest level (FINEST) sums a cell's column over the rows before the i-pairs, the
+// other levels the pairs of a row first.  A warp a coarse segment, eight gathers in sequence, was as
+// fast on the finest level of 150 cells an axis and slower below: solve of 75 x 62 x 53 1.02 -> 0.96 ms,
+// of 48^3 0.72 -> 0.67 (finest level: 10 -> 4 us a launch).
 constexpr int kQuadsPerBlock = kSegThreads / 128;
 
 // The quads' walk: quad `quad` of `nquads`, the block's quad quad_b (named barrier 1 + quad_b),
 // row `sub` of it; part = the block's [quads][4][2][16] sums in shared memory; start() as for
 // smooth_segments.
-template <typename V, typename R, bool COH = false, typename Start>
+template <typename V, typename R, bool FINEST, bool COH = false, typename Start>
 __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* __restrict__ A,
                                                        const V* __restrict__ b, const V* __restrict__ x,
                                                        const LGeom& gc, const SegArg& cseg, V* __restrict__ bc,
                                                        V* __restrict__ tc, const V* __restrict__ rdc,
-                                                       V (*part)[4][2][16], int quad, int nquads, int quad_b,
+                                                       V (*part)[4][2][FINEST ? 32 : 16], int quad, int nquads, int quad_b,
                                                        int sub, Start&& start) {
     const RecLoad<V, R> recf{A};
     auto rawf = [&](int q, int, int, int) -> V { return ldv<COH>(x, q); };
@@ -1434,15 +1385,22 @@ __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* 
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const V pair = sum[h] + __shfl_down_sync(kFull, sum[h], 1);
-            if ((lane & 1) == 0) part[quad_b][sub][h][lane >> 1] = pair;
+            if constexpr (FINEST) {
+                part[quad_b][sub][h][lane] = sum[h];
+            } else {
+                const V pair = sum[h] + __shfl_down_sync(kFull, sum[h], 1);
+                if ((lane & 1) == 0) part[quad_b][sub][h][lane >> 1] = pair;
+            }
         }
         // the quad's four warps meet on their own named barrier (1 + quad in the block)
         asm volatile("bar.sync %0, %1;" ::"r"(1 + quad_b), "r"(128) : "memory");
         if (sub == 0) {
             const int h = lane >> 4, q = lane & 15;
-            const V tot = ((part[quad_b][0][h][q] + part[quad_b][1][h][q]) + part[quad_b][2][h][q]) +
-                          part[quad_b][3][h][q];
+            auto rows = [&](int n) {
+                return ((part[quad_b][0][h][n] + part[quad_b][1][h][n]) + part[quad_b][2][h][n]) +
+                       part[quad_b][3][h][n];
+            };
+            const V tot = FINEST ? rows(2 * q) + rows(2 * q + 1) : rows(q);
             const int I = I0 + 16 * h + q;
             const int o = I + gc.s1 * J + gc.s2 * K;
             if (I < gc.n0 && EL_IN(o, (long long)gc.s2 * gc.n2, 32)) {
@@ -1458,16 +1416,16 @@ __device__ __forceinline__ void restrict_quad_segments(const LGeom& g, const R* 
     }
 }
 
-template <typename V, typename R>
+template <typename V, typename R, bool FINEST>
 __global__ void __launch_bounds__(kSegThreads, 4) restrict_quad_kernel(LGeom g, const R* __restrict__ A,
                                                                     const V* __restrict__ b, const V* __restrict__ x,
                                                                     LGeom gc, SegArg cseg, V* __restrict__ bc,
                                                                     V* __restrict__ tc, const V* __restrict__ rdc,
                                                                     const Scalars* s) {
-    __shared__ V part[kQuadsPerBlock][4][2][16];
+    __shared__ V part[kQuadsPerBlock][4][2][FINEST ? 32 : 16];
     const int wb = threadIdx.x >> 5;                  // warp in the block
     const int quad_b = wb >> 2, sub = wb & 3;         // quad in the block, row of the quad
-    restrict_quad_segments<V, R>(g, A, b, x, gc, cseg, bc, tc, rdc, part, blockIdx.x * kQuadsPerBlock + quad_b,
+    restrict_quad_segments<V, R, FINEST>(g, A, b, x, gc, cseg, bc, tc, rdc, part, blockIdx.x * kQuadsPerBlock + quad_b,
                                  gridDim.x * kQuadsPerBlock, quad_b, sub, [&] {
                                      pdl_wait();
                                      pdl_trigger();
@@ -1841,7 +1799,7 @@ __global__ void __launch_bounds__(kCycleThreads, 1) mg_coarse_cycle_kernel(const
         smooth_segments<float, float4, SM_ZERO2, DOT_NONE, true>(F.g, F.seg, F.rec, F.b, nullptr, F.g, nullptr, F.x, nullptr,
                                                                  wg, nw, now);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
-        restrict_quad_segments<float, float4, true>(F.g, F.rec, F.b, F.x, C.g, C.seg, C.b, nullptr, nullptr, part, quad, nquads,
+        restrict_quad_segments<float, float4, false, true>(F.g, F.rec, F.b, F.x, C.g, C.seg, C.b, nullptr, nullptr, part, quad, nquads,
                                                     quad_b, sub, now);
         if (!coarse_grid_barrier(a.bar, nblk)) return fail();
     }
@@ -1880,15 +1838,6 @@ static int dot_blocks(el_ctx* ctx, void (*kernel)(KArgs...), long long total_seg
 }
 
 static SegArg seg_arg(const SegList& l) { return SegArg{l.desc, l.count}; }
-
-// The finest level's restriction is bound by the latency of its gathers: as many warps as can
-// be resident (five CTAs of 256 threads per SM at its FP32 register budget), so that each walks a
-// short chain of coarse segments.
-static int restrict_blocks(el_ctx* ctx, long long total_segments) {
-    const long long warps = (long long)ctx->num_sms * 5 * (kSegThreads / 32);
-    const long long need = std::max<long long>(1, std::min<long long>(total_segments, warps));
-    return (int)((need * 32 + kSegThreads - 1) / kSegThreads);
-}
 
 // Cells a segment kernel of multigrid level `level` visits (for the byte counts of profiled
 // launches): the active segments' cells, as read back by record_active(), else `full`.
@@ -2109,16 +2058,15 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
             // reads b, x and records; writes the coarse b
             ProfScope prof(ctx, l == 0 ? EL_KC_RESTRICT : EL_KC_MG_COARSE, act(l, F) * (2 * vs + rb) + act(l + 1, C) * vs);
             const LGeom gf = make_geom(F.n0, F.n1, F.n2), gc = make_geom(C.n0, C.n1, C.n2);
-            if (l == 0)
-                launch_dependent(ctx, restrict_kernel<V, R0>, dim3(restrict_blocks(ctx, C.seg.total)), dim3(kSegThreads),
-                                 0, gf, (const R0*)F.rec, (const V*)F.b, (const V*)F.x, gc, seg_arg(C.seg), C.b, C.t,
-                                 (const V*)C.rd, (const Scalars*)s);
+            auto quads = [&](auto kernel, const auto* rec) {
+                const int blocks = one_wave(ctx, kernel, kSegThreads, seg_blocks(ctx, 4 * C.seg.total));
+                launch_dependent(ctx, kernel, dim3(blocks), dim3(kSegThreads), 0, gf, rec, (const V*)F.b, (const V*)F.x,
+                                 gc, seg_arg(C.seg), C.b, C.t, (const V*)C.rd, (const Scalars*)s);
+            };
+            if (l > 0)
+                quads(restrict_quad_kernel<V, RC, false>, (const RC*)F.rec);
             else
-                launch_dependent(ctx, restrict_quad_kernel<V, RC>,
-                                 dim3(one_wave(ctx, restrict_quad_kernel<V, RC>, kSegThreads,
-                                               seg_blocks(ctx, 4 * C.seg.total))),
-                                 dim3(kSegThreads), 0, gf, (const RC*)F.rec, (const V*)F.b, (const V*)F.x, gc,
-                                 seg_arg(C.seg), C.b, C.t, (const V*)C.rd, (const Scalars*)s);
+                quads(restrict_quad_kernel<V, R0, true>, (const R0*)F.rec);
         }
         launched += 2;
     }
