@@ -560,6 +560,24 @@ __global__ void __launch_bounds__(kDotThreads<V>) dir_spmv_rec_kernel(LGeom g, S
     }
 }
 
+// the end of an update: |r|^2 from the threads' shares, and whether it is small enough
+template <typename V>
+__device__ __forceinline__ void update_done(DotAcc<V> part, Scalars* s, double* partials, unsigned* counter) {
+    double acc[1] = {(double)part};
+    double tot[1];
+    if (grid_sum<1, kDotThreads<V>>(acc, partials, counter, tot)) {
+        s->rr = tot[0];
+        const int iter = s->iter + 1;
+        s->iter = iter;
+        if (!finite_d(tot[0])) {
+            s->bad = 1;
+            s->done = 1;
+        } else if (tot[0] < s->thresh || iter >= s->iter_limit) {
+            s->done = 1;
+        }
+    }
+}
+
 // K2: x += alpha p ; r -= alpha Ap ; |r|^2; FP64 also t = the V-cycle's first sweep from zero.
 template <typename V>
 __global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg seg, V* __restrict__ x,
@@ -612,19 +630,7 @@ __global__ void __launch_bounds__(kDotThreads<V>) update_kernel(LGeom g, SegArg 
         if (la) finish(ca, pa, apa, xa, ra);
         if (lb) finish(cb, pb, apb, xb, rb);
     }
-    double acc[1] = {(double)part};
-    double tot[1];
-    if (grid_sum<1, kDotThreads<V>>(acc, partials, counter, tot)) {
-        s->rr = tot[0];
-        const int iter = s->iter + 1;
-        s->iter = iter;
-        if (!finite_d(tot[0])) {
-            s->bad = 1;
-            s->done = 1;
-        } else if (tot[0] < s->thresh || iter >= s->iter_limit) {
-            s->done = 1;
-        }
-    }
+    update_done<V>(part, s, partials, counter);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1288,6 +1294,63 @@ __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegAr
         rec = load_rec7<V, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
     }
     return part;
+}
+
+// K2 of the FP32 solver and the V-cycle's first kernel in one: x += alpha p, r_out = r - alpha Ap, |r|^2,
+// and z = two sweeps from zero on r_out, which is formed again at the points of the stencil (so r_out
+// is another buffer).  The two are bound by launch and load latency on the scenes that do not take the
+// tile kernels (which do the same).  Mixed solve of 75 x 62 x 53 cells 0.96 -> 0.90 ms, 48^3 0.67 -> 0.64;
+// up to two waves of warps: 96^3 1.06 -> 1.03, 110 x 127 x 118 and 151 x 97 x 133 the same, and twelve
+// scenes at once 8.95 -> 9.05 ms, where its second reading of r and Ap is not hidden.
+template <typename R>
+__global__ void __launch_bounds__(kDotThreads<float>) update_smooth_kernel(LGeom g, SegArg seg, const R* __restrict__ A,
+                                                                          float* __restrict__ x,
+                                                                          const float* __restrict__ r,
+                                                                          float* __restrict__ r_out,
+                                                                          const float* __restrict__ p,
+                                                                          const float* __restrict__ ap,
+                                                                          float* __restrict__ z, Scalars* s,
+                                                                          double* partials, unsigned* counter) {
+    const RecLoad<float, R> recf{A};
+    const int lane = threadIdx.x & 31;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    int qs = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nseg = *seg.count;
+    int4 sd = qs < nseg ? seg.desc[qs] : make_int4(0, g.n0, 0, 0);
+    Near7 nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+    Rec7<float> rec = load_rec7<float, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+    pdl_wait();
+    pdl_trigger();
+    if (s->done) return;
+    const float alpha = (float)s->alpha, w1 = (float)kSweep1, w2 = (float)kSweep2;
+    float part = 0.f;
+    auto rawf = [&](int q, int, int, int) -> float2 { return make_float2(r[q], ap[q]); };
+    auto residual = [&](float2 v) -> float { return v.x - alpha * v.y; };
+    auto valf = [&](float2 v, const Co<float>& c) -> float {
+        return positive(c.d) ? mg_div(rn_mul(w1, residual(v)), c.d) : 0.f;
+    };
+    while (qs < nseg) {
+        const bool live = sd.y + lane < g.n0;
+        const int c = sd.x + lane;
+        const auto raw = load_raw7(g, nb, c, 0, 0, 0, live, rawf);
+        const float xc = live ? x[c] : 0.f, pc = live ? p[c] : 0.f;
+        const St7<float> st = value7<float>(nb, rec, raw, live, lane, valf);
+        if (live) {
+            const float rc = residual(raw.a0);
+            float zc = 0.f;
+            if (positive(st.d)) zc = rn_add(st.v0, mg_div(rn_mul(w2, rn_sub(rc, apply7(st))), st.d));
+            x[c] = xc + alpha * pc;
+            r_out[c] = rc;
+            z[c] = zc;
+            part += rc * rc;
+        }
+        qs += nwarps;
+        if (qs >= nseg) break;
+        sd = seg.desc[qs];
+        nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
+        rec = load_rec7<float, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+    }
+    update_done<float>(part, s, partials, counter);
 }
 
 template <typename V, typename R, int MODE, int DOT>
@@ -2003,9 +2066,10 @@ static int launch_coarse_cycle(el_ctx* ctx, std::vector<MGLevel<float>>& mg, int
 // z = M^-1 r with r = mg[0].b and z = mg[0].x; dot = DOT_INIT or DOT_BETA.  R0 / RC are the
 // record types of the finest / coarse levels.  from > 0: the levels below `from` only (level
 // from - 1 restricted onto mg[from].b before, and prolonged from mg[from].x after, by the caller).
+// smoothed: the finest level's two sweeps from zero are in mg[0].x already.
 template <typename V, typename R0, typename RC>
 static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegList& seg0, Scalars* s, int dot,
-                          int from = 0) {
+                          int from = 0, bool smoothed = false) {
     int launched = 0;
     const int L = (int)mg.size();
     auto segof = [&](int l) -> const SegList& { return l == 0 ? seg0 : mg[l].seg; };
@@ -2043,7 +2107,7 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
         MGLevel<V>& F = mg[l];
         MGLevel<V>& C = mg[l + 1];
         const double rb = l == 0 ? sizeof(R0) : sizeof(RC);
-        {
+        if (l > 0 || !smoothed) {
             // reads b and records (FP64: t and rd); writes x
             ProfScope prof(ctx, l == 0 ? EL_KC_SMOOTH : EL_KC_MG_COARSE, act(l, F) * ((vs == 8 ? 4 : 2) * vs + rb));
             // the two sweeps from zero; FP64: the first is in t already
@@ -2053,6 +2117,7 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
                 launch_smooth<V, R0, mode, DOT_NONE>(ctx, F, segof(l), first, nullptr, F.x, s);
             else
                 launch_smooth<V, RC, mode, DOT_NONE>(ctx, F, segof(l), first, nullptr, F.x, s);
+            ++launched;
         }
         {
             // reads b, x and records; writes the coarse b
@@ -2068,7 +2133,7 @@ static int enqueue_vcycle(el_ctx* ctx, std::vector<MGLevel<V>>& mg, const SegLis
             else
                 quads(restrict_quad_kernel<V, R0, true>, (const R0*)F.rec);
         }
-        launched += 2;
+        ++launched;
     }
     if (coop_from >= 0) {
         if constexpr (kBottomType) {
@@ -2197,10 +2262,11 @@ static int poll(el_ctx* ctx, Scalars* host_copy, int which) {
     return EL_OK;
 }
 
-// One PCG iteration of a multigrid-preconditioned solve (record operator A).
+// One PCG iteration of a multigrid-preconditioned solve (record operator A).  The direction alternates
+// between two buffers, in FP32 the residual too (mg[0].b follows it).
 template <typename V, typename RA, typename R0, typename RC>
-static int enqueue_mg_iteration(el_ctx* ctx, const RA* A, V* x, V* r, V* z, V*& p, V*& p_alt, V* ap, Scalars* s,
-                                int first, std::vector<MGLevel<V>>& mg) {
+static int enqueue_mg_iteration(el_ctx* ctx, const RA* A, V* x, V*& r, V*& r_alt, V* z, V*& p, V*& p_alt, V* ap,
+                                Scalars* s, int first, std::vector<MGLevel<V>>& mg) {
     const LGeom g = make_geom(ctx->ni, ctx->nj, ctx->nk);
     const SegList& seg = ctx->seg0;
     const double N = active_cells(ctx, 0, (double)ctx->ni * ctx->nj * ctx->nk), vs = sizeof(V);
@@ -2213,6 +2279,18 @@ static int enqueue_mg_iteration(el_ctx* ctx, const RA* A, V* x, V* r, V* z, V*& 
                          ctx->counter);
     }
     std::swap(p, p_alt);
+    if constexpr (sizeof(V) == 4) {
+        // (while kernel classes are timed, the update and the sweeps go as the kernels of their classes)
+        if (mg.size() > 1 && seg.total <= 128ll * ctx->num_sms && ctx->prof_mask == 0) {
+            auto kernel = update_smooth_kernel<R0>;
+            launch_dependent(ctx, kernel, dim3(dot_blocks<V>(ctx, kernel, seg.total)), dim3(kDotThreads<V>), 0, g,
+                             seg_arg(seg), (const R0*)mg[0].rec, x, (const V*)r, r_alt, (const V*)p, (const V*)ap, z, s,
+                             ctx->partials, ctx->counter);
+            std::swap(r, r_alt);
+            mg[0].b = r;
+            return 2 + enqueue_vcycle<V, R0, RC>(ctx, mg, seg, s, DOT_BETA, 0, true);
+        }
+    }
     {
         // reads x, r, p, Ap; writes x, r
         ProfScope prof(ctx, EL_KC_UPDATE, N * vs * 6);
@@ -2447,10 +2525,11 @@ static int solve_t(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st) 
         first_sweep_kernel<<<seg_blocks(ctx, ctx->seg0.total), kSegThreads, 0, ctx->stream>>>(
             g, seg_arg(ctx->seg0), ctx->r64, mg[0].rd, mg[0].t);
         ctx->launches += 1 + enqueue_vcycle<double, Rec64, Rec64>(ctx, mg, ctx->seg0, s0, DOT_INIT);
+        double* r = ctx->r64;
         double* p = ctx->p64;
         double* p_alt = ctx->p64b;
         rc = run_iterations(ctx, EL_SOLVER_MG_FP64, 0, prm.max_iter, check, h, [&](int first, int, bool) {
-            return enqueue_mg_iteration<double, Rec64, Rec64, Rec64>(ctx, ctx->A64rec, ctx->x64, ctx->r64, ctx->z64, p,
+            return enqueue_mg_iteration<double, Rec64, Rec64, Rec64>(ctx, ctx->A64rec, ctx->x64, r, r, ctx->z64, p,
                                                                     p_alt, ctx->ap64, s0, first, mg);
         });
         st->iterations = h->iter;
@@ -2502,7 +2581,7 @@ static int solve_t(el_ctx* ctx, const el_solve_params& prm, el_solve_stats* st) 
                 ctx->launches += enqueue_vcycle<float, ushort4, float4>(ctx, mg, ctx->seg0, s1, DOT_INIT);
             rc = run_iterations(ctx, EL_SOLVER_MIXED, 1, prm.max_iter - inner_total, check, &hi, [&](int first, int, bool) {
                 if (march) return enqueue_march_iteration(ctx, p, p_alt, r, r_alt, s1, first, mg);
-                return enqueue_mg_iteration<float, float4, ushort4, float4>(ctx, ctx->A32, ctx->x32, ctx->r32, ctx->z32,
+                return enqueue_mg_iteration<float, float4, ushort4, float4>(ctx, ctx->A32, ctx->x32, r, r_alt, ctx->z32,
                                                                             p, p_alt, ctx->ap32, s1, first, mg);
             });
             if (rc != EL_OK) break;
@@ -2650,7 +2729,7 @@ static int enqueue_solve_device_t(el_ctx* ctx, const el_solve_params& prm, int k
         ctx->partials, ctx->counter);
     auto iteration = [&](int first) {
         if (march) return enqueue_march_iteration(ctx, p, p_alt, r, r_alt, s1, first, mg);
-        return enqueue_mg_iteration<float, float4, ushort4, float4>(ctx, ctx->A32, ctx->x32, ctx->r32, ctx->z32, p,
+        return enqueue_mg_iteration<float, float4, ushort4, float4>(ctx, ctx->A32, ctx->x32, r, r_alt, ctx->z32, p,
                                                                    p_alt, ctx->ap32, s1, first, mg);
     };
     int body = 1 + (march ? enqueue_march_vcycle(ctx, mg, s1, DOT_INIT)
