@@ -167,24 +167,15 @@ struct SegArg {
 constexpr unsigned kFull = 0xffffffffu;
 
 // ---------------------------------------------------------------------------------------
-// segment lists: per-segment activity flag, then an ordered compaction
+// segment lists: per-segment activity flag (seg_flags_diag_kernel, coarsen_kernel), then an ordered
+// compaction.  Each launch costs two to three microseconds whatever its size, so a list of up to
+// kSegDirect segments is one: a block of seg_write_kernel adds up the flags before its own; a longer one
+// has its chunks counted first.  Flags, counts, a scan of the counts and the list in four launches a
+// level took 11 us a level, five levels and more a solve; coarse levels now take one launch, the finest
+// two or three (75 x 62 x 53: 0.90 -> 0.87 ms a solve, 151 x 97 x 133 1.61 -> 1.56).
 
 constexpr int kSegChunk = 1024;
-
-template <typename R>
-__global__ void seg_flags_rec_kernel(LGeom g, const R* __restrict__ rec, long long total, uint8_t* __restrict__ flags) {
-    const int lane = threadIdx.x & 31;
-    const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long id = w0; id < total; id += nw) {
-        int i, j, k;
-        seg_cell((int)id, g, lane, i, j, k);
-        bool act = false;
-        if (i < g.n0) act = ldrec(rec, i + g.s1 * j + g.s2 * k).d > 0;
-        const unsigned m = __ballot_sync(0xffffffffu, act);
-        if (lane == 0) flags[id] = m ? 1 : 0;
-    }
-}
+constexpr long long kSegDirect = 16 * kSegChunk;
 
 __global__ void seg_flags_diag_kernel(LGeom g, const double* __restrict__ diag, long long total,
                                       uint8_t* __restrict__ flags) {
@@ -217,6 +208,8 @@ __global__ void seg_flags_diag_kernel(LGeom g, const double* __restrict__ diag, 
 
 __global__ void seg_count_kernel(const uint8_t* __restrict__ flags, long long total, int* __restrict__ chunk) {
     __shared__ int sh[8];
+    pdl_wait();
+    pdl_trigger();
     const long long base = (long long)blockIdx.x * kSegChunk;
     int cnt = 0;
     for (int q = threadIdx.x; q < kSegChunk; q += blockDim.x) {
@@ -233,60 +226,45 @@ __global__ void seg_count_kernel(const uint8_t* __restrict__ flags, long long to
     }
 }
 
-// Exclusive scan of the chunk counts in one block of 1024 threads: each thread sums a span of
-// chunks, the span sums are scanned by warp shuffles (within a warp, then over the 32 warp
-// totals), and each thread rewrites its span with running offsets.
-__global__ void seg_scan_kernel(int* __restrict__ chunk, int nchunks, int* __restrict__ total_out) {
-    __shared__ int wsum[32];
-    const int per = (nchunks + blockDim.x - 1) / blockDim.x;
-    const int lo = threadIdx.x * per, hi = min(nchunks, lo + per);
-    int s = 0;
-    for (int q = lo; q < hi; ++q) s += chunk[q];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int x = s;  // inclusive scan within the warp
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-        int v = lane < nw ? wsum[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, v, o);
-            if (lane >= o) v += y;
-        }
-        wsum[lane] = v;  // inclusive over the warps
-    }
-    __syncthreads();
-    int run = x - s + (w > 0 ? wsum[w - 1] : 0);
-    if (threadIdx.x == blockDim.x - 1) *total_out = run + s;
-    for (int q = lo; q < hi; ++q) {
-        const int v = chunk[q];
-        chunk[q] = run;
-        run += v;
-    }
-}
-
 // The descriptors of a chunk's active segments, in order: each warp of the block takes an equal
 // run of the chunk's flags, counts its active ones, and writes them after the counts of the
-// warps before it.
+// warps before it and of the chunks before this one (chunk: their counts; null: from the flags).
+// The last block leaves the list's length.
 __global__ void seg_write_kernel(LGeom g, const uint8_t* __restrict__ flags, long long total,
-                                 const int* __restrict__ chunk, int4* __restrict__ desc) {
-    __shared__ int wcount[32];
+                                 const int* __restrict__ chunk, int4* __restrict__ desc, int* __restrict__ count) {
+    __shared__ int wcount[32], before[32];
+    pdl_wait();
+    pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int span = kSegChunk / nw;
     const long long wb = (long long)blockIdx.x * kSegChunk + (long long)w * span;
-    int cnt = 0;
+    int pre = 0, cnt = 0;
+    if (chunk) {
+        for (int q = threadIdx.x; q < (int)blockIdx.x; q += blockDim.x) pre += chunk[q];
+    } else {
+        const uint4* f4 = reinterpret_cast<const uint4*>(flags);
+        for (int q = threadIdx.x; q < (int)blockIdx.x * (kSegChunk / 16); q += blockDim.x) {
+            const uint4 f = f4[q];  // sixteen flags, each 0 or 1
+            pre += __popc(f.x) + __popc(f.y) + __popc(f.z) + __popc(f.w);
+        }
+    }
     for (int q = 0; q < span; q += 32) {
         const long long id = wb + q + lane;
         cnt += __popc(__ballot_sync(kFull, id < total && flags[id]));
     }
-    if (lane == 0) wcount[w] = cnt;
+    for (int o = 16; o > 0; o >>= 1) pre += __shfl_down_sync(kFull, pre, o);
+    if (lane == 0) {
+        wcount[w] = cnt;
+        before[w] = pre;
+    }
     __syncthreads();
-    int run = chunk[blockIdx.x];
+    int run = 0;
+    for (int v = 0; v < nw; ++v) run += before[v];
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) {
+        int all = run;
+        for (int v = 0; v < nw; ++v) all += wcount[v];
+        *count = all;
+    }
     for (int v = 0; v < w; ++v) run += wcount[v];
     for (int q = 0; q < span; q += 32) {
         const long long id = wb + q + lane;
@@ -333,15 +311,18 @@ __global__ void pack64_kernel(long long n, const double* __restrict__ d, const O
 // Coarse records A_c = 1/2 P^T A P over 2x2x2 blocks.  The FP32 hierarchy (float4 coarse
 // records, built from half4 or float4 records) sums in FP32 -- the eight children's values
 // carry at most 24 significant bits, and FP64 arithmetic runs at a small fraction of the FP32
-// rate on this GPU -- the FP64 hierarchy in FP64.
+// rate on this GPU -- the FP64 hierarchy in FP64.  A warp's 32 coarse cells are a row segment, whose
+// activity flag it writes.
 template <typename RF, typename RC>
 __global__ void coarsen_kernel(LGeom F, const RF* __restrict__ fr, LGeom C, RC* __restrict__ cr,
-                               double* __restrict__ rd) {
+                               double* __restrict__ rd, uint8_t* __restrict__ flags) {
+    pdl_wait();
+    pdl_trigger();
     using A = typename std::conditional<sizeof(RC) == sizeof(float4), float, double>::type;
     const int I = blockIdx.x * blockDim.x + threadIdx.x;
     const int J = blockIdx.y * blockDim.y + threadIdx.y;
     const int K = blockIdx.z;
-    if (I >= C.n0 || J >= C.n1) return;
+    if (J >= C.n1) return;  // a warp is a row's segment
     A d = 0, sx = 0, sy = 0, sz = 0, inner = 0;
     for (int kk = 0; kk < 2; ++kk)
         for (int jj = 0; jj < 2; ++jj)
@@ -358,6 +339,9 @@ __global__ void coarsen_kernel(LGeom F, const RF* __restrict__ fr, LGeom C, RC* 
     // an aggregate coupled to nothing outside it (an enclosed Neumann pocket) has a zero row
     // sum; its diagonal is raised to half the children's, which keeps the operator SPD
     if (d > A(0) && !(dc > A(1e-6) * d)) dc = A(0.5) * d;
+    const unsigned active = __ballot_sync(kFull, I < C.n0 && dc > A(0));
+    if (threadIdx.x == 0) flags[((long long)K * C.n1 + J) * C.nsr + blockIdx.x] = active ? 1 : 0;
+    if (I >= C.n0) return;
     const long long q = I + C.s1 * J + C.s2 * K;
     if constexpr (sizeof(RC) == sizeof(float4))
         cr[q] = make_float4(dc, A(0.5) * sx, A(0.5) * sy, A(0.5) * sz);
@@ -1944,17 +1928,12 @@ static int alloc_seglist(el_ctx* ctx, SegList& l, int n0, int n1, int n2) {
 // compaction of the flags into the ordered id list
 static int enqueue_compact(el_ctx* ctx, SegList& l, const LGeom& g) {
     const int nchunks = (int)((l.total + kSegChunk - 1) / kSegChunk);
-    seg_count_kernel<<<nchunks, 256, 0, ctx->stream>>>(l.flags, l.total, l.chunk);
-    seg_scan_kernel<<<1, 1024, 0, ctx->stream>>>(l.chunk, nchunks, l.count);
-    seg_write_kernel<<<nchunks, 256, 0, ctx->stream>>>(g, l.flags, l.total, l.chunk, l.desc);
-    return 3;
-}
-
-template <typename R>
-static int enqueue_seglist_rec(el_ctx* ctx, SegList& l, const LGeom& g, const R* rec) {
-    ProfScope prof(ctx, EL_KC_OTHER, (double)g.n0 * g.n1 * g.n2 * sizeof(R));
-    seg_flags_rec_kernel<R><<<seg_blocks(ctx, l.total), kSegThreads, 0, ctx->stream>>>(g, rec, l.total, l.flags);
-    return 1 + enqueue_compact(ctx, l, g);
+    const bool direct = l.total <= kSegDirect;
+    if (!direct)
+        launch_dependent(ctx, seg_count_kernel, dim3(nchunks), dim3(256), 0, (const uint8_t*)l.flags, l.total, l.chunk);
+    launch_dependent(ctx, seg_write_kernel, dim3(nchunks), dim3(256), 0, g, (const uint8_t*)l.flags, l.total,
+                     direct ? (const int*)nullptr : (const int*)l.chunk, l.desc, l.count);
+    return direct ? 1 : 2;
 }
 
 static int grid1d(el_ctx* ctx, long long n) {
@@ -2007,11 +1986,14 @@ static int enqueue_coarsen(el_ctx* ctx, std::vector<MGLevel<V>>& mg) {
             ProfScope prof(ctx, EL_KC_MG_COARSE, (double)F.n0 * F.n1 * F.n2 * (l == 0 ? sizeof(R0) : sizeof(RC)) +
                                                      (double)C.n0 * C.n1 * C.n2 * sizeof(RC));
             if (l == 0)
-                coarsen_kernel<R0, RC><<<grid, block, 0, ctx->stream>>>(gf, (const R0*)F.rec, gc, (RC*)C.rec, (double*)C.rd);
+                launch_dependent(ctx, coarsen_kernel<R0, RC>, grid, block, 0, gf, (const R0*)F.rec, gc, (RC*)C.rec,
+                                 (double*)C.rd, C.seg.flags);
             else
-                coarsen_kernel<RC, RC><<<grid, block, 0, ctx->stream>>>(gf, (const RC*)F.rec, gc, (RC*)C.rec, (double*)C.rd);
+                launch_dependent(ctx, coarsen_kernel<RC, RC>, grid, block, 0, gf, (const RC*)F.rec, gc, (RC*)C.rec,
+                                 (double*)C.rd, C.seg.flags);
         }
-        launched += 1 + enqueue_seglist_rec<RC>(ctx, C.seg, gc, (const RC*)C.rec);
+        ProfScope prof(ctx, EL_KC_OTHER, (double)C.seg.total * 17);  // flags read, descriptors written
+        launched += 1 + enqueue_compact(ctx, C.seg, gc);
     }
     return launched;
 }
