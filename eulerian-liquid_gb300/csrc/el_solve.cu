@@ -1234,16 +1234,18 @@ __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegAr
     const V omega = V(MODE == SM_PROLONG ? kSweep1 : kSweep2);
     DotAcc<V> part = 0;
     const RecLoad<V, R> recf{A};
-    // value of the current iterate at a cell, zero on inactive cells
     auto rawf = [&](int q, int qi, int qj, int qk) -> V {
         if (MODE == SM_ZERO2) return ldv<COH>(b, q);
         V v = ldv<COH>(x_in, q);
         if (MODE == SM_PROLONG) v += ldv<COH>(e, (qi >> 1) + gc.s1 * (qj >> 1) + gc.s2 * (qk >> 1));
         return v;
     };
-    auto valf = [&](V raw, const Co<V>& rec) -> V {
-        if (!positive(rec.d)) return V(0);
-        if constexpr (MODE == SM_ZERO2) return mg_div(rn_mul(w_first, raw), rec.d);
+    // the current iterate at a cell.  A stored value is read as it is: it is finite everywhere, and a
+    // coupling with a cell outside the system is zero; so the records of the +y and +z neighbours are
+    // not read for their diagonals (two of five records a cell: last sweep of 151 x 97 x 133 12.3 -> 11.0
+    // us, of a 128^3 level 8.0 -> 7.0)
+    auto valf = [&](V raw, [[maybe_unused]] const Co<V>& rec) -> V {
+        if constexpr (MODE == SM_ZERO2) return positive(rec.d) ? mg_div(rn_mul(w_first, raw), rec.d) : V(0);
         return raw;
     };
     const int lane = threadIdx.x & 31;
@@ -1251,7 +1253,7 @@ __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegAr
     const int nseg = *seg.count;
     int4 sd = qs < nseg ? seg.desc[qs] : make_int4(0, g.n0, 0, 0);
     Near7 nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
-    Rec7<V> rec = load_rec7<V, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+    Rec7<V> rec = load_rec7<V, MODE == SM_ZERO2>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
     if (!start()) return part;
     while (qs < nseg) {
         const bool live = sd.y + lane < g.n0;
@@ -1275,7 +1277,7 @@ __device__ __forceinline__ DotAcc<V> smooth_segments(const LGeom& g, const SegAr
         if (qs >= nseg) break;
         sd = seg.desc[qs];
         nb = near7(g, sd.x + lane, sd.y + lane, sd.z, sd.w, sd.y + lane < g.n0, lane);
-        rec = load_rec7<V, true>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
+        rec = load_rec7<V, MODE == SM_ZERO2>(g, nb, sd.x + lane, sd.y + lane < g.n0, recf);
     }
     return part;
 }
@@ -1337,8 +1339,9 @@ __global__ void __launch_bounds__(kDotThreads<float>) update_smooth_kernel(LGeom
     update_done<float>(part, s, partials, counter);
 }
 
+// (the sweeps with a dot product keep eight blocks an SM: the grid is part of the sum's order)
 template <typename V, typename R, int MODE, int DOT>
-__global__ void __launch_bounds__(kSegThreads) smooth_kernel(LGeom g, SegArg seg, const R* __restrict__ A,
+__global__ void __launch_bounds__(kSegThreads, DOT != DOT_NONE && sizeof(V) == 4 ? 8 : 1) smooth_kernel(LGeom g, SegArg seg, const R* __restrict__ A,
                                                              const V* __restrict__ b, const V* __restrict__ x_in,
                                                              LGeom gc, const V* __restrict__ e,
                                                              V* __restrict__ x_out, const V* __restrict__ rd,
