@@ -176,9 +176,11 @@ __device__ __forceinline__ bool el_in_bounds(long long idx, long long n, unsigne
 #endif
 
 // Programmatic dependent launch: a kernel launched with launch_dependent() may be scheduled
-// while the kernel before it on the stream is still running; its first act is pdl_wait(), which
-// returns once that kernel has completed and its memory operations are visible (at once for a
-// kernel launched the ordinary way).  pdl_trigger() lets the next such kernel be scheduled.
+// while the kernel before it on the stream is still running.  pdl_wait() returns once that kernel has
+// completed and its memory operations are visible (at once for a kernel launched the ordinary way);
+// before it a kernel writes nothing to global memory and reads only what the kernel before does not
+// write.  pdl_trigger() lets the next such kernel be scheduled, and comes after pdl_wait(): so when a
+// kernel starts, every kernel but the one before it has completed.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -312,7 +314,7 @@ struct el_ctx {
 
 namespace el {
 // launch `kernel` on the context's stream; with the context's `dependent_launch` set, as a
-// programmatic dependent launch (the kernel must begin with pdl_wait())
+// programmatic dependent launch (the kernel calls pdl_wait(), see there)
 template <typename... KArgs, typename... Args>
 cudaError_t launch_dependent(const el_ctx* ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                              Args&&... args) {

@@ -133,16 +133,6 @@ struct SegArg {
         const int c = sd.x + lane;                                                \
         const bool live = i < (g).n0;
 
-// the same over an explicit warp numbering (warp wg of nw warps)
-#define SEG_LOOP_ALL_W_BEGIN(seg, g, wg, nw)                                      \
-    const int lane = threadIdx.x & 31;                                            \
-    const int nseg = *(seg).count;                                                \
-    for (int qs = (wg); qs < nseg; qs += (nw)) {                                  \
-        const int4 sd = (seg).desc[qs];                                           \
-        const int i = sd.y + lane, j = sd.z, k = sd.w;                            \
-        const int c = sd.x + lane;                                                \
-        const bool live = i < (g).n0;
-
 // the same, with the next segment's descriptor loaded while the current one is processed (for
 // the kernels whose registers leave room for it)
 #define SEG_LOOP_ALL_PF_BEGIN(seg, g)                                             \
