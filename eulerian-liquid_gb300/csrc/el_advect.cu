@@ -14,6 +14,7 @@
 // shared memory, so that a box holds the clamped grid either way.
 #include <cstring>
 #include <limits>
+#include <type_traits>
 
 #include "el_internal.cuh"
 #include "el_tma.cuh"
@@ -161,8 +162,8 @@ __device__ __forceinline__ bool tri_inside(const GridView<T>& g, int i, int j, i
 }
 
 // the trilinear combination of 8 loaded points: x, then y, then z lerps; FP32 with the z = 0 and
-// z = 1 halves side by side in packed float2 arithmetic (each lane rounded as its scalar lerp)
-template <typename T>
+// z = 1 halves side by side in packed float2 arithmetic.  ZF: the form of its z lerp (LerpForm).
+template <typename T, int ZF = LERP_ANY>
 __device__ __forceinline__ T tri_mix(T fx, T fy, T fz, T c000, T c100, T c010, T c110, T c001, T c101, T c011,
                                      T c111) {
     if constexpr (sizeof(T) == 4) {
@@ -173,7 +174,7 @@ __device__ __forceinline__ T tri_mix(T fx, T fy, T fz, T c000, T c100, T c010, T
         const float2 x0 = lerp2(make_float2(c000, c001), make_float2(c100, c101), fx);
         const float2 x1 = lerp2(make_float2(c010, c011), make_float2(c110, c111), fx);
         const float2 y = lerp2(x0, x1, fy);
-        return lerp1(y.x, y.y, fz);
+        return lerp_form<ZF>(y.x, y.y, fz);
     } else {
         return tri_combine(fx, fy, fz, c000, c100, c010, c110, c001, c101, c011, c111);
     }
@@ -196,7 +197,7 @@ __device__ __forceinline__ T tri_mix(const Tri8<T>& v, T fx, T fy, T fz) {
 }
 
 // trilinear read of the sample's own grid, d cells away from sample (i, j, k)
-template <typename T>
+template <typename T, bool TILED>
 __device__ __forceinline__ T own_at(const GridView<T>& g, int i, int j, int k, const Vec3T<T>& d) {
     int bi, bj, bk;
     T fx, fy, fz;
@@ -206,8 +207,14 @@ __device__ __forceinline__ T own_at(const GridView<T>& g, int i, int j, int k, c
     bi = (int)((unsigned)bi + (unsigned)i);
     bj = (int)((unsigned)bj + (unsigned)j);
     bk = (int)((unsigned)bk + (unsigned)k);
-    if (tri_inside(g, bi, bj, bk)) return tri_mix(tri_load(g, bi, bj, bk), fx, fy, fz);
-    return tri_clamped(g, i, j, k, d.x, d.y, d.z);
+    // FP32: the forms are part of the level set's rounding (level_set_foot)
+    constexpr int X10 = sizeof(T) == 8 ? LERP_ANY : (TILED ? LERP_B : LERP_A);
+    constexpr int X00 = sizeof(T) == 8 ? LERP_ANY : LERP_A, R = sizeof(T) == 8 ? LERP_ANY : LERP_B;
+    if (tri_inside(g, bi, bj, bk)) {
+        const Tri8<T> v = tri_load(g, bi, bj, bk);
+        return tri_combine<X00, X10, R>(fx, fy, fz, v.c[0], v.c[1], v.c[2], v.c[3], v.c[4], v.c[5], v.c[6], v.c[7]);
+    }
+    return tri_clamped<X00, X10, R>(g, i, j, k, d.x, d.y, d.z);
 }
 
 // The clamped gathers of u, v, w for a position outside the grid (or a box): d cells away from sample
@@ -279,18 +286,30 @@ __device__ __forceinline__ Vec3T<T> cell_velocity(const Mac<T>& m, int i, int j,
 }
 
 // The foot point of cell (i, j, k), as the coordinate among the cells that own_at and sample_weno6
-// take: FP64 the displacement, relative to the cell; FP32 the absolute coordinate (relative to
-// index 0).  vel(axes, far) reads the velocity.
+// take after foot_coords: FP64 the displacement, relative to the cell; FP32 the absolute position
+// (relative to index 0).  vel(axes, far, stage) reads the velocity of stage 1 or 2.
+//
+// The FP32 level set is rounded at every operation as it always was: positions are absolute, WENO6
+// combines its three candidates, and which product of a lerp is rounded alone (LerpForm) is the
+// compiler's choice of one build written down.  The projection is why.  The ghost-fluid fractions
+// are ratios of the distances to the surface, so that where a cell lies within 1e-3 dx of it, another
+// rounding of phi, a more exact one too, gives another velocity: a cell with phi = -0.00092 dx, phi moved
+// by 2e-6 dx, has another pressure by 0.07 %, and its faces' v and w are off by 1e-3 of themselves.  Twelve
+// scenes of 0.4 to 2.3 million cells under six seeds, phi from WENO6 relative to its middle
+// candidate: twelve fields off by 1e-4 to 1e-3 at single faces (5e-3 under another seed); with
+// these roundings no field by 1e-4 under eight.  tests/test_gpu_level_set_bits.py holds the bits.
 template <typename T>
 __device__ __forceinline__ int foot_base(int i) {
     return sizeof(T) == 4 ? 0 : i;
 }
+template <int N>
+using Stage = std::integral_constant<int, N>;
 template <typename T, int TRACE, typename F>
 __device__ __forceinline__ Vec3T<T> level_set_foot(const Vec3T<T>& a, int i, int j, int k, T dt, T dx, T inv_dx, F&& vel) {
     if constexpr (sizeof(T) == 8) {
         const Vec3T<T> h{T(0), T(0), T(0)};
         return backtrace_from<T, TRACE>(a, -dt * inv_dx, [&](const Vec3T<T>& d) {
-            return vel(axes_rel(i, j, k, h, d), FarRel<T>{i, j, k, h, d});
+            return vel(axes_rel(i, j, k, h, d), FarRel<T>{i, j, k, h, d}, Stage<1>());
         });
     } else {
         const float h = -dt;
@@ -298,17 +317,30 @@ __device__ __forceinline__ Vec3T<T> level_set_foot(const Vec3T<T>& a, int i, int
         auto step = [](const Vec3T<float>& q, float s, const Vec3T<float>& v) {
             return Vec3T<float>{rn_fma(s, v.x, q.x), rn_fma(s, v.y, q.y), rn_fma(s, v.z, q.z)};
         };
-        auto at = [&](const Vec3T<float>& q) { return vel(axes_abs(q, dx, inv_dx), FarAbs{q, dx, inv_dx}); };
-        const Vec3T<float> b = at(step(p, 0.5f * h, a));
+        auto at = [&](const Vec3T<float>& q, auto stage) { return vel(axes_abs(q, dx, inv_dx), FarAbs{q, dx, inv_dx}, stage); };
+        const Vec3T<float> b = at(step(p, 0.5f * h, a), Stage<1>());
         Vec3T<float> q;
         if constexpr (TRACE == EL_TRACE_RK2) {
             q = step(p, h, b);
         } else {
-            const Vec3T<float> c = at(step(p, 0.75f * h, b));
+            const Vec3T<float> c = at(step(p, 0.75f * h, b), Stage<2>());
             q = step(step(step(p, h * (2.f / 9.f), a), h * (1.f / 3.f), b), h * (4.f / 9.f), c);
         }
-        return Vec3T<float>{coord_abs(q.x, dx, inv_dx).x, coord_abs(q.y, dx, inv_dx).x, coord_abs(q.z, dx, inv_dx).x};
+        return q;
     }
+}
+
+// a coordinate of level_set_foot's point among the cells: FP64 the displacement itself
+template <typename T>
+__device__ __forceinline__ T foot_coord(T p, T dx, T inv_dx) {
+    if constexpr (sizeof(T) == 8)
+        return p;
+    else
+        return rn_mul(rn_sub(p, 0.5f * dx), inv_dx);
+}
+template <typename T>
+__device__ __forceinline__ Vec3T<T> foot_coords(const Vec3T<T>& p, T dx, T inv_dx) {
+    return Vec3T<T>{foot_coord(p.x, dx, inv_dx), foot_coord(p.y, dx, inv_dx), foot_coord(p.z, dx, inv_dx)};
 }
 
 // out(x) = src(trace(x, -dt)) for every sample of src's grid (comp 0: cell centres, 1..3: a face
@@ -325,9 +357,9 @@ __global__ void __launch_bounds__(256) advect_kernel(GridView<T> src, int comp, 
     int bi = i, bj = j, bk = k;
     Vec3T<T> e;
     if (comp == 0) {
-        auto vel = [&](const Axes<T>& a, const auto& far) { return velocity_global(mac, a, far); };
-        const Vec3T<T> a = vel(axes_rel(i, j, k, zero, zero), FarRel<T>{i, j, k, zero, zero});
-        e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, vel);
+        auto vel = [&](const Axes<T>& a, const auto& far, auto) { return velocity_global(mac, a, far); };
+        const Vec3T<T> a = velocity_global(mac, axes_rel(i, j, k, zero, zero), FarRel<T>{i, j, k, zero, zero});
+        e = foot_coords(level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, vel), dx, inv_dx);
         bi = foot_base<T>(i);
         bj = foot_base<T>(j);
         bk = foot_base<T>(k);
@@ -342,7 +374,7 @@ __global__ void __launch_bounds__(256) advect_kernel(GridView<T> src, int comp, 
     if constexpr (SAMPLE == EL_SAMPLE_WENO6)
         r = sample_weno6(src, bi, bj, bk, e.x, e.y, e.z);
     else
-        r = own_at(src, bi, bj, bk, e);
+        r = own_at<T, false>(src, bi, bj, bk, e);
     const int oc = cell_index(src, i, j, k);
     if (EL_IN(oc, (long long)src.n0 * src.n1 * src.n2, 1)) out[oc] = r;
 }
@@ -372,14 +404,14 @@ constexpr int kBoxN = kBoxX * kBoxY * kBoxZ;
 // trilinear sample from a staged box at box-relative floor indices (x, y, z); false when the 8
 // points are not all inside the box.  CHECK = false: the caller knows they are (see
 // advect_velocity_tiled_kernel)
-template <typename T, bool CHECK = true>
+template <typename T, bool CHECK, int ZF = LERP_ANY>
 __device__ __forceinline__ bool staged_lerp(const T* box, int x, int y, int z, T fx, T fy, T fz, T& out) {
     if (CHECK && ((unsigned)x >= (unsigned)(kBoxX - 1) || (unsigned)y >= (unsigned)(kBoxY - 1) ||
                   (unsigned)z >= (unsigned)(kBoxZ - 1)))
         return false;
     const T* p = box + (z * kBoxY + y) * kBoxX + x;
     constexpr int SY = kBoxX, SZ = kBoxX * kBoxY;
-    out = tri_mix(fx, fy, fz, p[0], p[1], p[SY], p[SY + 1], p[SZ], p[SZ + 1], p[SZ + SY], p[SZ + SY + 1]);
+    out = tri_mix<T, ZF>(fx, fy, fz, p[0], p[1], p[SY], p[SY + 1], p[SZ], p[SZ + 1], p[SZ + SY], p[SZ + SY + 1]);
     return true;
 }
 
@@ -389,8 +421,8 @@ struct StagedMac {
     int bx0, by0, bz0;    // grid index of the boxes' first entry
 };
 
-// u, v, w at one position through the staged boxes
-template <typename T, bool CHECK, typename FAR>
+// u, v, w at one position through the staged boxes; ZU, ZV, ZW: the forms of their z lerps
+template <typename T, bool CHECK, int ZU = LERP_ANY, int ZV = LERP_ANY, int ZW = LERP_ANY, typename FAR>
 __device__ __forceinline__ Vec3T<T> velocity_staged(const Mac<T>& m, const StagedMac<T>& b, const Axes<T>& a,
                                                     const FAR& far) {
     auto rel = [](int g, int b0) { return (int)((unsigned)g - (unsigned)b0); };
@@ -398,9 +430,9 @@ __device__ __forceinline__ Vec3T<T> velocity_staged(const Mac<T>& m, const Stage
     const int xc = rel(x.c, b.bx0), xf = rel(x.f, b.bx0), yc = rel(y.c, b.by0), yf = rel(y.f, b.by0);
     const int zc = rel(z.c, b.bz0), zf = rel(z.f, b.bz0);
     Vec3T<T> v;
-    if (!staged_lerp<T, CHECK>(b.box, xf, yc, zc, x.wf, y.wc, z.wc, v.x) && CHECK) v.x = far.template at<0>(m.u);
-    if (!staged_lerp<T, CHECK>(b.box + kBoxN, xc, yf, zc, x.wc, y.wf, z.wc, v.y) && CHECK) v.y = far.template at<1>(m.v);
-    if (!staged_lerp<T, CHECK>(b.box + 2 * kBoxN, xc, yc, zf, x.wc, y.wc, z.wf, v.z) && CHECK)
+    if (!staged_lerp<T, CHECK, ZU>(b.box, xf, yc, zc, x.wf, y.wc, z.wc, v.x) && CHECK) v.x = far.template at<0>(m.u);
+    if (!staged_lerp<T, CHECK, ZV>(b.box + kBoxN, xc, yf, zc, x.wc, y.wf, z.wc, v.y) && CHECK) v.y = far.template at<1>(m.v);
+    if (!staged_lerp<T, CHECK, ZW>(b.box + 2 * kBoxN, xc, yc, zf, x.wc, y.wc, z.wf, v.z) && CHECK)
         v.z = far.template at<2>(m.w);
     return v;
 }
@@ -846,15 +878,17 @@ __global__ void __launch_bounds__(kTileX * kTileY) advect_phi_tiled_kernel(GridV
         const Vec3T<T> a = cell_velocity(mac, i, j, k);
         Vec3T<T> e;
         if (inside)
-            e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, [&](const Axes<T>& q, const auto& far) {
-                return velocity_staged<T, false>(mac, sm, q, far);
+            e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, [&](const Axes<T>& q, const auto& far, auto stage) {
+                constexpr int N = decltype(stage)::value;
+                constexpr int UV = N == 2 ? LERP_A : LERP_B, W = TRACE == EL_TRACE_RK2 ? LERP_A : LERP_B;
+                return velocity_staged<T, false, UV, UV, W>(mac, sm, q, far);
             });
         else
-            e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, [&](const Axes<T>& q, const auto& far) {
+            e = level_set_foot<T, TRACE>(a, i, j, k, dtv, dx, inv_dx, [&](const Axes<T>& q, const auto& far, auto) {
                 return velocity_staged<T, true>(mac, sm, q, far);
             });
         const int oc = cell_index(src, i, j, k);
-        const T r = own_at(src, foot_base<T>(i), foot_base<T>(j), foot_base<T>(k), e);
+        const T r = own_at<T, true>(src, foot_base<T>(i), foot_base<T>(j), foot_base<T>(k), foot_coords(e, dx, inv_dx));
         if (EL_IN(oc, (long long)src.n0 * src.n1 * src.n2, 3)) out[oc] = r;
     }
 }
@@ -866,30 +900,30 @@ __global__ void __launch_bounds__(kTileX * kTileY) advect_phi_tiled_kernel(GridV
 // grid's row pitch allows it (along x it then starts four cells left of the tile, a 16-byte
 // boundary, and holds 40 entries, of which the first is never read).
 //
-// The six-point combination, relative to its middle candidate.  Neighbouring candidates are cubics
+// The smoothness indicators of an x-pass depend only on the six values it reads, not on the
+// sample's fraction, so they are formed once per (row, floor index) of the box (34 floor indices of
+// each row) and shared by every sample whose stencil uses that row segment, instead of being formed
+// by each of the 36 x-passes of every sample.  The y- and z-passes combine per-sample values and are
+// evaluated in full.
+//
+// FP32: an entry is the three reciprocal squares (weno6_sq2) in 16 bytes; the expressions are those of
+// weno6_sq2, weno6_combine2 and, for the z-pass, weno6_eval, so that every sample within a cell of
+// its four planes has the same bits whatever the tile (level_set_foot says why).  Bound by
+// instruction issue; 256^3 1.43 ms (1.07 with the FP64 form below in float, which the bits rule out).
+//
+// FP64: the six-point combination relative to its middle candidate.  Neighbouring candidates are cubics
 // through three common nodes, so they differ by a fourth difference times a fixed polynomial:
 //   p_a - p_b = -D0 (x+1) x (x-1) / 6,   p_c - p_b = D1 x (x-1) (x-2) / 6,
 //   D0 = v4 - 4 v3 + 6 v2 - 4 v1 + v0,   D1 = v5 - 4 v4 + 6 v3 - 4 v2 + v1,
 // and with the nonlinear weights alpha_s = C_s / q_s, q_s = (eps + IS_s)^2, taken relative to the
 // middle one (ra = qb / qa, rc = qb / qc),
 //   sum(alpha p) / sum(alpha) = p_b + (Ka ra D0 + Kc rc D1) / (Cb + Ca ra + Cc rc),
-// Ka = -Ca (x+1) x (x-1) / 6, Kc = Cc x (x-1) (x-2) / 6: one candidate instead of three, and in FP64
-// one division instead of four.  ra, rc, ra D0 and rc D1 of an x-pass depend only on the six
-// values it reads, not on the sample's fraction: they are formed once per (row, floor index) of the
-// box (34 floor indices of each row) and shared by every sample whose stencil uses that row
-// segment, instead of being formed by each of the 36 x-passes of every sample.  In FP32 they are
-// one 16-byte entry {ra, ra D0, rc, rc D1}, so that the numerator and denominator of a pass are two
-// packed multiply-adds; in FP64 {ra, rc} and the plane of D0 (D1 is the next floor index's D0), three
-// doubles an entry.  The y- and z-passes combine per-sample values and are evaluated in full.
+// Ka = -Ca (x+1) x (x-1) / 6, Kc = Cc x (x-1) (x-2) / 6: one candidate instead of three, and one
+// division instead of four.  An entry is {ra, rc} and the plane of D0 (D1 is the next floor index's
+// D0), three doubles.  Bound by the FP64 operations (1400 a sample; 128^3: 11.2 -> 5.6 ms).
 //
-// FP32 is bound by instruction issue and the shared-memory loads (1380 instructions a sample, from
-// 2450; 256^3: 1.48 -> 1.07 ms, the per-sample kernel took 1.03 ms for 203 x 149 x 181 cells that
-// now take 0.45).  FP64 by its FP64 operations (1400 a sample; 128^3: 11.2 -> 5.6 ms, the pipe 88 %
-// busy).
-//
-// A foot point outside the box (a larger dt), and a result that is not finite, takes the global
-// sample_weno6 path: its weights alpha_s stay finite where ratios of the q_s overflow (level-set
-// jumps of 1e6 and more; an FP32 entry whose ratios could lose a weight to flushing is made NaN).
+// A foot point outside the box (a larger dt), and in FP64 a result that is not finite, takes the
+// global sample_weno6 path: its weights alpha_s stay finite where ratios of the q_s overflow.
 constexpr int kWX = 32, kWY = 8;
 constexpr int kWNodes = kWX + 8, kWBY = kWY + 7;  // nodes [tile - 4, tile + 4] x [tile - 3, tile + 4]
 constexpr int kWBases = kWX + 2;               // floor indices [tile - 1, tile + 32]
@@ -899,41 +933,39 @@ struct WenoTile {
     static constexpr int kBZ = WZ + 7;             // nodes [tile - 3, tile + 4] along z
     static constexpr int kRows = kWBY * kBZ;
     // FP32: rows of the box and of the entries a multiple of 32 banks apart, so that lanes whose
-    // foot points lie in neighbouring rows do not meet on a bank (203 x 149 x 181: 563 -> 488 us)
+    // foot points lie in neighbouring rows do not meet on a bank
     static constexpr int kBX = sizeof(T) == 4 ? 64 : kWNodes;
     static constexpr int kEP = sizeof(T) == 4 ? 40 : kWBases;
     static constexpr int kBoxN = kBX * kRows;      // phi box (a multiple of 16 bytes)
     static constexpr int kEntries = kRows * kWBases;
     static constexpr int kDiffs = kWBases + 1;     // FP64: D0 of the floor indices and of one more
-    static constexpr int kFoot = kWX * kWY * WZ;   // FP32: the samples' displacements, x, y, z planes
+    static constexpr int kFoot = kWX * kWY * WZ;   // FP32: the samples' foot points, x, y, z planes
     static constexpr int kBytes =
         kBoxN * (int)sizeof(T) + kRows * kEP * 16 + (sizeof(T) == 4 ? kFoot * 12 : kRows * kDiffs * 8);
     static constexpr int kNZ = NZ;                 // planes at a time
     static constexpr int kThreads = kWX * kWY * kNZ;
 };
 
-// the part of the combination that depends on x only
-template <typename T>
+// the part of the FP64 combination that depends on x only
 struct WenoX {
-    T L[4];          // p_b = sum_m L[m] v[m + 1]
-    T Ca, Cb, Cc, Ka, Kc;
+    double L[4];  // p_b = sum_m L[m] v[m + 1]
+    double Ca, Cb, Cc, Ka, Kc;
 };
 
-template <typename T>
-__device__ __forceinline__ WenoX<T> weno_x(T x) {
-    WenoX<T> w;
-    const T xp = x + T(1), xm = x - T(1), x2 = x - T(2);
+__device__ __forceinline__ WenoX weno_x(double x) {
+    WenoX w;
+    const double xp = x + 1.0, xm = x - 1.0, x2 = x - 2.0;
     // p_b in Newton form on nodes -1, 0, 1, 2
-    const T n2 = xp * x * T(0.5), n3 = xp * x * xm * T(1.0 / 6.0);
-    w.L[0] = T(1) - xp + n2 - n3;
-    w.L[1] = xp - T(2) * n2 + T(3) * n3;
-    w.L[2] = n2 - T(3) * n3;
+    const double n2 = xp * x * 0.5, n3 = xp * x * xm * (1.0 / 6.0);
+    w.L[0] = 1.0 - xp + n2 - n3;
+    w.L[1] = xp - 2.0 * n2 + 3.0 * n3;
+    w.L[2] = n2 - 3.0 * n3;
     w.L[3] = n3;
-    w.Ca = (T(2) - x) * (T(3) - x) * T(1.0 / 20.0);
-    w.Cb = (T(3) - x) * (x + T(2)) * T(1.0 / 10.0);
-    w.Cc = (x + T(2)) * xp * T(1.0 / 20.0);
+    w.Ca = (2.0 - x) * (3.0 - x) * (1.0 / 20.0);
+    w.Cb = (3.0 - x) * (x + 2.0) * (1.0 / 10.0);
+    w.Cc = (x + 2.0) * xp * (1.0 / 20.0);
     w.Ka = -w.Ca * n3;
-    w.Kc = w.Cc * (x * xm * x2 * T(1.0 / 6.0));
+    w.Kc = w.Cc * (x * xm * x2 * (1.0 / 6.0));
     return w;
 }
 
@@ -947,44 +979,27 @@ __device__ __forceinline__ float rcp_approx(float v) {
 // D0, D1.  Each 180 IS_s is 244 times a sum of squares of combinations of the first differences
 // (the quadratic form factored from its leading term; IS_2's is IS_0's read from the right):
 //   form(a, b, c) = (a + B b + G c)^2 + D (b + E c)^2 + Z c^2,
-// nine operations with the square, and in float the squares do not cancel where the quadratic
-// form's terms do.  The common factor (244 / 180)^2 drops out of the weights' ratios and, with eps
-// scaled alike, out of their normalisation.
-template <typename V, typename O>
-__device__ __forceinline__ void weno_q(const V (&v)[6], V& qa, V& qb, V& qc, V& D0, V& D1, O) {
-    V d[6];
+// nine operations with the square.  The common factor (244 / 180)^2 drops out of the weights' ratios
+// and, with eps scaled alike, out of their normalisation.
+__device__ __forceinline__ void weno_q(const double (&v)[6], double& qa, double& qb, double& qc, double& D0,
+                                       double& D1) {
+    double d[6];
 #pragma unroll
-    for (int m = 1; m < 6; ++m) d[m] = O::sub(v[m], v[m - 1]);
-    auto form = [&](V a, V b, V c, double B, double G, double D, double E, double Z) {
-        const V y1 = O::fma(O::k(G), c, O::fma(O::k(B), b, a)), y2 = O::fma(O::k(E), c, b);
-        V t = O::fma(O::mul(O::k(Z), c), c, O::k(1e-6 * 180.0 / 244.0));
-        t = O::fma(y1, y1, O::fma(O::mul(O::k(D), y2), y2, t));
-        return O::mul(t, t);
+    for (int m = 1; m < 6; ++m) d[m] = v[m] - v[m - 1];
+    auto form = [&](double a, double b, double c, double B, double G, double D, double E, double Z) {
+        const double y1 = fma(G, c, fma(B, b, a)), y2 = fma(E, c, b);
+        double t = fma(Z * c, c, 1e-6 * 180.0 / 244.0);
+        t = fma(y1, y1, fma(D * y2, y2, t));
+        return t * t;
     };
     constexpr double kB = -1171.0 / 488, kG = 683.0 / 488, kD = 152295.0 / 238144, kE = -1.0 / 1, kZ = 45.0 / 61;
     constexpr double kB1 = -781.0 / 488, kG1 = 293.0 / 488, kD1 = 327975.0 / 238144, kE1 = -10153.0 / 21865, kZ1 = 91377.0 / 266753;
     qa = form(d[1], d[2], d[3], kB, kG, kD, kE, kZ);
     qb = form(d[2], d[3], d[4], kB1, kG1, kD1, kE1, kZ1);
     qc = form(d[5], d[4], d[3], kB, kG, kD, kE, kZ);
-    D0 = O::fma(O::k(3.0), O::sub(d[2], d[3]), O::sub(d[4], d[1]));
-    D1 = O::fma(O::k(3.0), O::sub(d[3], d[4]), O::sub(d[5], d[2]));
+    D0 = fma(3.0, d[2] - d[3], d[4] - d[1]);
+    D1 = fma(3.0, d[3] - d[4], d[5] - d[2]);
 }
-
-template <typename T>
-struct ScalarOps {
-    static __device__ __forceinline__ T k(double c) { return T(c); }
-    static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
-    static __device__ __forceinline__ T sub(T a, T b) { return a - b; }
-    static __device__ __forceinline__ T fma(T a, T b, T c) { return rn_fma(a, b, c); }
-};
-struct PairOps {
-    static __device__ __forceinline__ float2 k(double c) { return make_float2((float)c, (float)c); }
-    static __device__ __forceinline__ float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-    static __device__ __forceinline__ float2 sub(float2 a, float2 b) {
-        return __ffma2_rn(b, make_float2(-1.f, -1.f), a);  // one rounding, no negations in registers
-    }
-    static __device__ __forceinline__ float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-};
 
 // num / den (den a positive normal double) in five FP64 operations instead of the nine of a
 // division: a float reciprocal of the leading bits, one Newton step, and one correction by the
@@ -1011,33 +1026,10 @@ __device__ __forceinline__ double inverse(double v) {
     return fma(r, fma(-v, r, 1.0), r);
 }
 
-// a y- or z-pass.  FP32: the weights alpha_s by reciprocals (as the general path's, finite for any
-// q_s); FP64: the ratios of the q_s by one division.
-__device__ __forceinline__ float weno_pass(const WenoX<float>& w, const float (&v)[6]) {
-    float qa, qb, qc, D0, D1;
-    weno_q(v, qa, qb, qc, D0, D1, ScalarOps<float>());
-    const float ia = rcp_approx(qa), ib = rcp_approx(qb), ic = rcp_approx(qc);
-    const float pb = fmaf(w.L[3], v[4], fmaf(w.L[2], v[3], fmaf(w.L[1], v[2], w.L[0] * v[1])));
-    const float den = fmaf(w.Cc, ic, fmaf(w.Ca, ia, w.Cb * ib));
-    const float num = fmaf(w.Kc * ic, D1, w.Ka * ia * D0);
-    return fmaf(num, rcp_approx(den), pb);
-}
-__device__ __forceinline__ float2 weno_pass(const WenoX<float>& w, const float2 (&v)[6]) {
-    using O = PairOps;
-    auto b2 = [](float x) { return make_float2(x, x); };
-    auto rcp2 = [](float2 q) { return make_float2(rcp_approx(q.x), rcp_approx(q.y)); };
-    float2 qa, qb, qc, D0, D1;
-    weno_q(v, qa, qb, qc, D0, D1, O());
-    const float2 ia = rcp2(qa), ib = rcp2(qb), ic = rcp2(qc);
-    const float2 pb = O::fma(b2(w.L[3]), v[4],
-                             O::fma(b2(w.L[2]), v[3], O::fma(b2(w.L[1]), v[2], O::mul(b2(w.L[0]), v[1]))));
-    const float2 den = O::fma(b2(w.Cc), ic, O::fma(b2(w.Ca), ia, O::mul(b2(w.Cb), ib)));
-    const float2 num = O::fma(O::mul(b2(w.Kc), ic), D1, O::mul(O::mul(b2(w.Ka), ia), D0));
-    return O::fma(num, rcp2(den), pb);
-}
-__device__ __forceinline__ double weno_pass(const WenoX<double>& w, const double (&v)[6]) {
+// a y- or z-pass: the ratios of the q_s by one division
+__device__ __forceinline__ double weno_pass(const WenoX& w, const double (&v)[6]) {
     double qa, qb, qc, D0, D1;
-    weno_q(v, qa, qb, qc, D0, D1, ScalarOps<double>());
+    weno_q(v, qa, qb, qc, D0, D1);
     const double inv = inverse(qa * qc);
     const double ra = qb * qc * inv, rc = qb * qa * inv;
     const double pb = fma(w.L[3], v[4], fma(w.L[2], v[3], fma(w.L[1], v[2], w.L[0] * v[1])));
@@ -1053,7 +1045,7 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* pbox = reinterpret_cast<T*>(align128(smem_raw));  // [z][y][x]
     const T* pb = pbox + 1;                              // the box from node tile - 3 along x
-    // FP32: float4 entries [row][floor index]; FP64: double2 entries, then D0 [row][kDiffs]
+    // FP32: float4 entries {qa, qb, qc, 0} [row][floor index]; FP64: double2 entries, then D0 [row][kDiffs]
     void* const entries = pbox + W::kBoxN;
     __shared__ uint64_t bar;
     const int x0 = blockIdx.x * kWX, y0 = blockIdx.y * kWY, z0 = blockIdx.z * WZ;
@@ -1079,7 +1071,7 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
         Vec3T<T> d{T(0), T(0), T(0)};
         if (column && k < src.n2)
             d = level_set_foot<T, TRACE>(cell_velocity(mac, i, j, k), i, j, k, dtv, dx, inv_dx,
-                                         [&](const Axes<T>& a, const auto& far) { return velocity_global(mac, a, far); });
+                                         [&](const Axes<T>& a, const auto& far, auto) { return velocity_global(mac, a, far); });
         if constexpr (sizeof(T) == 4) {
             sfoot[q * W::kThreads] = d.x;
             sfoot[q * W::kThreads + W::kFoot] = d.y;
@@ -1119,17 +1111,10 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
             float2 v[6];
 #pragma unroll
             for (int m = 0; m < 6; ++m) v[m] = make_float2(va[m], vb[m]);
-            float2 qa, qb, qc, D0, D1;
-            weno_q(v, qa, qb, qc, D0, D1, PairOps());
-            auto entry = [](float a, float b, float c, float d0, float d1) {
-                // q_s below 1e25: with q_s >= 1e-12 the ratios stay below 1e37, and so does the
-                // denominator (a reciprocal of 2^126 or more would be flushed to zero)
-                const float ra = fmaxf(fmaxf(a, b), c) < 1e25f ? b * rcp_approx(a) : __int_as_float(0x7fc00000);
-                const float rc = b * rcp_approx(c);
-                return make_float4(ra, ra * d0, rc, rc * d1);
-            };
-            q[r0 * W::kEP + b0] = entry(qa.x, qb.x, qc.x, D0.x, D1.x);
-            if (e1 != e0) q[r1 * W::kEP + b1] = entry(qa.y, qb.y, qc.y, D0.y, D1.y);
+            float2 qa, qb, qc;
+            weno6_sq2(v, qa, qb, qc);
+            q[r0 * W::kEP + b0] = make_float4(qa.x, qb.x, qc.x, 0.f);
+            if (e1 != e0) q[r1 * W::kEP + b1] = make_float4(qa.y, qb.y, qc.y, 0.f);
         }
     } else {
         double2* q = static_cast<double2*>(entries);
@@ -1139,7 +1124,7 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
             const T* p = pb + row * W::kBX + b;
             const double v[6] = {p[0], p[1], p[2], p[3], p[4], p[5]};
             double qa, qb, qc, D0, D1;
-            weno_q(v, qa, qb, qc, D0, D1, ScalarOps<double>());
+            weno_q(v, qa, qb, qc, D0, D1);
             const double inv = inverse(qa * qc);
             q[e] = make_double2(qb * qc * inv, qb * qa * inv);
             D[row * W::kDiffs + b] = D0;
@@ -1164,6 +1149,7 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
                 d.z = n == q ? foot[q].z : d.z;
             }
         }
+        d = foot_coords(d, dx, inv_dx);
         // stencil origin (floor - 2) relative to the box, per axis
         int px, py, pz;
         T fx, fy, fz;
@@ -1175,39 +1161,49 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
         pz = (int)((unsigned)pz + (unsigned)(foot_base<T>(k) - z0 + 1));
         T r = T(0);
         bool ok = false;
-        if ((unsigned)px < (unsigned)kWBases && (unsigned)py < (unsigned)(kWY + 2) && (unsigned)pz < (unsigned)(WZ + 2)) {
-            const WenoX<T> wx = weno_x(fx), wy = weno_x(fy);
-            T zl[6];
+        // (within a cell of the four planes the sample lies in, whatever the tile: beyond, the global path)
+        if ((unsigned)px < (unsigned)kWBases && (unsigned)py < (unsigned)(kWY + 2) && (unsigned)(pz - (kk & ~3)) < 6u) {
             if constexpr (sizeof(T) == 4) {
+                // the x-passes of rows dj and dj + 1, and the y-passes of planes dk and dk + 1, together
                 const float4* q = static_cast<const float4*>(entries);
-                const float2 Ka{wx.Ca, wx.Ka}, Kc{wx.Cc, wx.Kc}, Kb{wx.Cb, 0.f};
+                const WenoAxis<float> wx = weno_axis(fx), wy = weno_axis(fy);
+                float zl[6];
 #pragma unroll
                 for (int dk = 0; dk < 6; dk += 2) {
-                    float2 yl[6];  // .x: plane dk, .y: plane dk + 1, evaluated together
+                    float2 yl[6];  // .x: plane dk, .y: plane dk + 1
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const int row0 = (pz + dk + u) * kWBY + py;
 #pragma unroll
-                        for (int dj = 0; dj < 6; ++dj) {
-                            const float* v = pb + (row0 + dj) * W::kBX + px;
-                            const float4 e = q[(row0 + dj) * W::kEP + px];
-                            const float p = fmaf(wx.L[3], v[4], fmaf(wx.L[2], v[3], fmaf(wx.L[1], v[2], wx.L[0] * v[1])));
-                            // {denominator, numerator}
-                            const float2 t = __ffma2_rn(Kc, make_float2(e.z, e.w), __ffma2_rn(Ka, make_float2(e.x, e.y), Kb));
-                            const float y = fmaf(t.y, rcp_approx(t.x), p);
-                            if (u == 0)
-                                yl[dj].x = y;
-                            else
-                                yl[dj].y = y;
+                        for (int dj = 0; dj < 6; dj += 2) {
+                            const float* va = pb + (row0 + dj) * W::kBX + px;
+                            const float* vb = va + W::kBX;
+                            const float4 ea = q[(row0 + dj) * W::kEP + px], eb = q[(row0 + dj + 1) * W::kEP + px];
+                            float2 v[6];
+#pragma unroll
+                            for (int m = 0; m < 6; ++m) v[m] = make_float2(va[m], vb[m]);
+                            const float2 y = weno6_combine2(wx, v, make_float2(ea.x, eb.x), make_float2(ea.y, eb.y),
+                                                            make_float2(ea.z, eb.z));
+                            if (u == 0) {
+                                yl[dj].x = y.x;
+                                yl[dj + 1].x = y.y;
+                            } else {
+                                yl[dj].y = y.x;
+                                yl[dj + 1].y = y.y;
+                            }
                         }
                     }
-                    const float2 zv = weno_pass(wy, yl);
+                    const float2 zv = weno6_eval2(wy, yl);
                     zl[dk] = zv.x;
                     zl[dk + 1] = zv.y;
                 }
+                r = weno6_eval(weno_axis(fz), zl[0], zl[1], zl[2], zl[3], zl[4], zl[5]);
+                ok = true;
             } else {
+                const WenoX wx = weno_x(fx), wy = weno_x(fy);
                 const double2* q = static_cast<const double2*>(entries);
                 const double* D = reinterpret_cast<const double*>(q + W::kRows * W::kEP);
+                double zl[6];
 #pragma unroll
                 for (int dk = 0; dk < 6; ++dk) {
                     const int row0 = (pz + dk) * kWBY + py;
@@ -1231,9 +1227,9 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
                     zl[4] = dk == 4 ? zv : zl[4];
                     zl[5] = dk == 5 ? zv : zl[5];
                 }
+                r = weno_pass(weno_x(fz), zl);
+                ok = isfinite(r);
             }
-            r = weno_pass(weno_x(fz), zl);
-            ok = isfinite(r);
         }
         if (!ok) r = sample_weno6(src, foot_base<T>(i), foot_base<T>(j), foot_base<T>(k), d.x, d.y, d.z);
         const int oc = cell_index(src, i, j, k);
@@ -1333,9 +1329,9 @@ static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>&
 }
 
 // FP32: a CTA of 1024 threads per tile, four planes at a time.  Tiles of eight planes form 3.7
-// entries a sample against 5.5 of four planes (256^3: 1072 against 1230 us; 151 x 97 x 133: 156
-// against 177); where every tile of four planes has an SM of its own, those finish sooner (48^3:
-// 18.8 against 30.0 us).  512 and 768 threads a tile took 1187 and 1130 us at 256^3.
+// entries a sample against 5.5 of four planes (256^3: 1436 against 1569 us; 151 x 97 x 133: 216
+// against 232); where every tile of four planes has an SM of its own, those finish sooner (48^3:
+// 25.2 against 39.6 us).  512 threads a tile took 1453 us at 256^3, 768 on six planes 1449.
 constexpr int kSMs = 152;
 
 template <typename T, int TRACE>

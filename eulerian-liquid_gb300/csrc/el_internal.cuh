@@ -604,22 +604,35 @@ struct GridView {
     int n0, n1, n2;
 };
 
-// (1 - f) a + f b with one rounding a product or multiply-add, the same in every sampler.  FP64 forms
+// (1 - f) a + f b, with one multiply-add; which product is rounded alone is left to the compiler in
+// float (lerp_form where that matters).  FP64 forms
 // a + f (b - a): three fewer operations of the scarce FP64 pipe a trilinear read (float keeps the
 // products, which do not overflow for values near +-FLT_MAX).
 __device__ __forceinline__ float lerp1(float a, float b, float f) {
-    return rn_fma(f, b, rn_mul(rn_sub(1.f, f), a));
+    return (1.f - f) * a + f * b;
 }
 __device__ __forceinline__ double lerp1(double a, double b, double f) { return rn_fma(f, rn_sub(b, a), a); }
 
-// lerp(x, grid): x then y then z lerps of the 8 points (interpolation.h:35-72).  Split from the
-// reads so that every sampler (global or shared-memory data) rounds identically.
-template <typename T>
+// A float lerp's form: A rounds (1 - f) a alone, B rounds f b alone.
+enum LerpForm { LERP_ANY, LERP_A, LERP_B };
+template <int FORM, typename T>
+__device__ __forceinline__ T lerp_form(T a, T b, T f) {
+    if constexpr (FORM == LERP_A)
+        return rn_fma(f, b, rn_mul(rn_sub(T(1), f), a));
+    else if constexpr (FORM == LERP_B)
+        return rn_fma(rn_sub(T(1), f), a, rn_mul(f, b));
+    else
+        return lerp1(a, b, f);
+}
+
+// lerp(x, grid): x then y then z lerps of the 8 points (interpolation.h:35-72).  The forms: of the
+// first x lerp, of the second, and of the others.
+template <int X00 = LERP_ANY, int X10 = LERP_ANY, int R = LERP_ANY, typename T>
 __device__ __forceinline__ T tri_combine(T fx, T fy, T fz, T c000, T c100, T c010, T c110, T c001, T c101, T c011,
                                          T c111) {
-    const T lo = lerp1(lerp1(c000, c100, fx), lerp1(c010, c110, fx), fy);
-    const T hi = lerp1(lerp1(c001, c101, fx), lerp1(c011, c111, fx), fy);
-    return lerp1(lo, hi, fz);
+    const T lo = lerp_form<R>(lerp_form<X00>(c000, c100, fx), lerp_form<X10>(c010, c110, fx), fy);
+    const T hi = lerp_form<R>(lerp_form<R>(c001, c101, fx), lerp_form<R>(c011, c111, fx), fy);
+    return lerp_form<R>(lo, hi, fz);
 }
 
 // One axis of a position e cells away from sample index i (any e: the floor is limited to +-1e9, far
@@ -635,7 +648,7 @@ __device__ __forceinline__ int far_index(T e, int i, T& f) {
 
 // trilinear read (ex, ey, ez) cells away from sample (i, j, k): the clamped 8-point gather
 // (grid.h:369-377)
-template <typename T>
+template <int X00 = LERP_ANY, int X10 = LERP_ANY, int R = LERP_ANY, typename T>
 __device__ __forceinline__ T tri_clamped(const GridView<T>& g, int i, int j, int k, T ex, T ey, T ez) {
     T fx, fy, fz;
     const int bi = far_index(ex, i, fx), bj = far_index(ey, j, fy), bk = far_index(ez, k, fz);
@@ -646,7 +659,7 @@ __device__ __forceinline__ T tri_clamped(const GridView<T>& g, int i, int j, int
     const long long r10 = (long long)g.n0 * (j1 + (long long)g.n1 * k0);
     const long long r01 = (long long)g.n0 * (j0 + (long long)g.n1 * k1);
     const long long r11 = (long long)g.n0 * (j1 + (long long)g.n1 * k1);
-    return tri_combine(fx, fy, fz, __ldg(g.d + r00 + i0), __ldg(g.d + r00 + i1), __ldg(g.d + r10 + i0),
+    return tri_combine<X00, X10, R>(fx, fy, fz, __ldg(g.d + r00 + i0), __ldg(g.d + r00 + i1), __ldg(g.d + r10 + i0),
                        __ldg(g.d + r10 + i1), __ldg(g.d + r01 + i0), __ldg(g.d + r01 + i1), __ldg(g.d + r11 + i0),
                        __ldg(g.d + r11 + i1));
 }
@@ -730,6 +743,58 @@ __device__ __forceinline__ T weno6_combine(const WenoAxis<T>& w, T v0, T v1, T v
         const T aa = w.C[0] * qa, ab = w.C[1] * qb, ac = w.C[2] * qc;
         return __fdividef(aa * pa + ab * pb + ac * pc, aa + ab + ac);
     }
+}
+
+// weno6_combine for two FP32 passes at once (lanes .x and .y) in packed float2 arithmetic:
+// the candidates as FMA chains from the first product, the nonlinear combination
+// (aa pa + ab pb + ac pc) / (aa + ab + ac), each lane rounded as its scalar operations
+__device__ __forceinline__ float2 weno6_combine2(const WenoAxis<float>& w, const float2 (&v)[6], float2 qa, float2 qb,
+                                                 float2 qc) {
+    auto b2 = [](float x) { return make_float2(x, x); };
+    float2 p[3];
+#pragma unroll
+    for (int s = 0; s < 3; ++s) {
+        float2 t = __fmul2_rn(b2(w.L[s][0]), v[s]);
+        t = __ffma2_rn(b2(w.L[s][1]), v[s + 1], t);
+        t = __ffma2_rn(b2(w.L[s][2]), v[s + 2], t);
+        p[s] = __ffma2_rn(b2(w.L[s][3]), v[s + 3], t);
+    }
+    const float2 aa = __fmul2_rn(b2(w.C[0]), qa), ab = __fmul2_rn(b2(w.C[1]), qb), ac = __fmul2_rn(b2(w.C[2]), qc);
+    const float2 num = __ffma2_rn(ac, p[2], __ffma2_rn(ab, p[1], __fmul2_rn(aa, p[0])));
+    const float2 den = __fadd2_rn(__fadd2_rn(aa, ab), ac);
+    return make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
+}
+
+// weno6_sq for two FP32 passes at once in packed float2 arithmetic (the reciprocals per lane)
+__device__ __forceinline__ void weno6_sq2(const float2 (&v)[6], float2& qa, float2& qb, float2& qc) {
+    auto b2 = [](float x) { return make_float2(x, x); };
+    float2 d[6];
+#pragma unroll
+    for (int m = 1; m < 6; ++m) d[m] = __fadd2_rn(v[m], make_float2(-v[m - 1].x, -v[m - 1].y));  // exact negation
+    const float2 k = b2(1.0f / 180.0f);
+    auto form = [&](float2 a, float2 b, float2 c, float ca, float cb, float cc, float cbb, float cbc, float ccc) {
+        // (a (ca a + cb b + cc c) + b (cbb b + cbc c) + ccc c c) k
+        const float2 t1 = __ffma2_rn(b2(cc), c, __ffma2_rn(b2(cb), b, __fmul2_rn(b2(ca), a)));
+        const float2 t2 = __ffma2_rn(b2(cbc), c, __fmul2_rn(b2(cbb), b));
+        float2 t = __ffma2_rn(b, t2, __fmul2_rn(a, t1));
+        t = __ffma2_rn(__fmul2_rn(b2(ccc), c), c, t);
+        return __fmul2_rn(t, k);
+    };
+    const float2 ia = form(d[1], d[2], d[3], 244.f, -1171.f, 683.f, 1561.f, -1951.f, 814.f);
+    const float2 ib = form(d[2], d[3], d[4], 244.f, -781.f, 293.f, 961.f, -781.f, 244.f);
+    const float2 ic = form(d[3], d[4], d[5], 814.f, -1951.f, 683.f, 1561.f, -1171.f, 244.f);
+    const float2 eps = b2(1e-6f);
+    const float2 sa = __fadd2_rn(eps, ia), sb = __fadd2_rn(eps, ib), sc = __fadd2_rn(eps, ic);
+    const float2 sa2 = __fmul2_rn(sa, sa), sb2 = __fmul2_rn(sb, sb), sc2 = __fmul2_rn(sc, sc);
+    qa = make_float2(__fdividef(1.f, sa2.x), __fdividef(1.f, sa2.y));
+    qb = make_float2(__fdividef(1.f, sb2.x), __fdividef(1.f, sb2.y));
+    qc = make_float2(__fdividef(1.f, sc2.x), __fdividef(1.f, sc2.y));
+}
+
+__device__ __forceinline__ float2 weno6_eval2(const WenoAxis<float>& w, const float2 (&v)[6]) {
+    float2 qa, qb, qc;
+    weno6_sq2(v, qa, qb, qc);
+    return weno6_combine2(w, v, qa, qb, qc);
 }
 
 template <typename T>
