@@ -64,10 +64,11 @@ struct MacMaps {
 // the projected velocity a thousand times larger.
 
 // floor(e) and e - floor(e).  FP64: within two cells, where every stage of a step under the CFL limit
-// lies, from the high word by integer comparisons (a floor and its conversion are FP64-pipe
-// operations; -1 counts as below -1, with fraction 1: the same point).  FP32: e + 1.5 * 2^23 rounded toward -inf holds floor(e) in its low
-// mantissa bits (exact for |e| < 2^22); outside that range (and for NaN) the index lands millions
-// of cells away, i.e. outside every staged box and grid, and the sample takes the general path.
+// lies, by comparisons of the bits (a floor and its conversion are FP64-pipe operations).  -0 has floor 0
+// and -1 floor -1, both with fraction 0: a sample at rest is displaced by -dt / dx * 0 = -0 and keeps
+// its value whatever its neighbours hold.  FP32: e + 1.5 * 2^23 rounded toward -inf holds floor(e) in
+// its low mantissa bits (exact for |e| < 2^22); outside that range (and for NaN) the index lands
+// millions of cells away, i.e. outside every staged box and grid, and the sample takes the general path.
 template <typename T>
 __device__ __forceinline__ void floor_index(T e, int& idx, T& frac) {
     if constexpr (sizeof(T) == 4) {
@@ -76,9 +77,10 @@ __device__ __forceinline__ void floor_index(T e, int& idx, T& frac) {
         idx = (int)((unsigned)__float_as_int(r) - 0x4B400000u);
         frac = e - (r - big);
     } else {
-        const int hi = __double2hiint(e);
-        if ((hi & 0x7fffffff) < 0x40000000) {
-            const bool neg = hi < 0, far = (unsigned)(hi & 0x7fffffff) >= 0x3ff00000u;
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(e);
+        if ((bits & 0x7fffffffffffffffull) < 0x4000000000000000ull) {
+            const bool neg = bits > 0x8000000000000000ull;
+            const bool far = neg ? bits > 0xbff0000000000000ull : (bits & 0x7fffffffffffffffull) >= 0x3ff0000000000000ull;
             idx = neg ? (far ? -2 : -1) : (far ? 1 : 0);
             frac = e - __hiloint2double(neg ? (far ? (int)0xc0000000 : (int)0xbff00000) : (far ? 0x3ff00000 : 0), 0);
         } else {
@@ -823,8 +825,8 @@ __device__ __forceinline__ void velocity_tile(const Mac<T>& mac, const StagedMac
 // u, v, w of a tile, each advected through the (old) velocity itself.  FP32: bound by shared-memory
 // loads (66 a sample, seven trilinear reads) and issue (285 instructions a sample, from 617):
 // 256^3 RK3 0.96 -> 0.58 ms, three per-sample launches of 256 x 128 x 192 took 0.62 ms for what
-// now takes 0.24.  FP64: bound by its FP64 operations (155 a sample, from 350): 128^3 RK3 5.04 ->
-// 1.81 ms.
+// now takes 0.24.  FP64: bound by its FP64 operations (350 a sample before, now half of that): 128^3 RK3 5.04 ->
+// 2.03 ms.
 template <typename T, int TRACE>
 __global__ void __launch_bounds__(kTileX * kTileY, sizeof(T) == 4 ? 3 : 1) advect_velocity_tiled_kernel(
     Mac<T> mac, T* __restrict__ ou, T* __restrict__ ov, T* __restrict__ ow, DtArg dt, T inv_dx,

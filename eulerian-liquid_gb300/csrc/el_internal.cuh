@@ -605,13 +605,14 @@ struct GridView {
 };
 
 // (1 - f) a + f b, with one multiply-add; which product is rounded alone is left to the compiler in
-// float (lerp_form where that matters).  FP64 forms
-// a + f (b - a): three fewer operations of the scarce FP64 pipe a trilinear read (float keeps the
-// products, which do not overflow for values near +-FLT_MAX).
+// float (lerp_form where that matters).  Not a + f (b - a): the products are exact at f = 0 and 1 whatever
+// the other value holds, do not overflow between -max and max, and keep an infinite a = b.
 __device__ __forceinline__ float lerp1(float a, float b, float f) {
     return (1.f - f) * a + f * b;
 }
-__device__ __forceinline__ double lerp1(double a, double b, double f) { return rn_fma(f, rn_sub(b, a), a); }
+__device__ __forceinline__ double lerp1(double a, double b, double f) {
+    return rn_fma(f, b, rn_mul(rn_sub(1.0, f), a));
+}
 
 // A float lerp's form: A rounds (1 - f) a alone, B rounds f b alone.
 enum LerpForm { LERP_ANY, LERP_A, LERP_B };
