@@ -1308,8 +1308,10 @@ static int launch_phi_tiled(const GridView<T>& src, void* out, const Mac<T>& mac
                             cudaStream_t s) {
     const int smem = 3 * kBoxN * (int)sizeof(T) + 128;
     if (cudaFuncSetAttribute(advect_phi_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
+                             smem) != cudaSuccess) {
+        cudaGetLastError();  // the per-sample kernel takes over: not an error of the call
         return -1;
+    }
     const dim3 grid((src.n0 + kTileX - 1) / kTileX, (src.n1 + kTileY - 1) / kTileY, (src.n2 + kTileZ - 1) / kTileZ);
     advect_phi_tiled_kernel<T, TRACE><<<grid, dim3(kTileX, kTileY, 1), smem, s>>>(
         src, static_cast<T*>(out), mac, dt, dx, T(1) / dx, mac_maps(mac, copy));
@@ -1322,8 +1324,10 @@ static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>&
     using W = WenoTile<T, WZ, NZ>;
     const int smem = W::kBytes + 128;
     if (cudaFuncSetAttribute(advect_phi_weno_tiled_kernel<T, TRACE, WZ, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
+                             smem) != cudaSuccess) {
+        cudaGetLastError();  // the per-sample kernel takes over: not an error of the call
         return -1;
+    }
     const dim3 grid((src.n0 + kWX - 1) / kWX, (src.n1 + kWY - 1) / kWY, (src.n2 + WZ - 1) / WZ);
     advect_phi_weno_tiled_kernel<T, TRACE, WZ, NZ><<<grid, dim3(kWX, kWY, W::kNZ), smem, s>>>(
         src, static_cast<T*>(out), mac, dt, dx, T(1) / dx, box_map(src, copy, W::kBX, kWBY, W::kBZ));
@@ -1353,8 +1357,10 @@ static int launch_velocity_tiled(const Mac<T>& mac, void* ou, void* ov, void* ow
                                  cudaStream_t s) {
     const int smem = 3 * kBoxN * (int)sizeof(T) + 128;
     if (cudaFuncSetAttribute(advect_velocity_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem) != cudaSuccess)
+                             smem) != cudaSuccess) {
+        cudaGetLastError();  // the per-sample kernel takes over: not an error of the call
         return -1;
+    }
     // tiles of cells
     const dim3 grid((mac.v.n0 + kTileX - 1) / kTileX, (mac.u.n1 + kTileY - 1) / kTileY,
                     (mac.u.n2 + kTileZ - 1) / kTileZ);

@@ -1,0 +1,42 @@
+"""What the advection does when its tiled kernels cannot run: the library with el_advect.cu compiled
+against cpp/advect_fakes.cuh, which makes the kernels' set-up, or their wait for box copies, fail on
+the host's request."""
+
+import glob
+import importlib
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def said(el, tmp_path_factory):
+    build = importlib.import_module("eulerian_liquid_gb300.build")
+    build.build()
+    out = str(tmp_path_factory.mktemp("fakes"))
+    obj, lib = os.path.join(out, "el_advect.cu.o"), os.path.join(out, "libfakes.so")
+    run = dict(capture_output=True, text=True, timeout=600)
+    r = subprocess.run([build.nvcc(), *build.ARCH, *build.NVCC_FLAGS, "-include",
+                        os.path.join(HERE, "cpp", "advect_fakes.cuh"), "-c",
+                        os.path.join(build.CSRC, "el_advect.cu"), "-o", obj], **run)
+    assert r.returncode == 0, r.stderr
+    others = [o for o in glob.glob(os.path.join(build.OUT_DIR, "*.cu.o")) if os.path.basename(o) != "el_advect.cu.o"]
+    r = subprocess.run([build.nvcc(), *build.ARCH, "-shared", "-o", lib, obj, *others, "-lcudart_static", "-lrt",
+                        "-lpthread", "-ldl"], **run)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([sys.executable, os.path.join(HERE, "tile_failures_run.py"), lib], **run)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return json.loads(r.stdout.strip().splitlines()[-1])
+
+
+def test_setup_failure_falls_back(said):
+    """The per-sample kernels take over, and the call succeeds."""
+    assert said["setup_status"] == [0, 0]
+    assert said["setup_error"] < 2e-4  # FP32 WENO6 by the two paths (helpers.py)
