@@ -33,11 +33,12 @@ struct DtArg {
 
 __device__ __forceinline__ double dt_value(const DtArg& a) { return a.s ? a.s->dt : a.v; }
 
-// Set when a tile's wait for its box copies gave up (the tile's outputs are then NaN, so that
-// the step's solve fails on them); read and cleared by advect_fault_take().
+// Set when a wait for a tile's box copies of a context's advection gave up (the tile's outputs are then
+// NaN, so that the step's solve fails on them); read and cleared by advect_fault_take().  The stateless
+// operators, which no context's solve follows, leave the NaN alone (BoxMap::on 2).
 __device__ unsigned advect_wait_fault;
 
-// a box copy of one array (on = 0: the array is staged by plain loads)
+// a box copy of one array (on: BoxCopies; BOX_NONE: the array is staged by plain loads)
 struct BoxMap {
     CUtensorMap m;
     int on;
@@ -557,11 +558,11 @@ __device__ __forceinline__ void copy_boxes_begin(uint64_t* bar, unsigned bytes) 
 // wait gave up.  Then the fault is recorded and one thread waits once more (bounded) so that no
 // copy is still landing when the CTA ends.  Call after a barrier that follows the mbarrier's
 // initialisation.
-__device__ __forceinline__ bool copy_boxes_failed(uint64_t* bar) {
+__device__ __forceinline__ bool copy_boxes_failed(uint64_t* bar, bool report) {
     const bool ok = mbar_wait(bar, 0);
     if (!__syncthreads_or(!ok)) return false;
     if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
-        atomicOr(&advect_wait_fault, 1u);
+        if (report) atomicOr(&advect_wait_fault, 1u);
         mbar_wait(bar, 0);
     }
     __syncthreads();
@@ -629,7 +630,8 @@ __device__ __forceinline__ StagedMac<T> stage_mac(const Mac<T>& m, const MacMaps
     failed = false;
     if (ncopy) {
         __syncthreads();  // the mbarrier's initialisation is seen by every thread
-        failed = copy_boxes_failed(bar);
+        failed = copy_boxes_failed(bar, maps.c[0].on == BOX_REPORTED || maps.c[1].on == BOX_REPORTED ||
+                                            maps.c[2].on == BOX_REPORTED);
         if (!failed) {
             if (on0) finish_box<T, kBoxX, kBoxY, kBoxZ, true>(smem, m.u, bx0, by0, bz0, vmax);
             if (on1) finish_box<T, kBoxX, kBoxY, kBoxZ, true>(smem + kBoxN, m.v, bx0, by0, bz0, vmax);
@@ -1084,7 +1086,7 @@ __global__ void __launch_bounds__(WenoTile<T, WZ, NZ>::kThreads, 1)
     }
     if (pmap.on) {
         __syncthreads();  // the mbarrier's initialisation is seen by every thread
-        if (copy_boxes_failed(&bar)) {
+        if (copy_boxes_failed(&bar, pmap.on == BOX_REPORTED)) {
             nan_column(src, out, x0 + threadIdx.x, y0 + threadIdx.y, z0, WZ);
             return;
         }
@@ -1281,19 +1283,21 @@ static int advect_launch(int ni, int nj, int nk, double dx_d, int comp, void* ou
     return 1;
 }
 
-// The box map of one array for boxes of bx x by x bz (on = 0 when copies are off or the
+// The box map of one array for boxes of bx x by x bz (BOX_NONE when copies are off or the
 // array's pitch or address does not allow them: the kernel then stages it by plain loads).
 template <typename T>
-static BoxMap box_map(const GridView<T>& g, bool copy, unsigned bx, unsigned by, unsigned bz) {
+static BoxMap box_map(const GridView<T>& g, BoxCopies copy, unsigned bx, unsigned by, unsigned bz) {
     BoxMap b;
     std::memset(&b, 0, sizeof(b));
-    b.on = copy && tma_encode_3d(&b.m, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
-                                 (int)sizeof(T), g.d, g.n0, g.n1, g.n2, g.n0, bx, by, bz);
+    if (copy != BOX_NONE &&
+        tma_encode_3d(&b.m, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64,
+                      (int)sizeof(T), g.d, g.n0, g.n1, g.n2, g.n0, bx, by, bz))
+        b.on = copy;
     return b;
 }
 
 template <typename T>
-static MacMaps mac_maps(const Mac<T>& mac, bool copy) {
+static MacMaps mac_maps(const Mac<T>& mac, BoxCopies copy) {
     MacMaps m;
     m.c[0] = box_map(mac.u, copy, kBoxX, kBoxY, kBoxZ);
     m.c[1] = box_map(mac.v, copy, kBoxX, kBoxY, kBoxZ);
@@ -1304,7 +1308,7 @@ static MacMaps mac_maps(const Mac<T>& mac, bool copy) {
 // the tiled kernels: the level set (any scheme), and the velocity advecting itself (trilinear);
 // dynamic shared memory holds the boxes plus 128 bytes to align them
 template <typename T, int TRACE>
-static int launch_phi_tiled(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, bool copy,
+static int launch_phi_tiled(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, BoxCopies copy,
                             cudaStream_t s) {
     const int smem = 3 * kBoxN * (int)sizeof(T) + 128;
     if (cudaFuncSetAttribute(advect_phi_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1319,7 +1323,7 @@ static int launch_phi_tiled(const GridView<T>& src, void* out, const Mac<T>& mac
 }
 
 template <typename T, int TRACE, int WZ, int NZ>
-static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, bool copy,
+static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, BoxCopies copy,
                                 cudaStream_t s) {
     using W = WenoTile<T, WZ, NZ>;
     const int smem = W::kBytes + 128;
@@ -1341,7 +1345,7 @@ static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>&
 constexpr int kSMs = 152;
 
 template <typename T, int TRACE>
-static int launch_phi_weno_tiled(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, bool copy,
+static int launch_phi_weno_tiled(const GridView<T>& src, void* out, const Mac<T>& mac, DtArg dt, T dx, BoxCopies copy,
                                  cudaStream_t s) {
     if constexpr (sizeof(T) == 4) {
         const long long tiles4 = (long long)((src.n0 + kWX - 1) / kWX) * ((src.n1 + kWY - 1) / kWY) * ((src.n2 + 3) / 4);
@@ -1353,7 +1357,7 @@ static int launch_phi_weno_tiled(const GridView<T>& src, void* out, const Mac<T>
 }
 
 template <typename T, int TRACE>
-static int launch_velocity_tiled(const Mac<T>& mac, void* ou, void* ov, void* ow, DtArg dt, T dx, bool copy,
+static int launch_velocity_tiled(const Mac<T>& mac, void* ou, void* ov, void* ow, DtArg dt, T dx, BoxCopies copy,
                                  cudaStream_t s) {
     const int smem = 3 * kBoxN * (int)sizeof(T) + 128;
     if (cudaFuncSetAttribute(advect_velocity_tiled_kernel<T, TRACE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1371,7 +1375,7 @@ static int launch_velocity_tiled(const Mac<T>& mac, void* ou, void* ov, void* ow
 
 template <typename T>
 static int advect_phi_tiled_t(int ni, int nj, int nk, double dx_d, void* out, const void* in, const void* vu,
-                              const void* vv, const void* vw, DtArg dt, int trace, int sample, bool copy,
+                              const void* vv, const void* vw, DtArg dt, int trace, int sample, BoxCopies copy,
                               cudaStream_t s) {
     const T dx = (T)dx_d;
     Mac<T> mac{make_view<T>(vu, ni, nj, nk, 1), make_view<T>(vv, ni, nj, nk, 2),
@@ -1387,7 +1391,7 @@ static int advect_phi_tiled_t(int ni, int nj, int nk, double dx_d, void* out, co
 
 template <typename T>
 static int advect_velocity_tiled_t(int ni, int nj, int nk, double dx_d, void* ou, void* ov, void* ow, const void* vu,
-                                   const void* vv, const void* vw, DtArg dt, int trace, bool copy, cudaStream_t s) {
+                                   const void* vv, const void* vw, DtArg dt, int trace, BoxCopies copy, cudaStream_t s) {
     const T dx = (T)dx_d;
     Mac<T> mac{make_view<T>(vu, ni, nj, nk, 1), make_view<T>(vv, ni, nj, nk, 2),
                make_view<T>(vw, ni, nj, nk, 3)};
@@ -1398,7 +1402,7 @@ static int advect_velocity_tiled_t(int ni, int nj, int nk, double dx_d, void* ou
 // Level set through the tiled kernel; returns kernels launched, -1 on a launch set-up failure.
 // copy: stage the boxes by box copies where the arrays allow it (else plain loads throughout).
 int advect_phi_tiled(int dtype, int ni, int nj, int nk, double dx, void* out, const void* in, const void* vu,
-                     const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, int sample, bool copy,
+                     const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, int sample, BoxCopies copy,
                      cudaStream_t s) {
     DtArg dt{dts, dtv};
     if (dtype == EL_F64)
@@ -1408,7 +1412,7 @@ int advect_phi_tiled(int dtype, int ni, int nj, int nk, double dx, void* out, co
 
 // u, v, w advected through themselves with trilinear sampling, one tiled launch
 int advect_velocity_tiled(int dtype, int ni, int nj, int nk, double dx, void* ou, void* ov, void* ow, const void* vu,
-                          const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, bool copy,
+                          const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, BoxCopies copy,
                           cudaStream_t s) {
     DtArg dt{dts, dtv};
     if (dtype == EL_F64)

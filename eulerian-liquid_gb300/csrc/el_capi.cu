@@ -14,10 +14,10 @@ int advect_any(int dtype, int ni, int nj, int nk, double dx, int comp, void* out
                const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, int sample,
                cudaStream_t s, int rows = 4);
 int advect_phi_tiled(int dtype, int ni, int nj, int nk, double dx, void* out, const void* in, const void* vu,
-                     const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, int sample, bool copy,
+                     const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, int sample, BoxCopies copy,
                      cudaStream_t s);
 int advect_velocity_tiled(int dtype, int ni, int nj, int nk, double dx, void* ou, void* ov, void* ow, const void* vu,
-                          const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, bool copy,
+                          const void* vv, const void* vw, const Scalars* dts, double dtv, int trace, BoxCopies copy,
                           cudaStream_t s);
 bool advect_fault_take();
 int launch_weights(int dtype, int ni, int nj, int nk, const void* solid, void* wu, void* wv, void* ww,
@@ -490,7 +490,7 @@ static int advect_level_set_impl(el_ctx* ctx, const Scalars* dts, double dt, int
     int n = ctx->advect_tiled ? advect_phi_tiled(ctx->dtype, ctx->ni, ctx->nj, ctx->nk, ctx->dx, ctx->tmp[0],
                                                  ctx->field[EL_FIELD_PHI], ctx->field[EL_FIELD_U],
                                                  ctx->field[EL_FIELD_V], ctx->field[EL_FIELD_W], dts, dt, trace,
-                                                 sample, ctx->advect_tiled == 1, ctx->stream)
+                                                 sample, ctx->advect_tiled == 1 ? BOX_REPORTED : BOX_NONE, ctx->stream)
                               : -1;
     if (n < 0)
         n = advect_any(ctx->dtype, ctx->ni, ctx->nj, ctx->nk, ctx->dx, 0, ctx->tmp[0], ctx->field[EL_FIELD_PHI],
@@ -509,7 +509,8 @@ static int advect_velocity_impl(el_ctx* ctx, const Scalars* dts, double dt, int 
         ProfScope prof(ctx, EL_KC_ADVECT_VEL, 2 * vel_bytes);
         n = advect_velocity_tiled(ctx->dtype, ctx->ni, ctx->nj, ctx->nk, ctx->dx, ctx->tmp[1], ctx->tmp[2],
                                   ctx->tmp[3], ctx->field[EL_FIELD_U], ctx->field[EL_FIELD_V],
-                                  ctx->field[EL_FIELD_W], dts, dt, trace, ctx->advect_tiled == 1, ctx->stream);
+                                  ctx->field[EL_FIELD_W], dts, dt, trace,
+                                  ctx->advect_tiled == 1 ? BOX_REPORTED : BOX_NONE, ctx->stream);
     }
     if (n <= 0) {  // one launch per component
         n = 0;
@@ -864,7 +865,7 @@ EL_API int el_advect_collocated_grid(const el_grid* g, int dtype, void* out, con
         return EL_ERR_INVALID_ARGUMENT;
     // the tiled kernels, as advect_level_set (they stage nothing outside their launch)
     const int n = advect_phi_tiled(dtype, g->ni, g->nj, g->nk, g->dx, out, in, vu, vv, vw, nullptr, dt, trace, sample,
-                                   true, (cudaStream_t)stream);
+                                   BOX_UNREPORTED, (cudaStream_t)stream);
     if (n < 0)
         advect_any(dtype, g->ni, g->nj, g->nk, g->dx, 0, out, in, vu, vv, vw, nullptr, dt, trace, sample,
                    (cudaStream_t)stream);
@@ -887,8 +888,8 @@ EL_API int el_advect_staggered_grid(const el_grid* g, int dtype, void* ou, void*
     // a velocity advecting itself with trilinear reads: the tiled kernel, the three components in
     // one launch; any other field, and WENO6 reads, by the per-sample kernel
     if (sample == EL_SAMPLE_TRILINEAR && iu == vu && iv == vv && iw == vw &&
-        advect_velocity_tiled(dtype, g->ni, g->nj, g->nk, g->dx, ou, ov, ow, vu, vv, vw, nullptr, dt, trace, true,
-                              (cudaStream_t)stream) > 0)
+        advect_velocity_tiled(dtype, g->ni, g->nj, g->nk, g->dx, ou, ov, ow, vu, vv, vw, nullptr, dt, trace,
+                              BOX_UNREPORTED, (cudaStream_t)stream) > 0)
         return cudaGetLastError() == cudaSuccess ? EL_OK : EL_ERR_CUDA;
     for (int c = 0; c < 3; ++c)
         advect_any(dtype, g->ni, g->nj, g->nk, g->dx, c + 1, dst[c], src[c], vu, vv, vw, nullptr, dt, trace, sample,

@@ -598,6 +598,10 @@ __device__ bool grid_sum(double (&v)[NV], double* partials, unsigned* counter, d
 // ---------------------------------------------------------------------------------------
 // interpolation (include/nama/math/interpolation.h)
 
+// where the tiled advection kernels stage from: plain loads, or box copies whose fault a context's step
+// reports, or no one does
+enum BoxCopies { BOX_NONE = 0, BOX_REPORTED = 1, BOX_UNREPORTED = 2 };
+
 template <typename T>
 struct GridView {
     const T* __restrict__ d;

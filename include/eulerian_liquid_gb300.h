@@ -261,7 +261,9 @@ int el_update_velocity_using_pressure(el_ctx* ctx, double dt);
 
 /* ---- stateless operators on caller-owned device memory ------------------------------
  * The reference's free functions (include/nama/project/3d/fluid/advection.h:8-11,
- * boundary.h:8) over raw device pointers; no allocation, work enqueued on `stream`. */
+ * boundary.h:8) over raw device pointers; no allocation, work enqueued on `stream`.  The
+ * advections stage their tiles by asynchronous copies with bounded waits: a tile whose copy has
+ * not arrived when its wait gives up is left NaN. */
 typedef struct el_grid {
     int ni, nj, nk;
     double dx;

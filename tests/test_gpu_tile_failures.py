@@ -40,3 +40,13 @@ def test_setup_failure_falls_back(said):
     """The per-sample kernels take over, and the call succeeds."""
     assert said["setup_status"] == [0, 0]
     assert said["setup_error"] < 2e-4  # FP32 WENO6 by the two paths (helpers.py)
+
+
+def test_wait_failure_is_nan_and_not_another_callers(said):
+    """A context's step reports its own advection's wait as a timeout; a NaN in a step that no box copy had a
+    part in stays a NaN, whatever became of a stateless call before it (arrays of 40 cells a row: phi, v
+    and w by box copies, u by plain loads)."""
+    assert said["wait_status"] == [0, 0]
+    assert said["wait_nan"] == [True] * 4
+    assert "gave up" in said["wait_step_tiled"]
+    assert "gave up" not in said["nan_step_per_sample"] and "non-finite" in said["nan_step_per_sample"]

@@ -50,6 +50,32 @@ def main():
     said["setup_status"], got = stateless()
     setup_fails.value = 0
     said["setup_error"] = max(float(np.max(np.abs(g - w))) for g, w in zip(got, want))
+
+    def step(tiled, nan):
+        # 15 cells a row: u alone is staged by box copies, so that the level set keeps its fluid
+        sim = el.Simulator(15, 12, 20, dtype=el.EL_F32)
+        sim.set_tuning(advect_tiled=tiled)
+        sim.init_scene(dict(el.scenes.spheres_pool(16, 4), shape=(15, 12, 20)))
+        if nan:
+            u = np.zeros(sim.shape("u"), np.float32)
+            u[10, 2, 7] = np.nan
+            sim.upload("u", u)
+        try:
+            sim.step(0.005, sample_phi=el.SAMPLE_WENO6, solver=el.SOLVER_MIXED, tol=1e-6)
+            return "stepped"
+        except el.ELError as e:
+            return str(e)
+        finally:
+            sim.close()
+
+    # the waits give up: NaN from the stateless operators and no other trace of it; a context's step reports its own
+    assert lib.el_test_set_wait_fails(1) == 0
+    said["wait_status"], got = stateless()
+    said["wait_nan"] = [bool(np.all(np.isnan(a))) for a in got]
+    said["wait_step_tiled"] = step(1, False)
+    _, got = stateless()
+    assert lib.el_test_set_wait_fails(0) == 0
+    said["nan_step_per_sample"] = step(0, True)
     print(json.dumps(said))
 
 
