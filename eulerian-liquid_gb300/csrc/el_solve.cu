@@ -2801,6 +2801,7 @@ int solve_system_graph(el_ctx* ctx, const el_solve_params&, el_solve_stats* st) 
     if (rc != EL_OK) return rc;
     ctx->launches += ctx->solve_graph_kernels[0] + (long long)h->outer * ctx->solve_graph_kernels[1] +
                      (long long)h->inner_passes * ctx->solve_graph_kernels[2];
+    st->fluid_cells = h->count;
     st->iterations = h->inner_total;
     st->outer_iterations = h->outer;
     return finish_solve(ctx, h, st);
