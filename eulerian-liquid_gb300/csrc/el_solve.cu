@@ -63,6 +63,10 @@ __device__ __forceinline__ bool finite_d(double v) { return isfinite(v); }
 __device__ __forceinline__ bool positive(float v) { return v > 0.f; }
 __device__ __forceinline__ bool positive(double v) { return d_positive(v); }  // on the integer pipe
 
+// The reciprocal of a row's diagonal, 0 on an empty row.  A diagonal below 2^-1000 takes that scale
+// instead: its reciprocal could overflow, and a smaller one only leaves that row to the Krylov method.
+__device__ __forceinline__ double row_inverse(double d) { return positive(d) ? 1.0 / fmax(d, 0x1p-1000) : 0.0; }
+
 // ---------------------------------------------------------------------------------------
 // coefficient records
 
@@ -294,7 +298,7 @@ __global__ void pack64_kernel(long long n, const double* __restrict__ d, const O
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
         const double dc = d[c];
         a[c] = Rec64{dc, (double)ox[c], (double)oy[c], (double)oz[c]};
-        rd[c] = positive(dc) ? 1.0 / dc : 0.0;
+        rd[c] = row_inverse(dc);
     }
 }
 
@@ -337,7 +341,7 @@ __global__ void coarsen_kernel(LGeom F, const RF* __restrict__ fr, LGeom C, RC* 
         cr[q] = make_float4(dc, A(0.5) * sx, A(0.5) * sy, A(0.5) * sz);
     else {
         cr[q] = Rec64{dc, 0.5 * sx, 0.5 * sy, 0.5 * sz};
-        rd[q] = positive(dc) ? 1.0 / dc : 0.0;
+        rd[q] = row_inverse(dc);
     }
 }
 
@@ -840,9 +844,7 @@ __global__ void jacobi_start_kernel(LGeom g, SegArg seg, const double* __restric
                                     double* partials, unsigned* counter) {
     double acc[1] = {0.0};
     SEG_LOOP_BEGIN(seg, g)
-    const double d = diag[c];
-    // (a diagonal below 2^-1000 takes that scale instead: its reciprocal could overflow)
-    const double ic = d_positive(d) ? 1.0 / fmax(d, 0x1p-1000) : 0.0;
+    const double ic = row_inverse(diag[c]);
     const double rc = r[c];
     const double zc = rc * ic;
     inv_diag[c] = ic;
