@@ -699,9 +699,11 @@ __global__ void __launch_bounds__(kWgThreads, WGrad<CIN, COUT>::CTAS)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int ci = cis * 16 + h * 8 + (lane & 3) * 2, co = (cos * MB + m) * 16 + (lane >> 2);
-                *reinterpret_cast<float2*>(dst + (size_t)co * CIN + ci) = make_float2(acc[t][m][h][0], acc[t][m][h][1]);
-                *reinterpret_cast<float2*>(dst + (size_t)(co + 8) * CIN + ci) =
-                    make_float2(acc[t][m][h][2], acc[t][m][h][3]);
+                // (one float a store: the caller's workspace need not be aligned for two)
+                dst[(size_t)co * CIN + ci] = acc[t][m][h][0];
+                dst[(size_t)co * CIN + ci + 1] = acc[t][m][h][1];
+                dst[(size_t)(co + 8) * CIN + ci] = acc[t][m][h][2];
+                dst[(size_t)(co + 8) * CIN + ci + 1] = acc[t][m][h][3];
             }
     }
     if (bias_warp && (lane & 3) == 0) {
