@@ -713,7 +713,8 @@ __device__ __forceinline__ AxisPair axis_pair(float2 e, unsigned base, unsigned 
     p.w = __ffma2_rn(fl, make_float2(-1.f, -1.f), e);  // e - fl (packed additions take no negated operand)
     // the magic number's bits fold into the base (unsigned arithmetic wraps)
     const unsigned c = base - 0x4B400000u * stride;
-    // (as instructions: the compiler's own folding of this product was seen to lose the stride)
+    // as instructions: with the product written in C++, nvcc 13.0.88 folded it into an address without
+    // the stride (found by the index check of tri_pair in the debug build; not reduced to a small case)
     asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(p.a) : "r"(__float_as_int(r.x)), "r"(stride), "r"(c));
     asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(p.b) : "r"(__float_as_int(r.y)), "r"(stride), "r"(c));
     return p;
@@ -722,11 +723,12 @@ __device__ __forceinline__ AxisPair axis_pair(float2 e, unsigned base, unsigned 
 // byte strides of a box
 constexpr unsigned kSX = 4, kSY = 4 * kBoxX, kSZ = kSY * kBoxY;
 
-// the entry at shared-memory byte address `at` + OFF
+// the entry at shared-memory byte address `at` + OFF (the clobber keeps it behind the barrier that ends
+// the staging)
 template <int OFF>
 __device__ __forceinline__ float lds(unsigned at) {
     float v;
-    asm("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(at), "n"(OFF));
+    asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(at), "n"(OFF) : "memory");
     return v;
 }
 
@@ -737,7 +739,8 @@ __device__ __forceinline__ float2 tri_pair(unsigned box0, const AxisPair& x, con
     unsigned p = x.a + y.a + z.a, q = x.b + y.b + z.b;
     constexpr int SX = kSX, SY = kSY, SZ = kSZ, UP = BOX + SZ;
     if (!EL_IN(p - box0, 4 * kBoxN - SX - SY - SZ, 5) || !EL_IN(q - box0, 4 * kBoxN - SX - SY - 2 * SZ, 6)) p = q = box0;
-    // (every read is in the box, see the callers; a wrong address would be a fault, not a wrong value)
+    // Every read is in the box, see the callers.  An address that was not would read the box's end instead
+    // of faulting; the debug build records it (above).
     p = box0 + min(p - box0, (unsigned)(4 * kBoxN - SX - SY - SZ - 4));
     q = box0 + min(q - box0, (unsigned)(4 * kBoxN - SX - SY - 2 * SZ - 4));
     const float2 x00 = lerp1(make_float2(lds<BOX>(p), lds<UP>(q)), make_float2(lds<BOX + SX>(p), lds<UP + SX>(q)), x.w);
