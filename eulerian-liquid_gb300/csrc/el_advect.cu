@@ -1026,9 +1026,10 @@ __device__ __forceinline__ double div_newton(double num, double den) {
     const double r = rcp_newton(den), q = num * r;
     return fma(fma(-den, q, num), r, q);
 }
-// 1 / v to within an ulp (one more Newton step)
+// 1 / v to within an ulp (one more Newton step); NaN for a product that overflowed, whose 0 would silently
+// drop the weights formed with it (the result's NaN then takes the general path)
 __device__ __forceinline__ double inverse(double v) {
-    if (!in_float_range(v)) return 1.0 / v;
+    if (!in_float_range(v)) return v <= std::numeric_limits<double>::max() ? 1.0 / v : std::numeric_limits<double>::quiet_NaN();
     const double r = rcp_newton(v);
     return fma(r, fma(-v, r, 1.0), r);
 }
