@@ -16,6 +16,7 @@
 #include <limits>
 #include <type_traits>
 
+#include "el_div.cuh"
 #include "el_internal.cuh"
 #include "el_tma.cuh"
 
@@ -976,12 +977,6 @@ __device__ __forceinline__ WenoX weno_x(double x) {
     return w;
 }
 
-__device__ __forceinline__ float rcp_approx(float v) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-
 // q_s = (eps + IS_s)^2 of the three candidates, times a common factor, and the fourth differences
 // D0, D1.  Each 180 IS_s is 244 times a sum of squares of combinations of the first differences
 // (the quadratic form factored from its leading term; IS_2's is IS_0's read from the right):
@@ -1006,32 +1001,6 @@ __device__ __forceinline__ void weno_q(const double (&v)[6], double& qa, double&
     qc = form(d[5], d[4], d[3], kB, kG, kD, kE, kZ);
     D0 = fma(3.0, d[2] - d[3], d[4] - d[1]);
     D1 = fma(3.0, d[3] - d[4], d[5] - d[2]);
-}
-
-// num / den (den a positive normal double) in five FP64 operations instead of the nine of a
-// division: a float reciprocal of the leading bits, one Newton step, and one correction by the
-// residual (P. Markstein, IBM J. Res. Dev. 34, 1990); within an ulp.  Outside the floats' range the
-// division itself.
-__device__ __forceinline__ bool in_float_range(double v) {  // 2^-120 <= v < 2^120
-    return (unsigned)(__double2hiint(v) - 0x38700000) < 0x0f000000u;
-}
-__device__ __forceinline__ double rcp_newton(double v) {
-    const float f = __int_as_float(__funnelshift_l(__double2loint(v), __double2hiint(v) - 0x38000000, 3));
-    const unsigned b = (unsigned)__float_as_int(rcp_approx(f));
-    const double r = __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
-    return fma(r, fma(-v, r, 1.0), r);  // 44 bits
-}
-__device__ __forceinline__ double div_newton(double num, double den) {
-    if (!in_float_range(den)) return num / den;
-    const double r = rcp_newton(den), q = num * r;
-    return fma(fma(-den, q, num), r, q);
-}
-// 1 / v to within an ulp (one more Newton step); NaN for a product that overflowed, whose 0 would silently
-// drop the weights formed with it (the result's NaN then takes the general path)
-__device__ __forceinline__ double inverse(double v) {
-    if (!in_float_range(v)) return v <= std::numeric_limits<double>::max() ? 1.0 / v : std::numeric_limits<double>::quiet_NaN();
-    const double r = rcp_newton(v);
-    return fma(r, fma(-v, r, 1.0), r);
 }
 
 // a y- or z-pass: the ratios of the q_s by one division
