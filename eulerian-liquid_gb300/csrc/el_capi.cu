@@ -1019,7 +1019,9 @@ EL_API int el_solve_pressure_noalloc(const el_grid* g, const float* phi, float* 
     ctx.hscal = host_scalars;  // pageable host copy of the device scalars
 
     // the array keeps the previous call's contents: the reduction ticket and the scalars start
-    // at zero; everything else is written before it is read
+    // at zero; everything else is written before it is read, but for z and the two directions in row
+    // segments without fluid: a neighbour reads what an earlier call left there, times a zero
+    // coupling.  It is finite: a solve that met a NaN or infinity clears its vectors (reset_vectors)
     EL_CUDA_TRY(&ctx, cudaMemsetAsync(ctx.counter, 0, 64, ctx.stream));
     EL_CUDA_TRY(&ctx, cudaMemsetAsync(ctx.dscal, 0, 4 * sizeof(Scalars), ctx.stream));
     el_solve_stats local{};

@@ -227,10 +227,10 @@ struct el_ctx {
     // advection / extrapolation ping-pong buffers (same shapes as phi, u, v, w)
     void* tmp[4] = {};
     // extrapolation scratch per field slot (el_extrap.cu): two padded bitmasks of the valid
-    // cells and the list of a layer's cells; cells per slot of the current and the next layer
+    // cells, the mask as a flat bit stream, and four arrays of tile states
     unsigned* ex_bits[4][2] = {};
     unsigned* ex_flat[4] = {};
-    uint8_t* ex_tiles[4] = {};  // the tile states
+    uint8_t* ex_tiles[4] = {};
     size_t ex_bits_bytes = 0, ex_flat_bytes = 0, ex_tile_count = 0;
 
     // projection
