@@ -846,9 +846,13 @@ __global__ void __launch_bounds__(kTileX * kTileY, sizeof(T) == 4 ? 3 : 1) advec
     const StagedMac<T> sm = stage_mac(mac, maps, smem, &bar, x0, y0, z0, vmax, failed);
     if (failed) {
         const int i = x0 + threadIdx.x, j = y0 + threadIdx.y;
-        nan_column(mac.u, ou, i, j, z0, kTileZ + 1);
-        nan_column(mac.v, ov, i, j, z0, kTileZ + 1);
-        nan_column(mac.w, ow, i, j, z0, kTileZ + 1);
+        // the samples velocity_tile would have written: the tile's, and the last faces of a last tile
+        const bool more_w = z0 + kTileZ == mac.w.n2 - 1;
+        nan_column(mac.u, ou, i, j, z0, kTileZ);
+        nan_column(mac.v, ov, i, j, z0, kTileZ);
+        nan_column(mac.w, ow, i, j, z0, kTileZ + (more_w ? 1 : 0));
+        if (threadIdx.x == 0 && x0 + kTileX == mac.u.n0 - 1) nan_column(mac.u, ou, x0 + kTileX, j, z0, kTileZ);
+        if (threadIdx.y == 0 && y0 + kTileY == mac.v.n1 - 1) nan_column(mac.v, ov, i, y0 + kTileY, z0, kTileZ);
         return;
     }
     const T bm = box_max(vmax);  // ends the staging (a barrier)

@@ -50,3 +50,8 @@ def test_wait_failure_is_nan_and_not_another_callers(said):
     assert said["wait_nan"] == [True] * 4
     assert "gave up" in said["wait_step_tiled"]
     assert "gave up" not in said["nan_step_per_sample"] and "non-finite" in said["nan_step_per_sample"]
+
+
+def test_wait_failure_is_nan_on_the_last_faces(said):
+    """Grids of whole tiles: the last tiles also take the last faces along each axis."""
+    assert said["wait_nan_full_tiles"] == [True] * 4

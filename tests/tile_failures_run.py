@@ -22,13 +22,13 @@ def main():
     import torch
     lib = el.load()
     setup_fails = ctypes.c_int.in_dll(lib, "el_test_setup_fails")
-    rng = np.random.default_rng(1)
-    ni, nj, nk = 40, 18, 20
-    shapes = [(nk, nj, ni), (nk, nj, ni + 1), (nk, nj + 1, ni), (nk + 1, nj, ni)]
-    fields = [torch.from_numpy(rng.uniform(-0.5, 0.5, s).astype(np.float32)).cuda() for s in shapes]
-    dx = 1.0 / 40
 
-    def stateless():
+    def stateless(dims=(40, 18, 20)):
+        ni, nj, nk = dims
+        shapes = [(nk, nj, ni), (nk, nj, ni + 1), (nk, nj + 1, ni), (nk + 1, nj, ni)]
+        rng = np.random.default_rng(1)
+        fields = [torch.from_numpy(rng.uniform(-0.5, 0.5, s).astype(np.float32)).cuda() for s in shapes]
+        dx = 1.0 / ni
         out = [torch.zeros_like(a) for a in fields]
         vel = [a.data_ptr() for a in fields[1:]]
         status = []
@@ -72,6 +72,8 @@ def main():
     assert lib.el_test_set_wait_fails(1) == 0
     said["wait_status"], got = stateless()
     said["wait_nan"] = [bool(np.all(np.isnan(a))) for a in got]
+    _, got = stateless((64, 16, 24))
+    said["wait_nan_full_tiles"] = [bool(np.all(np.isnan(a))) for a in got]
     said["wait_step_tiled"] = step(1, False)
     _, got = stateless()
     assert lib.el_test_set_wait_fails(0) == 0
