@@ -681,14 +681,14 @@ __device__ __forceinline__ void velocity_sample(const Mac<T>& mac, const GridVie
         return sm.box[c * kBoxN + ((K + dk) * kBoxY + J + dj) * kBoxX + I + di];
     });
     const Vec3T<T> d = backtrace_from<T, TRACE>(a, s, [&](const Vec3T<T>& e) {
-        return velocity_staged<T, CHECK>(mac, sm, axes_rel(i, j, k, h, e), FarRel<T>{i, j, k, h, e});
+        return velocity_staged<T, CHECK, LERP_A, LERP_A, LERP_A>(mac, sm, axes_rel(i, j, k, h, e), FarRel<T>{i, j, k, h, e});
     });
     int x, y, z;
     T fx, fy, fz, r;
     floor_index(d.x, x, fx);
     floor_index(d.y, y, fy);
     floor_index(d.z, z, fz);
-    if (!staged_lerp<T, CHECK>(own, (int)((unsigned)I + (unsigned)x), (int)((unsigned)J + (unsigned)y),
+    if (!staged_lerp<T, CHECK, LERP_A>(own, (int)((unsigned)I + (unsigned)x), (int)((unsigned)J + (unsigned)y),
                                (int)((unsigned)K + (unsigned)z), fx, fy, fz, r) &&
         CHECK)
         r = tri_clamped(g, i, j, k, d.x, d.y, d.z);
