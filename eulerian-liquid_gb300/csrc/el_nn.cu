@@ -18,9 +18,9 @@
 // Backward data is the same kernel: grad_in = conv(grad_out masked by ReLU', W') with W' the
 // weights transposed in channels and mirrored in taps (packed separately); its output splits
 // back into the two concatenated inputs.  Backward weight is a second implicit GEMM,
-// M = output channels, N = input channels, K = voxels, per tap; each CTA keeps a group of taps'
-// accumulators in registers over a range of bricks and writes one partial, summed in a fixed
-// order by a reduction kernel (deterministic).
+// M = output channels, N = input channels, K = voxels, per tap; a CTA takes all 27 taps of 16 input
+// channels over a range of planes, accumulators in registers, and writes one partial, summed in a
+// fixed order by a reduction kernel (deterministic).
 #include <cuda_bf16.h>
 
 #include <cstdint>

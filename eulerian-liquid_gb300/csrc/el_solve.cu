@@ -2758,9 +2758,10 @@ int enqueue_solve_device(el_ctx* ctx, const el_solve_params& prm, int kernels[3]
 // Whether the mixed solve runs as one graph: the second and later of a row of solves with the same
 // parameters.  The host-driven solve stops the device at every poll (two a refinement sweep and one a
 // batch of iterations) and starts about twenty kernels a sweep one by one; the graph does neither, but
-// making it costs as much as several solves, so a solve whose parameters differ from the one before's
-// takes the host-driven path.  75 x 62 x 53 cells:
-// 1.13 -> 0.94 ms; a whole step of 48^3 1.13 -> 0.91, of 151 x 97 x 133 2.16 -> 1.99.
+// making it costs 0.03 to 0.25 ms, which a single solve does not earn back, so a solve whose parameters
+// differ from the one before's takes the host-driven path.  75 x 62 x 53 cells:
+// 0.98 -> 0.76 ms; a whole step of 48^3 0.94 -> 0.76, of 151 x 97 x 133 2.01 -> 1.88, of 256^3 6.95 -> 6.83
+// (parameters that alternate -> the same from call to call).
 bool solve_graph_ready(el_ctx* ctx, const el_solve_params& prm) {
     el_ctx::SolveKey key;
     key.tol = prm.tol;
