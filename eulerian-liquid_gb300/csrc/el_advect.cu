@@ -1318,7 +1318,8 @@ static int launch_phi_weno_tile(const GridView<T>& src, void* out, const Mac<T>&
 // FP32: a CTA of 1024 threads per tile, four planes at a time.  Tiles of eight planes form 3.7
 // entries a sample against 5.5 of four planes (256^3: 1436 against 1569 us; 151 x 97 x 133: 216
 // against 232); where every tile of four planes has an SM of its own, those finish sooner (48^3:
-// 25.2 against 39.6 us).  512 threads a tile took 1453 us at 256^3, 768 on six planes 1449.
+// 25.2 against 39.6 us), and so where the grid has no more planes (300 x 300 x 1: 37.9 against 42; 300 x
+// 300 x 2: 48.5).  512 threads a tile took 1453 us at 256^3, 768 on six planes 1449.
 static int device_sms() {
     int dev = 0, sms = 0;
     return cudaGetDevice(&dev) == cudaSuccess &&
@@ -1332,7 +1333,7 @@ static int launch_phi_weno_tiled(const GridView<T>& src, void* out, const Mac<T>
                                  cudaStream_t s) {
     if constexpr (sizeof(T) == 4) {
         const long long tiles4 = (long long)((src.n0 + kWX - 1) / kWX) * ((src.n1 + kWY - 1) / kWY) * ((src.n2 + 3) / 4);
-        if (tiles4 > device_sms()) return launch_phi_weno_tile<T, TRACE, 8, 4>(src, out, mac, dt, dx, copy, s);
+        if (src.n2 > 4 && tiles4 > device_sms()) return launch_phi_weno_tile<T, TRACE, 8, 4>(src, out, mac, dt, dx, copy, s);
         return launch_phi_weno_tile<T, TRACE, 4, 4>(src, out, mac, dt, dx, copy, s);
     } else {
         return launch_phi_weno_tile<T, TRACE, 4, 1>(src, out, mac, dt, dx, copy, s);
